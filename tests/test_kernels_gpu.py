@@ -1030,3 +1030,20 @@ def test_prefill_attention_on_tcgen05_refuses_odd_page_sizes(ops):
     table = torch.zeros(1, 1, dtype=torch.int32, device="cuda")
     assert not ops.paged_attention_prefill_tc(q, 128, torch.empty_like(q), pages, pages, table, z, z + 4, z + 4, 1, 1, 1, 128, 24,
                                               0.1, 0)
+
+
+@pytest.mark.parametrize("n,k", [(1, 4), (17, 132), (65, 128), (130, 516), (300, 33), (2500, 1040)])
+def test_gemm_f32_gives_the_same_bits_in_every_kernel(ops, n, k):
+    """A row alone, in the streaming kernel's row counts, at the edges of its tiles and of the register tiles, with K below, at and past
+    the eight parts and no multiple of a tile: the same bits as in a batch of 131, and within the bound of eight chains."""
+    g = torch.Generator().manual_seed(n + k)
+    a, w = torch.randn(131, k, generator=g), torch.randn(n, k, generator=g)
+    full = torch.empty(131, n, device="cuda")
+    ops.linear(dev(a), dev(w), full)
+    # a chain of n terms is within n * 2^-24 of sum |a_i w_i|: an eighth of K (16 at least) and the eight parts
+    bound = (-(-k // 128) * 16 + 9) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((full.cpu().double() - a.double() @ w.double().T).abs() <= bound).all())
+    for m in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 130):
+        out = torch.full((m + 1, n), 7.0, device="cuda")
+        ops.linear(dev(a[:m]), dev(w), out[:m])
+        assert torch.equal(out[:m], full[:m]) and bool((out[m] == 7.0).all()), m
