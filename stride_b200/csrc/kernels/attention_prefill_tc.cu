@@ -60,7 +60,18 @@ constexpr long long kStaggerCycles = 1000;
 // softmax warps, two CTAs per SM. Two heads: 8 service warps (three for keys, products, three for values, Q) and
 // 8 softmax warps, one CTA per SM: a single warp cannot issue a tile's copies as fast as two heads consume them.
 // REL: with a table of learned numbers per head and distance.
-template <int HD, int HEADS, bool TMA_KV, bool REL>
+// LATENT (one head per CTA, TMA): the expanded form of attention over a latent cache. A head's key is HD numbers of its own and 64
+// rotated ones that all heads share, its value HD numbers: keys and values come as rows [head: key, value] of a dense matrix
+// (map_k and map_v both describe it), the rotated parts as rows of another (map_k2), the requests' rows one after the other; the
+// query's rotated part has a matrix of its own too (map_q2). A key tile is 24 KB: one stage for keys and two for values leave room
+// for two CTAs per SM, and the scores run two tiles ahead, which hides the one stage. An optional gate (LatentGate) multiplies the
+// result. 2,048 tokens of 16 heads: 42 us, beside 12 us for the product that expands and 4 us for the
+// gather; on the latents themselves (latent_attention_tc.cu and two products a head) 745 + 2 x 243 us.
+struct LatentGate {
+    const __nv_bfloat16* values;        // null: none
+    int ld, per_output;                 // row stride; one number an output (else one a head)
+};
+template <int HD, int HEADS, bool TMA_KV, bool REL, bool LATENT = false>
 __global__ void __launch_bounds__(HEADS == 1 ? 256 : 512, HEADS == 1 ? 2 : 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __nv_bfloat16* __restrict__ k_pages,
@@ -68,15 +79,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                        const int32_t* __restrict__ block_table, int table_width, const int32_t* __restrict__ q_start,
                        const int32_t* __restrict__ q_len, const int32_t* __restrict__ ctx_len, int num_seqs, int nq, int nkv,
                        int page_shift, float scale_log2e, int window, float cap_in, const float* __restrict__ sinks,
-                       const float* __restrict__ slopes, const float* __restrict__ rel, int rel_len, int* __restrict__ status) {
+                       const float* __restrict__ slopes, const float* __restrict__ rel, int rel_len, int* __restrict__ status,
+                       const __grid_constant__ CUtensorMap map_q2, const __grid_constant__ CUtensorMap map_k2, LatentGate gate, int q2_stride) {
+    static_assert(!LATENT || (HEADS == 1 && TMA_KV && !REL), "the latent form");
     constexpr int HALVES = HD / 64;                       // 64-column boxes per row
     constexpr int HALF_BYTES = kQRows * 128;              // a [128 rows x 64 columns] bf16 box of Q
     constexpr int KV_HALF_BYTES = kKeys * 128;            // [64 keys x 64 columns] of K or V
-    constexpr int Q_BYTES = HALVES * HALF_BYTES;
-    constexpr int KV_BYTES = HALVES * KV_HALF_BYTES;      // one K tile or one V tile
+    constexpr int BOXES = HALVES + (LATENT ? 1 : 0);      // boxes per row of a query or key
+    constexpr int Q_BYTES = BOXES * HALF_BYTES;
+    constexpr int K_BYTES = BOXES * KV_HALF_BYTES;        // one K tile
+    constexpr int KV_BYTES = HALVES * KV_HALF_BYTES;      // one V tile
     constexpr uint32_t HEAD_COLS = 256;                   // per head: two score buffers (P over S) of 64 columns, O: HD columns
     constexpr uint32_t TMEM_COLS = HEAD_COLS * HEADS;
-    constexpr int KS = HEADS == 1 ? 2 : 4;                // stages of the key ring and of the value ring
+    constexpr int KSV = HEADS == 1 ? 2 : 4, KS = LATENT ? 1 : KSV;      // stages of the value ring and of the key ring
     // Service warps, in this order: LOADERS for the keys, one per head that issues the scores (the last of them, for
     // head 0, owns tensor memory), LOADERS for the values, one per head that issues the output products (the last of
     // them, for head 0, fetches Q first).
@@ -85,17 +100,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* q_s = smem;                            // HEADS query tiles
-    unsigned char* k_s = q_s + HEADS * Q_BYTES;           // KS key tiles, then KS value tiles
-    unsigned char* v_s = k_s + KS * KV_BYTES;
+    unsigned char* k_s = q_s + HEADS * Q_BYTES;           // KS key tiles, then KSV value tiles
+    unsigned char* v_s = k_s + KS * K_BYTES;
     __shared__ __align__(8) uint64_t q_full;
-    __shared__ __align__(8) uint64_t s_full[HEADS][2], p_full[HEADS][2], s_free[HEADS][2], k_full[KS], k_empty[KS], v_full[KS], v_empty[KS];
+    __shared__ __align__(8) uint64_t s_full[HEADS][2], p_full[HEADS][2], s_free[HEADS][2], k_full[KS], k_empty[KS], v_full[KSV], v_empty[KSV];
     __shared__ uint32_t tmem_base_slot;
 
     pdl_trigger();
     // Which request and which of its query tiles is this CTA? blockIdx.y counts the tiles, blockIdx.x the heads:
     // CTAs are handed out x first, so all heads of a tile start together, and within a request the last tile,
     // which has the most keys to walk, comes first: the long CTAs start first and do not form the tail.
-    int seq = -1, tile = 0;
+    int seq = -1, tile = 0, key_row0 = 0;          // key_row0: the dense row of the request's first key
     {
         int acc = 0;
         for (int s = 0; s < num_seqs; ++s) {
@@ -105,6 +120,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 tile = tiles - 1 - (blockIdx.y - acc);
                 break;
             }
+            if (LATENT) key_row0 += ctx_len[s];
             acc += tiles;
         }
     }
@@ -120,7 +136,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const int kt_first = first_key / kKeys;
     const int n_tiles = last_pos / kKeys - kt_first + 1;
     const int q_row0 = q_start[seq] + row0;                // row of the projection output that holds query 0 of this tile
-    const int32_t* table = block_table + static_cast<size_t>(seq) * table_width;
+    const int32_t* table = LATENT ? nullptr : block_table + static_cast<size_t>(seq) * table_width;
 
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(&q_full), 1);
@@ -135,6 +151,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // cp.async: one arrival per lane of the copying warps; TMA: the one that announces the tile's bytes
             mbar_init(smem_u32(&k_full[s]), TMA_KV ? 1 : 32 * LOADERS);
             mbar_init(smem_u32(&k_empty[s]), HEADS);             // one arrival per issuing warp
+        }
+        for (int s = 0; s < KSV; ++s) {
             mbar_init(smem_u32(&v_full[s]), TMA_KV ? 1 : 32 * LOADERS);
             mbar_init(smem_u32(&v_empty[s]), HEADS);
         }
@@ -164,6 +182,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         unsigned char* ring = is_k ? k_s : v_s;
         uint64_t* full = is_k ? k_full : v_full;
         uint64_t* empty = is_k ? k_empty : v_empty;
+        const int stages = is_k ? KS : KSV, tile_bytes = is_k ? K_BYTES : KV_BYTES;
         if constexpr (TMA_KV) {
             // Pages of 16 keys and more: a tile is 64 / page_size boxes of [page_size keys x 64 columns] per half
             // (one box of 64 keys when the page is larger), each issued by a lane of its own in the same
@@ -173,24 +192,42 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             // masked (K) or cleared (V) by the softmax warps, as with cp.async.
             if (part == 0) {
                 const CUtensorMap* map = is_k ? &map_k : &map_v;
+                if constexpr (LATENT) {
+                    // one box of 64 rows per 64 columns, each issued by a lane of its own; rows past the request's last key are
+                    // masked (K) or cleared (V) by the softmax warps, whatever they hold
+                    const int boxes = is_k ? BOXES : HALVES;
+                    const bool rotated = lane == HALVES;
+                    const int x = rotated ? 0 : head0 * 2 * HD + (is_k ? 0 : HD) + lane * 64;
+                    for (int j = 0; j < n_tiles; ++j) {
+                        const int st = j % stages;
+                        if (!mbar_wait(smem_u32(&empty[st]), (static_cast<uint32_t>(j / stages) & 1u) ^ 1u, status, is_k ? 11 : 18)) break;
+                        const uint32_t bar = smem_u32(&full[st]);
+                        if (lane == 0) mbar_expect_tx(bar, tile_bytes);
+                        __syncwarp();
+                        if (lane < boxes)
+                            tma_load_2d(smem_u32(ring + st * tile_bytes + lane * KV_HALF_BYTES), rotated ? &map_k2 : map, bar, x,
+                                        key_row0 + (kt_first + j) * kKeys);
+                    }
+                } else {
                 const int page_size = 1 << page_shift;
                 const int box_rows = min(page_size, kKeys);
                 const int boxes = kKeys / box_rows;
                 for (int j = 0; j < n_tiles; ++j) {
-                    const int st = j % KS;
-                    if (!mbar_wait(smem_u32(&empty[st]), (static_cast<uint32_t>(j / KS) & 1u) ^ 1u, status, is_k ? 11 : 18)) break;
+                    const int st = j % stages;
+                    if (!mbar_wait(smem_u32(&empty[st]), (static_cast<uint32_t>(j / stages) & 1u) ^ 1u, status, is_k ? 11 : 18)) break;
                     const uint32_t bar = smem_u32(&full[st]);
-                    if (lane == 0) mbar_expect_tx(bar, KV_BYTES);
+                    if (lane == 0) mbar_expect_tx(bar, tile_bytes);
                     __syncwarp();
                     if (lane < boxes) {
                         const int key0 = (kt_first + j) * kKeys + lane * box_rows;
                         const int page = key0 >> page_shift;
                         const int entry = page < table_width ? table[page] : -1;
                         const int y = entry < 0 ? -box_rows : (entry * nkv + kvh) * page_size + (key0 & (page_size - 1));
-                        const uint32_t dst = smem_u32(ring + st * KV_BYTES + lane * box_rows * 128);
+                        const uint32_t dst = smem_u32(ring + st * tile_bytes + lane * box_rows * 128);
 #pragma unroll
                         for (int h = 0; h < HALVES; ++h) tma_load_2d(dst + h * KV_HALF_BYTES, map, bar, h * 64, y);
                     }
+                }
                 }
             }
         } else {
@@ -241,7 +278,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             mbar_expect_tx(qb, HEADS * Q_BYTES);
             for (int hh = 0; hh < HEADS; ++hh)
                 for (int c = 0; c < HALVES; ++c)
-                    tma_load_2d(smem_u32(q_s + hh * Q_BYTES + c * HALF_BYTES), &map_q, qb, (head0 + hh) * HD + c * 64, q_row0);
+                    tma_load_2d(smem_u32(q_s + hh * Q_BYTES + c * HALF_BYTES), &map_q, qb, (head0 + hh) * (LATENT ? HD + 64 : HD) + c * 64, q_row0);
+            if (LATENT) tma_load_2d(smem_u32(q_s + HALVES * HALF_BYTES), &map_q2, qb, head0 * q2_stride, q_row0);
         }
         __syncwarp();
         const bool issuer = elect_one();
@@ -249,8 +287,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const uint32_t tmem_h = tmem_base + h * HEAD_COLS;
         bool ok = true;
         for (int j = 0; j < n_tiles && ok; ++j) {
-            const int st = j % KS;
-            ok = mbar_wait(smem_u32(&v_full[st]), static_cast<uint32_t>(j / KS) & 1u, status, 19);
+            const int st = j % KSV;
+            ok = mbar_wait(smem_u32(&v_full[st]), static_cast<uint32_t>(j / KSV) & 1u, status, 19);
             ok = ok && mbar_wait(smem_u32(&p_full[h][j & 1]), static_cast<uint32_t>(j >> 1) & 1u, status, 14);
             if (!ok) break;
             tc_fence_after();
@@ -281,9 +319,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             if (!ok) break;
             // (data whose arrival the mbarrier has reported needs no proxy fence before tcgen05.mma reads it)
             tc_fence_after();
-            const uint32_t k_addr = smem_u32(k_s + st * KV_BYTES);
+            const uint32_t k_addr = smem_u32(k_s + st * K_BYTES);
 #pragma unroll
-            for (int kk = 0; kk < HD / 16; ++kk) {      // 16 head columns per product
+            for (int kk = 0; kk < BOXES * 4; ++kk) {    // 16 head columns per product
                 const uint64_t a = smem_desc(q_addr + (kk / 4) * HALF_BYTES + (kk % 4) * 32, 16, 1024);
                 const uint64_t b = smem_desc(k_addr + (kk / 4) * KV_HALF_BYTES + (kk % 4) * 32, 16, 1024);
                 if (issuer) umma_bf16(tmem_base + h * HEAD_COLS + (j & 1) * kKeys, a, b, idesc_qk, kk > 0 ? 1u : 0u);
@@ -424,8 +462,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             if (k0 + kKeys - 1 > last_pos || k0 < first_key) {
                 // (with two heads both groups of warps clear the same rows with the same zeros: each must be
                 // sure of them before it lets its own product go)
-                const int vst = j % KS;
-                ok = mbar_wait(smem_u32(&v_full[vst]), static_cast<uint32_t>(j / KS) & 1u, status, 20);
+                const int vst = j % KSV;
+                ok = mbar_wait(smem_u32(&v_full[vst]), static_cast<uint32_t>(j / KSV) & 1u, status, 20);
                 if (!ok) break;
                 const int key = k0 + row;
                 if (row < kKeys && (key > last_pos || key < first_key)) {
@@ -455,6 +493,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 float v[32];
                 tmem_ld32(tmem_o + lane_base + c * 32, v);
                 if (row < rows) {
+                    if (LATENT && gate.values != nullptr) {
+                        const __nv_bfloat16* g = gate.values + static_cast<size_t>(q_row0 + row) * gate.ld;
+                        if (gate.per_output) {
+#pragma unroll
+                            for (int i = 0; i < 32; i += 8) {
+                                const uint4 raw = *reinterpret_cast<const uint4*>(g + head * HD + c * 32 + i);
+                                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&raw);
+#pragma unroll
+                                for (int k = 0; k < 8; ++k) v[i + k] *= 1.f / (1.f + expf(-to_f32(e[k])));
+                            }
+                        } else {
+                            const float f = 1.f / (1.f + expf(-to_f32(g[head])));
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) v[i] *= f;
+                        }
+                    }
 #pragma unroll
                     for (int q4 = 0; q4 < 4; ++q4) {
                         uint32_t w[4];
@@ -499,7 +553,7 @@ int launch_attn(const CUtensorMap* map_q, const CUtensorMap* map_k, const CUtens
     stride::launch(kernel, grid, block, smem, stream, *map_q, tma ? *map_k : *map_q, tma ? *map_v : *map_q, k_pages, v_pages, out,
                    block_table, table_width, q_start, q_len, ctx_len, num_seqs, nq, nkv, page_shift,
                    (softcap != 0.f ? fabsf(softcap) : scale) * 1.4426950408889634f, window, softcap != 0.f ? scale / softcap : 0.f, sinks, slopes, rel,
-                   rel_len, status);
+                   rel_len, status, *map_q, *map_q, LatentGate{nullptr, 0, 0}, 0);
     return STRIDE_LAUNCH_STATUS();
 }
 
@@ -580,4 +634,47 @@ extern "C" int stride_paged_prefill_attention_tc(const void* q, int q_stride, vo
     if (hd == 64) return pair ? STRIDE_ATTN_LAUNCH(64, 2) : STRIDE_ATTN_LAUNCH(64, 1);
     return pair ? STRIDE_ATTN_LAUNCH(128, 2) : STRIDE_ATTN_LAUNCH(128, 1);
 #undef STRIDE_ATTN_LAUNCH
+}
+
+// Attention over expanded latents for the first `num_seqs` requests of the step, which own the first `tokens` rows of the flat
+// batch. q: bf16 rows of q_ld numbers, head h's plain part at columns h * (hd + rot); q_rot: rows of q_rot_ld numbers, head h's
+// rotated part at columns h * q_rot_stride; both hold q_rows rows (tokens at least). kv: [kv_rows, heads, 2 * hd], a head's key and value, k_rot:
+// [kv_rows, rot]: the keys of request 0 from its position 0 on, then those of request 1, ... (kv_rows: rows that may be read;
+// rows past the last request's keys may hold anything). out: [tokens, heads * hd]. gate (bf16 or null): the result of row t is
+// multiplied by sigmoid(gate[t * gate_ld + h]), or, gate_per_output, by sigmoid(gate[t * gate_ld + column]). Returns -2 for other
+// sizes than hd 128 with rot 64 and for unaligned rows.
+extern "C" int stride_latent_prefill_tc(const void* q, int q_ld, const void* q_rot, int q_rot_ld, int q_rot_stride, int q_rows, const void* kv,
+                                        const void* k_rot, int kv_rows, void* out, const int32_t* q_start, const int32_t* q_len,
+                                        const int32_t* ctx_len, int num_seqs, int tokens, int heads, int hd, int rot, float scale,
+                                        const float* sinks, const void* gate, int gate_ld, int gate_per_output, int* status,
+                                        cudaStream_t stream) {
+    if (tokens < 0 || num_seqs < 0 || heads <= 0 || q_rows < tokens || kv_rows <= 0 || status == nullptr) return STRIDE_BAD_ARGUMENT;
+    if (q_ld < heads * (hd + rot) || q_rot_stride < rot || q_rot_ld < (heads - 1) * q_rot_stride + rot) return STRIDE_BAD_ARGUMENT;
+    if (hd != 128 || rot != 64 || heads > 65535 || (q_ld | q_rot_ld | q_rot_stride) % 8 || (gate && gate_per_output && gate_ld % 8)) return STRIDE_UNSUPPORTED;
+    if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(q_rot) | reinterpret_cast<uintptr_t>(kv) | reinterpret_cast<uintptr_t>(k_rot) |
+         reinterpret_cast<uintptr_t>(out) | (gate && gate_per_output ? reinterpret_cast<uintptr_t>(gate) : 0)) % 16)
+        return STRIDE_UNSUPPORTED;
+    if (tokens == 0 || num_seqs == 0) return 0;
+    constexpr int HD = 128, smem = 3 * tc::kQRows * 128 + 3 * tc::kKeys * 128 + 2 * 2 * tc::kKeys * 128 + 1024;       // Q, a key tile, two value tiles
+    const auto kernel = tc::attn_prefill_tc_kernel<HD, 1, true, false, true>;
+    static bool configured[64] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return STRIDE_BAD_ARGUMENT;
+    if (!configured[device]) {
+        const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return static_cast<int>(e);
+        configured[device] = true;
+    }
+    const int max_tiles = (tokens + tc::kQRows - 1) / tc::kQRows + num_seqs;
+    if (max_tiles > 65535) return STRIDE_UNSUPPORTED;
+    const long long kv_ld = static_cast<long long>(heads) * 2 * HD;
+    const CUtensorMap* map_q = tc::cached_map(q, q_rows, heads * (HD + 64), q_ld, tc::kQRows);
+    const CUtensorMap* map_q2 = tc::cached_map(q_rot, q_rows, (heads - 1) * q_rot_stride + 64, q_rot_ld, tc::kQRows);
+    const CUtensorMap* map_kv = tc::cached_map(kv, kv_rows, kv_ld, kv_ld, tc::kKeys);
+    const CUtensorMap* map_k2 = tc::cached_map(k_rot, kv_rows, 64, 64, tc::kKeys);
+    if (!map_q || !map_q2 || !map_kv || !map_k2) return STRIDE_UNSUPPORTED;
+    stride::launch(kernel, dim3(heads, max_tiles), dim3(256), smem, stream, *map_q, *map_kv, *map_kv, nullptr, nullptr, static_cast<__nv_bfloat16*>(out),
+                   nullptr, 0, q_start, q_len, ctx_len, num_seqs, heads, heads, 0, scale * 1.4426950408889634f, 0, 0.f, sinks, nullptr, nullptr, 0,
+                   status, *map_q2, *map_k2, tc::LatentGate{static_cast<const __nv_bfloat16*>(gate), gate_ld, gate_per_output}, q_rot_stride);
+    return STRIDE_LAUNCH_STATUS();
 }

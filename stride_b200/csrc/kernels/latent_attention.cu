@@ -79,6 +79,27 @@ latent_prepare_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ pr
     }
 }
 
+// ------------------------------------------------------------------------------------------------- gather
+// The latents and rotated key parts of the first `num_seqs` requests, position 0 on, request after request, out of their pages into
+// dense rows: what the product that expands keys and values reads. A warp a row, 16 bytes a lane.
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const uint4* __restrict__ latent_pages, const uint4* __restrict__ krot_pages, const int32_t* __restrict__ block_table,
+                     int table_width, const int32_t* __restrict__ ctx_len, int num_seqs, int page_size, int rank16, int rot16, int rows,
+                     uint4* __restrict__ latent, uint4* __restrict__ krot) {
+    pdl_trigger();
+    pdl_wait();
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    int key = row, seq = 0;
+    while (seq < num_seqs && key >= ctx_len[seq]) key -= ctx_len[seq++];
+    if (seq == num_seqs || key / page_size >= table_width) return;      // past the last request's keys: nothing is read from there
+    const int page = block_table[static_cast<size_t>(seq) * table_width + key / page_size];
+    if (page < 0) return;
+    const size_t slot = static_cast<size_t>(page) * page_size + key % page_size;
+    for (int i = lane; i < rank16; i += 32) latent[static_cast<size_t>(row) * rank16 + i] = latent_pages[slot * rank16 + i];
+    for (int i = lane; i < rot16; i += 32) krot[static_cast<size_t>(row) * rot16 + i] = krot_pages[slot * rot16 + i];
+}
+
 // ---------------------------------------------------------------------------------------------- head_gemm
 // C[t, a, n] = (sum_k A[t * lda + a * a_hs + k] * B[a * b_hs + k * b_ks + n * b_ns]) * (gate ? sigmoid(gate[t * ldg + a * g_hs + n * g_ns]) : 1)
 // (g_hs 1 and g_ns 0: one gate a head; g_hs N and g_ns 1: one gate an output)
@@ -331,6 +352,20 @@ int stride_head_gemm(const void* A, int lda, int a_hs, const void* B, long long 
     }
     else
         return STRIDE_BAD_ARGUMENT;
+    return STRIDE_LAUNCH_STATUS();
+}
+
+// Pages: latent [pages, page_size, rank], key part [pages, page_size, rot], bf16, rank and rot multiples of 8, 16-byte aligned.
+int stride_latent_gather(const void* latent_pages, const void* krot_pages, const int32_t* block_table, int table_width, const int32_t* ctx_len,
+                         int num_seqs, int page_size, int rank, int rot, int rows, void* latent, void* krot, cudaStream_t stream) {
+    if (num_seqs < 0 || page_size <= 0 || table_width <= 0 || rank <= 0 || rot <= 0 || rows < 0) return STRIDE_BAD_ARGUMENT;
+    if (rank % 8 || rot % 8 || (reinterpret_cast<uintptr_t>(latent_pages) | reinterpret_cast<uintptr_t>(krot_pages) | reinterpret_cast<uintptr_t>(latent) |
+                                reinterpret_cast<uintptr_t>(krot)) % 16)
+        return STRIDE_UNSUPPORTED;
+    if (num_seqs == 0 || rows == 0) return 0;
+    stride::launch(latent_gather_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, static_cast<const uint4*>(latent_pages),
+                   static_cast<const uint4*>(krot_pages), block_table, table_width, ctx_len, num_seqs, page_size, rank / 8, rot / 8, rows,
+                   static_cast<uint4*>(latent), static_cast<uint4*>(krot));
     return STRIDE_LAUNCH_STATUS();
 }
 

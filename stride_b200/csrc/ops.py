@@ -102,6 +102,11 @@ _SIGNATURES = {
                                               c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "stride_latent_attention": ("latent_attention", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                                      c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p]),
+    "stride_latent_gather": ("latent_attention", [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                                  c_void_p, c_void_p]),
+    "stride_latent_prefill_tc": ("attention_prefill_tc", [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
+                                                          c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
+                                                          c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "stride_latent_attention_tc": ("latent_attention_tc", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                                            c_float, c_int, c_int, c_void_p, c_void_p]),
@@ -1072,6 +1077,42 @@ def latent_attention_tc(qa, out, partial, latent_pages, krot_pages, block_table,
         _dev(q_len, "q_len", torch.int32), _dev(ctx_len, "ctx_len", torch.int32), _dev(seq_of_token, "seq_of_token", torch.int32),
         first_seq, num_seqs, first_token, tokens, max_q_len, heads, rank, rot, page_size, float(scale), splits, keys_per_split,
         _opt(sinks, "sinks", torch.float32), _stream()), "latent_attention_tc")
+
+
+def latent_prefill_supported(dtype, dim: int, vdim: int, rot: int, rank: int) -> bool:
+    """Sizes of the expanded form of latent attention (``latent_gather``, a product, ``latent_prefill_tc``)."""
+    return dtype == torch.bfloat16 and dim == 128 and vdim == 128 and rot == 64 and rank % 8 == 0
+
+
+def latent_gather(latent_pages, krot_pages, block_table, ctx_len, num_seqs: int, page_size: int, latent, krot) -> None:
+    """The cached latents and rotated key parts of the step's first ``num_seqs`` requests, every position of a request in order and the
+    requests one after the other, as rows of ``latent`` [rows, rank] and ``krot`` [rows, rot] (rows past the last request's keys
+    are left as they are)."""
+    _check(_fn("stride_latent_gather")(
+        _dev(latent_pages, "latent_pages", torch.bfloat16), _dev(krot_pages, "krot_pages", torch.bfloat16),
+        _dev(block_table, "block_table", torch.int32), block_table.shape[1], _dev(ctx_len, "ctx_len", torch.int32), num_seqs, page_size,
+        latent.shape[1], krot.shape[1], latent.shape[0], _dev(latent, "latent", torch.bfloat16), _dev(krot, "krot", torch.bfloat16),
+        _stream()), "latent_gather")
+
+
+def latent_prefill_tc(q, q_off: int, q_rot, q_rot_off: int, q_rot_stride: int, kv, krot, out, q_start, q_len, ctx_len, num_seqs: int,
+                      heads: int, scale: float, sinks=None, gate=None, gate_off: int = 0, gate_per_output: bool = False) -> None:
+    """Causal attention of the step's first ``num_seqs`` requests, which own the first rows of ``q``, over expanded keys and values: ``kv``
+    [rows, heads * 256] holds a head's 128 key and 128 value numbers, ``krot`` [rows, 64] the rotated key part, as ``latent_gather`` orders the
+    rows. Queries: 128 + 64 numbers a head in ``q`` from column ``q_off`` on, of which the 64 are taken (rotated) from ``q_rot``, head h at
+    column ``q_rot_off + h * q_rot_stride``. ``out`` [tokens, heads * 128] is multiplied by the sigmoid of ``gate`` (its columns from
+    ``gate_off`` on: one a head, or one an output)."""
+    tokens = out.shape[0]
+    if out.shape[1] != heads * 128 or kv.shape[1] != heads * 256 or krot.shape != (kv.shape[0], 64) or q.shape[0] < tokens or \
+            q_rot.shape[0] != q.shape[0] or (gate is not None and (gate.dtype != torch.bfloat16 or gate.shape[0] < tokens)):
+        raise KernelError("latent_prefill_tc: shapes do not agree")
+    st = _tc_buffers(q.device, 0)
+    _check(_fn("stride_latent_prefill_tc")(
+        _dev(q, "q", torch.bfloat16) + q_off * 2, q.shape[1], _dev(q_rot, "q_rot", torch.bfloat16) + q_rot_off * 2, q_rot.shape[1], q_rot_stride,
+        q.shape[0], _dev(kv, "kv", torch.bfloat16), _dev(krot, "krot", torch.bfloat16), kv.shape[0], _dev(out, "out", torch.bfloat16),
+        _dev(q_start, "q_start", torch.int32), _dev(q_len, "q_len", torch.int32), _dev(ctx_len, "ctx_len", torch.int32), num_seqs, tokens, heads,
+        128, 64, float(scale), _opt(sinks, "sinks", torch.float32), None if gate is None else _dev(gate, "gate") + gate_off * 2,
+        0 if gate is None else gate.shape[1], 1 if gate_per_output else 0, _dev(st["status"], "status"), _stream()), "latent_prefill_tc")
 
 
 # ---------------------------------------------------------------- recurrent block

@@ -123,7 +123,7 @@ class ModelRunner:
         return logits, timer.milliseconds()
 
     # ------------------------------------------------------------------- eager
-    def _context(self, staging, batch, num_tokens, num_rows, for_graph: int = 0):
+    def _context(self, staging, batch, num_tokens, num_rows, for_graph: int = 0, portion_bound: int = 0):
         items, row = [], 0
         for request, tokens, position, _want in batch.items():
             items.append((request, row, len(tokens), position, self.cache.state_slot(request)))
@@ -132,11 +132,12 @@ class ModelRunner:
         while tail_seq > 0 and items[tail_seq - 1][2] == 1:
             tail_seq -= 1
         tail_start = items[tail_seq][1] if tail_seq < len(items) else row
-        bound = for_graph if for_graph else batch.max_ctx       # a captured graph is sized for its context bucket
+        bound = for_graph or portion_bound or batch.max_ctx     # a captured graph is sized for its context bucket
+        portion_keys = portion_bound or sum(position + n for _request, _row, n, position, _slot in items[:tail_seq])
         return make_context(staging.dev, staging.layout, num_tokens, batch.num_seqs, num_rows, max_q_len=batch.max_q_len,
                             max_ctx=batch.max_ctx, decode_only=batch.decode_only, host_items=items,
                             decode_tail_start=0 if for_graph else tail_start, decode_tail_seq=0 if for_graph else tail_seq,
-                            context_bound=bound, seq_slots=staging.layout["seq_cap"] if for_graph else batch.num_seqs)
+                            context_bound=bound, portion_keys=0 if for_graph else portion_keys, seq_slots=staging.layout["seq_cap"] if for_graph else batch.num_seqs)
 
     def _pack(self, staging, batch):
         l = staging.layout
@@ -232,12 +233,14 @@ class ModelRunner:
     def _step_full_portion(self, batch):
         """One request's portion that fills the token budget (every step but the last of a long prompt cut into
         portions, when nothing else is running): always the same launches, whatever the position, so it is
-        replayed from a graph too, one for the portions that want no logits and one for those that want a row."""
-        key = ("portion", batch.num_rows)
+        replayed from a graph too, one for the portions that want no logits and one for those that want a row.
+        A part that sizes its launches by the keys a request holds (``sizes_by_context``) gets a graph a context bucket."""
+        bound = self._context_bucket(batch.max_ctx) if self.model.sizes_by_context else 0
+        key = ("portion", batch.num_rows) + ((bound,) if bound else ())
         entry = self._graphs.get(key)
         if entry is None:
             self._pack(self._eager, batch)
-            ctx = self._context(self._eager, batch, batch.num_tokens, batch.num_rows)
+            ctx = self._context(self._eager, batch, batch.num_tokens, batch.num_rows, portion_bound=bound)
             self._warm_up(ctx, batch)
             torch.cuda.synchronize()
             graph = torch.cuda.CUDAGraph()

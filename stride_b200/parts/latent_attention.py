@@ -5,9 +5,9 @@ key part ``k_r`` [rot_dim] that all heads share. Head a has the query ``[q_a | q
 second part rotated by position), the key ``[W_uk_a c | k_r]`` and the value ``W_uv_a c``; scores are causal,
 softmaxed, and the head's output may be gated by ``sigmoid(W_g h)_a`` before the output projection.
 
-The keys and values are never formed. With ``q~_a = W_uk_a^T q_a`` the score is ``(q~_a . c + q_rot_a . k_r) * scale``
+For single tokens the keys and values are never formed. With ``q~_a = W_uk_a^T q_a`` the score is ``(q~_a . c + q_rot_a . k_r) * scale``
 and the output ``W_uv_a (sum_j p_j c_j)``: attention runs on the cached vectors themselves, with one key/value
-"head" of width kv_rank + rot_dim for all query heads, in prompts and in decoding alike. Steps:
+"head" of width kv_rank + rot_dim for all query heads. Steps:
 
     one product     [W_q ; W_dkv ; W_g] h                          (``ops.linear``)
     latent_prepare  norm of the latent, rotations, cache write     (one kernel)
@@ -17,6 +17,16 @@ and the output ``W_uv_a (sum_j p_j c_j)``: attention runs on the cached vectors 
                                                                     and for the whole 32-bit path)
     head_gemm       W_uv per head, times the gate                  (one kernel)
     output product  W_o                                            (left to the residual stream)
+
+That form costs heads * (2 kv_rank + rot_dim) multiply-adds a (query, key) pair, the plain one heads * (dim + rot_dim + value_dim),
+3.4 times less at 128 + 64, 128 and a latent of 512, beside kv_rank * heads * (dim + value_dim) a key to expand it. So portions of prompts
+in bfloat16 expand, where the head sizes are those of the tcgen05 kernel (``_expands`` says from how many tokens on):
+
+    one product, latent_prepare  as above
+    latent_gather                the requests' latents out of their pages
+    one product                  [W_uk ; W_uv] c: every head's keys and values
+    latent_prefill_tc            attention over them, times the gate (tcgen05)
+    output product               as above
 
 Other forms, chosen by spec params: ``q_rank`` r > 0 sends the queries through a latent of their own,
 ``q = W_uq rms_norm(W_dq h)`` (tensors ``dq`` [r, hidden], ``dq.norm`` [r], ``uq`` in place of ``q``; the norm uses
@@ -46,6 +56,11 @@ from .base import CacheRequest, Mixer, Projection, TensorDecl, build_part, regis
 
 class LatentAttention(Mixer):
     lazy_output = True
+    # Portions go over expanded keys where tokens x keys reach this. A step of the six-layer Nidilix shape (two such layers), on the
+    # latents themselves / expanded: 100 tokens behind 2,000 2.11 / 1.94 ms, 24 behind 6,000 2.80 / 1.88 ms, 1,200 alone 3.49 / 2.73 ms;
+    # below it both are level (300 alone 2.08 / 2.12 ms: the launches), and the kernels of the folded form are fewer.
+    EXPAND_PAIRS = 1 << 16
+    MAX_EXPANDED_BYTES = 1 << 28      # keys and values of a step, expanded, at most
 
     def __init__(self, spec, runtime):
         super().__init__(spec, runtime)
@@ -80,11 +95,13 @@ class LatentAttention(Mixer):
         self.kv_off = -(-self.q_cols // 8) * 8
         self.g_off = self.kv_off + -(-self.kv_dim // 8) * 8
         self.proj_dim = -(-(self.g_off + self.g_dim) // 8) * 8
-        self.w_in = self.w_uk = self.w_uv = self.w_o = self.latent_w = self.w_uq = self.q_norm_w = self.sinks = None
+        self.w_in = self.w_ukv = self.w_o = self.latent_w = self.w_uq = self.q_norm_w = self.sinks = None
         # rotated entries in the order the kernels pair them: new entry 2i is old entry i, new entry 2i + 1 old entry i + dims / 2
         half = self.rot_dims // 2
         order = [j for i in range(half) for j in (i, i + half)] + list(range(self.rot_dims, self.rot))
         self.rot_order = torch.tensor(order, dtype=torch.long) if self.halves else None
+        self._expand = ops.latent_prefill_supported(runtime.dtype, self.dim, self.vdim, self.rot, self.rank)
+        self.sizes_by_context = self._expand
         self._fast = ops.latent_tc_supported(runtime.dtype, self.heads, self.rank, self.rot)
 
     # ----------------------------------------------------------------- weights
@@ -137,11 +154,15 @@ class LatentAttention(Mixer):
         if self.has_sinks:
             self.sinks = weights[self._n("sink")]
         self.w_in = w
-        self.w_uk, self.w_uv, self.w_o = weights[self._n("uk")], weights[self._n("uv")], weights[self._n("o")]
+        # [heads, dim + value_dim, rank]: a head's rows of W_uk, then of W_uv, so that one product expands both
+        self.w_ukv = torch.cat([weights[self._n("uk")].view(self.heads, self.dim, self.rank),
+                                weights[self._n("uv")].view(self.heads, self.vdim, self.rank)], 1).contiguous()
+        self.w_o = weights[self._n("o")]
         self.position.bind(weights)
 
     def named_tensors(self):
-        out = {self._n("uk"): self.w_uk, self._n("uv"): self.w_uv, self._n("o"): self.w_o}
+        out = {self._n("uk"): self.w_ukv[:, :self.dim].reshape(self.heads * self.dim, self.rank),
+               self._n("uv"): self.w_ukv[:, self.dim:].reshape(self.heads * self.vdim, self.rank), self._n("o"): self.w_o}
         if self.q_rank:
             out[self._n("dq")], out[self._n("dq.norm")] = self.w_in[:self.q_rank], self.q_norm_w
             out[self._n("uq")] = self._pair_rows(self.w_uq, self.dim, self.heads, self.dim + self.rot, inverse=True)
@@ -182,25 +203,50 @@ class LatentAttention(Mixer):
         ops.latent_prepare(proj, self.q_off, self.kv_off if self.own_latent else -1, qa, pos, seq,
                            ctx.slot_mapping[cache.group][:tokens] if cache.writes else None, cos, sin, self.latent_w, self.eps,
                            latent, key_rot, self.heads, self.dim, self.rot, self.rot_dims, self.rank, q=q if self.q_rank else None)
-        # q~[t, a, :] = q[t, a, :dim] @ W_uk[a]          W_uk [heads * dim, rank]: B_a[k, n] = W_uk[a * dim + k, n]
-        ops.head_gemm(q, q_ld, self.dim + self.rot, self.w_uk, self.dim * self.rank, self.rank, 1, qa, self.heads * width, width,
-                      tokens, self.heads, self.rank, self.dim, a_off=q_off)
-        mixed = self.rt.buffer("latent_mixed", tokens, self.heads * self.rank)
-        self._attend(qa, mixed, latent, key_rot, ctx, cache, tokens)
-        # o[t, a, :] = W_uv[a] mixed[t, a, :]            W_uv [heads * vdim, rank]: B_a[k, n] = W_uv[a * vdim + n, k]
         attn = self.rt.buffer("latent_out", tokens, self.heads * self.vdim)
-        gate = proj if self.gated else None
-        ops.head_gemm(mixed, self.heads * self.rank, self.rank, self.w_uv, self.vdim * self.rank, 1, self.rank, attn, self.heads * self.vdim,
-                      self.vdim, tokens, self.heads, self.vdim, self.rank, gate=gate, ldg=self.proj_dim, gate_off=self.g_off,
-                      gate_per_output=self.full_gate)
+        first = 0               # rows from here on go over the latents themselves
+        if self._expands(ctx, tokens):
+            first = min(ctx.decode_tail_start, tokens)
+            self._attend_expanded(q, q_off, qa, attn[:first], latent, key_rot, proj, ctx, cache)
+        if tokens > first:
+            rest, per_head = tokens - first, (self.dim + self.vdim) * self.rank
+            # q~[t, a, :] = q[t, a, :dim] @ W_uk[a]          B_a[k, n] = W_ukv[a, k, n]
+            ops.head_gemm(q[first:], q_ld, self.dim + self.rot, self.w_ukv, per_head, self.rank, 1, qa[first:], self.heads * width, width,
+                          rest, self.heads, self.rank, self.dim, a_off=q_off)
+            mixed = self.rt.buffer("latent_mixed", tokens, self.heads * self.rank)
+            self._attend(qa, mixed, latent, key_rot, ctx, cache, tokens, first)
+            # o[t, a, :] = W_uv[a] mixed[t, a, :]            B_a[k, n] = W_ukv[a, dim + n, k]
+            gate = proj[first:] if self.gated else None
+            ops.head_gemm(mixed[first:], self.heads * self.rank, self.rank, self.w_ukv.view(-1)[self.dim * self.rank:], per_head, 1, self.rank,
+                          attn[first:], self.heads * self.vdim, self.vdim, rest, self.heads, self.vdim, self.rank, gate=gate, ldg=self.proj_dim,
+                          gate_off=self.g_off, gate_per_output=self.full_gate)
         if lazy_output:
             return Projection(attn, self.w_o)
         out = self.rt.buffer("mixer_out", tokens, self.hidden)
         ops.linear(attn, self.w_o, out)
         return out
 
+    def _expands(self, ctx, tokens) -> bool:
+        """Whether this step's portions go over expanded keys and values."""
+        split, keys = min(ctx.decode_tail_start, tokens), ctx.portion_keys
+        return (self._expand and split * keys >= self.EXPAND_PAIRS
+                and keys * self.heads * 2 * (self.dim + self.vdim) <= self.MAX_EXPANDED_BYTES)
 
-    def _attend(self, qa, mixed, latent, key_rot, ctx, cache, tokens):
+    def _attend_expanded(self, q, q_off, qa, out, latent, key_rot, proj, ctx, cache):
+        keys, seqs = ctx.portion_keys, ctx.decode_tail_seq
+        rows = max(2048, 1 << (keys - 1).bit_length())          # few sizes, for the scratch and for the copies' descriptors
+        c = self.rt.scratch("latent_dense", rows * self.rank, self.rt.dtype)[:rows * self.rank].view(rows, self.rank)
+        k_rot = self.rt.scratch("latent_dense_rot", rows * self.rot, self.rt.dtype)[:rows * self.rot].view(rows, self.rot)
+        kv_dim = self.heads * (self.dim + self.vdim)
+        kv = self.rt.scratch("latent_expanded", rows * kv_dim, self.rt.dtype)[:rows * kv_dim].view(rows, kv_dim)
+        ops.latent_gather(latent, key_rot, ctx.block_table[cache.group], ctx.ctx_len, seqs, cache.page_size, c[:keys], k_rot[:keys])
+        ops.linear(c[:keys], self.w_ukv.view(kv_dim, self.rank), kv[:keys])
+        ops.latent_prefill_tc(q, q_off, qa, self.rank, self.rank + self.rot, kv, k_rot, out, ctx.q_start, ctx.q_len, ctx.ctx_len, seqs,
+                              self.heads, self.scale, sinks=self.sinks, gate=proj if self.gated else None, gate_off=self.g_off,
+                              gate_per_output=self.full_gate)
+
+    def _attend(self, qa, mixed, latent, key_rot, ctx, cache, tokens, first: int = 0):
+        """Attention over the latents themselves for the rows from ``first`` on (0, or where the decode tail starts)."""
         table = ctx.block_table[cache.group]
         if not self._fast:
             # the exact kernel: the whole 32-bit path, and sizes the tensor-core kernel refuses
@@ -209,7 +255,7 @@ class LatentAttention(Mixer):
             return
         geometry = (self.heads, self.rank, self.rot, cache.page_size, self.scale)
         split = min(ctx.decode_tail_start, tokens)          # portions before, single tokens after
-        if split > 0:
+        if split > first:
             ops.latent_attention_tc(qa, mixed, None, latent, key_rot, table, ctx.q_start, ctx.q_len, ctx.ctx_len, ctx.seq_of_token, 0,
                                     ctx.decode_tail_seq, 0, split, max(ctx.max_q_len, 2), *geometry, sinks=self.sinks)
         if tokens > split:

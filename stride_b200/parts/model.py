@@ -146,6 +146,11 @@ class DecoderModel:
         return out
 
     @property
+    def sizes_by_context(self) -> bool:
+        """True when a part sizes the launches of a prompt's portion by the keys that the requests hold."""
+        return any(getattr(p, "sizes_by_context", False) for layer in self.layers for p in getattr(layer, "parts", lambda: ())())
+
+    @property
     def graph_safe(self) -> bool:
         """False when a part needs the host's view of the step and therefore cannot
         be replayed from a captured graph."""

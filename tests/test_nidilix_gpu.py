@@ -201,6 +201,66 @@ def test_tensor_core_latent_attention_against_the_exact_kernel(gpu, heads, rank,
     close(got, want, 2e-2)
 
 
+@pytest.mark.parametrize("page,gate_kind,sinks", [(16, None, False), (8, "head", True), (64, "output", True)])
+def test_expanded_latent_attention_against_float64(gpu, page, gate_kind, sinks):
+    """Portions over expanded keys and values: a prompt, a portion behind a context, whole and broken tiles of queries and of keys, a
+    single token; keys scattered over shuffled pages; rows past the last request's keys are NaN."""
+    from stride_b200.csrc import ops
+    heads, rank, dim, rot, scale = 3, 40, 128, 64, 192 ** -0.5
+    g = torch.Generator().manual_seed(page)
+    lens = [(0, 75), (40, 9), (0, 128), (130, 65), (63, 1), (0, 129)]                                                # (cached, new)
+    total_pages = sum(-(-(c + n) // page) for c, n in lens) + 3
+    perm = torch.randperm(total_pages, generator=g).tolist()
+    latent = torch.randn(total_pages, 1, page, rank, generator=g).bfloat16().cuda()
+    key_rot = torch.randn(total_pages, 1, page, rot, generator=g).bfloat16().cuda()
+    table = torch.full((len(lens), max(-(-(c + n) // page) for c, n in lens)), -1, dtype=torch.int32)
+    q_start, q_len, ctx_len, at, flat = [], [], [], 0, []
+    for s, (c, n) in enumerate(lens):
+        pages = [perm.pop() for _ in range(-(-(c + n) // page))]
+        table[s, :len(pages)] = torch.tensor(pages)
+        q_start.append(at), q_len.append(n), ctx_len.append(c + n)
+        flat += [pages[j // page] * page + j % page for j in range(c + n)]
+        at += n
+    tokens, keys, rows = at, len(flat), 1000
+    dev = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    nan = lambda *shape: torch.full(shape, float("nan"), dtype=torch.bfloat16, device="cuda")
+    c, k_rot, kv = nan(rows, rank), nan(rows, rot), nan(rows, heads * 2 * dim)
+    ops.latent_gather(latent, key_rot, table.cuda(), dev(ctx_len), len(lens), page, c, k_rot)
+    at = torch.tensor(flat, device="cuda")
+    assert torch.equal(c[:keys], latent.view(-1, rank)[at]) and torch.equal(k_rot[:keys], key_rot.view(-1, rot)[at])
+    assert bool(c[keys:].isnan().all()) and bool(k_rot[keys:].isnan().all())
+    w = (torch.randn(heads * 2 * dim, rank, generator=g) * rank ** -0.5).bfloat16().cuda()
+    ops.linear(c[:keys].contiguous(), w, kv[:keys])
+    extra, per = 5, rank + rot                                  # rows of single tokens behind the portions; the queries' own columns
+    q = torch.randn(tokens + extra, 16 + heads * (dim + rot), generator=g).bfloat16().cuda()
+    q_rot = torch.randn(tokens + extra, heads * per, generator=g).bfloat16().cuda()
+    gate = None if gate_kind is None else torch.randn(tokens + extra, 8 + heads * dim, generator=g).bfloat16().cuda()
+    sink = torch.tensor([0.5, 3.0, -40.0], device="cuda") if sinks else None
+    out = nan(tokens + 1, heads * dim)
+    ops.latent_prefill_tc(q, 16, q_rot, rank, per, kv, k_rot, out[:tokens], dev(q_start), dev(q_len), dev(ctx_len), len(lens), heads, scale,
+                          sinks=sink, gate=gate, gate_off=8, gate_per_output=gate_kind == "output")
+    torch.cuda.synchronize()
+    ops.check_kernel_status()
+    assert bool(out[tokens].isnan().all())
+    want, key0 = torch.zeros(tokens, heads, dim, dtype=torch.float64, device="cuda"), 0
+    for s, (before, n) in enumerate(lens):
+        own = kv[key0:key0 + before + n].double().view(-1, heads, 2 * dim)
+        k = torch.cat([own[..., :dim], k_rot[key0:key0 + before + n].double()[:, None].expand(-1, heads, -1)], -1)
+        r = slice(q_start[s], q_start[s] + n)
+        qs = torch.cat([q[r, 16:].double().view(n, heads, -1)[..., :dim], q_rot[r].double().view(n, heads, per)[..., rank:]], -1)
+        z = torch.einsum("nhd,jhd->hnj", qs, k) * scale
+        z = z.masked_fill(torch.arange(before + n, device="cuda")[None, :] > torch.arange(before, before + n, device="cuda")[:, None], float("-inf"))
+        if sinks:
+            z = torch.cat([z, sink.double()[:, None, None].expand(heads, n, 1)], -1)
+        want[r] = torch.einsum("hnj,jhd->nhd", torch.softmax(z, -1)[..., :before + n], own[..., dim:])
+        key0 += before + n
+    if gate is not None:
+        used = torch.sigmoid(gate[:tokens, 8:].double())
+        want = want * (used[:, :heads, None] if gate_kind == "head" else used[:, :heads * dim].view(tokens, heads, dim))
+    # a probability and the result are rounded to 8 bits: at most 2^-8 of the largest value each
+    close(out[:tokens], want.view(tokens, -1), 1e-2)
+
+
 # ----------------------------------------------------------- each mixer alone, in a model of nothing else
 ONLY_RECURRENT = cases.config(72, 101, [(cases.recurrent(88, 4, 5), None), (cases.recurrent(40, 1, 2), None)], mult=1.0)
 ONLY_ATTENTION = cases.config(72, 101, [(cases.attention(3, 24, 8, 4, 16, 48), None),
