@@ -16,6 +16,7 @@
 //                 every token of a long sequence
 //   rglru_scan    the recurrence over each request's tokens, the output, and the new state (S and the tail)
 #include "common.cuh"
+#include "mma.cuh"
 
 namespace stride {
 
@@ -26,6 +27,63 @@ __device__ __forceinline__ float gelu_tanh_f(float z) {
 }
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
+
+// A long step with four taps: a thread owns four channels of eight consecutive tokens and keeps the last three rows in registers,
+// so that a row is read once and not four times. 2,048 tokens x 2,560 channels: 12 us, 41 us with a thread a number.
+constexpr int CT = 8;
+__global__ void __launch_bounds__(128)
+rglru_conv_rows_kernel(const __nv_bfloat16* __restrict__ xy, int ld, int x_off, const float* __restrict__ bias_x, const __nv_bfloat16* __restrict__ conv_w,
+                       const float* __restrict__ conv_b, const float* __restrict__ state, const int32_t* __restrict__ seq_of_token,
+                       const int32_t* __restrict__ q_start, const int32_t* __restrict__ state_slot, float* __restrict__ u, int tokens, int width) {
+    constexpr int TAPS = 4;
+    pdl_trigger();
+    const int c = (blockIdx.x * 128 + threadIdx.x) * 4, t0 = blockIdx.y * CT;
+    if (c >= width) return;
+    float w[4][TAPS], bias[4], first[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) w[e][j] = to_f32(conv_w[static_cast<size_t>(c + e) * TAPS + j]);
+        bias[e] = bias_x[c + e];
+        first[e] = conv_b[c + e];
+    }
+    pdl_wait();
+    uint2 raw[CT + TAPS - 1];
+#pragma unroll
+    for (int i = 0; i < CT + TAPS - 1; ++i) {
+        const int t = t0 + i - (TAPS - 1);
+        raw[i] = t >= 0 && t < tokens ? *reinterpret_cast<const uint2*>(xy + static_cast<size_t>(t) * ld + x_off + c) : make_uint2(0, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < CT; ++i) {
+        const int t = t0 + i;
+        if (t >= tokens) break;
+        const int seq = seq_of_token[t];
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        if (seq >= 0) {
+            const int local = t - q_start[seq];
+            const float* tail = state + static_cast<size_t>(state_slot[seq]) * TAPS * width;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[e] = first[e];
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) {
+                const int src = local - (TAPS - 1) + j;
+                float v[4];
+                if (src >= 0) {
+                    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[i + j].x));
+                    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[i + j].y));
+                    v[0] = lo.x + bias[0]; v[1] = lo.y + bias[1]; v[2] = hi.x + bias[2]; v[3] = hi.y + bias[3];
+                } else {
+                    const float4 q = *reinterpret_cast<const float4*>(tail + static_cast<size_t>(TAPS - 1 + src) * width + c);
+                    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[e] = fmaf(w[e][j], v[e], acc[e]);
+            }
+        }
+        *reinterpret_cast<float4*>(u + static_cast<size_t>(t) * width + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    }
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -126,54 +184,125 @@ rglru_gates_kernel(const float* __restrict__ u, const T* __restrict__ wa_t, cons
     }
 }
 
-// The same products for a long step: GT tokens x 128 output channels of one block a CTA, each thread one channel and
-// the whole sum over the block's inputs; the tokens' inputs lie [input][token] in shared memory, so that a thread takes
-// the eight tokens of an input with two 16-byte loads for sixteen multiply-adds.
-template <typename T>
-__global__ void __launch_bounds__(128)
-rglru_gates_wide_kernel(const float* __restrict__ u, const T* __restrict__ wa_t, const T* __restrict__ wi_t, const float* __restrict__ ba,
-                        const float* __restrict__ bi, const float* __restrict__ lam, float decay, float* __restrict__ a_out,
-                        float* __restrict__ gx_out, int tokens, int width, int bw) {
+// The same products for a long step in bfloat16 mode, on the tensor cores. The inputs are float32: each is cut into three bfloat16
+// numbers that add up to it (24 bits), the weights are bfloat16 as stored. The tensor cores cut off what falls below their
+// accumulator's last place, always towards zero, which over a long sum is twice the error of rounded multiply-adds (2.4e-7 against
+// 1.2e-7 at 72 inputs): so the first parts' products of 16 inputs start from zero and are added up with rounded additions, and only
+// those of the second and third parts, 2^-8 and less of them, stay in an accumulator. A CTA: 64 tokens x 64 output channels
+// of one block, both gates; eight warps, 32 tokens x 16 channels each; 64 inputs at a time through shared memory. Bound by
+// the exponentials of its epilogue (22 us) and the products; 2,048 tokens x 10 blocks of 256: 114 us, 243 us with multiply-adds
+// (8 tokens x 128 channels a CTA).
+template <bool VEC>
+__global__ void __launch_bounds__(256, 2)
+rglru_gates_mma_kernel(const float* __restrict__ u, const __nv_bfloat16* __restrict__ wa_t, const __nv_bfloat16* __restrict__ wi_t,
+                       const float* __restrict__ ba, const float* __restrict__ bi, const float* __restrict__ lam, float decay,
+                       float* __restrict__ a_out, float* __restrict__ gx_out, int tokens, int width, int bw) {
+    constexpr int LD = 72;                              // 64 numbers and 16 bytes: rows of a fragment meet no bank twice
+    __shared__ __align__(16) __nv_bfloat16 us[3][64][LD];      // [part][token][input]
+    __shared__ __align__(16) __nv_bfloat16 ws[2][64][LD];      // [gate][input][channel]
     pdl_trigger();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int b = blockIdx.y, t0 = blockIdx.z * 64, c0 = blockIdx.x * 64;
+    const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
+    const __nv_bfloat16* const wg[2] = {wa_t + static_cast<size_t>(b) * bw * bw, wi_t + static_cast<size_t>(b) * bw * bw};
+    const float* const ub = u + static_cast<size_t>(b) * bw;
+    float acc[2][4][4] = {}, low[2][4][4] = {};         // [16 tokens][gate, 8 channels][fragment]
     pdl_wait();
-    extern __shared__ __align__(16) float us[];         // [bw][GT]
-    const int b = blockIdx.y;
-    const int t0 = blockIdx.z * GT;
-    const int oc = blockIdx.x * 128 + threadIdx.x;
-    for (int i = threadIdx.x; i < GT * bw; i += 128) {
-        const int tt = i / bw, k = i % bw;
-        us[k * GT + tt] = t0 + tt < tokens ? u[static_cast<size_t>(t0 + tt) * width + b * bw + k] : 0.f;
-    }
-    __syncthreads();
-    if (oc >= bw) return;
-    float accr[GT], acci[GT];
+    for (int k0 = 0; k0 < bw; k0 += 64) {
+        if (k0) __syncthreads();
+        for (int p = tid; p < 64 * 16; p += 256) {      // 4 inputs of a token
+            const int r = p >> 4, k = (p & 15) * 4;
+            float x[4] = {0.f, 0.f, 0.f, 0.f};
+            if (t0 + r < tokens) {
+                const float* src = ub + static_cast<size_t>(t0 + r) * width + k0 + k;
+                if (VEC) {
+                    if (k0 + k < bw) {
+                        const float4 v = *reinterpret_cast<const float4*>(src);
+                        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+                    }
+                } else {
 #pragma unroll
-    for (int tt = 0; tt < GT; ++tt) accr[tt] = acci[tt] = 0.f;
-    const T* wa = wa_t + static_cast<size_t>(b) * bw * bw + oc;
-    const T* wi = wi_t + static_cast<size_t>(b) * bw * bw + oc;
-#pragma unroll 4
-    for (int k = 0; k < bw; ++k) {
-        const float wr = to_f32(wa[static_cast<size_t>(k) * bw]), wg = to_f32(wi[static_cast<size_t>(k) * bw]);
-        const float4 x0 = *reinterpret_cast<const float4*>(us + k * GT), x1 = *reinterpret_cast<const float4*>(us + k * GT + 4);
-        const float x[GT] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+                    for (int e = 0; e < 4; ++e)
+                        if (k0 + k + e < bw) x[e] = src[e];
+                }
+            }
 #pragma unroll
-        for (int tt = 0; tt < GT; ++tt) {
-            accr[tt] = fmaf(wr, x[tt], accr[tt]);
-            acci[tt] = fmaf(wg, x[tt], acci[tt]);
+            for (int part = 0; part < 3; ++part) {
+                __nv_bfloat162 h[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    h[e] = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
+                    const float lo = __bfloat162float(h[e].x), hi = __bfloat162float(h[e].y);
+                    x[2 * e] = isinf(lo) ? 0.f : x[2 * e] - lo;             // an infinity is whole in its first part
+                    x[2 * e + 1] = isinf(hi) ? 0.f : x[2 * e + 1] - hi;
+                }
+                *reinterpret_cast<uint2*>(&us[part][r][k]) = make_uint2(*reinterpret_cast<uint32_t*>(&h[0]), *reinterpret_cast<uint32_t*>(&h[1]));
+            }
+        }
+        for (int p = tid; p < 2 * 64 * 8; p += 256) {   // 8 channels of an input
+            const int gate = p >> 9, k = (p >> 3) & 63, c = (p & 7) * 8;
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (k0 + k < bw) {
+                const __nv_bfloat16* src = wg[gate] + static_cast<size_t>(k0 + k) * bw + c0 + c;
+                if (VEC) {
+                    if (c0 + c < bw) v = *reinterpret_cast<const uint4*>(src);
+                } else {
+                    __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&v);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (c0 + c + i < bw) e[i] = src[i];
+                }
+            }
+            *reinterpret_cast<uint4*>(&ws[gate][k][c]) = v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 64; k += 16) {
+            uint32_t bf[2][4];                          // per gate: (channels 0-7: inputs 0-7, 8-15), (channels 8-15: the same)
+#pragma unroll
+            for (int gate = 0; gate < 2; ++gate) ldmatrix_x4_trans(bf[gate], smem_addr(&ws[gate][k + (lane & 15)][wn + (lane >> 4) * 8]));
+#pragma unroll
+            for (int part = 2; part >= 0; --part)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    uint32_t af[4];
+                    ldmatrix_x4(af, smem_addr(&us[part][wm + i * 16 + (lane & 15)][k + (lane >> 4) * 8]));
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        if (part) {
+                            mma_bf16_16816(low[i][n], af, bf[n >> 1][(n & 1) * 2], bf[n >> 1][(n & 1) * 2 + 1]);
+                        } else {
+                            float d[4] = {0.f, 0.f, 0.f, 0.f};
+                            mma_bf16_16816(d, af, bf[n >> 1][(n & 1) * 2], bf[n >> 1][(n & 1) * 2 + 1]);
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) acc[i][n][e] += d[e];
+                        }
+                    }
+                }
         }
     }
-    const int c = b * bw + oc;
-    const float rate = decay * softplus_f(lam[c]);
-    const float br = ba[c], bg = bi[c];
 #pragma unroll
-    for (int tt = 0; tt < GT; ++tt) {
-        if (t0 + tt >= tokens) break;
-        const float r = sigmoid_f(accr[tt] + br), g = sigmoid_f(acci[tt] + bg);
-        const float log_a = -rate * r;
-        const size_t at = static_cast<size_t>(t0 + tt) * width + c;
-        a_out[at] = expm1f(log_a);
-        gx_out[at] = sqrtf(-expm1f(2.f * log_a)) * g * us[oc * GT + tt];
-    }
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int oc = c0 + wn + n * 8 + 2 * t + e;
+            if (oc >= bw) continue;
+            const int c = b * bw + oc;
+            const float rate = decay * softplus_f(lam[c]), br = ba[c], bg = bi[c];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int row = t0 + wm + i * 16 + g + 8 * h;
+                    if (row >= tokens) continue;
+                    const float r = sigmoid_f(acc[i][n][2 * h + e] + low[i][n][2 * h + e] + br);
+                    const float q = sigmoid_f(acc[i][2 + n][2 * h + e] + low[i][2 + n][2 * h + e] + bg);
+                    const float log_a = -rate * r;
+                    const size_t at = static_cast<size_t>(row) * width + c;
+                    a_out[at] = expm1f(log_a);
+                    gx_out[at] = sqrtf(-expm1f(2.f * log_a)) * q * u[at];
+                }
+        }
 }
 
 template <typename T>
@@ -328,6 +457,14 @@ int stride_rglru_conv(const void* xy, int ld, int x_off, const float* bias_x, co
     if (tokens < 0 || width <= 0 || taps <= 0 || ld <= 0 || x_off < 0) return STRIDE_BAD_ARGUMENT;
     if (taps > kMaxTaps) return STRIDE_UNSUPPORTED;
     if (tokens == 0) return 0;
+    // (short steps spread better with a thread a number)
+    if (dtype == STRIDE_DTYPE_BF16 && taps == 4 && tokens >= 128 && width % 4 == 0 && ld % 4 == 0 && x_off % 4 == 0 &&
+        (reinterpret_cast<uintptr_t>(xy) | reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(state)) % 16 == 0) {
+        stride::launch(rglru_conv_rows_kernel, dim3((width / 4 + 127) / 128, (tokens + CT - 1) / CT), dim3(128), 0, stream,
+                       static_cast<const __nv_bfloat16*>(xy), ld, x_off, bias_x, static_cast<const __nv_bfloat16*>(conv_w), conv_b, state, seq_of_token,
+                       q_start, state_slot, u, tokens, width);
+        return STRIDE_LAUNCH_STATUS();
+    }
     const dim3 grid(tokens, (width + 255) / 256);
     if (dtype == STRIDE_DTYPE_F32)
         stride::launch(rglru_conv_kernel<float>, grid, dim3(256), 0, stream, static_cast<const float*>(xy), ld, x_off, bias_x,
@@ -350,19 +487,19 @@ int stride_rglru_gates(const float* u, const void* wa_t, const void* wi_t, const
     if (smem > 48 * 1024) {     // blocks of more than 1,280 channels: ask for the shared memory beyond the default limit
         const int want = static_cast<int>(smem);
         if (cudaFuncSetAttribute(rglru_gates_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, want) != cudaSuccess ||
-            cudaFuncSetAttribute(rglru_gates_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, want) != cudaSuccess ||
-            cudaFuncSetAttribute(rglru_gates_wide_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, want) != cudaSuccess)
+            cudaFuncSetAttribute(rglru_gates_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, want) != cudaSuccess)
             return STRIDE_UNSUPPORTED;
     }
     const dim3 grid((bw + GC - 1) / GC, blocks, (tokens + GT - 1) / GT);
     if (grid.z > 65535 || grid.y > 65535) return STRIDE_UNSUPPORTED;
     if (tokens > 64 && dtype == STRIDE_DTYPE_BF16) {
-        // Long steps in bfloat16 mode: one thread sums all of a block's inputs. (The 32-bit path keeps one form for
-        // every step, so that a token's sums have the same order however the step was cut.)
-        const dim3 wide((bw + 127) / 128, blocks, (tokens + GT - 1) / GT);
-        stride::launch(rglru_gates_wide_kernel<__nv_bfloat16>, wide, dim3(128), static_cast<size_t>(GT) * bw * sizeof(float), stream, u,
-                       static_cast<const __nv_bfloat16*>(wa_t), static_cast<const __nv_bfloat16*>(wi_t), ba, bi, lam, decay, a_out, gx_out,
-                       tokens, width, bw);
+        // Long steps in bfloat16 mode. (The 32-bit path keeps one form for every step, so that a token's sums have the same order
+        // however the step was cut.)
+        const dim3 tiles((bw + 63) / 64, blocks, (tokens + 63) / 64);
+        const bool vec = bw % 8 == 0 && (reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(wa_t) | reinterpret_cast<uintptr_t>(wi_t)) % 16 == 0;
+        const auto kernel = vec ? rglru_gates_mma_kernel<true> : rglru_gates_mma_kernel<false>;
+        stride::launch(kernel, tiles, dim3(256), 0, stream, u, static_cast<const __nv_bfloat16*>(wa_t), static_cast<const __nv_bfloat16*>(wi_t), ba, bi,
+                       lam, decay, a_out, gx_out, tokens, width, bw);
         return STRIDE_LAUNCH_STATUS();
     }
     if (dtype == STRIDE_DTYPE_F32)

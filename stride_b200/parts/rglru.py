@@ -24,6 +24,7 @@ import torch
 
 from ..csrc import ops
 from .base import Mixer, Projection, StateRequest, TensorDecl, register_part
+from .runtime import sequence_slots
 
 
 class RecurrentGatedUnit(Mixer):
@@ -84,7 +85,7 @@ class RecurrentGatedUnit(Mixer):
         gx = self.rt.buffer("rglru_gx", tokens, w, torch.float32)
         ops.rglru_gates(u, self.wa_t, self.wi_t, self.ba, self.bi, self.lam, self.decay, a, gx, self.blocks)
         mixed = self.rt.buffer("rglru_out", tokens, w)
-        seqs = ctx.q_len.shape[0]
+        seqs = sequence_slots(ctx)
         if x.dtype == torch.bfloat16 and ctx.max_q_len >= ops.SCAN_PIECES_MIN_TOKENS:
             # a long portion: the recurrence in pieces of 64 tokens, parallel over the pieces
             piece = self.rt.scratch("rglru_pieces", (tokens // 64 + seqs + 1) * 2 * w)

@@ -201,6 +201,58 @@ def test_tensor_core_latent_attention_against_the_exact_kernel(gpu, heads, rank,
     close(got, want, 2e-2)
 
 
+@pytest.mark.parametrize("tokens,blocks,bw", [(65, 1, 8), (130, 3, 72), (127, 2, 30), (192, 1, 256), (66, 2, 1)])
+def test_recurrent_gates_of_long_steps_against_float64(gpu, tokens, blocks, bw):
+    """Three bfloat16 parts of a float32 input on the tensor cores: no further from 64 bits than the multiply-adds of short steps (a half more
+    is left for the luck of the draw), at broken tiles of tokens, channels and inputs, and rows that cannot be copied in 16 bytes."""
+    from stride_b200.csrc import ops
+    g = torch.Generator().manual_seed(tokens + bw)
+    width, decay = blocks * bw, 8.0
+    u = (torch.randn(tokens, width, generator=g) * torch.exp(torch.randn(tokens, 1, generator=g))).cuda()
+    wa, wi = ((torch.randn(blocks, bw, bw, generator=g) * bw ** -0.5).bfloat16().cuda() for _ in range(2))      # [block, in, out]
+    ba, bi, lam = (torch.randn(width, generator=g).cuda() for _ in range(3))
+    u64 = u.double().view(tokens, blocks, bw)
+    r, q = (torch.sigmoid(torch.einsum("tbi,bio->tbo", u64, w.double()).reshape(tokens, width) + z.double()) for w, z in ((wa, ba), (wi, bi)))
+    log_a = -decay * torch.nn.functional.softplus(lam.double()) * r
+    want = torch.expm1(log_a), torch.sqrt(-torch.expm1(2 * log_a)) * q * u.double()
+    got = [torch.full((tokens + 1, width), 7.0, device="cuda") for _ in range(2)]
+    ops.rglru_gates(u, wa, wi, ba, bi, lam, decay, got[0][:tokens], got[1][:tokens], blocks)
+    short = [torch.empty(tokens, width, device="cuda") for _ in range(2)]
+    for at in range(0, tokens, 64):
+        ops.rglru_gates(u[at:at + 64], wa, wi, ba, bi, lam, decay, short[0][at:at + 64], short[1][at:at + 64], blocks)
+    error = lambda x, y: float((x.double() - y).norm() / y.norm())
+    for x, s, y in zip(got, short, want):
+        assert bool((x[tokens] == 7.0).all())
+        assert error(x[:tokens], y) <= 1.5 * error(s, y) + 2.0 ** -26 and error(s, y) < 1e-6, (error(x[:tokens], y), error(s, y))
+
+
+@pytest.mark.parametrize("width", [4, 516])
+def test_recurrent_convolution_of_long_steps(gpu, width):
+    """Four taps over rows kept in registers: requests that start, go on behind a tail and end inside a run of eight tokens, padding, and
+    a step whose length is no multiple of eight."""
+    from stride_b200.csrc import ops
+    g = torch.Generator().manual_seed(width)
+    lens, taps = [(0, 5), (3, 1), (9, 2), (0, 70), (7, 57)], 4                          # (cached, new)
+    tokens = sum(n for _c, n in lens) + 2
+    xy = torch.randn(tokens, 2 * width, generator=g).bfloat16()
+    bias_x, conv_b = torch.randn(width, generator=g), torch.randn(width, generator=g)
+    conv_w = torch.randn(width, taps, generator=g).bfloat16()
+    state = torch.randn(len(lens) + 1, taps, width, generator=g)
+    seq_of, q_start, slots, want, at = [], [], [], torch.zeros(tokens, width, dtype=torch.float64), 0
+    for s, (_c, n) in enumerate(lens):
+        slots.append(len(lens) - s)
+        q_start.append(at)
+        seq_of += [s] * n
+        rows = torch.cat([state[slots[-1], :taps - 1].double(), xy[at:at + n, width:].double() + bias_x.double()])
+        for i in range(n):
+            want[at + i] = conv_b.double() + (rows[i:i + taps].T * conv_w.double()).sum(1)
+        at += n
+    dev = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    u = torch.full((tokens, width), 7.0, device="cuda")
+    ops.rglru_conv(xy.cuda(), width, bias_x.cuda(), conv_w.cuda(), conv_b.cuda(), state.cuda(), dev(seq_of + [-1, -1]), dev(q_start), dev(slots), u)
+    assert float((u.cpu().double() - want).abs().max()) <= 6 * 2.0 ** -24 * 40.0        # five sums, none of their terms above 40 here
+
+
 @pytest.mark.parametrize("page,gate_kind,sinks", [(16, None, False), (8, "head", True), (64, "output", True)])
 def test_expanded_latent_attention_against_float64(gpu, page, gate_kind, sinks):
     """Portions over expanded keys and values: a prompt, a portion behind a context, whole and broken tiles of queries and of keys, a
