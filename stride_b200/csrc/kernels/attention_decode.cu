@@ -168,15 +168,15 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
         cp_async_commit();
     };
     const bool holds_newest = pos < lo + split_keys;      // the key written by the kernel before this one is in this split
-    if (!holds_newest) {
+    // (by tiles with TMA: only the tile of the token's own position waits; cp.async groups must be committed in order)
+    auto waits = [&](int j) { return TMA ? tile_base(j) + kTileKeys > pos : holds_newest; };
 #pragma unroll
-        for (int st = 0; st < kStages; ++st) issue(st);
-    }
+    for (int st = 0; st < kStages; ++st)
+        if (!waits(st)) issue(st);
     pdl_wait();
-    if (holds_newest) {
 #pragma unroll
-        for (int st = 0; st < kStages; ++st) issue(st);
-    }
+    for (int st = 0; st < kStages; ++st)
+        if (waits(st)) issue(st);
 
     // The query group as the A operand: row r is query head kvh * group + r.
     uint32_t qa[KSTEPS][4];
@@ -328,6 +328,7 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
         l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
     }
 
+    const int s_lo = first / split_keys, n = pos / split_keys - s_lo + 1;      // live splits
     // Merge the four warps through shared memory (the key and value tiles are no longer needed).
     __syncthreads();
     float* red = reinterpret_cast<float*>(smem);
@@ -362,6 +363,14 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
             acc += f * src[d];
             sum += f * src[HD + 1];
         }
+        if (n == 1) {       // no other split: what the merge below would make of it
+            if (sinks != nullptr) sum += exp2f(fmaf(sinks[kvh * group + row], 1.4426950408889634f, -mm));
+            float inv = 1.f / sum;
+            if (gate_col >= 0)
+                inv /= 1.f + expf(-__bfloat162float(q[static_cast<size_t>(t) * q_stride + gate_col + kvh * group + row]));
+            out[(static_cast<size_t>(t) * nq + kvh * group + row) * HD + d] = __float2bfloat16_rn(acc * inv);
+            continue;
+        }
         const size_t slot = (static_cast<size_t>(t) * nq + kvh * group + row) * num_splits + split;
         part_o[slot * HD + d] = acc;
         if (d == 0) {
@@ -371,7 +380,7 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
     }
 
     // ---- the CTA that finishes last for this (token, key head) merges the splits
-    const int s_lo = first / split_keys, n = pos / split_keys - s_lo + 1;      // live splits
+    if (n == 1) return;
     __shared__ int is_last;
     __threadfence();
     __syncthreads();
