@@ -22,6 +22,9 @@
 //                 1 / g_j can overflow where a channel forgets nearly everything within a chunk: a CTA whose chunk has a
 //                 channel with g below e^-60 forms its scores with exp(log g_i - log g_j) per channel instead, which only
 //                 costs time. A constant decay never divides: decay^(i - j) is taken from a table of powers.
+//
+// The chunks also run the matrix LSTM of mlstm.cu (mlstm_chunks): its gates are one number a head and token, with a running
+// maximum; n goes along as one more column. 1,999 tokens of 16 heads of 128 x 128: 127 us, 622 us token after token.
 #include "memory_scan.cuh"
 
 namespace stride {
@@ -33,6 +36,17 @@ constexpr int kChunkThreads = 256;
 constexpr int kLd = kChunk + 4;         // row stride of the transposed tiles: 16-byte reads, stores without bank conflicts
 constexpr float kSafeLog = -60.f;
 
+// The gates of a chunk's tokens of one head of the matrix LSTM (lstm_gates_kernel): with b the running sum of the forget gates'
+// logarithms inside the chunk, li the input gates' logarithms, m the running maximum (m_0 at the chunk's start, m_e at its end), token
+// j weighs exp(b_i - b_j + li_j - m_i) in token i's output, the memory at the start exp(b_i + m_0 - m_i).
+struct LstmChunk {
+    float b_hi[kChunk], b_lo[kChunk];   // b in two parts: a difference of two sums is as good as the sum of the logarithms between them
+    float li[kChunk], m[kChunk];
+    float carry[kChunk];                // exp(b_i + m_0 - m_i)
+    float take[kChunk];                 // exp(b_e - b_j + li_j - m_e): token j's weight in the memory at the chunk's end
+    float decay, pad[3];                // carry at the end
+};
+
 struct ChunkArgs {
     const void* q;          // [tokens, ld], head h at column h * D
     const void* k;
@@ -41,6 +55,8 @@ struct ChunkArgs {
     float* cum;             // channel decays: [tokens, H * D], the running logarithm of the decays inside the chunk
     const float* bias;      // channel decays: [H * D]
     const float* powers;    // constant decay: [H, kChunk + 1], decay^n
+    const LstmChunk* lstm;  // matrix LSTM: [seqs * max_pieces, H]
+    float* piece_n;         // matrix LSTM: [seqs * max_pieces, H, D]
     float q_scale, inv_tau;
     float* o;               // [tokens, H * DV]
     float* piece_s;         // [seqs * max_pieces, H, D, DV]
@@ -78,6 +94,88 @@ chunk_decay_kernel(const ChunkArgs p) {
                 at[static_cast<size_t>(t0 + u) * HD] = sum;
             }
     }
+}
+
+struct LstmGates {
+    const float* gates;     // [tokens, ld] float32: column h the input gate's projection, column H + h the forget gate's
+    int ld;
+    const float* bias_i;
+    const float* bias_f;
+    float cap;
+    float* state;           // m of head h at m_off + h of a slot's row
+    long long state_stride, m_off;
+    const int32_t* state_slot;
+    LstmChunk* chunks;
+};
+
+// The gates' logarithms, their running sums in a chunk and the running maximum through a whole portion, m_t = max(lf_t + m_(t-1), li_t):
+// with A the sum and B the largest contribution of a run of tokens, two runs make A = A1 + A2, B = max(B1 + A2, B2), and
+// m = max(m_0 + A, B), so 256 tokens (four chunks) are one scan over a CTA. Sums and exponents in float64. Grid (heads, requests).
+static __global__ void __launch_bounds__(256)
+lstm_gates_kernel(const LstmGates p, const int32_t* __restrict__ q_start, const int32_t* __restrict__ q_len, int H, int max_pieces) {
+    __shared__ double w_sum[8], w_top[8], s_b[4], s_m[4];
+    pdl_trigger();
+    pdl_wait();
+    const int h = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int len = q_len[seq], start = q_start[seq];
+    if (len <= 0) return;
+    float* const m_g = p.state + static_cast<size_t>(p.state_slot[seq]) * p.state_stride + p.m_off + h;
+    const float bi = p.bias_i[h], bf = p.bias_f[h];
+    double m_in = *m_g;
+    float zi = 0.f, zf = 0.f;
+    auto fetch = [&](int t) {
+        if (t >= len) return;
+        const size_t row = static_cast<size_t>(start + t) * p.ld;
+        zi = p.gates[row + h];
+        zf = p.gates[row + H + h];
+    };
+    fetch(tid);
+    for (int t0 = 0; t0 < len; t0 += 256) {
+        const bool live = t0 + tid < len;
+        const float li = live ? p.cap * tanhf((zi + bi) / p.cap) : -INFINITY;
+        const float lf = live ? log_sigmoid_f(p.cap * tanhf((zf + bf) / p.cap)) : 0.f;      // a token past the end leaves m as it is
+        fetch(t0 + 256 + tid);
+        double sum = lf, top = li;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double s = __shfl_up_sync(0xffffffffu, sum, o), b = __shfl_up_sync(0xffffffffu, top, o);
+            if (lane >= o) {
+                top = fmax(b + sum, top);
+                sum += s;
+            }
+        }
+        if (lane == 31) { w_sum[warp] = sum; w_top[warp] = top; }
+        __syncthreads();
+        double b = sum;                                 // inside the chunk
+        if (warp & 1) b += w_sum[warp - 1];
+        double m_before = m_in, m_end = m_in;           // before this warp's tokens, behind the last of the 256
+        for (int w = 0; w < 8; ++w) {
+            m_end = fmax(m_end + w_sum[w], w_top[w]);
+            if (w < warp) m_before = m_end;
+        }
+        const double m = fmax(m_before + sum, top);
+        const int c = warp >> 1;                        // this thread's chunk of the four
+        // the chunk's end is its last token, or the portion's; both hold b and m of it (tokens past the end add nothing)
+        if ((warp & 1) && lane == 31) { s_b[c] = b; s_m[c] = m; }
+        __syncthreads();
+        const double m_start = c ? s_m[c - 1] : m_in, b_end = s_b[c], m_last = s_m[c];
+        const int piece = t0 / kChunk + c;
+        if (piece * kChunk < len) {
+            LstmChunk& r = p.chunks[(static_cast<size_t>(seq) * max_pieces + piece) * H + h];
+            const int i = tid & (kChunk - 1);
+            const float hi = static_cast<float>(b);
+            r.b_hi[i] = hi;
+            r.b_lo[i] = static_cast<float>(b - hi);
+            r.li[i] = live ? li : 0.f;
+            r.m[i] = static_cast<float>(m);
+            r.carry[i] = live ? expf(static_cast<float>(b + m_start - m)) : 0.f;
+            r.take[i] = live ? expf(static_cast<float>(b_end - b + li - m_last)) : 0.f;
+            if (i == 0) r.decay = expf(static_cast<float>(b_end + m_start - m_last));
+        }
+        m_in = m_end;
+        __syncthreads();
+    }
+    if (tid == 0) *m_g = static_cast<float>(m_in);
 }
 
 // Eight neighbouring values of a row of the projection.
@@ -149,6 +247,7 @@ chunk_sum_kernel(const ChunkArgs p) {
     const size_t row0 = static_cast<size_t>(p.q_start[seq] + first);
     const float* powers = RULE == kConstantDecay ? p.powers + h * (kChunk + 1) : nullptr;
     const float* cum = RULE == kChannelDecay ? p.cum + row0 * HD + h * D : nullptr;
+    const LstmChunk* lstm = RULE == kLstm ? p.lstm + static_cast<size_t>(z) * p.H + h : nullptr;
     if (p.vec) {
         constexpr int PACKS = kChunk * DP / 8 / kChunkThreads > 0 ? kChunk * DP / 8 / kChunkThreads : 1;
         uint4 raw[PACKS];
@@ -166,6 +265,10 @@ chunk_sum_kernel(const ChunkArgs p) {
                 const float f = j < nt ? powers[nt - 1 - j] : 0.f;
 #pragma unroll
                 for (int e = 0; e < 8; ++e) k[e] = silu_quick(k[e]) * f;
+            } else if (RULE == kLstm) {
+                const float f = j < kChunk ? lstm->take[j] : 0.f;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) k[e] *= f;
             } else if (j < nt && d < D) {
                 const float4* end = reinterpret_cast<const float4*>(cum + static_cast<size_t>(nt - 1) * HD + d);
                 const float4* own = reinterpret_cast<const float4*>(cum + static_cast<size_t>(j) * HD + d);
@@ -191,6 +294,7 @@ chunk_sum_kernel(const ChunkArgs p) {
             if (d < D) {
                 k = load_any(p.k, (row0 + j) * p.ld + h * D + d, p.in_bf16);
                 k = RULE == kConstantDecay ? silu_f(k) * powers[nt - 1 - j]
+                    : RULE == kLstm        ? k * lstm->take[j]
                                            : k * expf(cum[static_cast<size_t>(nt - 1) * HD + d] - cum[static_cast<size_t>(j) * HD + d]);
             }
             ks[idx] = k;
@@ -200,8 +304,20 @@ chunk_sum_kernel(const ChunkArgs p) {
     if (blockIdx.x == 0)
         for (int d = threadIdx.x; d < D; d += kChunkThreads)
             p.piece_p[(static_cast<size_t>(z) * p.H + h) * D + d] =
-                RULE == kConstantDecay ? powers[nt] : expf(cum[static_cast<size_t>(nt - 1) * HD + d]);
+                RULE == kConstantDecay ? powers[nt] : RULE == kLstm ? lstm->decay : expf(cum[static_cast<size_t>(nt - 1) * HD + d]);
     __syncthreads();
+    if (RULE == kLstm && blockIdx.x == 0) {         // the chunk's own share of n: the weighted keys without values
+        for (int d = threadIdx.x; d < D; d += kChunkThreads) {
+            float n4[4] = {0.f, 0.f, 0.f, 0.f};
+            int j = 0;
+            for (; j + 4 <= nt; j += 4) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) n4[e] += ks[(j + e) * DP + d];
+            }
+            for (; j < nt; ++j) n4[0] += ks[j * DP + d];
+            p.piece_n[(static_cast<size_t>(z) * p.H + h) * D + d] = (n4[0] + n4[1]) + (n4[2] + n4[3]);
+        }
+    }
     const int warp = threadIdx.x >> 5, cg = (threadIdx.x & 15) * 4, half = (threadIdx.x >> 4) & 1;
     float* out = p.piece_s + (static_cast<size_t>(z) * p.H + h) * D * DV;
     for (int pass = 0; pass < DP / PASS_ROWS; ++pass) {
@@ -310,6 +426,8 @@ chunk_out_kernel(const ChunkArgs p) {
     const size_t row0 = static_cast<size_t>(p.q_start[seq] + first);
     const float* powers = RULE == kConstantDecay ? p.powers + h * (kChunk + 1) : nullptr;
     const float* cum = RULE == kChannelDecay ? p.cum + row0 * HD + h * D : nullptr;
+    const LstmChunk* lstm = RULE == kLstm ? p.lstm + static_cast<size_t>(z) * p.H + h : nullptr;
+    __shared__ float den_s[RULE == kLstm ? 4 : 1][RULE == kLstm ? kChunk : 1];
     bool safe = true;
     if (RULE == kChannelDecay) {
         int low = 0;
@@ -341,6 +459,9 @@ chunk_out_kernel(const ChunkArgs p) {
                     q[e] = silu_quick(q[e]);
                     k[e] = silu_quick(k[e]);
                 }
+            } else if (RULE == kLstm) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) q[e] *= p.q_scale;
             } else if (i < nt && d < D) {
                 const float4* own = reinterpret_cast<const float4*>(cum + static_cast<size_t>(i) * HD + d);
                 const float4 c0 = own[0], c1 = own[1];
@@ -372,7 +493,7 @@ chunk_out_kernel(const ChunkArgs p) {
                     k = silu_f(k);
                 } else {
                     q *= p.q_scale;
-                    if (safe) {
+                    if (RULE == kChannelDecay && safe) {
                         const float c = cum[static_cast<size_t>(i) * HD + d];
                         q *= expf(c);
                         k *= expf(-c);
@@ -412,7 +533,7 @@ chunk_out_kernel(const ChunkArgs p) {
         float a[4][4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) a[e][0] = a[e][1] = a[e][2] = a[e][3] = 0.f;
-        if (RULE == kConstantDecay || safe) {
+        if (RULE != kChannelDecay || safe) {
             if (tx <= ty) {
 #pragma unroll 8
                 for (int d = 0; d < DP; ++d) {
@@ -446,6 +567,11 @@ chunk_out_kernel(const ChunkArgs p) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int n = 4 * ty + e - (4 * tx + f);
+                if (RULE == kLstm) {
+                    const int i = 4 * ty + e, j = 4 * tx + f;
+                    w[e] = n < 0 || i >= nt ? 0.f : a[e][f] * expf((lstm->b_hi[i] - lstm->b_hi[j]) + (lstm->b_lo[i] - lstm->b_lo[j]) + (lstm->li[j] - lstm->m[i]));
+                    continue;
+                }
                 w[e] = n < 0 ? 0.f : RULE == kConstantDecay ? a[e][f] * powers[n] : a[e][f];
             }
             *reinterpret_cast<float4*>(aT + (4 * tx + f) * kLd + 4 * ty) = make_float4(w[0], w[1], w[2], w[3]);
@@ -457,6 +583,20 @@ chunk_out_kernel(const ChunkArgs p) {
             const int i = idx % kChunk, d = idx / kChunk;
             if (d < D && i < nt) qT[d * kLd + i] *= expf(cum[static_cast<size_t>(i) * HD + d]);
         }
+    }
+    if (RULE == kLstm) {            // n . q of every token, a quarter of its terms a thread
+        const int i = threadIdx.x & (kChunk - 1), part = threadIdx.x / kChunk;
+        const float* n = p.piece_n + (static_cast<size_t>(z) * p.H + h) * D;
+        float own[2] = {0.f, 0.f}, past[2] = {0.f, 0.f};
+        for (int j = part * (kChunk / 4); j < (part + 1) * (kChunk / 4); j += 2) {
+            own[0] += aT[j * kLd + i];
+            own[1] += aT[(j + 1) * kLd + i];
+        }
+        for (int d = part * (DP / 4); d < min(D, (part + 1) * (DP / 4)); d += 2) {
+            past[0] = fmaf(qT[d * kLd + i], n[d], past[0]);
+            if (d + 1 < D) past[1] = fmaf(qT[(d + 1) * kLd + i], n[d + 1], past[1]);
+        }
+        den_s[part][i] = (own[0] + own[1]) + lstm->carry[i] * (past[0] + past[1]);
     }
     // outputs: warp w tokens 8 w .. + 7, lane columns 4 lane .. + 3
     float acc[8][4];
@@ -491,6 +631,14 @@ chunk_out_kernel(const ChunkArgs p) {
             for (int e = 0; e < 4; ++e) acc[r][e] *= f;
         }
     }
+    if (RULE == kLstm) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const float f = lstm->carry[8 * warp + r];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[r][e] *= f;
+        }
+    }
     stage_values<kChunkCols, RULE>(p, kT, row0, nt, h, col0);
     __syncthreads();
     const int last = min(nt, 8 * warp + 8);         // later tokens have no weight in this warp's rows
@@ -500,6 +648,12 @@ chunk_out_kernel(const ChunkArgs p) {
     for (int r = 0; r < 8; ++r) {
         const int i = 8 * warp + r;
         if (i >= nt) break;
+        if (RULE == kLstm) {
+            const float dot = (den_s[0][i] + den_s[1][i]) + (den_s[2][i] + den_s[3][i]);
+            const float f = 1.f / (fmaxf(fabsf(dot), expf(-lstm->m[i])) + 1e-6f);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[r][e] *= f;
+        }
         float* dst = p.o + ((row0 + i) * p.H + h) * DV + col0 + 4 * lane;
         if (s_vec) {
             if (col0 + 4 * lane < DV) *reinterpret_cast<float4*>(dst) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
@@ -602,6 +756,10 @@ int launch_chunks(const ChunkArgs& p, float* state, long long state_stride, cons
     else
         stride::launch(pieces_combine_kernel, dim3((p.H * p.D * p.DV + 255) / 256, num_seqs), dim3(256), 0, stream, p.piece_s,
                        static_cast<const float*>(p.piece_p), state, state_stride, p.q_len, state_slot, p.H, p.D, p.DV, kChunk, p.max_pieces);
+    if (RULE == kLstm)      // n is one more column of the memory
+        stride::launch(pieces_combine_kernel, dim3((p.H * p.D + 255) / 256, num_seqs), dim3(256), 0, stream, p.piece_n,
+                       static_cast<const float*>(p.piece_p), state + static_cast<size_t>(p.H) * p.D * p.DV, state_stride, p.q_len, state_slot, p.H,
+                       p.D, 1, kChunk, p.max_pieces);
     stride::launch(chunk_out_kernel<DP, RULE>, grid, block, out_bytes, stream, p);
     return STRIDE_LAUNCH_STATUS();
 }
@@ -714,6 +872,53 @@ int stride_decay_chunks(const void* q, const void* k, const void* v, int ld, flo
     p.vec = p.in_bf16 && D % 8 == 0 && DV % 8 == 0 && ld % 8 == 0 && aligned(q) && aligned(k) && aligned(v) && (powers || aligned(logit));
     return powers ? dispatch_chunks<kConstantDecay>(p, state, state_stride, state_slot, num_seqs, stream)
                   : dispatch_chunks<kChannelDecay>(p, state, state_stride, state_slot, num_seqs, stream);
+}
+
+// Scratch of stride_mlstm_chunks in floats.
+long long stride_mlstm_chunks_scratch(int num_seqs, int max_pieces, int H, int D, int DV) {
+    return static_cast<long long>(num_seqs) * max_pieces * H * (static_cast<long long>(D) * (DV + 2) + static_cast<long long>(sizeof(LstmChunk) / 4));
+}
+
+// The matrix LSTM (mlstm.cu has the recurrence and the layout of the state) over long portions, chunk by chunk. Arguments as
+// stride_mlstm_scan; scratch: 16-byte aligned. Returns -2 for more than 256 rows a head or too many chunks.
+int stride_mlstm_chunks(const void* proj, int ld, int q_off, int k_off, int v_off, const float* gates, int ld_gates, const float* bias_i,
+                        const float* bias_f, float cap, float q_scale, float* o, float* state, long long state_stride, const int32_t* q_start,
+                        const int32_t* q_len, const int32_t* state_slot, int num_seqs, int H, int D, int DV, int dtype, int max_pieces, float* scratch,
+                        cudaStream_t stream) {
+    if (num_seqs < 0 || H <= 0 || D <= 0 || DV <= 0 || ld <= 0 || ld_gates < 2 * H || !(cap > 0.f) || q_off < 0 || k_off < 0 || v_off < 0 ||
+        max_pieces <= 0 || !scratch)
+        return STRIDE_BAD_ARGUMENT;
+    if (dtype != STRIDE_DTYPE_F32 && dtype != STRIDE_DTYPE_BF16) return STRIDE_BAD_ARGUMENT;
+    if (state_stride < static_cast<long long>(H) * D * DV + static_cast<long long>(H) * D + H) return STRIDE_BAD_ARGUMENT;
+    if (D > 256 || static_cast<long long>(num_seqs) * max_pieces > 65535 || H > 65535 || reinterpret_cast<uintptr_t>(scratch) % 16) return STRIDE_UNSUPPORTED;
+    if (num_seqs == 0) return 0;
+    const int item = dtype == STRIDE_DTYPE_BF16 ? 2 : 4;
+    const size_t records = static_cast<size_t>(num_seqs) * max_pieces * H;
+    auto at = [&](int off) { return static_cast<const unsigned char*>(proj) + static_cast<size_t>(off) * item; };
+    ChunkArgs p = {};
+    p.q = at(q_off);
+    p.k = at(k_off);
+    p.v = at(v_off);
+    p.ld = ld;
+    p.in_bf16 = dtype == STRIDE_DTYPE_BF16 ? 1 : 0;
+    p.q_scale = q_scale;
+    p.o = o;
+    LstmChunk* chunks = reinterpret_cast<LstmChunk*>(scratch);
+    p.lstm = chunks;
+    p.piece_s = scratch + records * (sizeof(LstmChunk) / 4);
+    p.piece_p = p.piece_s + records * D * DV;
+    p.piece_n = p.piece_p + records * D;
+    p.q_start = q_start;
+    p.q_len = q_len;
+    p.H = H;
+    p.D = D;
+    p.DV = DV;
+    p.max_pieces = max_pieces;
+    auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
+    p.vec = p.in_bf16 && D % 8 == 0 && DV % 8 == 0 && ld % 8 == 0 && aligned(p.q) && aligned(p.k) && aligned(p.v);
+    const LstmGates g{gates, ld_gates, bias_i, bias_f, cap, state, state_stride, static_cast<long long>(H) * D * DV + static_cast<long long>(H) * D, state_slot, chunks};
+    stride::launch(lstm_gates_kernel, dim3(H, num_seqs), dim3(256), 0, stream, g, q_start, q_len, H, max_pieces);
+    return dispatch_chunks<kLstm>(p, state, state_stride, state_slot, num_seqs, stream);
 }
 
 }  // extern "C"

@@ -11,6 +11,7 @@ enum MemoryRule {
     kBonusMemory = 1,       // o = (S + diag(bonus) k v^T)^T a ; S <- diag(exp(-exp(w + w0))) S + k v^T
     kChannelDecay = 2,      // S <- diag(sigmoid(w + w0)^(1 / tau)) S + k v^T ; o = q_scale S^T a
     kConstantDecay = 3,     // S <- (1 + fade) S + silu(k) silu(v)^T ; o = S^T silu(a)
+    kLstm = 5,              // the matrix LSTM (mlstm.cu), in decay_memory.cu's chunks only
     kTokenDecay = 4,        // d = softplus(beta + dt_bias), S <- exp(-exp(a_log) d) S + d k v^T ; o = S^T a + skip v (a number a head and token)
 };
 

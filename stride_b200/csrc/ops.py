@@ -182,6 +182,9 @@ _SIGNATURES = {
     "stride_decay_chunks": ("decay_memory", [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_float, c_void_p,
                                              c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                              c_void_p, c_void_p]),
+    "stride_mlstm_chunks": ("decay_memory", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_float, c_void_p,
+                                             c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                             c_void_p]),
     "stride_mlstm_scan": ("mlstm", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_float, c_void_p,
                                     c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "stride_pointwise": ("pointwise", [c_void_p, c_void_p, c_int, c_float, c_longlong, c_int, c_void_p]),
@@ -240,7 +243,7 @@ _CLASS_OF = {
     "stride_head_norm_gate": "per-head norm and gate",
     "stride_stream_concat": "repeated block: input", "stride_add_row_vector": "repeated block: input",
     "stride_rms_norm_cols": "latent norm", "stride_conv_head_norm": "convolution + head norms + cache write",
-    "stride_conv_tail": "convolution + head norms + cache write", "stride_mlstm_scan": "matrix LSTM: recurrence",
+    "stride_conv_tail": "convolution + head norms + cache write", "stride_mlstm_scan": "matrix LSTM: recurrence", "stride_mlstm_chunks": "matrix LSTM: recurrence",
     "stride_conv_row_norm": "convolution + row norms + cache write", "stride_copies_step": "residual copies + norm",
     "stride_decay_scan": "fading memory: recurrence", "stride_decay_chunks": "fading memory: recurrence",
     "stride_decay_step": "fading memory: recurrence",
@@ -654,6 +657,35 @@ def mlstm_scan(proj, q_off: int, k_off: int, v_off: int, gates, bias_i, bias_f, 
         _dev(o, "o", torch.float32), *_state_rows(state), _dev(q_start, "q_start", torch.int32),
         _dev(q_len, "q_len", torch.int32), _dev(state_slot, "state_slot", torch.int32), int(num_seqs), H, D, DV, _code(proj.dtype),
         _stream()), "mlstm_scan")
+
+
+# Portions of at least this many tokens run chunk by chunk in bfloat16 models (0: none do).
+MLSTM_CHUNKS_MIN_TOKENS = int(_os.environ.get("STRIDE_B200_MLSTM_CHUNKS_MIN", "96"))
+
+
+def mlstm_chunks_scratch_floats(num_seqs: int, max_q_len: int, H: int, D: int, DV: int) -> int:
+    f = _bound.get("stride_mlstm_chunks_scratch")
+    if f is None:
+        f = build.load_kernel_library("decay_memory").stride_mlstm_chunks_scratch
+        f.argtypes = [c_int] * 5
+        f.restype = c_longlong
+        _bound["stride_mlstm_chunks_scratch"] = f
+    return int(f(num_seqs, -(-max_q_len // DECAY_CHUNK), H, D, DV))
+
+
+def mlstm_chunks(proj, q_off: int, k_off: int, v_off: int, gates, bias_i, bias_f, cap: float, q_scale: float, o, state, q_start, q_len,
+                 state_slot, num_seqs: int, H: int, D: int, DV: int, max_q_len: int, scratch) -> None:
+    """``mlstm_scan`` with the chunks of every portion side by side (sums in another order)."""
+    if state.shape[1] < mlstm_state_floats(H, D, DV) or o.shape[1] != H * DV or gates.shape[1] < 2 * H:
+        raise KernelError("mlstm_chunks: shapes do not agree")
+    if scratch.numel() < mlstm_chunks_scratch_floats(num_seqs, max_q_len, H, D, DV):
+        raise KernelError("mlstm_chunks: the scratch is too short")
+    _check(_fn("stride_mlstm_chunks")(
+        _dev(proj, "proj"), proj.shape[1], int(q_off), int(k_off), int(v_off), _dev(gates, "gates", torch.float32), gates.shape[1],
+        _dev(bias_i, "bias_i", torch.float32), _dev(bias_f, "bias_f", torch.float32), float(cap), float(q_scale),
+        _dev(o, "o", torch.float32), *_state_rows(state), _dev(q_start, "q_start", torch.int32),
+        _dev(q_len, "q_len", torch.int32), _dev(state_slot, "state_slot", torch.int32), int(num_seqs), H, D, DV, _code(proj.dtype),
+        -(-max_q_len // DECAY_CHUNK), _dev(scratch, "scratch", torch.float32), _stream()), "mlstm_chunks")
 
 
 # ------------------------------------------------------------ fading memories (linear attention with decay)

@@ -92,8 +92,19 @@ class MatrixLstmMixer(Mixer):
         gates = self.rt.buffer("mlstm_gates", tokens, self.gate_cols, f32)
         ops.linear(x, self.w_gates, gates)                  # float32 sums: what enters the recurrence is never rounded to 16 bits
         o = self.rt.buffer("mlstm_o", tokens, self.HV, f32)
-        ops.mlstm_scan(proj, 0, self.k_off, self.v_off, gates, self.bias_i, self.bias_f, self.cap, self.D ** -0.5, o, cache.state,
-                       ctx.q_start, ctx.q_len, ctx.state_slot, sequence_slots(ctx), self.H, self.D, self.DV)
+        columns, gate_args, sizes = (0, self.k_off, self.v_off), (gates, self.bias_i, self.bias_f, self.cap, self.D ** -0.5), (self.H, self.D, self.DV)
+        portions, slots = ctx.decode_tail_seq, sequence_slots(ctx)      # the requests before the trailing single tokens; all of them
+        first = 0
+        # (float32 models keep the one chain, whose sums do not depend on the cutting)
+        if (x.dtype == torch.bfloat16 and portions and 0 < ops.MLSTM_CHUNKS_MIN_TOKENS <= ctx.max_q_len
+                and portions * -(-ctx.max_q_len // ops.DECAY_CHUNK) <= 65535):
+            scratch = self.rt.scratch("mlstm_chunks", ops.mlstm_chunks_scratch_floats(portions, ctx.max_q_len, *sizes))
+            ops.mlstm_chunks(proj, *columns, *gate_args, o, cache.state, ctx.q_start, ctx.q_len, ctx.state_slot, portions, *sizes, ctx.max_q_len,
+                             scratch)
+            first = portions
+        if slots > first:
+            ops.mlstm_scan(proj, *columns, *gate_args, o, cache.state, ctx.q_start[first:], ctx.q_len[first:], ctx.state_slot[first:], slots - first,
+                           *sizes)
         mixed = self.rt.buffer("mlstm_mixed", tokens, self.HV)
         ops.head_norm_gate(o, self.norm_w, True, proj, "sigmoid_compute", mixed, self.H, self.DV, self.norm_eps, gate_off=self.g_off)
         if lazy_output:

@@ -265,6 +265,60 @@ def test_matrix_lstm_scan(gpu, dtype, tol, H, D, DV, cap):
     assert torch.equal(state_dev[:, floats:].cpu(), state[:, floats:])      # nothing beyond a row's memory is touched
 
 
+@pytest.mark.parametrize("H,D,DV,cap,ld_pad", [(2, 24, 16, 6.0, 0), (1, 128, 136, 15.0, 0), (3, 10, 14, 4.0, 3), (1, 200, 20, 15.0, 0)])
+def test_matrix_lstm_chunks(gpu, H, D, DV, cap, ld_pad):
+    """Long portions chunk by chunk (one chunk, whole and broken ones, more than the 256 tokens of a turn of the gates' scan; with a past
+    and fresh): no further from the recurrence in float64 than the chain of tokens (half as much again is left for the luck of the
+    draw), in outputs and in the state rows."""
+    from stride_b200.csrc import ops
+    g = torch.Generator().manual_seed(H * D + DV)
+    new, slots = [130, 64, 289, 1], [1, 2, 0, 3]
+    tokens = sum(new) + 1
+    k_off, v_off = H * D, 2 * H * D + 8
+    ld = v_off + H * DV + ld_pad
+    proj = torch.randn(tokens, ld, generator=g).bfloat16()
+    gates = torch.randn(tokens, 2 * H + 3, generator=g) * 2.0
+    bias_i, bias_f = torch.randn(H, generator=g), 2.0 + torch.randn(H, generator=g)
+    floats = H * D * DV + H * D + H
+    state = torch.zeros(4, (floats + 7) // 4 * 4)
+    state[1, :H * D * DV + H * D] = torch.randn(H * D * DV + H * D, generator=g)
+    state[1, H * D * DV + H * D:floats] = torch.rand(H, generator=g) * 3.0
+    state[2, :floats] = state[1, :floats] * 0.5
+    want, want_state, at = torch.zeros(tokens - 1, H * DV, dtype=torch.float64), state.double().clone(), 0
+    for n, slot in zip(new, slots):
+        x = proj[at:at + n].double()
+        for a in range(H):
+            S = state[slot, a * D * DV:(a + 1) * D * DV].double().view(D, DV).clone()
+            nn = state[slot, H * D * DV + a * D:H * D * DV + (a + 1) * D].double().clone()
+            top = float(state[slot, H * D * DV + H * D + a])
+            for t in range(n):
+                q, k, v = x[t, a * D:(a + 1) * D] * D ** -0.5, x[t, k_off + a * D:k_off + (a + 1) * D], x[t, v_off + a * DV:v_off + (a + 1) * DV]
+                li = cap * math.tanh((float(gates[at + t, a]) + float(bias_i[a])) / cap)
+                lf = plain.log_sigmoid(cap * math.tanh((float(gates[at + t, H + a]) + float(bias_f[a])) / cap))
+                new_top = max(lf + top, li)
+                keep, take = math.exp(lf + top - new_top), math.exp(li - new_top)
+                S, nn, top = keep * S + take * torch.outer(k, v), keep * nn + take * k, new_top
+                want[at + t, a * DV:(a + 1) * DV] = (S.T @ q) / (max(abs(float(nn @ q)), math.exp(-top)) + 1e-6)
+            want_state[slot, a * D * DV:(a + 1) * D * DV] = S.reshape(-1)
+            want_state[slot, H * D * DV + a * D:H * D * DV + (a + 1) * D] = nn
+            want_state[slot, H * D * DV + H * D + a] = top
+        at += n
+    results = []
+    for chunks in (False, True):
+        state_dev, o = state.cuda(), torch.full((tokens, H * DV), float("nan"), device="cuda")
+        args = (proj.cuda(), 0, k_off, v_off, gates.cuda(), bias_i.cuda(), bias_f.cuda(), cap, D ** -0.5, o, state_dev,
+                dev([0, new[0], new[0] + new[1], sum(new[:3]), 0]), dev(new + [0]), dev(slots + [0]), 5, H, D, DV)
+        if chunks:
+            scratch = torch.full((ops.mlstm_chunks_scratch_floats(5, max(new), H, D, DV),), float("nan"), device="cuda")
+            ops.mlstm_chunks(*args, max(new), scratch)
+        else:
+            ops.mlstm_scan(*args)
+        assert bool(o[-1].isnan().all()) and torch.equal(state_dev[:, floats:].cpu(), state[:, floats:])
+        error = lambda x, y: float((x.double().cpu() - y).norm() / y.norm())
+        results.append((error(o[:-1], want), error(state_dev[:, :floats], want_state[:, :floats])))
+    assert all(c <= 1.5 * r + 2.0 ** -24 and r < 1e-4 for r, c in zip(*results)), results
+
+
 @pytest.mark.parametrize("dtype,tol", [("float32", 3e-6), ("bfloat16", 1e-2)])
 def test_latent_norm_between_two_products(gpu, dtype, tol):
     from stride_b200.csrc import ops
