@@ -36,6 +36,13 @@ namespace stride {
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Asks L2 for the lines of [first, first + bytes): for weights, which no kernel writes, ahead of pdl_wait(). Thread `who` of `of`.
+__device__ __forceinline__ void prefetch_l2(const void* first, size_t bytes, int who, int of) {
+    const uintptr_t base = reinterpret_cast<uintptr_t>(first), begin = base & ~uintptr_t(127);
+    for (uintptr_t line = begin + static_cast<size_t>(who) * 128; line < base + bytes; line += static_cast<size_t>(of) * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
+}
+
 inline bool pdl_enabled() {
     static const bool on = [] {
         const char* e = getenv("STRIDE_B200_PDL");

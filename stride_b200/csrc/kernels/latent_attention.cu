@@ -165,6 +165,14 @@ head_gemm_tc_kernel(const __nv_bfloat16* __restrict__ A, int lda, int a_hs, cons
                     int b_ns, __nv_bfloat16* __restrict__ C, int ldc, int c_hs, const __nv_bfloat16* __restrict__ gate, int ldg, int g_hs,
                     int g_ns, int M, int N, int K) {
     pdl_trigger();
+    if (blockIdx.z == 0) {      // the CTA's part of the weights, a row of 64 or of K numbers a thread
+        const __nv_bfloat16* b = B + static_cast<size_t>(blockIdx.y) * b_hs + static_cast<size_t>(blockIdx.x) * TN * b_ns;
+        const int cols = min(TN, N - static_cast<int>(blockIdx.x) * TN);
+        if (b_ns == 1)
+            for (int k = threadIdx.x; k < K; k += 128) prefetch_l2(b + static_cast<size_t>(k) * b_ks, cols * 2, 0, 1);
+        else if (b_ks == 1)
+            for (int n = threadIdx.x; n < cols; n += 128) prefetch_l2(b + static_cast<size_t>(n) * b_ns, static_cast<size_t>(K) * 2, 0, 1);
+    }
     pdl_wait();
     __shared__ TileSmem sm;
     const int a = blockIdx.y;

@@ -367,6 +367,12 @@ moe_route_rule_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* 
     __shared__ float z[kRouteMaxRows];
     __shared__ float choice[kMaxExperts], gscore[kMaxExperts];
     pdl_trigger();
+    // every CTA reads all of w: each asks for its share while the kernel before this one ends (8 tokens x 33 rows of 2,048: 9.4 us
+    // among the kernels of a step, 13.5 without)
+    {
+        const size_t bytes = static_cast<size_t>(rows) * hidden * 2, share = (bytes / gridDim.x + 127) / 128 * 128, at = blockIdx.x * share;
+        if (at < bytes) prefetch_l2(reinterpret_cast<const unsigned char*>(w) + at, bytes - at < share ? bytes - at : share, threadIdx.x, kRouteThreads);
+    }
     pdl_wait();
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool padded = seq_of_token && seq_of_token[t] < 0;

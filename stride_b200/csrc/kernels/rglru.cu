@@ -126,6 +126,14 @@ rglru_gates_kernel(const float* __restrict__ u, const T* __restrict__ wa_t, cons
                    const float* __restrict__ bi, const float* __restrict__ lam, float decay, float* __restrict__ a_out,
                    float* __restrict__ gx_out, int tokens, int width, int bw) {
     pdl_trigger();
+    if (blockIdx.z == 0) {      // the CTA's columns of both matrices, a row a thread
+        const size_t at = static_cast<size_t>(blockIdx.y) * bw * bw + blockIdx.x * GC;
+        const int cols = min(GC, bw - static_cast<int>(blockIdx.x) * GC);
+        for (int k = threadIdx.x; k < bw; k += GC * GS) {
+            prefetch_l2(wa_t + at + static_cast<size_t>(k) * bw, cols * sizeof(T), 0, 1);
+            prefetch_l2(wi_t + at + static_cast<size_t>(k) * bw, cols * sizeof(T), 0, 1);
+        }
+    }
     pdl_wait();
     extern __shared__ float us[];                   // [GT][bw], then the slices' sums [GS][2][GT][GC]
     float* part = us + GT * bw;
@@ -146,7 +154,7 @@ rglru_gates_kernel(const float* __restrict__ u, const T* __restrict__ wa_t, cons
     if (oc < bw) {
         const T* wa = wa_t + static_cast<size_t>(b) * bw * bw + oc;
         const T* wi = wi_t + static_cast<size_t>(b) * bw * bw + oc;
-#pragma unroll 4
+#pragma unroll 16       // 32 loads in flight: 3 tokens of 10 blocks of 256 in 11.7 us, 19.6 with 8
         for (int k = k_lo; k < k_hi; ++k) {
             const float wr = to_f32(wa[static_cast<size_t>(k) * bw]), wg = to_f32(wi[static_cast<size_t>(k) * bw]);
 #pragma unroll
