@@ -30,7 +30,9 @@ namespace stream_gemm {
 
 constexpr int kStepCols = 32;    // columns of K per warp step (a quad's four 16-byte pieces)
 constexpr int kUnroll = 2;       // steps per batch (one cp.async group)
-constexpr int kMaxTiles = 4;     // 16-row tiles per CTA at most
+// 16-row tiles per CTA at most: five hold an 148th of 11,840 rows (with four a gate/up matrix of 11,008 rows went in 172 CTAs, two
+// rounds: 14.7 us a product of 2,048 columns against 10.3). With 9 to 16 tokens four: the ring and the partial sums of five do not fit.
+constexpr int max_row_tiles(int nt) { return nt == 1 ? 5 : 4; }
 
 __device__ __forceinline__ void cp_async_16_or_zero(void* smem, const void* gmem, bool valid) {
     const int bytes = valid ? 16 : 0;        // 0 source bytes: the 16 destination bytes are filled with zeros
@@ -177,6 +179,10 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     // ---- TMA: stage i of this warp holds columns (i * WARPS + warp) * 64 .. + 63
     const int k_stages = (k + 63) / 64;
     const int my_stages = k_stages > warp ? (k_stages - warp + WARPS - 1) / WARPS : 0;
+    // Stages asked for at a time. A warp whose share of K fits the ring has all of it on the way at once (K = 2048: 5.8 against 6.4 us
+    // for a 2048 x 2048 matrix among the kernels of a step; K = 4096: a step of the 8B layers 1 % faster); a longer one leaves a stage
+    // free (K = 8256: 9.3 us, with all four 11.3).
+    const int ahead = my_stages <= 2 * STAGES ? STAGES : STAGES - 1;
     unsigned char* my_ring = ring_bytes + warp * STAGES * STAGE_BYTES;
     bool alive = true;                                      // false once a bounded wait has run out
     auto request_stage = [&](int i, bool weights, bool tokens) {
@@ -206,7 +212,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (int i = 0; i < STAGES - 1; ++i) request_stage(i, true, false);
         pdl_wait();       // x is written by the kernel before this one
 #pragma unroll
-        for (int i = 0; i < STAGES - 1; ++i) request_stage(i, false, true);
+        for (int i = 0; i < STAGES; ++i)
+            if (i < ahead) request_stage(i, i == STAGES - 1, true);
     } else {
     #pragma unroll
         for (int b = 0; b < STAGES - 1; ++b) request_weights(b);
@@ -286,7 +293,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 }
             }
             __syncwarp();                                   // every lane is done with the stage before it is refilled
-            request_stage(i + STAGES - 1, true, true);
+            request_stage(i + ahead, true, true);           // into the stage just read, or the one before
         }
     } else {
         for (int b = 0; b < my_batches; ++b) {
@@ -470,14 +477,14 @@ inline bool stream_tma_enabled() {
 }
 
 // Rows (MODE 2: rotation pairs) per CTA and the number of CTAs: one CTA per SM with equal shares when a CTA's
-// kMaxTiles tiles can hold such a share, else full CTAs of kMaxTiles tiles; a short K (small models) gets one tile
+// max_tiles tiles can hold such a share, else full CTAs of max_tiles tiles; a short K (small models) gets one tile
 // per CTA and fewer warps. With TMA copies a MODE 2 CTA stays inside one head: `ctas_per_head` CTAs of `per_cta`
 // pairs each (the last one of a head may hold fewer).
 struct Shape {
     int per_cta, ctas, tiles, warps, ctas_per_head;
     bool tma;
 };
-inline Shape shape_for(int n, int k, int mode, int hd, bool tma_possible) {
+inline Shape shape_for(int n, int k, int mode, int hd, bool tma_possible, int max_tiles) {
     const int batches = ((k + kStepCols - 1) / kStepCols + kUnroll - 1) / kUnroll;
     const int units = mode == 2 ? n / 2 : n, per_tile = mode == 2 ? 8 : 16;
     Shape s{};
@@ -491,14 +498,14 @@ inline Shape shape_for(int n, int k, int mode, int hd, bool tma_possible) {
     }
     s.warps = 8;
     s.per_cta = (units + sm_count() - 1) / sm_count();
-    if (s.per_cta > kMaxTiles * per_tile) s.per_cta = kMaxTiles * per_tile;
+    if (s.per_cta > max_tiles * per_tile) s.per_cta = max_tiles * per_tile;
     s.tma = tma_possible && stream_tma_enabled();
     if (s.tma && mode == 2) {
         const int half = hd / 2;
         int per_head = (half + s.per_cta / 2) / s.per_cta;          // rounded: CTAs a head is cut into
         if (per_head < 1) per_head = 1;
         const int pairs = (half + per_head - 1) / per_head;
-        if (pairs > kMaxTiles * per_tile) {
+        if (pairs > max_tiles * per_tile) {
             s.tma = false;
         } else {
             s.ctas_per_head = per_head;
@@ -516,13 +523,13 @@ inline Shape shape_for(int n, int k, int mode, int hd, bool tma_possible) {
 template <int NT, int MODE>
 int launch_stream(const __nv_bfloat16* x, const __nv_bfloat16* w, void* out, int m, int n, int k, cudaStream_t stream, int* status,
                   const QkvEpilogue& qkv = QkvEpilogue{}, const RowNorm& norm = RowNorm{}) {
-    Shape s = shape_for(n, k, MODE, qkv.hd, status != nullptr);
+    Shape s = shape_for(n, k, MODE, qkv.hd, status != nullptr, max_row_tiles(NT));
     const CUtensorMap* map_w = nullptr;
     const CUtensorMap* map_x = nullptr;
     if (s.tma) {
         map_w = tc::cached_map(w, n, k, k, s.per_cta);
         map_x = tc::cached_map(x, m, k, k, NT * 8);
-        if (map_w == nullptr || map_x == nullptr) s = shape_for(n, k, MODE, qkv.hd, false);
+        if (map_w == nullptr || map_x == nullptr) s = shape_for(n, k, MODE, qkv.hd, false, max_row_tiles(NT));
     }
 #define STRIDE_STREAM_LAUNCH(MT_, WARPS_, TMA_)                                                                                 \
     launch_warps<NT, MT_, WARPS_, MODE, TMA_>(map_w, map_x, x, w, out, m, n, k, s.per_cta, s.ctas_per_head, s.ctas, qkv, norm, status, \
@@ -534,14 +541,16 @@ int launch_stream(const __nv_bfloat16* x, const __nv_bfloat16* w, void* out, int
             case 1: return STRIDE_STREAM_LAUNCH(1, 8, true);
             case 2: return STRIDE_STREAM_LAUNCH(2, 8, true);
             case 3: return STRIDE_STREAM_LAUNCH(3, 8, true);
-            default: return STRIDE_STREAM_LAUNCH(4, 8, true);
+            case 4: return STRIDE_STREAM_LAUNCH(4, 8, true);
+            default: return STRIDE_STREAM_LAUNCH(max_row_tiles(NT), 8, true);
         }
     }
     switch (s.tiles) {
         case 1: return STRIDE_STREAM_LAUNCH(1, 8, false);
         case 2: return STRIDE_STREAM_LAUNCH(2, 8, false);
         case 3: return STRIDE_STREAM_LAUNCH(3, 8, false);
-        default: return STRIDE_STREAM_LAUNCH(4, 8, false);
+        case 4: return STRIDE_STREAM_LAUNCH(4, 8, false);
+        default: return STRIDE_STREAM_LAUNCH(max_row_tiles(NT), 8, false);
     }
 #undef STRIDE_STREAM_LAUNCH
 }
@@ -622,7 +631,7 @@ extern "C" int stride_gemm_stream_add_norm(const void* x, const void* w, void* x
     if (tokens < 0 || n_out <= 0 || k <= 0 || residual == nullptr || norm_weight == nullptr || partials == nullptr || ctas_out == nullptr)
         return STRIDE_BAD_ARGUMENT;
     if (tokens > 16 || k % 8 || (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) % 16) return STRIDE_UNSUPPORTED;
-    const stream_gemm::Shape shape = stream_gemm::shape_for(n_out, k, 3, 0, status != nullptr);
+    const stream_gemm::Shape shape = stream_gemm::shape_for(n_out, k, 3, 0, status != nullptr, stream_gemm::max_row_tiles(tokens <= 8 ? 1 : 2));
     if (partials_capacity < static_cast<long long>(shape.ctas) * 16) return STRIDE_BAD_ARGUMENT;
     *ctas_out = shape.ctas;
     if (tokens == 0) return 0;

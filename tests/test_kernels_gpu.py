@@ -1047,3 +1047,28 @@ def test_gemm_f32_gives_the_same_bits_in_every_kernel(ops, n, k):
         out = torch.full((m + 1, n), 7.0, device="cuda")
         ops.linear(dev(a[:m]), dev(w), out[:m])
         assert torch.equal(out[:m], full[:m]) and bool((out[m] == 7.0).all()), m
+
+
+@pytest.mark.parametrize("n,k", [(9500, 2048), (11008, 2112), (11841, 1024), (2048, 4096), (520, 4160), (1000, 8256)])
+def test_the_weight_streaming_product_at_its_edges(ops, n, k):
+    """Five row tiles a CTA (up to 8 tokens; four above), a fifth tile with one row, rows beyond an equal share of 148, a warp's share of K
+    that just fills the ring, that is asked for a ring ahead, and longer ones; bounds as for the other products of few tokens."""
+    g = torch.Generator().manual_seed(n + k)
+    w = dev((torch.randn(n, k, generator=g) * 0.05).bfloat16())
+    for tokens in (1, 8, 9, 16):
+        x = dev((torch.randn(tokens, k, generator=g) * 0.5).bfloat16())
+        want = x.double() @ w.double().T
+        scale = float(want.abs().max())
+        for out_dtype, tol in ((torch.float32, 2e-5), (torch.bfloat16, 1e-2)):
+            out = torch.full((tokens + 1, n), 7.0, dtype=out_dtype, device="cuda")
+            assert ops.linear_stream(x, w, out[:tokens]), "the kernel refused the shape"
+            ops.check_kernel_status()
+            assert float((out[:tokens].double() - want).abs().max()) <= tol * scale and bool((out[tokens] == 7.0).all())
+        residual, weight = torch.randn(tokens, n, generator=g).cuda(), torch.rand(n, generator=g).cuda()
+        before, xt = residual.double(), torch.empty(tokens, n, dtype=torch.bfloat16, device="cuda")
+        partials = torch.full((16 * (n // 16 + 149),), float("nan"), device="cuda")
+        count = ops.linear_add_norm(x, w, residual, weight, xt, partials)
+        assert count > 0
+        assert float((residual.double() - (before + want)).abs().max()) <= 1e-2 * scale
+        squares = partials.view(-1, 16)[:count, :tokens].double().sum(0)
+        assert torch.allclose(squares, residual.double().square().sum(1), rtol=1e-5)
