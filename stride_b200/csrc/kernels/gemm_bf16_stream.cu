@@ -34,6 +34,39 @@ constexpr int kUnroll = 2;       // steps per batch (one cp.async group)
 // rounds: 14.7 us a product of 2,048 columns against 10.3). With 9 to 16 tokens four: the ring and the partial sums of five do not fit.
 constexpr int max_row_tiles(int nt) { return nt == 1 ? 5 : 4; }
 
+// Stages of two pieces of K, for up to kPairTiles row tiles. (2048 x 2048: 4.4 us among the kernels of a step, 5.5 piece by piece;
+// steps of the 2048-wide designs 3 to 9 % faster, the most at K = 8256. With two row tiles the ring is too coarse: the 8B layers lose 1.5 % a step.)
+constexpr int kPairStages = 2;
+constexpr int kPairTiles = 1;
+
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z, int u) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(u)
+        : "memory");
+}
+
+// The first k / 512 * 512 columns of a [rows, k] bfloat16 matrix (k 512 at least) as [turn][8 warps][rows][64 columns], in boxes of two
+// turns of one warp by box_rows rows with the 128-byte swizzle. Rows and turns past the end read as zero.
+inline const CUtensorMap* cached_turns(const void* base, long long rows, long long k, int box_rows) {
+    static std::unordered_map<tc::MapKey, CUtensorMap, tc::MapKeyHash> cache;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    const tc::MapKey key{base, rows, k, k, box_rows};
+    const auto it = cache.find(key);
+    if (it != cache.end()) return &it->second;
+    tc::EncodeFn fn = tc::encode_fn();
+    if (!fn) return nullptr;
+    const cuuint64_t dims[4] = {64, static_cast<cuuint64_t>(rows), 8, static_cast<cuuint64_t>(k / 512)};
+    const cuuint64_t strides[3] = {static_cast<cuuint64_t>(k) * 2, 128, 1024};
+    const cuuint32_t box[4] = {64, static_cast<cuuint32_t>(box_rows), 1, 2}, elem[4] = {1, 1, 1, 1};
+    CUtensorMap m;
+    if (fn(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return nullptr;
+    return &cache.emplace(key, m).first->second;
+}
+
 __device__ __forceinline__ void cp_async_16_or_zero(void* smem, const void* gmem, bool valid) {
     const int bytes = valid ? 16 : 0;        // 0 source bytes: the 16 destination bytes are filled with zeros
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_addr(smem)), "l"(gmem), "r"(bytes));
@@ -90,15 +123,21 @@ struct RowNorm {
 // stage's mbarrier and read their fragments with ldmatrix. Many warps issuing small boxes stream faster than
 // cp.async does on this GPU (see attention_decode.cu). MODE 2 then keeps a CTA's pairs inside one head (two boxes per
 // stage: the pairs' first halves and their second halves), `per_cta` pairs at `ctas_per_head` CTAs a head.
-template <int NT, int MT, int WARPS, int MODE, bool TMA>
+// CH: pieces of 64 columns a stage (TMA). A copy costs an SM some 100 cycles to start whatever its size, and a stage of one piece of
+// 14 rows is 1.8 KB of weights and 1 KB of tokens: the copies of a 2048 x 8256 product alone took 13 us to start. Viewed as
+// [turn of the warps][warp][row][64 columns] the pieces of a warp's two next turns are one box, [turn][row] packed tight in shared
+// memory (the swizzle follows the address): the sums keep their order. Columns past the last whole turn come piece by piece.
+template <int NT, int MT, int WARPS, int MODE, bool TMA, int CH>
 __global__ void __launch_bounds__(WARPS * 32)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                   const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x2,
                    const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, void* __restrict__ out, int m, int n,
                    int k, int per_cta, int ctas_per_head, const QkvEpilogue qkv, const RowNorm norm, int* __restrict__ status) {
-    constexpr int STAGES = ring_stages(NT, MT, WARPS);
+    constexpr int STAGES = CH == 1 ? ring_stages(NT, MT, WARPS) : kPairStages;
     constexpr int THREADS = WARPS * 32;
     constexpr int PIECES = 2 * MT + NT;      // per step: rows g and g + 8 of every tile, then one piece of x per token tile
-    constexpr int W_BYTES = MT * 2048, X_BYTES = NT * 1024, STAGE_BYTES = W_BYTES + X_BYTES;      // TMA: a stage of one warp
+    static_assert(CH == 1 || (TMA && WARPS == 8), "the view of two turns is of eight warps");
+    constexpr int W_BYTES = CH * MT * 2048, X_BYTES = CH * NT * 1024, STAGE_BYTES = W_BYTES + X_BYTES;      // TMA: a stage of one warp
     extern __shared__ __align__(1024) unsigned char ring_raw[];
     unsigned char* ring_bytes = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ring_raw) + 1023) & ~uintptr_t(1023));
     uint4* ring = reinterpret_cast<uint4*>(ring_bytes);  // cp.async: [STAGES][kUnroll][PIECES][THREADS]
@@ -176,9 +215,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[mt][nt][i] = 0.f;
 
-    // ---- TMA: stage i of this warp holds columns (i * WARPS + warp) * 64 .. + 63
-    const int k_stages = (k + 63) / 64;
-    const int my_stages = k_stages > warp ? (k_stages - warp + WARPS - 1) / WARPS : 0;
+    // ---- TMA: turn j of this warp is columns (j * WARPS + warp) * 64 .. + 63; a stage holds CH turns, or the one past the whole turns
+    const int k_pieces = (k + 63) / 64;
+    const int my_turns = k_pieces > warp ? (k_pieces - warp + WARPS - 1) / WARPS : 0;
+    const int whole = CH == 1 ? my_turns : k / (64 * WARPS), whole_stages = (whole + CH - 1) / CH;
+    const int my_stages = whole_stages + (my_turns > whole ? 1 : 0);
     // Stages asked for at a time. A warp whose share of K fits the ring has all of it on the way at once (K = 2048: 5.8 against 6.4 us
     // for a 2048 x 2048 matrix among the kernels of a step; K = 4096: a step of the 8B layers 1 % faster); a longer one leaves a stage
     // free (K = 8256: 9.3 us, with all four 11.3).
@@ -187,21 +228,27 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     bool alive = true;                                      // false once a bounded wait has run out
     auto request_stage = [&](int i, bool weights, bool tokens) {
         if (lane != 0 || i >= my_stages || !alive) return;
-        const int st = i % STAGES, col = (i * WARPS + warp) * 64;
+        const int st = i % STAGES;
+        const bool single = CH == 1 || i >= whole_stages;
+        const int turns = single ? 1 : CH, col = ((CH == 1 ? i : whole) * WARPS + warp) * 64;
+        auto load = [&](uint32_t to, const CUtensorMap& one, const CUtensorMap& two, uint32_t on, int row) {
+            if (single) tc::tma_load_2d(to, &one, on, col, row);
+            else tma_load_4d(to, &two, on, 0, row, warp, i * CH);
+        };
         const uint32_t bar = tc::smem_u32(&stage_bar[warp][st]), dst = tc::smem_u32(my_ring + st * STAGE_BYTES);
         if (weights) {
             // one arrival per stage use: the bytes of every box of the stage are announced with the first copies
             if (MODE == 2) {
-                tc::mbar_expect_tx(bar, 2 * per_cta * 128 + NT * 8 * 128);
+                tc::mbar_expect_tx(bar, turns * (2 * per_cta * 128 + NT * 8 * 128));
                 const int head = first / half, i0 = first - head * half;
-                tc::tma_load_2d(dst, &map_w, bar, col, head * qkv.hd + i0);
-                tc::tma_load_2d(dst + MT * 1024, &map_w, bar, col, head * qkv.hd + half + i0);
+                load(dst, map_w, map_w2, bar, head * qkv.hd + i0);
+                load(dst + CH * MT * 1024, map_w, map_w2, bar, head * qkv.hd + half + i0);
             } else {
-                tc::mbar_expect_tx(bar, per_cta * 128 + NT * 8 * 128);
-                tc::tma_load_2d(dst, &map_w, bar, col, first);
+                tc::mbar_expect_tx(bar, turns * (per_cta * 128 + NT * 8 * 128));
+                load(dst, map_w, map_w2, bar, first);
             }
         }
-        if (tokens) tc::tma_load_2d(dst + W_BYTES, &map_x, bar, col, 0);
+        if (tokens) load(dst + W_BYTES, map_x, map_x2, bar, 0);
     };
     if (TMA) {
         if (lane == 0)
@@ -261,9 +308,12 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (alive) alive = tc::mbar_wait(tc::smem_u32(&stage_bar[warp][st]), static_cast<uint32_t>(i / STAGES) & 1u, status, 41);
             __syncwarp();
             if (alive) {
-                const uint32_t ws = smem_addr(my_ring + st * STAGE_BYTES), xs = ws + W_BYTES;
+                const uint32_t ws = smem_addr(my_ring + st * STAGE_BYTES);
 #pragma unroll
-                for (int kp = 0; kp < 2; ++kp) {            // two 16-column steps per ldmatrix of x
+                for (int kc = 0; kc < 2 * CH; ++kc) {       // two 16-column steps per ldmatrix of x
+                    const int c = kc >> 1, kp = kc & 1;     // piece of the stage, half of the piece
+                    if (CH > 1 && c >= CH - 1 && i >= whole_stages) break;
+                    const uint32_t xs = ws + W_BYTES + c * NT * 1024;
                     uint32_t bx[NT][4];
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt) {       // tokens nt*8 + lr, chunks 4 kp + lm: b0, b1 of step 2 kp, then of 2 kp + 1
@@ -279,10 +329,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                             uint32_t base = ws;
                             if (MODE == 2) {                // rows 0-7: the pairs' first halves (first box), rows 8-15: their second halves
                                 row = mt * 8 + lr;
-                                base += (lm & 1) * (MT * 1024);
+                                base += (lm & 1) * (CH * MT * 1024);
                             } else {
                                 row = mt * 16 + (lm & 1) * 8 + lr;
                             }
+                            row += c * per_cta;
                             const int chunk = 2 * kk + (lm >> 1);
                             uint32_t a[4];
                             ldmatrix_x4(a, base + row * 128 + ((chunk ^ (row & 7)) << 4));
@@ -439,13 +490,13 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
 }
 
-template <int NT, int MT, int WARPS, int MODE, bool TMA>
-int launch_warps(const CUtensorMap* map_w, const CUtensorMap* map_x, const __nv_bfloat16* x, const __nv_bfloat16* w, void* out, int m,
+template <int NT, int MT, int WARPS, int MODE, bool TMA, int CH = 1>
+int launch_warps(const CUtensorMap* map_w, const CUtensorMap* map_x, const CUtensorMap* map_w2, const CUtensorMap* map_x2, const __nv_bfloat16* x, const __nv_bfloat16* w, void* out, int m,
                  int n, int k, int per_cta, int ctas_per_head, int ctas, const QkvEpilogue& qkv, const RowNorm& norm, int* status,
                  cudaStream_t stream) {
-    constexpr int smem = (TMA ? ring_stages(NT, MT, WARPS) * WARPS * (MT * 2048 + NT * 1024)
+    constexpr int smem = (TMA ? (CH == 1 ? ring_stages(NT, MT, WARPS) : kPairStages) * WARPS * CH * (MT * 2048 + NT * 1024)
                               : ring_stages(NT, MT, WARPS) * kUnroll * (2 * MT + NT) * WARPS * 32 * 16) + 1024;
-    auto kernel = gemm_stream_kernel<NT, MT, WARPS, MODE, TMA>;
+    auto kernel = gemm_stream_kernel<NT, MT, WARPS, MODE, TMA, CH>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -454,6 +505,7 @@ int launch_warps(const CUtensorMap* map_w, const CUtensorMap* map_x, const __nv_
     }
     static const CUtensorMap no_map = {};
     stride::launch(kernel, dim3(static_cast<unsigned>(ctas)), dim3(WARPS * 32), smem, stream, TMA ? *map_w : no_map, TMA ? *map_x : no_map,
+                   CH > 1 ? *map_w2 : no_map, CH > 1 ? *map_x2 : no_map,
                    x, w, out, m, n, k, per_cta, ctas_per_head, qkv, norm, status);
     return STRIDE_LAUNCH_STATUS();
 }
@@ -526,16 +578,27 @@ int launch_stream(const __nv_bfloat16* x, const __nv_bfloat16* w, void* out, int
     Shape s = shape_for(n, k, MODE, qkv.hd, status != nullptr, max_row_tiles(NT));
     const CUtensorMap* map_w = nullptr;
     const CUtensorMap* map_x = nullptr;
+    const CUtensorMap* map_w2 = nullptr;
+    const CUtensorMap* map_x2 = nullptr;
+    bool pairs = false;
     if (s.tma) {
         map_w = tc::cached_map(w, n, k, k, s.per_cta);
         map_x = tc::cached_map(x, m, k, k, NT * 8);
+        if (s.tiles <= kPairTiles && k >= 512) {
+            map_w2 = cached_turns(w, n, k, s.per_cta);
+            map_x2 = cached_turns(x, m, k, NT * 8);
+            pairs = map_w2 != nullptr && map_x2 != nullptr;
+        }
         if (map_w == nullptr || map_x == nullptr) s = shape_for(n, k, MODE, qkv.hd, false, max_row_tiles(NT));
     }
 #define STRIDE_STREAM_LAUNCH(MT_, WARPS_, TMA_)                                                                                 \
-    launch_warps<NT, MT_, WARPS_, MODE, TMA_>(map_w, map_x, x, w, out, m, n, k, s.per_cta, s.ctas_per_head, s.ctas, qkv, norm, status, \
+    launch_warps<NT, MT_, WARPS_, MODE, TMA_>(map_w, map_x, nullptr, nullptr, x, w, out, m, n, k, s.per_cta, s.ctas_per_head, s.ctas, qkv, norm, status, \
                                               stream)
     if (s.warps == 4) return STRIDE_STREAM_LAUNCH(1, 4, false);
     if (s.warps == 2) return STRIDE_STREAM_LAUNCH(1, 2, false);
+    if (s.tma && pairs) {
+        return launch_warps<NT, 1, 8, MODE, true, 2>(map_w, map_x, map_w2, map_x2, x, w, out, m, n, k, s.per_cta, s.ctas_per_head, s.ctas, qkv, norm, status, stream);
+    }
     if (s.tma) {
         switch (s.tiles) {
             case 1: return STRIDE_STREAM_LAUNCH(1, 8, true);
