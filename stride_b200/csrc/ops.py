@@ -42,7 +42,7 @@ _SIGNATURES = {
     "stride_gemm_nt_f32": ("gemm_f32", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "stride_paged_attention_generic": ("attention_generic", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
-                                                             c_int, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
+                                                             c_int, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "stride_gemm_tc_skinny": ("gemm_bf16_tc", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_longlong,
                                                c_void_p, c_int, c_void_p, c_void_p]),
     "stride_gemm_tc_clustered": ("gemm_bf16_tc", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
@@ -1801,12 +1801,13 @@ def _rel_args(rel, nq: int) -> tuple:
 
 def paged_attention(q, q_stride: int, out, k_pages, v_pages, block_table, seq_of_token, positions, nq: int, nkv: int,
                     hd: int, page_size: int, scale: float, window: int = 0, softcap: float = 0.0, sinks=None, slopes=None,
-                    vd: int | None = None, rel=None) -> None:
+                    vd: int | None = None, rel=None, portions: bool = False) -> None:
     """Attention of every token in the flat batch over its request's pages.
     ``q`` holds head h of token t at ``q[t * q_stride + h * hd]``. ``softcap`` c > 0 caps the scaled scores at
     c tanh(s / c); ``sinks`` (float32 [nq]) adds exp(sink) of the head to the softmax's denominator; ``slopes`` (float32
     [nq]) takes slope_h times the key's distance off every score; ``vd`` is the values' width where it is not ``hd``;
-    ``rel`` (float32 [nq, n]) adds ``rel[h, min(distance, n - 1)]`` to every score of head h."""
+    ``rel`` (float32 [nq, n]) adds ``rel[h, min(distance, n - 1)]`` to every score of head h. ``portions``: neighbouring
+    tokens mostly belong to one request (only the time depends on it)."""
     tokens = out.shape[0]
     vd = hd if vd is None else int(vd)
     if out.shape[1] != nq * vd or k_pages.shape[-1] != hd or v_pages.shape[-1] != vd:
@@ -1815,8 +1816,8 @@ def paged_attention(q, q_stride: int, out, k_pages, v_pages, block_table, seq_of
         _dev(q, "q"), q_stride, _dev(out, "out"), _dev(k_pages, "k_pages"), _dev(v_pages, "v_pages"),
         _dev(block_table, "block_table", torch.int32), block_table.shape[1], _dev(seq_of_token, "seq_of_token", torch.int32),
         _dev(positions, "positions", torch.int32), tokens, nq, nkv, hd, vd, page_size, float(scale), int(window), float(softcap),
-        _opt(sinks, "sinks", torch.float32), _opt(slopes, "slopes", torch.float32), *_rel_args(rel, nq), _code(q.dtype), _stream()),
-        "paged_attention")
+        _opt(sinks, "sinks", torch.float32), _opt(slopes, "slopes", torch.float32), *_rel_args(rel, nq), 1 if portions else 0,
+        _code(q.dtype), _stream()), "paged_attention")
 
 
 def fast_attention_supported(dtype, nq: int, nkv: int, hd: int) -> bool:

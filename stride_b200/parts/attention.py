@@ -481,7 +481,8 @@ class PagedAttention(Mixer):
         if not self._fast:
             # the exact kernel: the whole 32-bit path, and bfloat16 sizes the tensor-core kernels refuse
             ops.paged_attention(qkv, self.qkv_dim, attn, cache.k_pages, cache.v_pages, table, ctx.seq_of_token[:tokens],
-                                ctx.positions[:tokens], *geometry, self.softcap, self.sinks, self.slopes, self.vd, self.rel)
+                                ctx.positions[:tokens], *geometry, self.softcap, self.sinks, self.slopes, self.vd, self.rel,
+                                portions=ctx.max_q_len >= 8)
             return tokens
         split = min(ctx.decode_tail_start, tokens)          # portions before, single decoded tokens after
         if split > 0:

@@ -1072,3 +1072,32 @@ def test_the_weight_streaming_product_at_its_edges(ops, n, k):
         assert float((residual.double() - (before + want)).abs().max()) <= 1e-2 * scale
         squares = partials.view(-1, 16)[:count, :tokens].double().sum(0)
         assert torch.allclose(squares, residual.double().square().sum(1), rtol=1e-5)
+
+
+@pytest.mark.parametrize("nq,nkv,hd,window,rules", [(4, 2, 32, 0, False), (6, 1, 128, 40, True), (3, 3, 4, 0, True), (5, 1, 100, 33, False)])
+def test_attention_f32_in_tiles_gives_the_bits_of_single_rows(ops, nq, nkv, hd, window, rules):
+    """Eight rows a CTA against a row a CTA: runs that start and end inside a tile, single tokens, a padded row, a group of heads that
+    needs two CTAs, windows whose older pages are gone from the table, caps, sinks and slopes; and both against the formula."""
+    g = torch.Generator().manual_seed(nq * hd)
+    page = 8
+    q, k_pages, v_pages, table, seq_of, pos, want = _paged_case(g, torch.float32, [(0, 100), (40, 9), (131, 1), (7, 1), (0, 33), (64, 2)], nq, nkv, hd,
+                                                                page, window or None)
+    if window:          # pages that no query of the step sees any more
+        for s in range(table.shape[0]):
+            first = int(pos[seq_of == s].min()) - window + 1
+            for p in range(max(0, first // page)):
+                table[s, p] = -1
+    tokens = q.shape[0]
+    seq_of = torch.cat([seq_of, torch.tensor([-1], dtype=torch.int32)])
+    pos = torch.cat([pos, torch.tensor([0], dtype=torch.int32)])
+    q = torch.cat([q, q[:1]])
+    extra = dict(softcap=20.0, sinks=dev(torch.randn(nq, generator=g)), slopes=dev(torch.rand(nq, generator=g) * 0.1)) if rules else {}
+    outs = []
+    for portions in (False, True):
+        out = torch.full((tokens + 1, nq * hd), float("nan"), device="cuda")
+        ops.paged_attention(dev(q), nq * hd, out, dev(k_pages), dev(v_pages), dev(table), dev(seq_of), dev(pos), nq, nkv, hd, page, hd ** -0.5, window,
+                            portions=portions, **extra)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and float(outs[0][tokens].abs().max()) == 0.0
+    if not rules:
+        close(outs[0][:tokens], want.reshape(tokens, -1), torch.float32)
