@@ -9,7 +9,7 @@
 // in tensor memory and frees each stage with tcgen05.commit; four warps read the accumulator back with tcgen05.ld, a
 // row a thread, apply the activation and store. Rows of the tile past the expert's last row and features past its
 // last feature are computed from whatever lies there (the next expert's rows, zeros past the end) and not stored.
-// Two CTAs fit one SM, so one tile's epilogue runs under the other's products.
+// BLOCK_N 256 (two stages) or 128 (three): two CTAs fit one SM, so one tile's epilogue runs under the other's products.
 //
 // act 0: none; 1: the square of the positive part; 2: the rows of W come as (gate, up) pairs, row 2i beside row
 // 2i + 1, and the tile leaves g' sigmoid(alpha g') (u' + 1), g' = min(g, limit), u' = clamp(u, -limit, limit), N / 2 wide;
@@ -97,19 +97,18 @@ grouped_gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     const uint32_t tmem_base = tmem_base_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
-            const int w_row = e * N + n0;
-            for (int i = 0; i < num_kb; ++i) {
-                const int s = i % STAGES;
-                if (i >= STAGES && !mbar_wait(smem_u32(&empty_bar[s]), ((i / STAGES) & 1) ^ 1, status, 11)) break;
-                const uint32_t bar = smem_u32(&full_bar[s]);
-                mbar_expect_tx(bar, STAGE_BYTES);
-                const uint32_t a_dst = smem_u32(smem + s * STAGE_BYTES);
-                tma_load_2d(a_dst, &map_a, bar, i * kGroupK, m0);
-                tma_load_2d(a_dst + A_BYTES, &map_w, bar, i * kGroupK, w_row);
-            }
+        // one thread needs some 300 cycles a copy, two lanes of a warp together no more than one: lane 0 brings the rows, lane 1 the weights
+        const CUtensorMap* map = lane == 0 ? &map_a : &map_w;
+        const int row = lane == 0 ? m0 : e * N + n0;
+        for (int i = 0; i < num_kb; ++i) {
+            const int s = i % STAGES;
+            if (i >= STAGES && !mbar_wait(smem_u32(&empty_bar[s]), ((i / STAGES) & 1) ^ 1, status, 11)) break;
+            const uint32_t bar = smem_u32(&full_bar[s]);
+            if (lane == 0) mbar_expect_tx(bar, STAGE_BYTES);
+            __syncwarp();
+            if (lane < 2) tma_load_2d(smem_u32(smem + s * STAGE_BYTES) + lane * A_BYTES, map, bar, i * kGroupK, row);
+            __syncwarp();
         }
-        __syncwarp();
     } else if (warp == 1) {
         if (lane == 0) {
             constexpr uint32_t idesc = instr_desc_bf16(kGroupM, BLOCK_N, false);
@@ -207,10 +206,9 @@ gather_rows_kernel(const uint4* __restrict__ x, int ldx16, const int32_t* __rest
     }
 }
 
-template <typename OutT>
+template <int BLOCK_N, int STAGES, typename OutT>
 int launch_grouped(const CUtensorMap* map_a, const CUtensorMap* map_w, const int32_t* offsets, int experts, OutT* C, int ldc, int max_rows,
                    int N, int K, int act, float limit, float alpha, const float* row_weight, int vec_ok, int* status, cudaStream_t stream) {
-    constexpr int BLOCK_N = 128, STAGES = 3;
     constexpr int smem = STAGES * (kGroupM * kGroupK * 2 + BLOCK_N * kGroupK * 2) + 1024;
     static bool configured[64] = {};
     int device = 0;
@@ -248,16 +246,21 @@ int stride_grouped_gemm_tc5(const void* A, int lda, const void* W, const int32_t
     if (K % 8 || lda % 8 || (reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) % 16) return STRIDE_UNSUPPORTED;
     if (static_cast<long long>(experts) * N > 2147483647LL) return STRIDE_UNSUPPORTED;
     const CUtensorMap* map_a = tc::cached_map(A, max_rows, K, lda, tc::kGroupM);
-    const CUtensorMap* map_w = tc::cached_map(W, static_cast<long long>(experts) * N, K, K, 128);
+    // Tiles of 256 features read the rows half as often, which counts where K is short and the result float32. With fewer such
+    // tiles than SMs the narrow ones spread better. (8,192 rows over 32 experts, 768 x 2,048 / 2,048 x 768 float32: 48 and 49 us,
+    // 47 and 58 with tiles of 128 and one thread for both copies; one CTA an SM with four stages 51 and 54.)
+    const bool wide = N % 256 == 0 && static_cast<long long>((max_rows + tc::kGroupM - 1) / tc::kGroupM) * (N / 256) >= 148;
+    const CUtensorMap* map_w = tc::cached_map(W, static_cast<long long>(experts) * N, K, K, wide ? 256 : 128);
     if (!map_a || !map_w) return STRIDE_UNSUPPORTED;
     // rows of four outputs are stored whole when every row of C starts on a 16-byte boundary
     const int elem = out_is_f32 ? 4 : 2;
     const int vec_ok = (reinterpret_cast<uintptr_t>(C) % 16 == 0 && (static_cast<long long>(ldc) * elem) % 16 == 0) ? 1 : 0;
-    if (out_is_f32)
-        return tc::launch_grouped<float>(map_a, map_w, offsets, experts, static_cast<float*>(C), ldc, max_rows, N, K, act, limit, alpha,
-                                         row_weight, vec_ok, status, stream);
-    return tc::launch_grouped<__nv_bfloat16>(map_a, map_w, offsets, experts, static_cast<__nv_bfloat16*>(C), ldc, max_rows, N, K, act, limit,
-                                             alpha, row_weight, vec_ok, status, stream);
+#define STRIDE_GROUPED(BLOCK_N_, STAGES_, OUT_)                                                                                       \
+    tc::launch_grouped<BLOCK_N_, STAGES_>(map_a, map_w, offsets, experts, static_cast<OUT_*>(C), ldc, max_rows, N, K, act, limit, alpha, \
+                                          row_weight, vec_ok, status, stream)
+    if (wide) return out_is_f32 ? STRIDE_GROUPED(256, 2, float) : STRIDE_GROUPED(256, 2, __nv_bfloat16);
+    return out_is_f32 ? STRIDE_GROUPED(128, 3, float) : STRIDE_GROUPED(128, 3, __nv_bfloat16);
+#undef STRIDE_GROUPED
 }
 
 // xs[p] = x[perm[p]] for the rows p that the plan filled; rows of `row_bytes` (a multiple of 16), x with row stride ldx_bytes.

@@ -251,6 +251,12 @@ def test_expert_products_on_the_tcgen05_tiles(gpu, n, k, act, out_dtype):
     assert torch.equal(out[rows:].cpu().double(), want[rows:]), "rows past the last expert's were written"
 
 
+@pytest.mark.parametrize("n,k,act,out_dtype", [(6400, 72, 2, torch.bfloat16), (6400, 1032, 0, torch.float32), (6656, 64, 1, torch.bfloat16)])
+def test_expert_products_on_the_wide_tcgen05_tiles(gpu, n, k, act, out_dtype):
+    """The same where tiles of 256 features are enough to fill the device: one block of K, a few, and many turns of its ring."""
+    test_expert_products_on_the_tcgen05_tiles(gpu, n, k, act, out_dtype)
+
+
 def test_rows_laid_out_expert_by_expert(gpu):
     from stride_b200.csrc import ops
     g = torch.Generator().manual_seed(3)
