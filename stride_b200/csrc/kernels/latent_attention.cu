@@ -3,7 +3,8 @@
 // plain part folded through W_uk (q~_a = W_uk_a^T q_a [rank]) the score of a key is
 //   s = (q~_a . c + q_rot_a . k_r) * scale
 // and the head's output W_uv_a (sum_j p_j c_j): every head reads the same [rank + rot] numbers per key and nothing
-// but c and k_r is ever kept or expanded. Three kernels:
+// but c and k_r is kept. (Portions of prompts may expand keys and values for the length of a pass instead:
+// latent_gather here, attention_prefill_tc.cu.) Kernels:
 //
 //   latent_prepare    norms the latent (float32 statistics, plain weight), rotates the shared key part and the
 //                     rotated part of every query head (pairs (2i, 2i+1), angle from a float32 table), writes the
