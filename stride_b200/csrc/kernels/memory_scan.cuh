@@ -390,6 +390,14 @@ int launch_scan_as(const ScanArgs& p, int num_seqs, cudaStream_t stream) {
                              dim3((p.DV + cta_cols - 1) / cta_cols, p.H, num_seqs), dim3(kScanThreads), 0, stream, p);
     } else if (p.DV >= 4 * COLS) {
         const dim3 grid((p.DV + 4 * COLS - 1) / (4 * COLS), p.H, num_seqs);
+        // The delta rule's token costs a thread two rounds of shuffles: with two columns a thread the chain is shorter, as long as the
+        // twice as many CTAs still run side by side, three an SM (16 heads of 128 x 128, four / two columns: 2,048 tokens of one request
+        // 881 / 788 us, 1,750 of three 417 / 385, 1,500 of six, 768 CTAs, 222 / 290; single tokens of three 8.6 / 7.1).
+        const long long narrow = (p.DV + 2 * COLS - 1) / (2 * COLS);
+        if (RULE == kDeltaRule && !p.mode && narrow * p.H * num_seqs <= 3 * 148) {
+            stride::launch_alone(scan_kernel<LANES, R, 2, CHUNK, RULE, false>, dim3(static_cast<unsigned>(narrow), p.H, num_seqs), dim3(kScanThreads), 0, stream, p);
+            return STRIDE_LAUNCH_STATUS();
+        }
         if (p.mode) stride::launch_alone(scan_kernel<LANES, R, 4, CHUNK, RULE, true>, grid, dim3(kScanThreads), 0, stream, p);
         else stride::launch_alone(scan_kernel<LANES, R, 4, CHUNK, RULE, false>, grid, dim3(kScanThreads), 0, stream, p);
     } else {

@@ -33,6 +33,7 @@ import torch
 
 from ..csrc import ops
 from .base import Mixer, Projection, StateRequest, TensorDecl, register_part
+from .runtime import sequence_slots
 
 
 def _pad8(n: int) -> int:
@@ -117,7 +118,7 @@ class GatedDeltaMixer(Mixer):
         v = self.rt.buffer("delta_v", tokens, self.HV, f32)
         beta = self.rt.buffer("delta_beta", tokens, self.H, f32)
         decay = self.rt.buffer("delta_decay", tokens, self.HD, f32)
-        seqs = ctx.q_len.shape[0]
+        seqs = sequence_slots(ctx)
         ops.delta_prepare(proj, self.conv_w, two, self.a_log, self.dt_bias, state, self.s_floats, ctx.seq_of_token[:tokens], ctx.q_start,
                           ctx.state_slot, qk, v, beta, decay, self.G, self.H, self.D, self.DV, self.taps, self.unit_eps)
         o = self.rt.buffer("delta_o", tokens, self.HV, f32)
@@ -207,7 +208,7 @@ class BonusMemoryMixer(Mixer):
         wlog = self.rt.buffer("wkv_wlog", tokens, self.HD, f32)
         ops.linear(low, self.w_2, wlog)
         o = self.rt.buffer("wkv_o", tokens, self.HD, f32)
-        seqs, scratch = ctx.q_len.shape[0], None
+        seqs, scratch = sequence_slots(ctx), None
         if x.dtype == torch.bfloat16 and ctx.max_q_len >= ops.SCAN_PIECES_MIN_TOKENS:
             # a long portion: the recurrence in pieces, parallel over the pieces (the 32-bit path keeps the one chain, whose
             # sums do not depend on the cutting)

@@ -411,3 +411,34 @@ def test_greedy_generation_through_the_engine(gpu, tmp_models):
                     check_invariants=True)
     outs = engine.generate(copy.deepcopy(prompts), SamplingParams(temperature=0.0, max_tokens=new, ignore_eos=True))
     assert [o.tokens for o in outs] == expected
+
+
+@pytest.mark.parametrize("D,DV,n", [(128, 128, 21), (128, 72, 9), (100, 130, 3)])
+def test_delta_rule_scan_has_the_same_bits_with_two_and_four_columns_a_thread(gpu, D, DV, n):
+    """Few requests take the form with two columns a thread, a launch with room for many the one with four; and both against the
+    recurrence in float64 (a token adds a rounding or so to a sum of D terms of size one)."""
+    from stride_b200.csrc import ops
+    g = torch.Generator().manual_seed(D + DV)
+    H, slots = 2, 64
+    unit = lambda t: t / t.norm(dim=-1, keepdim=True)
+    qk = torch.cat([unit(torch.randn(n, H, D, generator=g)).reshape(n, -1) for _ in range(2)], 1)
+    v, beta = torch.randn(n, H * DV, generator=g), torch.rand(n, H, generator=g)
+    decay = -torch.rand(n, H * D, generator=g) * 0.2
+    state = torch.randn(1, H * D * DV, generator=g)
+    proj = torch.zeros(n, 8)
+    dev = lambda t: torch.as_tensor(t, dtype=torch.int32).cuda()
+    lens, zeros = dev([n] + [0] * (slots - 1)), dev([0] * slots)
+    outs = []
+    for seqs in (1, slots):
+        o, s = torch.full((n, H * DV), float("nan"), device="cuda"), state.cuda()
+        ops.delta_scan(qk.cuda(), v.cuda(), beta.cuda(), decay.cuda(), o, s, H * D * DV, proj.cuda(), zeros, lens, zeros, seqs, H, H, D, DV, 1)
+        outs.append((o, s))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    for h in range(H):
+        S = state[0, h * D * DV:(h + 1) * D * DV].double().view(D, DV)
+        for t in range(n):
+            q, k = qk[t, h * D:(h + 1) * D].double(), qk[t, (H + h) * D:(H + h + 1) * D].double()
+            S = (1.0 + decay[t, h * D:(h + 1) * D].double())[:, None] * S
+            S = S + torch.outer(k, beta[t, h].double() * (v[t, h * DV:(h + 1) * DV].double() - S.T @ k))
+            want = S.T @ q
+            assert float((outs[0][0][t, h * DV:(h + 1) * DV].cpu().double() - want).abs().max()) <= (n + 40) * 2.0 ** -22
