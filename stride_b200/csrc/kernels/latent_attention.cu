@@ -203,6 +203,112 @@ head_gemm_tc_kernel(const __nv_bfloat16* __restrict__ A, int lda, int a_hs, cons
         }
 }
 
+// The same for portions: 128 tokens x 128 columns a CTA, eight warps of 64 x 32, 64 columns of K at a time by cp.async, twice buffered;
+// weights whose output index is the contiguous one stay as they lie and are read with transposing fragment loads (the kernel above takes them
+// number by number). The terms come in the same order, so the bits are the same. 2,048 tokens of 16 heads, 128 x 512 and
+// 512 x 128: at most 31 us each, 243 with the tiles of 64 x 64.
+constexpr int WM = 128, WN = 128, WLD = TK + 8, WLDT = WN + 8;
+constexpr int kWideStage = WM * WLD + (WN * WLD > TK * WLDT ? WN * WLD : TK * WLDT);       // elements
+template <bool N_CONTIGUOUS>
+__global__ void __launch_bounds__(256, 2)
+head_gemm_wide_kernel(const __nv_bfloat16* __restrict__ A, int lda, int a_hs, const __nv_bfloat16* __restrict__ B, long long b_hs, int b_ld,
+                      __nv_bfloat16* __restrict__ C, int ldc, int c_hs, const __nv_bfloat16* __restrict__ gate, int ldg, int g_hs, int g_ns, int M,
+                      int N, int K) {
+    extern __shared__ __align__(16) unsigned char wide_smem[];
+    __nv_bfloat16* const sm = reinterpret_cast<__nv_bfloat16*>(wide_smem);
+    pdl_trigger();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int a = blockIdx.y, m0 = blockIdx.z * WM, n0 = blockIdx.x * WN, wm = (warp >> 2) * 64, wn = (warp & 3) * 32;
+    const __nv_bfloat16* const Ah = A + static_cast<size_t>(a) * a_hs;
+    const __nv_bfloat16* const Bh = B + static_cast<size_t>(a) * b_hs;
+    auto copy = [&](__nv_bfloat16* dst, const __nv_bfloat16* src, bool live) {      // 16 bytes, zeros past the end
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src), "r"(live ? 16 : 0)
+                     : "memory");
+    };
+    auto load = [&](int k0, int buf) {
+        __nv_bfloat16* const as = sm + buf * kWideStage;
+        __nv_bfloat16* const bs = as + WM * WLD;
+        for (int i = tid; i < WM * TCH; i += 256) {
+            const int r = i / TCH, k = (i % TCH) * 8;
+            const bool live = m0 + r < M && k0 + k < K;
+            copy(as + r * WLD + k, live ? Ah + static_cast<size_t>(m0 + r) * lda + k0 + k : A, live);
+        }
+        if (N_CONTIGUOUS) {
+            for (int i = tid; i < TK * (WN / 8); i += 256) {
+                const int k = i / (WN / 8), n = (i % (WN / 8)) * 8;
+                const bool live = n0 + n < N && k0 + k < K;
+                copy(bs + k * WLDT + n, live ? Bh + static_cast<size_t>(k0 + k) * b_ld + n0 + n : B, live);
+            }
+        } else {
+            for (int i = tid; i < WN * TCH; i += 256) {
+                const int n = i / TCH, k = (i % TCH) * 8;
+                const bool live = n0 + n < N && k0 + k < K;
+                copy(bs + n * WLD + k, live ? Bh + static_cast<size_t>(n0 + n) * b_ld + k0 + k : B, live);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[4][4][4] = {};
+    pdl_wait();
+    load(0, 0);
+    int buf = 0;
+    for (int k0 = 0; k0 < K; k0 += TK, buf ^= 1) {
+        if (k0 + TK < K) {
+            load(k0 + TK, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const __nv_bfloat16* const as = sm + buf * kWideStage;
+        const __nv_bfloat16* const bs = as + WM * WLD;
+#pragma unroll
+        for (int kk = 0; kk < TK; kk += 16) {
+            uint32_t af[4][4], bf[4][2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ldmatrix_x4(af[i], as + (wm + i * 16 + (lane & 15)) * WLD + kk + (lane >> 4) * 8);
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {
+                uint32_t r[4];
+                if (N_CONTIGUOUS) {
+                    const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(bs + (kk + (lane & 15)) * WLDT + wn + j * 8 + (lane >> 4) * 8));
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+                } else {
+                    ldmatrix_x4(r, bs + (wn + j * 8 + (lane & 7) + ((lane >> 4) << 3)) * WLD + kk + ((lane >> 3) & 1) * 8);
+                }
+                bf[j][0] = r[0]; bf[j][1] = r[1]; bf[j + 1][0] = r[2]; bf[j + 1][1] = r[3];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) mma_bf16_16816(acc[i][j], af[i], bf[j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int m = m0 + wm + i * 16 + g + 8 * h;
+            if (m >= M) continue;
+            float f = 1.f;
+            if (gate && !g_ns) f = 1.f / (1.f + expf(-to_f32(gate[static_cast<size_t>(m) * ldg + static_cast<size_t>(a) * g_hs])));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int n = n0 + wn + j * 8 + 2 * t;          // N is even: both columns or none
+                if (n >= N) continue;
+                float v[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    if (gate && g_ns) f = 1.f / (1.f + expf(-to_f32(gate[static_cast<size_t>(m) * ldg + static_cast<size_t>(a) * g_hs + static_cast<size_t>(n + e) * g_ns])));
+                    v[e] = acc[i][j][2 * h + e] * f;
+                }
+                *reinterpret_cast<__nv_bfloat162*>(C + static_cast<size_t>(m) * ldc + static_cast<size_t>(a) * c_hs + n) = __floats2bfloat162_rn(v[0], v[1]);
+            }
+        }
+}
+
 // ------------------------------------------------------------------------------------------- exact attention
 constexpr int kLatWarps = 4;
 constexpr int kMaxRank = 512;          // latent width the exact kernel keeps in registers (rank / 32 per lane)
@@ -354,6 +460,20 @@ int stride_head_gemm(const void* A, int lda, int a_hs, const void* B, long long 
                        static_cast<const float*>(B), b_hs, b_ks, b_ns, static_cast<float*>(C), ldc, c_hs, static_cast<const float*>(gate),
                        ldg, g_hs, g_ns, M, N, K);
     else if (dtype == STRIDE_DTYPE_BF16) {
+        const long long b_ld = b_ns == 1 ? b_ks : b_ns;
+        const bool wide = M >= 128 && (b_ns == 1 || b_ks == 1) && K % 8 == 0 && N % 8 == 0 && lda % 8 == 0 && a_hs % 8 == 0 && b_hs % 8 == 0 && b_ld % 8 == 0 &&
+                          ldc % 2 == 0 && c_hs % 2 == 0 && (reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) % 16 == 0 &&
+                          reinterpret_cast<uintptr_t>(C) % 4 == 0;
+        if (wide) {
+            constexpr int bytes = 2 * kWideStage * 2;
+            const auto kernel = b_ks == 1 ? head_gemm_wide_kernel<false> : head_gemm_wide_kernel<true>;
+            const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            if (e != cudaSuccess) return static_cast<int>(e);
+            stride::launch(kernel, dim3((N + WN - 1) / WN, heads, (M + WM - 1) / WM), dim3(256), bytes, stream, static_cast<const __nv_bfloat16*>(A), lda, a_hs,
+                           static_cast<const __nv_bfloat16*>(B), b_hs, static_cast<int>(b_ld), static_cast<__nv_bfloat16*>(C), ldc, c_hs,
+                           static_cast<const __nv_bfloat16*>(gate), ldg, g_hs, g_ns, M, N, K);
+            return STRIDE_LAUNCH_STATUS();
+        }
         const dim3 tc_grid((N + TN - 1) / TN, heads, (M + TM - 1) / TM);
         stride::launch(head_gemm_tc_kernel, tc_grid, dim3(128), 0, stream, static_cast<const __nv_bfloat16*>(A), lda, a_hs,
                        static_cast<const __nv_bfloat16*>(B), b_hs, b_ks, b_ns, static_cast<__nv_bfloat16*>(C), ldc, c_hs,

@@ -436,3 +436,29 @@ def test_greedy_generation_through_the_engine(gpu, tmp_models):
                     check_invariants=True)
     outs = engine.generate(copy.deepcopy(prompts), SamplingParams(temperature=0.0, max_tokens=new, ignore_eos=True))
     assert [o.tokens for o in outs] == expected
+
+
+@pytest.mark.parametrize("n,k,n_contiguous,gate", [(128, 64, True, None), (136, 72, True, "head"), (40, 200, False, "output"), (256, 512, False, "head")])
+def test_per_head_products_of_portions_have_the_bits_of_short_ones(gpu, n, k, n_contiguous, gate):
+    """128 tokens and more (broken tiles of tokens, columns and K) against the same rows in launches of 64, bit for bit, and against float64."""
+    from stride_b200.csrc import ops
+    heads, tokens = 3, 201
+    g = torch.Generator().manual_seed(n + k)
+    a = torch.randn(tokens, heads * (k + 8), generator=g).bfloat16().cuda()
+    b = torch.randn(heads, *((k, n) if n_contiguous else (n, k)), generator=g).bfloat16().cuda()
+    gates = torch.randn(tokens, 8 + heads * n, generator=g).bfloat16().cuda()
+    strides = (n, 1) if n_contiguous else (1, k)
+    extra = {} if gate is None else dict(ldg=gates.shape[1], gate_off=8, gate_per_output=gate == "output")
+    def run(lo, hi):
+        c = torch.full((hi - lo + 1, heads * n), 7.0, dtype=torch.bfloat16, device="cuda")
+        ops.head_gemm(a[lo:hi], a.shape[1], k + 8, b, n * k, *strides, c, heads * n, n, hi - lo, heads, n, k,
+                      gate=None if gate is None else gates[lo:hi], **extra)
+        assert bool((c[hi - lo] == 7.0).all())
+        return c[:hi - lo]
+    whole = run(0, tokens)
+    assert torch.equal(whole, torch.cat([run(lo, min(tokens, lo + 64)) for lo in range(0, tokens, 64)]))
+    want = torch.einsum("thk,hkn->thn", a.double().view(tokens, heads, -1)[..., :k], b.double() if n_contiguous else b.double().transpose(1, 2))
+    if gate is not None:
+        f = torch.sigmoid(gates[:, 8:].double())
+        want = want * (f[:, :heads, None] if gate == "head" else f.view(tokens, heads, n))
+    close(whole, want.reshape(tokens, -1), 1e-2)
