@@ -45,7 +45,7 @@ class StepContext:
     # for a step that runs once, every slot of its batch bucket for a captured graph. 0: not given (every slot of the arrays).
     seq_slots: int = 0
     # Keys that the requests in front of the decode tail hold together after this step, or an upper bound of it for as long as
-    # this context's launches may be replayed. 0: not given.
+    # this context's launches may be replayed. 0: not given (a part must then not size a launch by it).
     portion_keys: int = 0
     # Host copy of the step's items for parts that loop in Python:
     # (request, first flat row, number of tokens, position of the first token, state slot)

@@ -123,7 +123,9 @@ class ModelRunner:
         return logits, timer.milliseconds()
 
     # ------------------------------------------------------------------- eager
-    def _context(self, staging, batch, num_tokens, num_rows, for_graph: int = 0, portion_bound: int = 0):
+    def _context(self, staging, batch, num_tokens, num_rows, for_graph: int = 0, portion_bound: int | None = None):
+        """``for_graph``: the context bucket of a captured decode step. ``portion_bound``: of a captured portion, 0 where the model asks
+        for none; None: the step runs once, and what it holds now is what its launches may be sized by."""
         items, row = [], 0
         for request, tokens, position, _want in batch.items():
             items.append((request, row, len(tokens), position, self.cache.state_slot(request)))
@@ -133,7 +135,8 @@ class ModelRunner:
             tail_seq -= 1
         tail_start = items[tail_seq][1] if tail_seq < len(items) else row
         bound = for_graph or portion_bound or batch.max_ctx     # a captured graph is sized for its context bucket
-        portion_keys = portion_bound or sum(position + n for _request, _row, n, position, _slot in items[:tail_seq])
+        held = [position + n for _request, _row, n, position, _slot in items[:tail_seq]]
+        portion_keys = sum(held) if portion_bound is None else portion_bound
         return make_context(staging.dev, staging.layout, num_tokens, batch.num_seqs, num_rows, max_q_len=batch.max_q_len,
                             max_ctx=batch.max_ctx, decode_only=batch.decode_only, host_items=items,
                             decode_tail_start=0 if for_graph else tail_start, decode_tail_seq=0 if for_graph else tail_seq,

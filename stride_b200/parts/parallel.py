@@ -40,6 +40,7 @@ class ParallelMixer(Mixer):
             self.state_floats = at
         self.hidden = int(spec.hidden)
         self.graph_safe = all(getattr(m, "graph_safe", True) for m, _ in self.branches)
+        self.sizes_by_context = any(getattr(m, "sizes_by_context", False) for m, _ in self.branches)
 
     def declare(self):
         d = {}

@@ -1,0 +1,145 @@
+"""Latent attention whose portions go over expanded keys and values, as a model and the engine drive it: full portions replayed from
+captured graphs at positions far past the captured one, and a latent layer inside a parallel mixer. Against the plain float64 implementation (``plain_nidilix``)."""
+
+import dataclasses
+
+import pytest
+import torch
+
+import nidilix_cases as cases
+import plain_nidilix as plain
+from helpers import compare_logits, seeded_tokens, write_model_dir
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+
+
+def two_layers(rank):
+    """The head sizes of the tcgen05 kernel; the second layer borrows the first one's latents."""
+    heads = cases.attention(3, 128, 64, 64, 128, rank)
+    return cases.config(96, 131, [(heads, None), (cases.attention(3, 128, 64, 64, 128, rank, kv_from=0), None)], mult=0.5)
+
+
+class Case:
+    def __init__(self, tmp_models, rank, seed=41):
+        self.cfg = two_layers(rank)
+        state = cases.seeded_state(self.cfg, seed)
+        self.folder = write_model_dir(str(tmp_models / f"latent_expanded_{rank}"), self.cfg, state, torch.bfloat16)
+        self.state = {k: v.bfloat16() for k, v in state.items()}
+        self.want = {}
+
+    def logits(self, tokens):
+        key = tuple(tokens)
+        if key not in self.want:
+            self.want[key] = plain.forward(self.cfg, self.state, list(tokens))
+        return self.want[key]
+
+
+@pytest.fixture(scope="module")
+def models(tmp_models):
+    return {rank: Case(tmp_models, rank) for rank in (48,)}
+
+
+@pytest.fixture
+def expansions(monkeypatch):
+    """The expanded kernel's calls, the rows of each; every portion is worth expanding."""
+    from stride_b200.csrc import ops
+    from stride_b200.parts.latent_attention import LatentAttention
+    monkeypatch.setattr(LatentAttention, "EXPAND_PAIRS", 1)
+    calls, run = [], ops.latent_prefill_tc
+    monkeypatch.setattr(ops, "latent_prefill_tc", lambda *a, **k: (calls.append(a[7].shape[0]), run(*a, **k))[1])
+    return calls
+
+
+def engine_for(case, **options):
+    from stride_b200 import Engine
+    options = {"block_size": 16, "num_blocks": 80, "max_batch_tokens": 256, "max_batch_seqs": 6, "max_model_len": 400, **options}
+    return Engine(case.folder, dtype="bfloat16", **options)
+
+
+def check(got, case, tokens, rows, label):
+    ok, msg = compare_logits(got.cpu(), case.logits(tokens)[rows], "bfloat16")
+    assert ok, f"{label}: {msg}"
+
+
+def open_request(engine, key, n):
+    engine.cache.open(key, "u")
+    assert engine.cache.ensure(key, n, 0)
+
+
+def full_portions(engine, case, key, tokens, size):
+    """A prompt in portions that fill the token budget; logits of the last row of each."""
+    open_request(engine, key, len(tokens))
+    for at in range(0, len(tokens), size):
+        want = [size - 1] if at + size >= len(tokens) or at % (2 * size) else []
+        got = engine.forward([(key, tokens[at:at + size], at, want)])
+        if want:
+            check(got, case, tokens, [at + size - 1], f"request {key}, portion at {at}")
+    engine.cache.close(key)
+
+
+@pytest.mark.parametrize("bucketed", [True, False])
+def test_full_portions_replayed_from_graphs(gpu, models, expansions, monkeypatch, bucketed):
+    """Four portions of 64 tokens, with a context bucket that ends behind each of them; then another prompt over the same graphs.
+    A model that gives no bound for its captured portions (a layer without ``parts``, say) stays on the latents: a graph captured at
+    the first portion must not go on to expand that portion's keys alone."""
+    from stride_b200.engine.runner import ModelRunner
+    from stride_b200.parts.model import DecoderModel
+    monkeypatch.setattr(ModelRunner, "CONTEXT_BUCKET_BASE", 64)
+    if not bucketed:
+        monkeypatch.setattr(DecoderModel, "sizes_by_context", False)
+    case = models[48]
+    engine = engine_for(case, max_batch_tokens=64)
+    for key in (1, 2):
+        full_portions(engine, case, key, seeded_tokens(256, case.cfg["vocab"], 900 + key), 64)
+    bounds = {k[2:] for k in engine.runner._graphs if k[0] == "portion"}
+    assert (len(bounds) >= 3 and len(expansions) > 0) if bucketed else (bounds == {()} and not expansions)
+    assert engine.runner.graph_replays == 8
+
+
+def register_parallel():
+    from stride_b200.config import MixerSpec, register_architecture
+    from stride_b200.config.nidilix import NidilixConfig
+
+    class InParallel:
+        """The Nidilix design with every mixer as the one branch of a parallel mixer."""
+
+        def __init__(self, d):
+            self.d = dict(d)
+
+        @classmethod
+        def from_dict(cls, d):
+            return cls(d)
+
+        def to_dict(self):
+            return dict(self.d)
+
+        def to_model_spec(self):
+            spec = NidilixConfig.from_dict(dict(self.d, architecture="Nidilix")).to_model_spec()
+            layers = tuple(dataclasses.replace(l, mixer=MixerSpec("parallel", hidden=spec.hidden, prefix=l.mixer.prefix,
+                                                                  params=(("branches", ((l.mixer, 1.0),)),))) for l in spec.layers)
+            return dataclasses.replace(spec, layers=layers)
+
+    register_architecture("ToyLatentInParallel", InParallel)
+
+
+def test_a_latent_branch_of_a_parallel_mixer_in_full_portions(gpu, models, expansions, monkeypatch, tmp_models):
+    from stride_b200.engine.runner import ModelRunner
+    register_parallel()
+    monkeypatch.setattr(ModelRunner, "CONTEXT_BUCKET_BASE", 64)
+    cfg = dict(two_layers(48), architecture="ToyLatentInParallel")
+    cfg["layers"] = cfg["layers"][:1]
+    case = Case.__new__(Case)
+    case.cfg, case.want = dict(cfg, architecture="Nidilix"), {}
+    state = cases.seeded_state(case.cfg, 43)
+    case.folder = write_model_dir(str(tmp_models / "latent_in_parallel"), cfg, state, torch.bfloat16)
+    case.state = {k: v.bfloat16() for k, v in state.items()}
+    engine = engine_for(case, max_batch_tokens=64)
+    assert engine.model.sizes_by_context
+    full_portions(engine, case, 1, seeded_tokens(256, cfg["vocab"], 911), 64)
+    assert expansions and engine.runner.graph_replays == 4
