@@ -134,7 +134,8 @@ class ModelRunner:
         while tail_seq > 0 and items[tail_seq - 1][2] == 1:
             tail_seq -= 1
         tail_start = items[tail_seq][1] if tail_seq < len(items) else row
-        bound = for_graph or portion_bound or batch.max_ctx     # a captured graph is sized for its context bucket
+        # a captured graph is sized for its context bucket, or for what the block table holds
+        bound = batch.max_ctx if not for_graph and portion_bound is None else for_graph or portion_bound or self.table_width * self.cache.page_size
         held = [position + n for _request, _row, n, position, _slot in items[:tail_seq]]
         portion_keys = sum(held) if portion_bound is None else portion_bound
         return make_context(staging.dev, staging.layout, num_tokens, batch.num_seqs, num_rows, max_q_len=batch.max_q_len,

@@ -248,6 +248,16 @@ def test_a_long_prompt_alone_is_prefilled_in_full_portions_from_a_graph(case, dt
     assert engine.runner.graph_replays > replays
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_a_token_budget_of_one(case, dtype):
+    """Every token of a prompt is a full portion of its own: the graph captured at position 0 must hold for all that follow."""
+    from stride_b200 import SamplingParams
+    prompt = seeded_tokens(150, case["cfg"]["vocab_size"], 779)
+    engine = engine_for(case, dtype, max_batch_tokens=1, max_batch_seqs=1)
+    out = engine.generate([prompt], SamplingParams(temperature=0.0, max_tokens=4))[0]
+    assert_greedy(case, dtype, prompt, out.tokens, "a token at a time")
+
+
 def test_add_request_refuses_more_than_max_queued_waiting_requests(case):
     from stride_b200 import EngineBusy, SamplingParams
     engine = engine_for(case, "float32", max_queued=2)
