@@ -24,7 +24,7 @@
 //                 costs time. A constant decay never divides: decay^(i - j) is taken from a table of powers.
 //
 // The chunks also run the matrix LSTM of mlstm.cu (mlstm_chunks): its gates are one number a head and token, with a running
-// maximum; n goes along as one more column. 1,999 tokens of 16 heads of 128 x 128: 127 us, 622 us token after token.
+// maximum; n goes along as one more column. 2,000 tokens of 16 heads of 128 x 128: 131 us, 634 us token after token.
 #include "memory_scan.cuh"
 
 namespace stride {
@@ -35,6 +35,11 @@ constexpr int kSumCols = 64;            // the same in the kernel of the chunks'
 constexpr int kChunkThreads = 256;
 constexpr int kLd = kChunk + 4;         // row stride of the transposed tiles: 16-byte reads, stores without bank conflicts
 constexpr float kSafeLog = -60.f;
+// The matrix LSTM's sums over channels and over a chunk's tokens go in runs of this many terms, which are then added up: as one chain
+// of 128 terms they were further from 64 bits than the token-by-token kernel, whose sums are spread over lanes (16 heads of 128 x 128,
+// gates as a projection makes them: median error of a row 1.2 of that kernel's as one chain, 0.9 in runs; 2,000 tokens 122 us and
+// 131 us).
+constexpr int kRun = 16;
 
 // The gates of a chunk's tokens of one head of the matrix LSTM (lstm_gates_kernel): with b the running sum of the forget gates'
 // logarithms inside the chunk, li the input gates' logarithms, m the running maximum (m_0 at the chunk's start, m_e at its end), token
@@ -410,7 +415,7 @@ __host__ __device__ constexpr int chunk_out_floats() { return DP * kLd + chunk_s
 template <int DP, int RULE>
 __global__ void __launch_bounds__(kChunkThreads, DP <= 128 ? 2 : 1)
 chunk_out_kernel(const ChunkArgs p) {
-    constexpr int SLAB = 64 < DP ? 64 : DP;         // rows of S staged at a time
+    constexpr int SLAB = RULE == kLstm ? 32 : 64 < DP ? 64 : DP;        // rows of S staged at a time (the runs' sums take registers)
     constexpr int SLAB_PACKS = SLAB * kChunkCols / 4 / kChunkThreads;
     extern __shared__ __align__(16) float smem[];
     float* qT = smem;                               // [DP][kLd]: column i is token i's query (times g_i)
@@ -535,6 +540,7 @@ chunk_out_kernel(const ChunkArgs p) {
         for (int e = 0; e < 4; ++e) a[e][0] = a[e][1] = a[e][2] = a[e][3] = 0.f;
         if (RULE != kChannelDecay || safe) {
             if (tx <= ty) {
+                float run[4][4] = {};
 #pragma unroll 8
                 for (int d = 0; d < DP; ++d) {
                     const float4 q4 = *reinterpret_cast<const float4*>(qT + d * kLd + 4 * ty);
@@ -543,7 +549,19 @@ chunk_out_kernel(const ChunkArgs p) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e)
 #pragma unroll
-                        for (int f = 0; f < 4; ++f) a[e][f] = fmaf(qv[e], kv[f], a[e][f]);
+                        for (int f = 0; f < 4; ++f) {
+                            float& to = RULE == kLstm ? run[e][f] : a[e][f];
+                            to = fmaf(qv[e], kv[f], to);
+                        }
+                    if (RULE == kLstm && d % kRun == kRun - 1) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+#pragma unroll
+                            for (int f = 0; f < 4; ++f) {
+                                a[e][f] += run[e][f];
+                                run[e][f] = 0.f;
+                            }
+                    }
                 }
             }
         } else if (tx <= ty) {
@@ -614,13 +632,31 @@ chunk_out_kernel(const ChunkArgs p) {
             acc[r][3] = fmaf(a[r], b.w, acc[r][3]);
         }
     };
+    float sum[8][4] = {};                           // matrix LSTM: the sums of the runs
+    auto end_run = [&] {
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                sum[r][e] += acc[r][e];
+                acc[r][e] = 0.f;
+            }
+    };
     for (int d0 = 0; d0 < DP && d0 < D; d0 += SLAB) {
 #pragma unroll
         for (int n = 0; n < SLAB_PACKS; ++n) *reinterpret_cast<float4*>(kT + (n * kChunkThreads + threadIdx.x) * 4) = ahead[n];
         __syncthreads();
         if (d0 + SLAB < D) fetch_slab(d0 + SLAB);
+        if constexpr (RULE == kLstm) {
+            for (int d1 = 0; d1 < SLAB; d1 += kRun) {
 #pragma unroll 4
-        for (int d = 0; d < SLAB; ++d) step(qT + (d0 + d) * kLd + 8 * warp, kT + d * kChunkCols + 4 * lane);
+                for (int d = d1; d < d1 + kRun; ++d) step(qT + (d0 + d) * kLd + 8 * warp, kT + d * kChunkCols + 4 * lane);
+                end_run();
+            }
+        } else {
+#pragma unroll 4
+            for (int d = 0; d < SLAB; ++d) step(qT + (d0 + d) * kLd + 8 * warp, kT + d * kChunkCols + 4 * lane);
+        }
         __syncthreads();
     }
     if (RULE == kConstantDecay) {
@@ -636,14 +672,22 @@ chunk_out_kernel(const ChunkArgs p) {
         for (int r = 0; r < 8; ++r) {
             const float f = lstm->carry[8 * warp + r];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[r][e] *= f;
+            for (int e = 0; e < 4; ++e) sum[r][e] *= f;
         }
     }
     stage_values<kChunkCols, RULE>(p, kT, row0, nt, h, col0);
     __syncthreads();
     const int last = min(nt, 8 * warp + 8);         // later tokens have no weight in this warp's rows
+    if constexpr (RULE == kLstm) {
+        for (int j0 = 0; j0 < last; j0 += kRun) {
 #pragma unroll 4
-    for (int j = 0; j < last; ++j) step(aT + j * kLd + 8 * warp, kT + j * kChunkCols + 4 * lane);
+            for (int j = j0; j < min(last, j0 + kRun); ++j) step(aT + j * kLd + 8 * warp, kT + j * kChunkCols + 4 * lane);
+            end_run();
+        }
+    } else {
+#pragma unroll 4
+        for (int j = 0; j < last; ++j) step(aT + j * kLd + 8 * warp, kT + j * kChunkCols + 4 * lane);
+    }
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int i = 8 * warp + r;
@@ -652,7 +696,7 @@ chunk_out_kernel(const ChunkArgs p) {
             const float dot = (den_s[0][i] + den_s[1][i]) + (den_s[2][i] + den_s[3][i]);
             const float f = 1.f / (fmaxf(fabsf(dot), expf(-lstm->m[i])) + 1e-6f);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[r][e] *= f;
+            for (int e = 0; e < 4; ++e) acc[r][e] = sum[r][e] * f;
         }
         float* dst = p.o + ((row0 + i) * p.H + h) * DV + col0 + 4 * lane;
         if (s_vec) {

@@ -677,3 +677,50 @@ def test_greedy_generation_through_the_engine(gpu, tmp_models):
                     check_invariants=True)
     outs = engine.generate(copy.deepcopy(prompts), SamplingParams(temperature=0.0, max_tokens=new, ignore_eos=True))
     assert [o.tokens for o in outs] == expected
+
+
+def lstm_case(H, D, DV, lens, seed):
+    """Projections and gates as a model's products make them, the arguments of the scan for them from empty memories, and the float64
+    outputs [tokens, H, DV]."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    tokens, floats = sum(lens), H * D * DV + H * D + H
+    proj = (torch.randn(tokens, 2 * H * D + H * DV, generator=g, device="cuda") * 0.9).bfloat16()
+    gates = torch.randn(tokens, 2 * H, generator=g, device="cuda") * 0.9
+    bias, cap, want, at = torch.ones(H, device="cuda"), 15.0, [], 0
+    for n in filter(None, lens):
+        x = proj[at:at + n].double()
+        q, k, v = x[:, :H * D].view(n, H, D) * D ** -0.5, x[:, H * D:2 * H * D].view(n, H, D), x[:, 2 * H * D:].view(n, H, DV)
+        li, f = (cap * torch.tanh((z.double() + 1.0) / cap) for z in (gates[at:at + n, :H], gates[at:at + n, H:]))
+        lf = torch.nn.functional.logsigmoid(f)
+        b, m, tops = torch.cumsum(lf, 0), torch.zeros(H, dtype=torch.float64, device="cuda"), []
+        for t in range(n):
+            m = torch.maximum(lf[t] + m, li[t])
+            tops.append(m)
+        tops = torch.stack(tops)
+        w = (b[:, None] - b[None, :] + li[None, :] - tops[:, None]).masked_fill(torch.triu(torch.ones(n, n, dtype=torch.bool, device="cuda"), 1)[..., None], float("-inf")).exp()
+        s = torch.einsum("ihd,jhd->ijh", q, k) * w
+        want.append(torch.einsum("ijh,jhv->ihv", s, v) / (torch.maximum(s.sum(1).abs(), torch.exp(-tops)) + 1e-6)[..., None])
+        at += n
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+
+    def run(chunks=True):
+        from stride_b200.csrc import ops
+        state, o = torch.zeros(len(lens), floats, device="cuda"), torch.full((tokens, H * DV), float("nan"), device="cuda")
+        args = (proj, 0, H * D, 2 * H * D, gates, bias, bias, cap, D ** -0.5, o, state, dev(starts), dev(lens), dev(list(range(len(lens)))), len(lens), H, D, DV)
+        if chunks:
+            scratch = torch.full((ops.mlstm_chunks_scratch_floats(len(lens), max(lens), H, D, DV),), float("nan"), device="cuda")
+            ops.mlstm_chunks(*args, max(lens), scratch)
+        else:
+            ops.mlstm_scan(*args)
+        return o, state
+
+    return run, torch.cat(want)
+
+
+@pytest.mark.parametrize("H,D,DV,lens", [(8, 128, 128, [500]), (8, 128, 128, [96, 130]), (4, 256, 128, [200]), (6, 100, 72, [300, 64])])
+def test_matrix_lstm_chunks_are_no_further_from_float64_than_the_chain(gpu, H, D, DV, lens):
+    """The median over a step's (token, head) rows, which single rows whose divisor all but vanishes do not move (over eight seeds the
+    ratio lay within 0.75 and 0.92)."""
+    run, want = lstm_case(H, D, DV, lens, 5)
+    error = lambda o: float(((o.double().view(want.shape) - want).norm(dim=-1) / want.norm(dim=-1)).median())
+    assert error(run()[0]) <= error(run(chunks=False)[0])
