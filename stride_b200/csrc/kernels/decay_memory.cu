@@ -60,12 +60,17 @@ struct ChunkArgs {
     float* cum;             // channel decays: [tokens, H * D], the running logarithm of the decays inside the chunk
     const float* bias;      // channel decays: [H * D]
     const float* powers;    // constant decay: [H, kChunk + 1], decay^n
-    const LstmChunk* lstm;  // matrix LSTM: [seqs * max_pieces, H]
-    float* piece_n;         // matrix LSTM: [seqs * max_pieces, H, D]
+    // matrix LSTM: the chunks lie one request's behind the other's, records of them at most, so that a long portion beside many short
+    // ones costs no room for chunks that are not there
+    const LstmChunk* lstm;  // [records, H]
+    float* piece_n;         // [records, H, D]
+    const int2* where;      // [records]: a chunk's request and first token, -1 past the last chunk (null: of one request, in order)
+    const int32_t* base;    // [seqs]: a request's first chunk (null: of one request)
+    int records;
     float q_scale, inv_tau;
     float* o;               // [tokens, H * DV]
-    float* piece_s;         // [seqs * max_pieces, H, D, DV]
-    float* piece_p;         // [seqs * max_pieces, H, D]
+    float* piece_s;         // [seqs * max_pieces (matrix LSTM: records), H, D, DV]
+    float* piece_p;         // [the same, H, D]
     const int32_t* q_start;
     const int32_t* q_len;
     int H, D, DV, max_pieces;
@@ -111,18 +116,37 @@ struct LstmGates {
     long long state_stride, m_off;
     const int32_t* state_slot;
     LstmChunk* chunks;
+    int2* where;
+    int32_t* base;
+    int records;
 };
 
 // The gates' logarithms, their running sums in a chunk and the running maximum through a whole portion, m_t = max(lf_t + m_(t-1), li_t):
 // with A the sum and B the largest contribution of a run of tokens, two runs make A = A1 + A2, B = max(B1 + A2, B2), and
 // m = max(m_0 + A, B), so 256 tokens (four chunks) are one scan over a CTA. Sums and exponents in float64. Grid (heads, requests).
 static __global__ void __launch_bounds__(256)
-lstm_gates_kernel(const LstmGates p, const int32_t* __restrict__ q_start, const int32_t* __restrict__ q_len, int H, int max_pieces) {
+lstm_gates_kernel(const LstmGates p, const int32_t* __restrict__ q_start, const int32_t* __restrict__ q_len, int H) {
     __shared__ double w_sum[8], w_top[8], s_b[4], s_m[4];
+    __shared__ int w_pieces[8];
     pdl_trigger();
     pdl_wait();
     const int h = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int len = q_len[seq], start = q_start[seq];
+    const int len = q_len[seq], start = q_start[seq], pieces = len > 0 ? (len + kChunk - 1) / kChunk : 0;
+    int before_it = 0;                                  // chunks of the requests before this one
+    for (int s = tid; s < seq; s += 256) before_it += max(0, q_len[s] + kChunk - 1) / kChunk;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before_it += __shfl_xor_sync(0xffffffffu, before_it, o);
+    if (lane == 0) w_pieces[warp] = before_it;
+    __syncthreads();
+    int base = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) base += w_pieces[w];
+    if (h == 0 && gridDim.y > 1) {
+        if (tid == 0) p.base[seq] = base;
+        for (int c = tid; c < pieces && base + c < p.records; c += 256) p.where[base + c] = make_int2(seq, c * kChunk);
+        if (seq == static_cast<int>(gridDim.y) - 1)
+            for (int c = base + pieces + tid; c < p.records; c += 256) p.where[c] = make_int2(-1, 0);
+    }
     if (len <= 0) return;
     float* const m_g = p.state + static_cast<size_t>(p.state_slot[seq]) * p.state_stride + p.m_off + h;
     const float bi = p.bias_i[h], bf = p.bias_f[h];
@@ -165,8 +189,8 @@ lstm_gates_kernel(const LstmGates p, const int32_t* __restrict__ q_start, const 
         __syncthreads();
         const double m_start = c ? s_m[c - 1] : m_in, b_end = s_b[c], m_last = s_m[c];
         const int piece = t0 / kChunk + c;
-        if (piece * kChunk < len) {
-            LstmChunk& r = p.chunks[(static_cast<size_t>(seq) * max_pieces + piece) * H + h];
+        if (piece < pieces && base + piece < p.records) {
+            LstmChunk& r = p.chunks[static_cast<size_t>(base + piece) * H + h];
             const int i = tid & (kChunk - 1);
             const float hi = static_cast<float>(b);
             r.b_hi[i] = hi;
@@ -234,6 +258,21 @@ __device__ __forceinline__ void stage_values(const ChunkArgs& p, float* vs, size
     }
 }
 
+// Which request's chunk z is, and its first token there; false: none. (The matrix LSTM's table is written by the kernel before.)
+template <int RULE>
+__device__ __forceinline__ bool locate_chunk(const ChunkArgs& p, int z, int& seq, int& first) {
+    if (RULE == kLstm && p.where) {
+        pdl_wait();
+        const int2 at = p.where[z];
+        seq = at.x;
+        first = at.y;
+        return seq >= 0;
+    }
+    seq = z / p.max_pieces;
+    first = (z % p.max_pieces) * kChunk;
+    return true;
+}
+
 // piece_s[z, h] = sum_j (k_j G / g_j) v_j^T, piece_p[z, h] = G. DP: D padded. Grid (tiles of kSumCols columns, heads, chunks).
 template <int DP, int RULE>
 __global__ void __launch_bounds__(kChunkThreads)
@@ -244,10 +283,11 @@ chunk_sum_kernel(const ChunkArgs p) {
     float* vs = smem + kChunk * DP;         // [kChunk][kSumCols]
     pdl_trigger();
     const int z = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * kSumCols;
-    const int seq = z / p.max_pieces, first = (z % p.max_pieces) * kChunk;
+    int seq, first;
+    if (!locate_chunk<RULE>(p, z, seq, first)) return;
     const int nt = min(p.q_len[seq] - first, kChunk);
     if (nt <= 0) return;
-    pdl_wait();
+    if (RULE != kLstm || !p.where) pdl_wait();
     const int D = p.D, DV = p.DV, HD = p.H * D;
     const size_t row0 = static_cast<size_t>(p.q_start[seq] + first);
     const float* powers = RULE == kConstantDecay ? p.powers + h * (kChunk + 1) : nullptr;
@@ -371,7 +411,8 @@ chunk_sum_kernel(const ChunkArgs p) {
 // pieces_combine_kernel, with four neighbouring columns a thread.
 static __global__ void __launch_bounds__(256)
 chunk_combine_kernel(float4* __restrict__ piece_s, const float* __restrict__ piece_p, float* __restrict__ state, long long state_stride,
-                     const int32_t* __restrict__ q_len, const int32_t* __restrict__ state_slot, int H, int D, int DV, int max_pieces) {
+                     const int32_t* __restrict__ q_len, const int32_t* __restrict__ state_slot, int H, int D, int DV, int max_pieces,
+                     const int32_t* __restrict__ base) {
     pdl_trigger();
     const int seq = blockIdx.y;
     const int len = q_len[seq];
@@ -382,6 +423,7 @@ chunk_combine_kernel(float4* __restrict__ piece_s, const float* __restrict__ pie
     float4* S_g = reinterpret_cast<float4*>(state + static_cast<size_t>(state_slot[seq]) * state_stride) + entry;
     float4 S = *S_g;
     const int pieces = (len + kChunk - 1) / kChunk;
+    const size_t z0 = base ? static_cast<size_t>(base[seq]) : static_cast<size_t>(seq) * max_pieces;
     constexpr int AHEAD = 8;        // chunks whose loads are in flight together
     for (int c0 = 0; c0 < pieces; c0 += AHEAD) {
         float4 own[AHEAD];
@@ -389,14 +431,14 @@ chunk_combine_kernel(float4* __restrict__ piece_s, const float* __restrict__ pie
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u)
             if (c0 + u < pieces) {
-                const size_t z = static_cast<size_t>(seq) * max_pieces + c0 + u;
+                const size_t z = z0 + c0 + u;
                 own[u] = piece_s[z * entries + entry];
                 decay[u] = piece_p[z * H * D + row];
             }
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u)
             if (c0 + u < pieces) {
-                piece_s[(static_cast<size_t>(seq) * max_pieces + c0 + u) * entries + entry] = S;
+                piece_s[(z0 + c0 + u) * entries + entry] = S;
                 S.x = fmaf(decay[u], S.x, own[u].x);
                 S.y = fmaf(decay[u], S.y, own[u].y);
                 S.z = fmaf(decay[u], S.z, own[u].z);
@@ -423,10 +465,11 @@ chunk_out_kernel(const ChunkArgs p) {
     float* aT = kT + chunk_second_floats<DP>();     // [kChunk j][kLd i]: scores
     pdl_trigger();
     const int z = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * kChunkCols;
-    const int seq = z / p.max_pieces, first = (z % p.max_pieces) * kChunk;
+    int seq, first;
+    if (!locate_chunk<RULE>(p, z, seq, first)) return;
     const int nt = min(p.q_len[seq] - first, kChunk);
     if (nt <= 0) return;
-    pdl_wait();
+    if (RULE != kLstm || !p.where) pdl_wait();
     const int D = p.D, DV = p.DV, HD = p.H * D;
     const size_t row0 = static_cast<size_t>(p.q_start[seq] + first);
     const float* powers = RULE == kConstantDecay ? p.powers + h * (kChunk + 1) : nullptr;
@@ -784,7 +827,7 @@ cudaError_t more_shared_memory(void (*kernel)(A...), int bytes) {
 
 template <int DP, int RULE>
 int launch_chunks(const ChunkArgs& p, float* state, long long state_stride, const int32_t* state_slot, int num_seqs, cudaStream_t stream) {
-    const int zs = num_seqs * p.max_pieces;
+    const int zs = RULE == kLstm ? p.records : num_seqs * p.max_pieces;
     const dim3 grid((p.DV + kChunkCols - 1) / kChunkCols, p.H, zs), block(kChunkThreads);
     const dim3 sum_grid((p.DV + kSumCols - 1) / kSumCols, p.H, zs);
     constexpr int sum_bytes = (kChunk * DP + kChunk * kSumCols) * 4, out_bytes = chunk_out_floats<DP>() * 4;
@@ -796,14 +839,14 @@ int launch_chunks(const ChunkArgs& p, float* state, long long state_stride, cons
     if (p.DV % 4 == 0 && state_stride % 4 == 0 && reinterpret_cast<uintptr_t>(state) % 16 == 0)
         stride::launch(chunk_combine_kernel, dim3((p.H * p.D * p.DV / 4 + 255) / 256, num_seqs), dim3(256), 0, stream,
                        reinterpret_cast<float4*>(p.piece_s), static_cast<const float*>(p.piece_p), state, state_stride, p.q_len, state_slot, p.H,
-                       p.D, p.DV, p.max_pieces);
+                       p.D, p.DV, p.max_pieces, p.base);
     else
         stride::launch(pieces_combine_kernel, dim3((p.H * p.D * p.DV + 255) / 256, num_seqs), dim3(256), 0, stream, p.piece_s,
-                       static_cast<const float*>(p.piece_p), state, state_stride, p.q_len, state_slot, p.H, p.D, p.DV, kChunk, p.max_pieces);
+                       static_cast<const float*>(p.piece_p), state, state_stride, p.q_len, state_slot, p.H, p.D, p.DV, kChunk, p.max_pieces, p.base);
     if (RULE == kLstm)      // n is one more column of the memory
         stride::launch(pieces_combine_kernel, dim3((p.H * p.D + 255) / 256, num_seqs), dim3(256), 0, stream, p.piece_n,
                        static_cast<const float*>(p.piece_p), state + static_cast<size_t>(p.H) * p.D * p.DV, state_stride, p.q_len, state_slot, p.H,
-                       p.D, 1, kChunk, p.max_pieces);
+                       p.D, 1, kChunk, p.max_pieces, p.base);
     stride::launch(chunk_out_kernel<DP, RULE>, grid, block, out_bytes, stream, p);
     return STRIDE_LAUNCH_STATUS();
 }
@@ -918,26 +961,28 @@ int stride_decay_chunks(const void* q, const void* k, const void* v, int ld, flo
                   : dispatch_chunks<kChannelDecay>(p, state, state_stride, state_slot, num_seqs, stream);
 }
 
-// Scratch of stride_mlstm_chunks in floats.
-long long stride_mlstm_chunks_scratch(int num_seqs, int max_pieces, int H, int D, int DV) {
-    return static_cast<long long>(num_seqs) * max_pieces * H * (static_cast<long long>(D) * (DV + 2) + static_cast<long long>(sizeof(LstmChunk) / 4));
+// Scratch of stride_mlstm_chunks in floats for `records` chunks in all.
+static long long lstm_table_floats(int num_seqs, int records) { return (2LL * records + 3) / 4 * 4 + (num_seqs + 3LL) / 4 * 4; }
+long long stride_mlstm_chunks_scratch(int num_seqs, int records, int H, int D, int DV) {
+    return static_cast<long long>(records) * H * (static_cast<long long>(D) * (DV + 2) + static_cast<long long>(sizeof(LstmChunk) / 4)) +
+           lstm_table_floats(num_seqs, records);
 }
 
 // The matrix LSTM (mlstm.cu has the recurrence and the layout of the state) over long portions, chunk by chunk. Arguments as
-// stride_mlstm_scan; scratch: 16-byte aligned. Returns -2 for more than 256 rows a head or too many chunks.
+// stride_mlstm_scan; records: the sum of the requests' chunks (of 64 tokens, the last one broken) at least; scratch: 16-byte aligned. Returns -2 for more than 256 rows a head or too many chunks.
 int stride_mlstm_chunks(const void* proj, int ld, int q_off, int k_off, int v_off, const float* gates, int ld_gates, const float* bias_i,
                         const float* bias_f, float cap, float q_scale, float* o, float* state, long long state_stride, const int32_t* q_start,
-                        const int32_t* q_len, const int32_t* state_slot, int num_seqs, int H, int D, int DV, int dtype, int max_pieces, float* scratch,
+                        const int32_t* q_len, const int32_t* state_slot, int num_seqs, int H, int D, int DV, int dtype, int records, float* scratch,
                         cudaStream_t stream) {
     if (num_seqs < 0 || H <= 0 || D <= 0 || DV <= 0 || ld <= 0 || ld_gates < 2 * H || !(cap > 0.f) || q_off < 0 || k_off < 0 || v_off < 0 ||
-        max_pieces <= 0 || !scratch)
+        records <= 0 || !scratch)
         return STRIDE_BAD_ARGUMENT;
     if (dtype != STRIDE_DTYPE_F32 && dtype != STRIDE_DTYPE_BF16) return STRIDE_BAD_ARGUMENT;
     if (state_stride < static_cast<long long>(H) * D * DV + static_cast<long long>(H) * D + H) return STRIDE_BAD_ARGUMENT;
-    if (D > 256 || static_cast<long long>(num_seqs) * max_pieces > 65535 || H > 65535 || reinterpret_cast<uintptr_t>(scratch) % 16) return STRIDE_UNSUPPORTED;
+    if (D > 256 || records > 65535 || num_seqs > 65535 || H > 65535 || reinterpret_cast<uintptr_t>(scratch) % 16) return STRIDE_UNSUPPORTED;
     if (num_seqs == 0) return 0;
     const int item = dtype == STRIDE_DTYPE_BF16 ? 2 : 4;
-    const size_t records = static_cast<size_t>(num_seqs) * max_pieces * H;
+    const size_t rows = static_cast<size_t>(records) * H;
     auto at = [&](int off) { return static_cast<const unsigned char*>(proj) + static_cast<size_t>(off) * item; };
     ChunkArgs p = {};
     p.q = at(q_off);
@@ -949,19 +994,24 @@ int stride_mlstm_chunks(const void* proj, int ld, int q_off, int k_off, int v_of
     p.o = o;
     LstmChunk* chunks = reinterpret_cast<LstmChunk*>(scratch);
     p.lstm = chunks;
-    p.piece_s = scratch + records * (sizeof(LstmChunk) / 4);
-    p.piece_p = p.piece_s + records * D * DV;
-    p.piece_n = p.piece_p + records * D;
+    int2* where = reinterpret_cast<int2*>(scratch + rows * (sizeof(LstmChunk) / 4));
+    int32_t* base = reinterpret_cast<int32_t*>(where) + (2LL * records + 3) / 4 * 4;
+    p.where = num_seqs > 1 ? where : nullptr;
+    p.base = num_seqs > 1 ? base : nullptr;
+    p.records = records;
+    p.piece_s = scratch + rows * (sizeof(LstmChunk) / 4) + lstm_table_floats(num_seqs, records);
+    p.piece_p = p.piece_s + rows * D * DV;
+    p.piece_n = p.piece_p + rows * D;
     p.q_start = q_start;
     p.q_len = q_len;
     p.H = H;
     p.D = D;
     p.DV = DV;
-    p.max_pieces = max_pieces;
+    p.max_pieces = records;
     auto aligned = [](const void* x) { return reinterpret_cast<uintptr_t>(x) % 16 == 0; };
     p.vec = p.in_bf16 && D % 8 == 0 && DV % 8 == 0 && ld % 8 == 0 && aligned(p.q) && aligned(p.k) && aligned(p.v);
-    const LstmGates g{gates, ld_gates, bias_i, bias_f, cap, state, state_stride, static_cast<long long>(H) * D * DV + static_cast<long long>(H) * D, state_slot, chunks};
-    stride::launch(lstm_gates_kernel, dim3(H, num_seqs), dim3(256), 0, stream, g, q_start, q_len, H, max_pieces);
+    const LstmGates g{gates, ld_gates, bias_i, bias_f, cap, state, state_stride, static_cast<long long>(H) * D * DV + static_cast<long long>(H) * D, state_slot, chunks, where, base, records};
+    stride::launch(lstm_gates_kernel, dim3(H, num_seqs), dim3(256), 0, stream, g, q_start, q_len, H);
     return dispatch_chunks<kLstm>(p, state, state_stride, state_slot, num_seqs, stream);
 }
 

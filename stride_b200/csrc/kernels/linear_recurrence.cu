@@ -495,7 +495,7 @@ int stride_bonus_scan(const void* r, const void* k, const void* v, const float* 
     if (code != 0) return code;
     const int entries = H * D * D;
     stride::launch(pieces_combine_kernel, dim3((entries + 255) / 256, num_seqs), dim3(256), 0, stream, p.piece_s,
-                   static_cast<const float*>(p.piece_p), state, state_stride, q_len, state_slot, H, D, D, piece, max_pieces);
+                   static_cast<const float*>(p.piece_p), state, state_stride, q_len, state_slot, H, D, D, piece, max_pieces, nullptr);
     code = STRIDE_LAUNCH_STATUS();
     if (code != 0) return code;
     p.mode = 2;

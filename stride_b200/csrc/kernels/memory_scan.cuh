@@ -346,7 +346,7 @@ scan_kernel(const ScanArgs p) {
 static __global__ void __launch_bounds__(256)
 pieces_combine_kernel(float* __restrict__ piece_s, const float* __restrict__ piece_p, float* __restrict__ state, long long state_stride,
                       const int32_t* __restrict__ q_len, const int32_t* __restrict__ state_slot, int H, int D, int DV, int piece,
-                      int max_pieces) {
+                      int max_pieces, const int32_t* __restrict__ base) {
     pdl_trigger();
     pdl_wait();
     const int seq = blockIdx.y;
@@ -358,20 +358,22 @@ pieces_combine_kernel(float* __restrict__ piece_s, const float* __restrict__ pie
     float* S_g = state + static_cast<size_t>(state_slot[seq]) * state_stride + entry;
     float S = *S_g;
     const int pieces = (len + piece - 1) / piece;
+    // a request's first piece: one of max_pieces a request, or as `base` says
+    const size_t z0 = base ? static_cast<size_t>(base[seq]) : static_cast<size_t>(seq) * max_pieces;
     constexpr int AHEAD = 8;        // pieces whose loads are in flight together
     for (int c0 = 0; c0 < pieces; c0 += AHEAD) {
         float own[AHEAD], decay[AHEAD];
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u)
             if (c0 + u < pieces) {
-                const size_t z = static_cast<size_t>(seq) * max_pieces + c0 + u;
+                const size_t z = z0 + c0 + u;
                 own[u] = piece_s[z * H * D * DV + entry];
                 decay[u] = piece_p[z * H * D + row];
             }
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u)
             if (c0 + u < pieces) {
-                piece_s[(static_cast<size_t>(seq) * max_pieces + c0 + u) * H * D * DV + entry] = S;
+                piece_s[(z0 + c0 + u) * H * D * DV + entry] = S;
                 S = fmaf(decay[u], S, own[u]);
             }
     }

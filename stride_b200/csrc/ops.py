@@ -663,29 +663,37 @@ def mlstm_scan(proj, q_off: int, k_off: int, v_off: int, gates, bias_i, bias_f, 
 MLSTM_CHUNKS_MIN_TOKENS = int(_os.environ.get("STRIDE_B200_MLSTM_CHUNKS_MIN", "96"))
 
 
-def mlstm_chunks_scratch_floats(num_seqs: int, max_q_len: int, H: int, D: int, DV: int) -> int:
+# Room for the chunks of a step, at most (a record is the memory's size a head and chunk: 1.1 MB for 16 heads of 128 x 128).
+MLSTM_CHUNKS_MAX_BYTES = 1 << 29
+
+
+def mlstm_chunks_scratch_floats(num_seqs: int, max_q_len: int, H: int, D: int, DV: int, records: int | None = None) -> int:
+    """``records``: chunks in all (None: as many a request as the longest one has)."""
     f = _bound.get("stride_mlstm_chunks_scratch")
     if f is None:
         f = build.load_kernel_library("decay_memory").stride_mlstm_chunks_scratch
         f.argtypes = [c_int] * 5
         f.restype = c_longlong
         _bound["stride_mlstm_chunks_scratch"] = f
-    return int(f(num_seqs, -(-max_q_len // DECAY_CHUNK), H, D, DV))
+    return int(f(num_seqs, num_seqs * -(-max_q_len // DECAY_CHUNK) if records is None else records, H, D, DV))
 
 
 def mlstm_chunks(proj, q_off: int, k_off: int, v_off: int, gates, bias_i, bias_f, cap: float, q_scale: float, o, state, q_start, q_len,
-                 state_slot, num_seqs: int, H: int, D: int, DV: int, max_q_len: int, scratch) -> None:
-    """``mlstm_scan`` with the chunks of every portion side by side (sums in another order)."""
+                 state_slot, num_seqs: int, H: int, D: int, DV: int, max_q_len: int, scratch, records: int | None = None) -> None:
+    """``mlstm_scan`` with the chunks of every portion side by side (sums in another order). ``records``: at least the sum of the
+    requests' chunks (of ``DECAY_CHUNK`` tokens, the last one broken); None: as many a request as ``max_q_len`` has."""
+    if records is None:
+        records = num_seqs * -(-max_q_len // DECAY_CHUNK)
     if state.shape[1] < mlstm_state_floats(H, D, DV) or o.shape[1] != H * DV or gates.shape[1] < 2 * H:
         raise KernelError("mlstm_chunks: shapes do not agree")
-    if scratch.numel() < mlstm_chunks_scratch_floats(num_seqs, max_q_len, H, D, DV):
+    if scratch.numel() < mlstm_chunks_scratch_floats(num_seqs, max_q_len, H, D, DV, records):
         raise KernelError("mlstm_chunks: the scratch is too short")
     _check(_fn("stride_mlstm_chunks")(
         _dev(proj, "proj"), proj.shape[1], int(q_off), int(k_off), int(v_off), _dev(gates, "gates", torch.float32), gates.shape[1],
         _dev(bias_i, "bias_i", torch.float32), _dev(bias_f, "bias_f", torch.float32), float(cap), float(q_scale),
         _dev(o, "o", torch.float32), *_state_rows(state), _dev(q_start, "q_start", torch.int32),
         _dev(q_len, "q_len", torch.int32), _dev(state_slot, "state_slot", torch.int32), int(num_seqs), H, D, DV, _code(proj.dtype),
-        -(-max_q_len // DECAY_CHUNK), _dev(scratch, "scratch", torch.float32), _stream()), "mlstm_chunks")
+        int(records), _dev(scratch, "scratch", torch.float32), _stream()), "mlstm_chunks")
 
 
 # ------------------------------------------------------------ fading memories (linear attention with decay)

@@ -85,6 +85,22 @@ class MatrixLstmMixer(Mixer):
     def state_request(self):
         return StateRequest((ops.mlstm_state_floats(self.H, self.D, self.DV),), torch.float32)
 
+    @staticmethod
+    def _room(records: int) -> int:
+        return 1 << (records - 1).bit_length()      # few sizes: a scratch that was outgrown stays allocated
+
+    def _chunks(self, ctx, tokens) -> int:
+        """The chunks of the step's portions where these run chunk by chunk, else 0. (float32 models keep the one chain, whose sums do
+        not depend on the cutting.)"""
+        portions = ctx.decode_tail_seq
+        if not portions or not 0 < ops.MLSTM_CHUNKS_MIN_TOKENS <= ctx.max_q_len:
+            return 0
+        count = min(ctx.decode_tail_start, tokens)
+        lens = ctx.portion_lens
+        records = sum(-(-n // ops.DECAY_CHUNK) for n in lens) if lens else count // ops.DECAY_CHUNK + portions
+        room = ops.mlstm_chunks_scratch_floats(portions, ctx.max_q_len, self.H, self.D, self.DV, records=self._room(records)) * 4
+        return records if records <= 65535 and room <= ops.MLSTM_CHUNKS_MAX_BYTES else 0
+
     def forward(self, x, ctx, cache, lazy_output: bool = False):
         tokens, f32 = x.shape[0], torch.float32
         proj = self.rt.buffer("mlstm_proj", tokens, self.c_in)
@@ -95,12 +111,11 @@ class MatrixLstmMixer(Mixer):
         columns, gate_args, sizes = (0, self.k_off, self.v_off), (gates, self.bias_i, self.bias_f, self.cap, self.D ** -0.5), (self.H, self.D, self.DV)
         portions, slots = ctx.decode_tail_seq, sequence_slots(ctx)      # the requests before the trailing single tokens; all of them
         first = 0
-        # (float32 models keep the one chain, whose sums do not depend on the cutting)
-        if (x.dtype == torch.bfloat16 and portions and 0 < ops.MLSTM_CHUNKS_MIN_TOKENS <= ctx.max_q_len
-                and portions * -(-ctx.max_q_len // ops.DECAY_CHUNK) <= 65535):
-            scratch = self.rt.scratch("mlstm_chunks", ops.mlstm_chunks_scratch_floats(portions, ctx.max_q_len, *sizes))
+        records = self._chunks(ctx, tokens) if x.dtype == torch.bfloat16 else 0
+        if records:
+            room = ops.mlstm_chunks_scratch_floats(portions, ctx.max_q_len, *sizes, records=self._room(records))
             ops.mlstm_chunks(proj, *columns, *gate_args, o, cache.state, ctx.q_start, ctx.q_len, ctx.state_slot, portions, *sizes, ctx.max_q_len,
-                             scratch)
+                             self.rt.scratch("mlstm_chunks", room), records=records)
             first = portions
         if slots > first:
             ops.mlstm_scan(proj, *columns, *gate_args, o, cache.state, ctx.q_start[first:], ctx.q_len[first:], ctx.state_slot[first:], slots - first,

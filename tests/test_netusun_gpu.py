@@ -703,13 +703,13 @@ def lstm_case(H, D, DV, lens, seed):
         at += n
     starts = [sum(lens[:i]) for i in range(len(lens))]
 
-    def run(chunks=True):
+    def run(records=None, chunks=True):
         from stride_b200.csrc import ops
         state, o = torch.zeros(len(lens), floats, device="cuda"), torch.full((tokens, H * DV), float("nan"), device="cuda")
         args = (proj, 0, H * D, 2 * H * D, gates, bias, bias, cap, D ** -0.5, o, state, dev(starts), dev(lens), dev(list(range(len(lens)))), len(lens), H, D, DV)
         if chunks:
-            scratch = torch.full((ops.mlstm_chunks_scratch_floats(len(lens), max(lens), H, D, DV),), float("nan"), device="cuda")
-            ops.mlstm_chunks(*args, max(lens), scratch)
+            scratch = torch.full((ops.mlstm_chunks_scratch_floats(len(lens), max(lens), H, D, DV, records),), float("nan"), device="cuda")
+            ops.mlstm_chunks(*args, max(lens), scratch, records)
         else:
             ops.mlstm_scan(*args)
         return o, state
@@ -724,3 +724,32 @@ def test_matrix_lstm_chunks_are_no_further_from_float64_than_the_chain(gpu, H, D
     run, want = lstm_case(H, D, DV, lens, 5)
     error = lambda o: float(((o.double().view(want.shape) - want).norm(dim=-1) / want.norm(dim=-1)).median())
     assert error(run()[0]) <= error(run(chunks=False)[0])
+
+
+def test_matrix_lstm_chunks_lie_close(gpu):
+    """A long portion beside short and empty ones: room for the chunks that there are, and the same bits in it as in one with a long
+    portion's chunks for every request."""
+    from stride_b200.csrc import ops
+    lens = [7, 130, 1, 64, 0, 5, 200, 65, 0]
+    run, _want = lstm_case(3, 24, 16, lens, 9)
+    records = sum(-(-n // ops.DECAY_CHUNK) for n in lens)
+    whole, close_by = run(), run(records)
+    assert torch.equal(whole[0], close_by[0]) and torch.equal(whole[1], close_by[1])
+    assert not bool(whole[0].isnan().any())
+    spread, packed = (ops.mlstm_chunks_scratch_floats(201, 1000, 16, 128, 128, r) * 4 for r in (None, 216))
+    assert packed < 0.26e9 < 3.5e9 < spread
+
+
+def test_matrix_lstm_chunks_stay_within_their_room(gpu):
+    """A step whose chunks would need more room than allowed goes token by token."""
+    from types import SimpleNamespace
+
+    from stride_b200.parts.mlstm import MatrixLstmMixer
+    part = SimpleNamespace(H=16, D=128, DV=128, _room=MatrixLstmMixer._room)
+
+    def chunks(lens, given=True):
+        ctx = SimpleNamespace(decode_tail_seq=len(lens), max_q_len=max(lens), decode_tail_start=sum(lens), portion_lens=tuple(lens) if given else ())
+        return MatrixLstmMixer._chunks(part, ctx, sum(lens))
+
+    assert chunks([2000]) == 32 and chunks([200] * 8) == 32 and chunks([95]) == 0 and chunks([2000], given=False) >= 32
+    assert chunks([16384]) == 256 and chunks([20000]) == 0          # 256 chunks of 1.1 MB are allowed, 512 (the next size) are not
