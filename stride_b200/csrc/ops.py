@@ -667,6 +667,19 @@ MLSTM_CHUNKS_MIN_TOKENS = int(_os.environ.get("STRIDE_B200_MLSTM_CHUNKS_MIN", "9
 MLSTM_CHUNKS_MAX_BYTES = 1 << 29
 
 
+def mlstm_chunks_pay(portions: int, longest: int, tokens: int, records: int, H: int, D: int, DV: int) -> bool:
+    """Whether ``portions`` (``tokens`` in all, the longest of ``longest``, ``records`` chunks) are faster chunk by chunk than token by
+    token, by estimates in us fitted to the measured times below. The chain takes its longest request's tokens one after the other, or
+    what the tokens and the requests' states take the device; the chunks cost their launches and the passes over what the chunks and
+    states hold, a broken chunk as much as a whole one, more once that outgrows L2. Chain / chunks, 16 heads of 128 x 128: one
+    request of 128 tokens 45 / 51 us, of 200 70 / 52, of 2,000 634 / 128; 8 of 200 370 / 125; one of 100 beside 60 of 8 273 / 423, one of
+    1,000 beside 100 of 5 623 / 859. 32 heads: one of 96 65 / 53; 8 heads of 256 x 256: one of 300 beside 30 of 20 394 / 510."""
+    size, wide = H * D * DV / 262144, 0.78 if D > 128 else 1.0
+    chain = max(longest * max(0.2 + 0.1 * size, 0.3 * size * wide), size * wide * (0.22 * tokens + 2.9 * portions))
+    held = (records + portions) * size
+    return 13 + 0.19 * min(D, 128) + 0.25 * records + held * (2.6 if held < 75 else 3.7) < chain
+
+
 def mlstm_chunks_scratch_floats(num_seqs: int, max_q_len: int, H: int, D: int, DV: int, records: int | None = None) -> int:
     """``records``: chunks in all (None: as many a request as the longest one has)."""
     f = _bound.get("stride_mlstm_chunks_scratch")

@@ -99,7 +99,9 @@ class MatrixLstmMixer(Mixer):
         lens = ctx.portion_lens
         records = sum(-(-n // ops.DECAY_CHUNK) for n in lens) if lens else count // ops.DECAY_CHUNK + portions
         room = ops.mlstm_chunks_scratch_floats(portions, ctx.max_q_len, self.H, self.D, self.DV, records=self._room(records)) * 4
-        return records if records <= 65535 and room <= ops.MLSTM_CHUNKS_MAX_BYTES else 0
+        if records > 65535 or room > ops.MLSTM_CHUNKS_MAX_BYTES:
+            return 0
+        return records if ops.mlstm_chunks_pay(portions, ctx.max_q_len, count, records, self.H, self.D, self.DV) else 0
 
     def forward(self, x, ctx, cache, lazy_output: bool = False):
         tokens, f32 = x.shape[0], torch.float32

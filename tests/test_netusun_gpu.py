@@ -740,8 +740,8 @@ def test_matrix_lstm_chunks_lie_close(gpu):
     assert packed < 0.26e9 < 3.5e9 < spread
 
 
-def test_matrix_lstm_chunks_stay_within_their_room(gpu):
-    """A step whose chunks would need more room than allowed goes token by token."""
+def test_matrix_lstm_takes_the_chunks_where_they_pay_and_fit(gpu):
+    """One long portion beside many short ones stays token by token, as do steps whose chunks would need more room than allowed."""
     from types import SimpleNamespace
 
     from stride_b200.parts.mlstm import MatrixLstmMixer
@@ -751,5 +751,7 @@ def test_matrix_lstm_chunks_stay_within_their_room(gpu):
         ctx = SimpleNamespace(decode_tail_seq=len(lens), max_q_len=max(lens), decode_tail_start=sum(lens), portion_lens=tuple(lens) if given else ())
         return MatrixLstmMixer._chunks(part, ctx, sum(lens))
 
-    assert chunks([2000]) == 32 and chunks([200] * 8) == 32 and chunks([95]) == 0 and chunks([2000], given=False) >= 32
+    assert chunks([2000]) == 32 and chunks([200]) == 4 and chunks([200] * 8) == 32
+    assert chunks([95]) == 0 and chunks([100] + [8] * 60) == 0 and chunks([1000] + [5] * 200) == 0
+    assert chunks([2000], given=False) >= 32
     assert chunks([16384]) == 256 and chunks([20000]) == 0          # 256 chunks of 1.1 MB are allowed, 512 (the next size) are not
