@@ -66,10 +66,11 @@ constexpr long long kStaggerCycles = 1000;
 // query's rotated part has a matrix of its own too (map_q2). A key tile is 24 KB: one stage for keys and two for values leave room
 // for two CTAs per SM, and the scores run two tiles ahead, which hides the one stage. An optional gate (LatentGate) multiplies the
 // result. 2,048 tokens of 16 heads: 42 us, beside 12 us for the product that expands and 4 us for the
-// gather; on the latents themselves (latent_attention_tc.cu and two products a head) 745 + 2 x 243 us.
+// gather; on the latents themselves (latent_attention_tc.cu and two products a head) 745 + 24 + 19 us.
 struct LatentGate {
     const __nv_bfloat16* values;        // null: none
     int ld, per_output;                 // row stride; one number an output (else one a head)
+    int head_stride, v_off;             // of an expanded row: head h's key at column h * head_stride, its value v_off behind it
 };
 template <int HD, int HEADS, bool TMA_KV, bool REL, bool LATENT = false>
 __global__ void __launch_bounds__(HEADS == 1 ? 256 : 512, HEADS == 1 ? 2 : 1)
@@ -197,7 +198,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     // masked (K) or cleared (V) by the softmax warps, whatever they hold
                     const int boxes = is_k ? BOXES : HALVES;
                     const bool rotated = lane == HALVES;
-                    const int x = rotated ? 0 : head0 * 2 * HD + (is_k ? 0 : HD) + lane * 64;
+                    const int x = rotated ? 0 : head0 * gate.head_stride + (is_k ? 0 : gate.v_off) + lane * 64;
                     for (int j = 0; j < n_tiles; ++j) {
                         const int st = j % stages;
                         if (!mbar_wait(smem_u32(&empty[st]), (static_cast<uint32_t>(j / stages) & 1u) ^ 1u, status, is_k ? 11 : 18)) break;
@@ -553,7 +554,7 @@ int launch_attn(const CUtensorMap* map_q, const CUtensorMap* map_k, const CUtens
     stride::launch(kernel, grid, block, smem, stream, *map_q, tma ? *map_k : *map_q, tma ? *map_v : *map_q, k_pages, v_pages, out,
                    block_table, table_width, q_start, q_len, ctx_len, num_seqs, nq, nkv, page_shift,
                    (softcap != 0.f ? fabsf(softcap) : scale) * 1.4426950408889634f, window, softcap != 0.f ? scale / softcap : 0.f, sinks, slopes, rel,
-                   rel_len, status, *map_q, *map_q, LatentGate{nullptr, 0, 0}, 0);
+                   rel_len, status, *map_q, *map_q, LatentGate{}, 0);
     return STRIDE_LAUNCH_STATUS();
 }
 
@@ -638,19 +639,22 @@ extern "C" int stride_paged_prefill_attention_tc(const void* q, int q_stride, vo
 
 // Attention over expanded latents for the first `num_seqs` requests of the step, which own the first `tokens` rows of the flat
 // batch. q: bf16 rows of q_ld numbers, head h's plain part at columns h * (hd + rot); q_rot: rows of q_rot_ld numbers, head h's
-// rotated part at columns h * q_rot_stride; both hold q_rows rows (tokens at least). kv: [kv_rows, heads, 2 * hd], a head's key and value, k_rot:
+// rotated part at columns h * q_rot_stride; both hold q_rows rows (tokens at least). kv: [kv_rows, heads * 2 * hd], head h's key at
+// column h * kv_head_stride, its value kv_v_off behind it (multiples of 8), k_rot:
 // [kv_rows, rot]: the keys of request 0 from its position 0 on, then those of request 1, ... (kv_rows: rows that may be read;
 // rows past the last request's keys may hold anything). out: [tokens, heads * hd]. gate (bf16 or null): the result of row t is
 // multiplied by sigmoid(gate[t * gate_ld + h]), or, gate_per_output, by sigmoid(gate[t * gate_ld + column]). Returns -2 for other
 // sizes than hd 128 with rot 64 and for unaligned rows.
 extern "C" int stride_latent_prefill_tc(const void* q, int q_ld, const void* q_rot, int q_rot_ld, int q_rot_stride, int q_rows, const void* kv,
-                                        const void* k_rot, int kv_rows, void* out, const int32_t* q_start, const int32_t* q_len,
+                                        int kv_head_stride, int kv_v_off, const void* k_rot, int kv_rows, void* out, const int32_t* q_start, const int32_t* q_len,
                                         const int32_t* ctx_len, int num_seqs, int tokens, int heads, int hd, int rot, float scale,
                                         const float* sinks, const void* gate, int gate_ld, int gate_per_output, int* status,
                                         cudaStream_t stream) {
     if (tokens < 0 || num_seqs < 0 || heads <= 0 || q_rows < tokens || kv_rows <= 0 || status == nullptr) return STRIDE_BAD_ARGUMENT;
     if (q_ld < heads * (hd + rot) || q_rot_stride < rot || q_rot_ld < (heads - 1) * q_rot_stride + rot) return STRIDE_BAD_ARGUMENT;
-    if (hd != 128 || rot != 64 || heads > 65535 || (q_ld | q_rot_ld | q_rot_stride) % 8 || (gate && gate_per_output && gate_ld % 8)) return STRIDE_UNSUPPORTED;
+    if (kv_head_stride < hd || kv_v_off < hd || (heads - 1) * static_cast<long long>(kv_head_stride) + kv_v_off + hd > 2LL * heads * hd)
+        return STRIDE_BAD_ARGUMENT;
+    if (hd != 128 || rot != 64 || heads > 65535 || (q_ld | q_rot_ld | q_rot_stride | kv_head_stride | kv_v_off) % 8 || (gate && gate_per_output && gate_ld % 8)) return STRIDE_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(q_rot) | reinterpret_cast<uintptr_t>(kv) | reinterpret_cast<uintptr_t>(k_rot) |
          reinterpret_cast<uintptr_t>(out) | (gate && gate_per_output ? reinterpret_cast<uintptr_t>(gate) : 0)) % 16)
         return STRIDE_UNSUPPORTED;
@@ -675,6 +679,6 @@ extern "C" int stride_latent_prefill_tc(const void* q, int q_ld, const void* q_r
     if (!map_q || !map_q2 || !map_kv || !map_k2) return STRIDE_UNSUPPORTED;
     stride::launch(kernel, dim3(heads, max_tiles), dim3(256), smem, stream, *map_q, *map_kv, *map_kv, nullptr, nullptr, static_cast<__nv_bfloat16*>(out),
                    nullptr, 0, q_start, q_len, ctx_len, num_seqs, heads, heads, 0, scale * 1.4426950408889634f, 0, 0.f, sinks, nullptr, nullptr, 0,
-                   status, *map_q2, *map_k2, tc::LatentGate{static_cast<const __nv_bfloat16*>(gate), gate_ld, gate_per_output}, q_rot_stride);
+                   status, *map_q2, *map_k2, tc::LatentGate{static_cast<const __nv_bfloat16*>(gate), gate_ld, gate_per_output, kv_head_stride, kv_v_off}, q_rot_stride);
     return STRIDE_LAUNCH_STATUS();
 }

@@ -104,7 +104,7 @@ _SIGNATURES = {
                                                      c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p]),
     "stride_latent_gather": ("latent_attention", [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                                   c_void_p, c_void_p]),
-    "stride_latent_prefill_tc": ("attention_prefill_tc", [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
+    "stride_latent_prefill_tc": ("attention_prefill_tc", [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p,
                                                           c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
                                                           c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "stride_latent_attention_tc": ("latent_attention_tc", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
@@ -1149,9 +1149,11 @@ def latent_gather(latent_pages, krot_pages, block_table, ctx_len, num_seqs: int,
 
 
 def latent_prefill_tc(q, q_off: int, q_rot, q_rot_off: int, q_rot_stride: int, kv, krot, out, q_start, q_len, ctx_len, num_seqs: int,
-                      heads: int, scale: float, sinks=None, gate=None, gate_off: int = 0, gate_per_output: bool = False) -> None:
+                      heads: int, scale: float, sinks=None, gate=None, gate_off: int = 0, gate_per_output: bool = False,
+                      kv_head_stride: int = 256, kv_v_off: int = 128) -> None:
     """Causal attention of the step's first ``num_seqs`` requests, which own the first rows of ``q``, over expanded keys and values: ``kv``
-    [rows, heads * 256] holds a head's 128 key and 128 value numbers, ``krot`` [rows, 64] the rotated key part, as ``latent_gather`` orders the
+    [rows, heads * 256] holds head h's 128 key numbers from column ``h * kv_head_stride`` on and its 128 value numbers ``kv_v_off`` columns
+    further, ``krot`` [rows, 64] the rotated key part, as ``latent_gather`` orders the
     rows. Queries: 128 + 64 numbers a head in ``q`` from column ``q_off`` on, of which the 64 are taken (rotated) from ``q_rot``, head h at
     column ``q_rot_off + h * q_rot_stride``. ``out`` [tokens, heads * 128] is multiplied by the sigmoid of ``gate`` (its columns from
     ``gate_off`` on: one a head, or one an output)."""
@@ -1162,7 +1164,7 @@ def latent_prefill_tc(q, q_off: int, q_rot, q_rot_off: int, q_rot_stride: int, k
     st = _tc_buffers(q.device, 0)
     _check(_fn("stride_latent_prefill_tc")(
         _dev(q, "q", torch.bfloat16) + q_off * 2, q.shape[1], _dev(q_rot, "q_rot", torch.bfloat16) + q_rot_off * 2, q_rot.shape[1], q_rot_stride,
-        q.shape[0], _dev(kv, "kv", torch.bfloat16), _dev(krot, "krot", torch.bfloat16), kv.shape[0], _dev(out, "out", torch.bfloat16),
+        q.shape[0], _dev(kv, "kv", torch.bfloat16), int(kv_head_stride), int(kv_v_off), _dev(krot, "krot", torch.bfloat16), kv.shape[0], _dev(out, "out", torch.bfloat16),
         _dev(q_start, "q_start", torch.int32), _dev(q_len, "q_len", torch.int32), _dev(ctx_len, "ctx_len", torch.int32), num_seqs, tokens, heads,
         128, 64, float(scale), _opt(sinks, "sinks", torch.float32), None if gate is None else _dev(gate, "gate") + gate_off * 2,
         0 if gate is None else gate.shape[1], 1 if gate_per_output else 0, _dev(st["status"], "status"), _stream()), "latent_prefill_tc")

@@ -96,7 +96,7 @@ class LatentAttention(Mixer):
         self.kv_off = -(-self.q_cols // 8) * 8
         self.g_off = self.kv_off + -(-self.kv_dim // 8) * 8
         self.proj_dim = -(-(self.g_off + self.g_dim) // 8) * 8
-        self.w_in = self.w_ukv = self.w_o = self.latent_w = self.w_uq = self.q_norm_w = self.sinks = None
+        self.w_in = self.w_ukv = self.w_uk = self.w_uv = self.w_o = self.latent_w = self.w_uq = self.q_norm_w = self.sinks = None
         # rotated entries in the order the kernels pair them: new entry 2i is old entry i, new entry 2i + 1 old entry i + dims / 2
         half = self.rot_dims // 2
         order = [j for i in range(half) for j in (i, i + half)] + list(range(self.rot_dims, self.rot))
@@ -159,15 +159,14 @@ class LatentAttention(Mixer):
         if self.has_sinks:
             self.sinks = weights[self._n("sink")]
         self.w_in = w
-        # [heads, dim + value_dim, rank]: a head's rows of W_uk, then of W_uv, so that one product expands both
-        self.w_ukv = torch.cat([weights[self._n("uk")].view(self.heads, self.dim, self.rank),
-                                weights[self._n("uv")].view(self.heads, self.vdim, self.rank)], 1).contiguous()
+        # W_uk's rows, then W_uv's, so that one product expands both
+        self.w_ukv = torch.cat([weights[self._n("uk")], weights[self._n("uv")]]).contiguous()
+        self.w_uk, self.w_uv = self.w_ukv[:self.heads * self.dim], self.w_ukv[self.heads * self.dim:]
         self.w_o = weights[self._n("o")]
         self.position.bind(weights)
 
     def named_tensors(self):
-        out = {self._n("uk"): self.w_ukv[:, :self.dim].reshape(self.heads * self.dim, self.rank),
-               self._n("uv"): self.w_ukv[:, self.dim:].reshape(self.heads * self.vdim, self.rank), self._n("o"): self.w_o}
+        out = {self._n("uk"): self.w_uk, self._n("uv"): self.w_uv, self._n("o"): self.w_o}
         if self.q_rank:
             out[self._n("dq")], out[self._n("dq.norm")] = self.w_in[:self.q_rank], self.q_norm_w
             out[self._n("uq")] = self._pair_rows(self.w_uq, self.dim, self.heads, self.dim + self.rot, inverse=True)
@@ -214,17 +213,16 @@ class LatentAttention(Mixer):
             first = min(ctx.decode_tail_start, tokens)
             self._attend_expanded(q, q_off, qa, attn[:first], latent, key_rot, proj, ctx, cache)
         if tokens > first:
-            rest, per_head = tokens - first, (self.dim + self.vdim) * self.rank
-            # q~[t, a, :] = q[t, a, :dim] @ W_uk[a]          B_a[k, n] = W_ukv[a, k, n]
-            ops.head_gemm(q[first:], q_ld, self.dim + self.rot, self.w_ukv, per_head, self.rank, 1, qa[first:], self.heads * width, width,
-                          rest, self.heads, self.rank, self.dim, a_off=q_off)
-            mixed = self.rt.buffer("latent_mixed", tokens, self.heads * self.rank)
+            mixed, gate, rows = self.rt.buffer("latent_mixed", tokens, self.heads * self.rank), proj if self.gated else None, slice(first, tokens)
+            q_in, q_out, o_in, o_out = (q, qa, mixed, attn) if not first else (q[rows], qa[rows], mixed[rows], attn[rows])
+            # q~[t, a, :] = q[t, a, :dim] @ W_uk[a]          W_uk [heads * dim, rank]: B_a[k, n] = W_uk[a * dim + k, n]
+            ops.head_gemm(q_in, q_ld, self.dim + self.rot, self.w_uk, self.dim * self.rank, self.rank, 1, q_out, self.heads * width, width,
+                          tokens - first, self.heads, self.rank, self.dim, a_off=q_off)
             self._attend(qa, mixed, latent, key_rot, ctx, cache, tokens, first)
-            # o[t, a, :] = W_uv[a] mixed[t, a, :]            B_a[k, n] = W_ukv[a, dim + n, k]
-            gate = proj[first:] if self.gated else None
-            ops.head_gemm(mixed[first:], self.heads * self.rank, self.rank, self.w_ukv.view(-1)[self.dim * self.rank:], per_head, 1, self.rank,
-                          attn[first:], self.heads * self.vdim, self.vdim, rest, self.heads, self.vdim, self.rank, gate=gate, ldg=self.proj_dim,
-                          gate_off=self.g_off, gate_per_output=self.full_gate)
+            # o[t, a, :] = W_uv[a] mixed[t, a, :]            W_uv [heads * vdim, rank]: B_a[k, n] = W_uv[a * vdim + n, k]
+            ops.head_gemm(o_in, self.heads * self.rank, self.rank, self.w_uv, self.vdim * self.rank, 1, self.rank, o_out, self.heads * self.vdim,
+                          self.vdim, tokens - first, self.heads, self.vdim, self.rank, gate=gate if gate is None or not first else gate[rows],
+                          ldg=self.proj_dim, gate_off=self.g_off, gate_per_output=self.full_gate)
         if lazy_output:
             return Projection(attn, self.w_o)
         out = self.rt.buffer("mixer_out", tokens, self.hidden)
@@ -245,10 +243,10 @@ class LatentAttention(Mixer):
         kv_dim = self.heads * (self.dim + self.vdim)
         kv = self.rt.scratch("latent_expanded", rows * kv_dim, self.rt.dtype)[:rows * kv_dim].view(rows, kv_dim)
         ops.latent_gather(latent, key_rot, ctx.block_table[cache.group], ctx.ctx_len, seqs, cache.page_size, c[:keys], k_rot[:keys])
-        ops.linear(c[:keys], self.w_ukv.view(kv_dim, self.rank), kv[:keys])
+        ops.linear(c[:keys], self.w_ukv, kv[:keys])
         ops.latent_prefill_tc(q, q_off, qa, self.rank, self.rank + self.rot, kv, k_rot, out, ctx.q_start, ctx.q_len, ctx.ctx_len, seqs,
                               self.heads, self.scale, sinks=self.sinks, gate=proj if self.gated else None, gate_off=self.g_off,
-                              gate_per_output=self.full_gate)
+                              gate_per_output=self.full_gate, kv_head_stride=self.dim, kv_v_off=self.heads * self.dim)
 
     def _attend(self, qa, mixed, latent, key_rot, ctx, cache, tokens, first: int = 0):
         """Attention over the latents themselves for the rows from ``first`` on (0, or where the decode tail starts)."""

@@ -143,3 +143,20 @@ def test_a_latent_branch_of_a_parallel_mixer_in_full_portions(gpu, models, expan
     assert engine.model.sizes_by_context
     full_portions(engine, case, 1, seeded_tokens(256, cfg["vocab"], 911), 64)
     assert expansions and engine.runner.graph_replays == 4
+
+
+def test_weights_are_handed_out_as_they_are_held(gpu, models):
+    """A change to what ``get_weight`` gives is a change to the model, also of the two matrices that one product expands with."""
+    case = models[48]
+    engine = engine_for(case)
+    tokens = seeded_tokens(20, case.cfg["vocab"], 731)
+    open_request(engine, 1, 20)
+    before = engine.forward([(1, tokens, 0, [19])]).clone()
+    for name in ("l0.mix.uk", "l0.mix.uv"):
+        weight = engine.get_weight(name)
+        assert weight.shape == case.state[name].shape and torch.equal(weight.cpu(), case.state[name])
+        weight.zero_()
+        assert not bool(engine.get_weight(name).any())
+        after = engine.forward([(1, tokens, 0, [19])]).clone()
+        assert not torch.equal(before, after)
+        before = after
