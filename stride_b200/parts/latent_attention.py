@@ -253,8 +253,8 @@ class LatentAttention(Mixer):
         table = ctx.block_table[cache.group]
         if not self._fast:
             # the exact kernel: the whole 32-bit path, and sizes the tensor-core kernel refuses
-            ops.latent_attention(qa, mixed, latent, key_rot, table, ctx.seq_of_token[:tokens], ctx.positions[:tokens], self.heads, self.rank,
-                                 self.rot, cache.page_size, self.scale, sinks=self.sinks)
+            ops.latent_attention(qa[first:], mixed[first:], latent, key_rot, table, ctx.seq_of_token[first:tokens], ctx.positions[first:tokens],
+                                 self.heads, self.rank, self.rot, cache.page_size, self.scale, sinks=self.sinks)
             return
         geometry = (self.heads, self.rank, self.rot, cache.page_size, self.scale)
         split = min(ctx.decode_tail_start, tokens)          # portions before, single tokens after

@@ -42,7 +42,7 @@ class Case:
 
 @pytest.fixture(scope="module")
 def models(tmp_models):
-    return {rank: Case(tmp_models, rank) for rank in (48,)}
+    return {rank: Case(tmp_models, rank) for rank in (48, 40)}       # 40: the tensor-core kernel over the latents refuses it
 
 
 @pytest.fixture
@@ -160,3 +160,28 @@ def test_weights_are_handed_out_as_they_are_held(gpu, models):
         after = engine.forward([(1, tokens, 0, [19])]).clone()
         assert not torch.equal(before, after)
         before = after
+
+
+@pytest.mark.parametrize("rank", [48, 40])
+def test_portions_beside_single_tokens(gpu, models, expansions, monkeypatch, rank):
+    """A whole prompt; then a portion behind it and another request's first one beside two single tokens, which go over the latents:
+    through the tensor-core kernel, or (a rank it refuses) the exact one, which is given their rows alone."""
+    from stride_b200.csrc import ops
+    from stride_b200.parts.latent_attention import LatentAttention
+    monkeypatch.setattr(LatentAttention, "EXPAND_PAIRS", 1)
+    exact, run = [], ops.latent_attention
+    monkeypatch.setattr(ops, "latent_attention", lambda *a, **k: (exact.append(a[0].shape[0]), run(*a, **k))[1])
+    case, vocab = models[rank], models[rank].cfg["vocab"]
+    engine = engine_for(case)
+    tokens = {key: seeded_tokens(n, vocab, 700 + key) for key, n in ((1, 150), (2, 90), (3, 40), (4, 70))}
+    for key, t in tokens.items():
+        open_request(engine, key, len(t))
+    check(engine.forward([(1, tokens[1][:120], 0, list(range(120)))]), case, tokens[1], list(range(120)), "whole prompt")
+    assert expansions == [120, 120]             # two layers
+    engine.forward([(2, tokens[2][:89], 0, []), (3, tokens[3][:39], 0, [])])
+    exact.clear()
+    got = engine.forward([(1, tokens[1][120:], 120, list(range(30))), (4, tokens[4], 0, list(range(70))), (2, tokens[2][89:], 89, [0]),
+                          (3, tokens[3][39:], 39, [0])])
+    assert expansions[-1] == 100 and exact == ([2, 2] if rank == 40 else [])
+    for key, rows, at in ((1, range(120, 150), 0), (4, range(70), 30), (2, [89], 100), (3, [39], 101)):
+        check(got[at:at + len(rows)], case, tokens[key], list(rows), f"request {key} of the mixed step")
