@@ -47,6 +47,8 @@ class StepContext:
     # Keys that the requests in front of the decode tail hold together after this step, or an upper bound of it for as long as
     # this context's launches may be replayed. 0: not given (a part must then not size a launch by it).
     portion_keys: int = 0
+    # The same of the one among them that holds the most.
+    portion_longest: int = 0
     # Tokens that each of the requests in front of the decode tail brings (a captured portion always brings the same). (): not given.
     portion_lens: tuple = ()
     # Host copy of the step's items for parts that loop in Python:

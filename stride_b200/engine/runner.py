@@ -138,10 +138,11 @@ class ModelRunner:
         bound = batch.max_ctx if not for_graph and portion_bound is None else for_graph or portion_bound or self.table_width * self.cache.page_size
         held = [position + n for _request, _row, n, position, _slot in items[:tail_seq]]
         portion_keys = sum(held) if portion_bound is None else portion_bound
+        longest = max(held, default=0) if portion_bound is None else portion_bound
         return make_context(staging.dev, staging.layout, num_tokens, batch.num_seqs, num_rows, max_q_len=batch.max_q_len,
                             max_ctx=batch.max_ctx, decode_only=batch.decode_only, host_items=items,
                             decode_tail_start=0 if for_graph else tail_start, decode_tail_seq=0 if for_graph else tail_seq,
-                            context_bound=bound, portion_keys=0 if for_graph else portion_keys,
+                            context_bound=bound, portion_keys=0 if for_graph else portion_keys, portion_longest=0 if for_graph else longest,
                             portion_lens=() if for_graph else tuple(item[2] for item in items[:tail_seq]),
                             seq_slots=staging.layout["seq_cap"] if for_graph else batch.num_seqs)
 

@@ -21,7 +21,7 @@ and the output ``W_uv_a (sum_j p_j c_j)``: attention runs on the cached vectors 
 That form costs heads * (2 kv_rank + rot_dim) multiply-adds a (query, key) pair, the plain one heads * (dim + rot_dim + value_dim),
 3.4 times less at 128 + 64, 128 and a latent of 512, beside kv_rank * heads * (dim + value_dim) a key to expand it. So portions of prompts
 in bfloat16 expand, where the head sizes are those of the tcgen05 kernel and the queries have no latent (``_expands`` says from how many
-tokens on):
+keys on):
 
     one product, latent_prepare  as above
     latent_gather                the requests' latents out of their pages
@@ -57,11 +57,15 @@ from .base import CacheRequest, Mixer, Projection, TensorDecl, build_part, regis
 
 class LatentAttention(Mixer):
     lazy_output = True
-    # Portions go over expanded keys where tokens x keys reach this. A step of the six-layer Nidilix shape (two such layers), on the
-    # latents themselves / expanded: 100 tokens behind 2,000 2.11 / 1.94 ms, 24 behind 6,000 2.80 / 1.88 ms, 1,200 alone 3.49 / 2.73 ms;
-    # below it both are level (300 alone 2.08 / 2.12 ms: the launches), and the kernels of the folded form are fewer.
-    EXPAND_PAIRS = 1 << 16
-    MAX_EXPANDED_BYTES = 1 << 28      # keys and values of a step, expanded, at most
+    # Portions go over expanded keys where one of their requests holds this many: the folded form walks a request's keys in one CTA, a
+    # tile of 64 after the other at some 12 us each, however few the tokens. Two such layers of 16 heads and nothing else, a step on the
+    # latents / expanded: 33 tokens behind 2,000 841 / 449 us, 10 behind 30,000 9.3 / 1.5 ms, 2,000 alone 1738 / 577 us. Below it the
+    # folded form has fewer launches (256 alone 429 / 466 us, 64 requests of 8 561 / 651). Many requests make the product that
+    # expands long while the walk stays what the longest one's is (16 of 16 tokens behind 1,000 556 / 513 us): at most
+    # EXPAND_SHARE times the longest one's keys in all.
+    EXPAND_KEYS = 512
+    EXPAND_SHARE = 16
+    MAX_EXPANDED_BYTES = 1 << 28      # keys and values of a step, expanded, at most (the buffer, whose rows are a power of two)
 
     def __init__(self, spec, runtime):
         super().__init__(spec, runtime)
@@ -229,15 +233,18 @@ class LatentAttention(Mixer):
         ops.linear(attn, self.w_o, out)
         return out
 
+    def _expanded_rows(self, keys) -> int:
+        return max(2048, 1 << (keys - 1).bit_length())          # few sizes, for the scratch and for the copies' descriptors
+
     def _expands(self, ctx, tokens) -> bool:
         """Whether this step's portions go over expanded keys and values."""
-        split, keys = min(ctx.decode_tail_start, tokens), ctx.portion_keys
-        return (self._expand and split * keys >= self.EXPAND_PAIRS
-                and keys * self.heads * 2 * (self.dim + self.vdim) <= self.MAX_EXPANDED_BYTES)
+        keys, longest = ctx.portion_keys, ctx.portion_longest
+        return (self._expand and ctx.decode_tail_start > 0 and longest >= self.EXPAND_KEYS and keys <= self.EXPAND_SHARE * longest
+                and self._expanded_rows(keys) * self.heads * 2 * (self.dim + self.vdim) <= self.MAX_EXPANDED_BYTES)
 
     def _attend_expanded(self, q, q_off, qa, out, latent, key_rot, proj, ctx, cache):
         keys, seqs = ctx.portion_keys, ctx.decode_tail_seq
-        rows = max(2048, 1 << (keys - 1).bit_length())          # few sizes, for the scratch and for the copies' descriptors
+        rows = self._expanded_rows(keys)
         c = self.rt.scratch("latent_dense", rows * self.rank, self.rt.dtype)[:rows * self.rank].view(rows, self.rank)
         k_rot = self.rt.scratch("latent_dense_rot", rows * self.rot, self.rt.dtype)[:rows * self.rot].view(rows, self.rot)
         kv_dim = self.heads * (self.dim + self.vdim)

@@ -47,10 +47,10 @@ def models(tmp_models):
 
 @pytest.fixture
 def expansions(monkeypatch):
-    """The expanded kernel's calls, the rows of each; every portion is worth expanding."""
+    """The expanded kernel's calls, the rows of each; requests of 64 keys and more are worth expanding."""
     from stride_b200.csrc import ops
     from stride_b200.parts.latent_attention import LatentAttention
-    monkeypatch.setattr(LatentAttention, "EXPAND_PAIRS", 1)
+    monkeypatch.setattr(LatentAttention, "EXPAND_KEYS", 64)
     calls, run = [], ops.latent_prefill_tc
     monkeypatch.setattr(ops, "latent_prefill_tc", lambda *a, **k: (calls.append(a[7].shape[0]), run(*a, **k))[1])
     return calls
@@ -168,7 +168,7 @@ def test_portions_beside_single_tokens(gpu, models, expansions, monkeypatch, ran
     through the tensor-core kernel, or (a rank it refuses) the exact one, which is given their rows alone."""
     from stride_b200.csrc import ops
     from stride_b200.parts.latent_attention import LatentAttention
-    monkeypatch.setattr(LatentAttention, "EXPAND_PAIRS", 1)
+    monkeypatch.setattr(LatentAttention, "EXPAND_KEYS", 1)
     exact, run = [], ops.latent_attention
     monkeypatch.setattr(ops, "latent_attention", lambda *a, **k: (exact.append(a[0].shape[0]), run(*a, **k))[1])
     case, vocab = models[rank], models[rank].cfg["vocab"]
@@ -185,3 +185,31 @@ def test_portions_beside_single_tokens(gpu, models, expansions, monkeypatch, ran
     assert expansions[-1] == 100 and exact == ([2, 2] if rank == 40 else [])
     for key, rows, at in ((1, range(120, 150), 0), (4, range(70), 30), (2, [89], 100), (3, [39], 101)):
         check(got[at:at + len(rows)], case, tokens[key], list(rows), f"request {key} of the mixed step")
+
+
+def test_the_rule_and_the_byte_limit(gpu, models, expansions, monkeypatch):
+    """Short requests, too many keys beside the longest one's, and a buffer past the limit stay on the latents."""
+    from stride_b200.parts.latent_attention import LatentAttention
+    case = models[48]
+    tokens = {key: seeded_tokens(n, case.cfg["vocab"], 720 + key) for key, n in ((1, 80), (2, 30), (3, 30))}
+
+    def run(expanded, keys=80, share=16, limit=1 << 28):
+        for name, value in (("EXPAND_KEYS", keys), ("EXPAND_SHARE", share), ("MAX_EXPANDED_BYTES", limit)):
+            monkeypatch.setattr(LatentAttention, name, value)
+        engine = engine_for(case)
+        for key, t in tokens.items():
+            open_request(engine, key, len(t))
+        before = len(expansions)
+        got = engine.forward([(key, t, 0, list(range(len(t)))) for key, t in tokens.items()])
+        at = 0
+        for key, t in tokens.items():
+            check(got[at:at + len(t)], case, t, list(range(len(t))), f"request {key}")
+            at += len(t)
+        assert (len(expansions) > before) == expanded
+
+    run(True)
+    run(False, keys=81)
+    run(False, share=1)
+    # 140 keys take a buffer of 2,048 rows of 3 heads of 256 numbers
+    run(True, limit=2048 * 3 * 512)
+    run(False, limit=2048 * 3 * 512 - 1)
