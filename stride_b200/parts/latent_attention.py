@@ -20,8 +20,8 @@ and the output ``W_uv_a (sum_j p_j c_j)``: attention runs on the cached vectors 
 
 That form costs heads * (2 kv_rank + rot_dim) multiply-adds a (query, key) pair, the plain one heads * (dim + rot_dim + value_dim),
 3.4 times less at 128 + 64, 128 and a latent of 512, beside kv_rank * heads * (dim + value_dim) a key to expand it. So portions of prompts
-in bfloat16 expand, where the head sizes are those of the tcgen05 kernel and the queries have no latent (``_expands`` says from how many
-keys on):
+in bfloat16 expand, where the head sizes are those of the tcgen05 kernel (``_expands`` says from how many keys on, ``__init__`` in which
+models):
 
     one product, latent_prepare  as above
     latent_gather                the requests' latents out of their pages
@@ -105,11 +105,11 @@ class LatentAttention(Mixer):
         half = self.rot_dims // 2
         order = [j for i in range(half) for j in (i, i + half)] + list(range(self.rot_dims, self.rot))
         self.rot_order = torch.tensor(order, dtype=torch.long) if self.halves else None
-        # A layer whose queries come through a latent of their own stays on the latents in prompts too. Both forms are as far from 64 bits
-        # (24 passes of the Netusun shape: 0.0055 and 0.0052 where nothing magnifies it), but the design that has such layers divides
-        # by a sum that can vanish further up (the matrix LSTM): what the other rounding changed then grew to 0.03 to 0.06 of the
-        # logits in 4 of those passes, more than two runs of this path may differ by.
-        self._expand = not self.q_rank and ops.latent_prefill_supported(runtime.dtype, self.dim, self.vdim, self.rot, self.rank)
+        # In a model with a matrix LSTM the layer stays on the latents in prompts too. Both forms are as far from 64 bits (layers alone:
+        # 0.0018 of the result each, expanded a hundredth closer), but the matrix LSTM divides by a sum that can vanish: what the other
+        # rounding changed in front of it then grew to 0.03 to 0.06 of the logits in 4 of 24 passes of the Netusun shape, more than
+        # two runs of this path may differ by.
+        self._expand = "mlstm" not in runtime.mixer_kinds and ops.latent_prefill_supported(runtime.dtype, self.dim, self.vdim, self.rot, self.rank)
         self.sizes_by_context = self._expand
         self._fast = ops.latent_tc_supported(runtime.dtype, self.heads, self.rank, self.rot)
 

@@ -22,11 +22,20 @@ from .copies import CopiedStream
 from .runtime import ResidualStream, Runtime
 
 
+def mixer_kinds(spec) -> set:
+    """The kind of a mixer and, of a parallel one, of the branches inside it."""
+    if spec is None:
+        return set()
+    branches = dict(spec.params).get("branches", ()) if spec.kind == "parallel" else ()
+    return {spec.kind}.union(*(mixer_kinds(branch) for branch, _scale in branches))
+
+
 class DecoderModel:
     def __init__(self, spec, runtime: Runtime):
         self.spec = spec
         self.rt = runtime
         self.hidden, self.vocab = spec.hidden, spec.vocab
+        runtime.mixer_kinds = frozenset(kind for layer in spec.layers for kind in mixer_kinds(getattr(layer, "mixer", None)))
         self.embedding = build_part("embedding", spec.embedding_spec(), runtime)
         self.layers = [build_part("layer", ls, runtime) for ls in spec.layers]
         self.final_norm = build_part("norm", spec.final_norm, runtime)

@@ -22,6 +22,9 @@ def sequence_slots(ctx) -> int:
 
 
 class Runtime:
+    # Kinds of the model's mixers (those inside a parallel mixer too), for a part whose form depends on what else the model holds.
+    mixer_kinds: frozenset = frozenset()
+
     def __init__(self, device, dtype: torch.dtype, token_capacity: int, row_capacity: int):
         self.device = torch.device(device)
         self.dtype = dtype

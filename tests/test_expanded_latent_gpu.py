@@ -1,5 +1,6 @@
-"""Latent attention whose portions go over expanded keys and values, as a model and the engine drive it: full portions replayed from
-captured graphs at positions far past the captured one, and a latent layer inside a parallel mixer. Against the plain float64 implementation (``plain_nidilix``)."""
+"""Latent attention whose portions go over expanded keys and values, as a model and the engine drive it: whole prompts, portions
+beside single tokens, the byte limit, full portions replayed from captured graphs at positions far past the captured one, and a
+latent layer inside a parallel mixer. Against the plain float64 implementation (``plain_nidilix``)."""
 
 import dataclasses
 
@@ -145,23 +146,6 @@ def test_a_latent_branch_of_a_parallel_mixer_in_full_portions(gpu, models, expan
     assert expansions and engine.runner.graph_replays == 4
 
 
-def test_weights_are_handed_out_as_they_are_held(gpu, models):
-    """A change to what ``get_weight`` gives is a change to the model, also of the two matrices that one product expands with."""
-    case = models[48]
-    engine = engine_for(case)
-    tokens = seeded_tokens(20, case.cfg["vocab"], 731)
-    open_request(engine, 1, 20)
-    before = engine.forward([(1, tokens, 0, [19])]).clone()
-    for name in ("l0.mix.uk", "l0.mix.uv"):
-        weight = engine.get_weight(name)
-        assert weight.shape == case.state[name].shape and torch.equal(weight.cpu(), case.state[name])
-        weight.zero_()
-        assert not bool(engine.get_weight(name).any())
-        after = engine.forward([(1, tokens, 0, [19])]).clone()
-        assert not torch.equal(before, after)
-        before = after
-
-
 @pytest.mark.parametrize("rank", [48, 40])
 def test_portions_beside_single_tokens(gpu, models, expansions, monkeypatch, rank):
     """A whole prompt; then a portion behind it and another request's first one beside two single tokens, which go over the latents:
@@ -213,3 +197,45 @@ def test_the_rule_and_the_byte_limit(gpu, models, expansions, monkeypatch):
     # 140 keys take a buffer of 2,048 rows of 3 heads of 256 numbers
     run(True, limit=2048 * 3 * 512)
     run(False, limit=2048 * 3 * 512 - 1)
+
+
+def test_weights_are_handed_out_as_they_are_held(gpu, models):
+    """A change to what ``get_weight`` gives is a change to the model, also of the two matrices that one product expands with."""
+    case = models[48]
+    engine = engine_for(case)
+    tokens = seeded_tokens(20, case.cfg["vocab"], 731)
+    open_request(engine, 1, 20)
+    before = engine.forward([(1, tokens, 0, [19])]).clone()
+    for name in ("l0.mix.uk", "l0.mix.uv"):
+        weight = engine.get_weight(name)
+        assert weight.shape == case.state[name].shape and torch.equal(weight.cpu(), case.state[name])
+        weight.zero_()
+        assert not bool(engine.get_weight(name).any())
+        after = engine.forward([(1, tokens, 0, [19])]).clone()
+        assert not torch.equal(before, after)
+        before = after
+
+
+@pytest.mark.parametrize("lstm", [False, True])
+def test_query_latents_expand_unless_the_model_holds_a_matrix_lstm(gpu, expansions, monkeypatch, tmp_models, lstm):
+    import netusun_cases
+    import plain_netusun
+    from stride_b200.parts.latent_attention import LatentAttention
+    monkeypatch.setattr(LatentAttention, "EXPAND_KEYS", 1)
+    layers = [(netusun_cases.latent(3, 128, 64, 128, 48, 32), netusun_cases.dense(72))]
+    if lstm:
+        layers.append((netusun_cases.lstm(2, 24, 16), None))
+    cfg = netusun_cases.config(96, 131, layers)
+    state = netusun_cases.seeded_state(cfg, 47)
+    folder = write_model_dir(str(tmp_models / f"latent_netusun_{lstm}"), cfg, state, torch.bfloat16)
+    case = Case.__new__(Case)
+    case.folder = folder
+    engine = engine_for(case)
+    tokens = seeded_tokens(140, 131, 733)
+    open_request(engine, 1, 140)
+    got = engine.forward([(1, tokens, 0, list(range(0, 140, 7)))]).cpu()
+    assert bool(expansions) == (not lstm)
+    if not lstm:
+        want = plain_netusun.forward(cfg, {k: v.bfloat16().double() for k, v in state.items()}, tokens)[list(range(0, 140, 7))]
+        error = float((got.double() - want).norm() / want.norm())
+        assert error <= 0.03, error         # bfloat16 through one layer; a lost key or rotation changes rows outright
