@@ -24,6 +24,7 @@ namespace stride {
 
 constexpr int kWarps = 4;
 constexpr int kMaxHeadDim = 256;
+constexpr int kMaxTileDim = 128;        // widths of keys and values of the kernel with the keys in shared memory
 
 template <typename T>
 __device__ __forceinline__ float dot_row(const float* __restrict__ q, const T* __restrict__ k, int hd);
@@ -164,7 +165,7 @@ paged_attention_tile_f32_kernel(const float* __restrict__ q, int q_stride, float
                                 const int32_t* __restrict__ seq_of_token, const int32_t* __restrict__ positions, int tokens, int nq, int nkv,
                                 int hd, int vd, int page_size, float scale, int window, float softcap, const float* __restrict__ sinks,
                                 const float* __restrict__ slopes, const float* __restrict__ rel, int rel_len, int GH) {
-    constexpr int THREADS = NW * 32, MAXV = 4;          // vd up to 128
+    constexpr int THREADS = NW * 32, MAXV = kMaxTileDim / 32;
     extern __shared__ __align__(16) float tile_smem[];
     const int kld = hd + 4;
     float* const ks = tile_smem;                        // [2][32][hd + 4]
@@ -317,6 +318,20 @@ paged_attention_tile_f32_kernel(const float* __restrict__ q, int q_stride, float
     }
 }
 
+template <int TQ, int NW, int NR>
+int launch_tiles(const float* q, int q_stride, float* out, const float* k_pages, const float* v_pages, const int32_t* block_table, int table_width,
+                 const int32_t* seq_of_token, const int32_t* positions, int tokens, int nq, int nkv, int hd, int vd, int page_size, float scale,
+                 int window, float softcap, const float* sinks, const float* slopes, const float* rel, int rel_len, int gh, int ctas_y,
+                 cudaStream_t stream) {
+    const auto floats = [](int hd, int vd) { return 2 * 32 * (hd + 4) + 2 * 32 * vd + NW * NR * hd; };
+    const cudaError_t e = allow_shared<paged_attention_tile_f32_kernel<TQ, NW, NR>>(floats(kMaxTileDim, kMaxTileDim) * 4);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    stride::launch(paged_attention_tile_f32_kernel<TQ, NW, NR>, dim3((tokens + TQ - 1) / TQ, ctas_y), dim3(NW * 32), floats(hd, vd) * 4, stream, q,
+                   q_stride, out, k_pages, v_pages, block_table, table_width, seq_of_token, positions, tokens, nq, nkv, hd, vd, page_size, scale,
+                   window, softcap, sinks, slopes, rel, rel_len, gh);
+    return STRIDE_LAUNCH_STATUS();
+}
+
 }  // namespace stride
 
 using namespace stride;
@@ -334,22 +349,17 @@ extern "C" int stride_paged_attention_generic(const void* q, int q_stride, void*
     if (nq % nkv) return STRIDE_BAD_ARGUMENT;
     if (hd > kMaxHeadDim || vd > kMaxHeadDim) return STRIDE_UNSUPPORTED;
     if (tokens == 0) return 0;
-    const bool tile = dtype == STRIDE_DTYPE_F32 && hd % 4 == 0 && vd % 4 == 0 && hd <= 128 && vd <= 128 &&
+    const bool tile = dtype == STRIDE_DTYPE_F32 && hd % 4 == 0 && vd % 4 == 0 && hd <= kMaxTileDim && vd <= kMaxTileDim &&
                       (reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages)) % 16 == 0;
     if (tile) {
         const int gh = min(nq / nkv, 4), ctas_y = nkv * ((nq / nkv + gh - 1) / gh);
         if (ctas_y <= 65535) {
-            auto run = [&](auto kernel, int tq, int rows, int threads) {
-                const int bytes = (2 * 32 * (hd + 4) + 2 * 32 * vd + rows * hd) * 4;
-                const cudaError_t e = bytes > 48 * 1024 ? cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)
-                                                        : cudaSuccess;
-                if (e != cudaSuccess) return static_cast<int>(e);
-                stride::launch(kernel, dim3((tokens + tq - 1) / tq, ctas_y), dim3(threads), bytes, stream, static_cast<const float*>(q), q_stride,
-                               static_cast<float*>(out), static_cast<const float*>(k_pages), static_cast<const float*>(v_pages), block_table, table_width,
-                               seq_of_token, positions, tokens, nq, nkv, hd, vd, page_size, scale, window, softcap, sinks, slopes, rel, rel_len, gh);
-                return STRIDE_LAUNCH_STATUS();
-            };
-            return portions ? run(paged_attention_tile_f32_kernel<8, 8, 4>, 8, 32, 256) : run(paged_attention_tile_f32_kernel<1, 4, 1>, 1, 4, 128);
+            return portions ? launch_tiles<8, 8, 4>(static_cast<const float*>(q), q_stride, static_cast<float*>(out), static_cast<const float*>(k_pages),
+                                                    static_cast<const float*>(v_pages), block_table, table_width, seq_of_token, positions, tokens, nq,
+                                                    nkv, hd, vd, page_size, scale, window, softcap, sinks, slopes, rel, rel_len, gh, ctas_y, stream)
+                            : launch_tiles<1, 4, 1>(static_cast<const float*>(q), q_stride, static_cast<float*>(out), static_cast<const float*>(k_pages),
+                                                    static_cast<const float*>(v_pages), block_table, table_width, seq_of_token, positions, tokens, nq,
+                                                    nkv, hd, vd, page_size, scale, window, softcap, sinks, slopes, rel, rel_len, gh, ctas_y, stream);
         }
     }
     dim3 grid(tokens, (nq + kWarps - 1) / kWarps);

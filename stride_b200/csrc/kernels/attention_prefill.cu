@@ -267,12 +267,8 @@ int launch_prefill(const __nv_bfloat16* q, int q_stride, __nv_bfloat16* out, con
                    const int32_t* q_len, const int32_t* ctx_len, int num_seqs, int max_tiles, int nq, int nkv, int page_size,
                    float scale, int window, float softcap, const float* sinks, const float* slopes, const float* rel, int rel_len, cudaStream_t stream) {
     const int smem = 2 * 2 * kKTile * HD * 2;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(paged_prefill_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return static_cast<int>(e);
-        configured = true;
-    }
+    const cudaError_t e = allow_shared<paged_prefill_kernel<HD>>(smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
     dim3 grid(max_tiles, nq);
     stride::launch(paged_prefill_kernel<HD>, dim3(grid), dim3(128), smem, stream, q, q_stride, out, k_pages, v_pages, block_table, table_width, q_start,
                                                           q_len, ctx_len, num_seqs, nq, nkv, page_size,

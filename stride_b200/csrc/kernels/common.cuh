@@ -13,6 +13,8 @@
 
 #include <cstdlib>
 
+#include "shared_limit.hpp"
+
 #define STRIDE_DTYPE_F32 0
 #define STRIDE_DTYPE_BF16 1
 

@@ -497,12 +497,8 @@ int launch_warps(const CUtensorMap* map_w, const CUtensorMap* map_x, const CUten
     constexpr int smem = (TMA ? (CH == 1 ? ring_stages(NT, MT, WARPS) : kPairStages) * WARPS * CH * (MT * 2048 + NT * 1024)
                               : ring_stages(NT, MT, WARPS) * kUnroll * (2 * MT + NT) * WARPS * 32 * 16) + 1024;
     auto kernel = gemm_stream_kernel<NT, MT, WARPS, MODE, TMA, CH>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return static_cast<int>(e);
-        configured = true;
-    }
+    const cudaError_t e = allow_shared<gemm_stream_kernel<NT, MT, WARPS, MODE, TMA, CH>>(smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
     static const CUtensorMap no_map = {};
     stride::launch(kernel, dim3(static_cast<unsigned>(ctas)), dim3(WARPS * 32), smem, stream, TMA ? *map_w : no_map, TMA ? *map_x : no_map,
                    CH > 1 ? *map_w2 : no_map, CH > 1 ? *map_x2 : no_map,

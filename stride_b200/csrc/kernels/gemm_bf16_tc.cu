@@ -365,13 +365,9 @@ int launch(const CUtensorMap* map_a, const CUtensorMap* map_b, OutT* out, int ld
            float* partials, int* tickets, int* status, cudaStream_t stream, const float* norm_partials = nullptr, int norm_count = 0,
            float norm_eps = 0.f, int act = 0, float act_limit = 0.f, float act_alpha = 1.f) {
     constexpr int smem = STAGES * (kBlockM * kBlockK * 2 + BLOCK_N * kBlockK * 2) + 1024;
-    static bool configured = false;
     auto kernel = gemm_tn_bf16_kernel<BLOCK_N, STAGES, TRANSPOSED, TRANSPOSED, OutT, GATED>;   // swapped use: A holds weights
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return static_cast<int>(e);
-        configured = true;
-    }
+    const cudaError_t e = allow_shared<gemm_tn_bf16_kernel<BLOCK_N, STAGES, TRANSPOSED, TRANSPOSED, OutT, GATED>>(smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
     const int k_blocks = (K + kBlockK - 1) / kBlockK;
     const int per_split = (k_blocks + splits - 1) / splits;
     dim3 grid((M + kBlockM - 1) / kBlockM, (N + BLOCK_N - 1) / BLOCK_N, splits);

@@ -272,8 +272,8 @@ struct Args {
 template <int MT, int STAGES>
 int run_stream(const Args& g, cudaStream_t stream) {
     constexpr int bytes = (STAGES * (16 + MT) * (PARTS * 32 + 4) + PARTS * MT * 16) * 4, fit = 220 * 1024 / (bytes + 1024);
-    static const cudaError_t set = cudaFuncSetAttribute(gemm_nt_f32_stream_kernel<MT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (set != cudaSuccess) return static_cast<int>(set);
+    const cudaError_t e = allow_shared<gemm_nt_f32_stream_kernel<MT, STAGES>>(bytes);
+    if (e != cudaSuccess) return static_cast<int>(e);
     const int grid = min((g.N + 15) / 16, 148 * fit);
     stride::launch(gemm_nt_f32_stream_kernel<MT, STAGES>, dim3(grid), dim3(128), bytes, stream, g.A, g.W, g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc);
     return STRIDE_LAUNCH_STATUS();

@@ -467,7 +467,7 @@ int stride_head_gemm(const void* A, int lda, int a_hs, const void* B, long long 
         if (wide) {
             constexpr int bytes = 2 * kWideStage * 2;
             const auto kernel = b_ks == 1 ? head_gemm_wide_kernel<false> : head_gemm_wide_kernel<true>;
-            const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            const cudaError_t e = b_ks == 1 ? allow_shared<head_gemm_wide_kernel<false>>(bytes) : allow_shared<head_gemm_wide_kernel<true>>(bytes);
             if (e != cudaSuccess) return static_cast<int>(e);
             stride::launch(kernel, dim3((N + WN - 1) / WN, heads, (M + WM - 1) / WM), dim3(256), bytes, stream, static_cast<const __nv_bfloat16*>(A), lda, a_hs,
                            static_cast<const __nv_bfloat16*>(B), b_hs, static_cast<int>(b_ld), static_cast<__nv_bfloat16*>(C), ldc, c_hs,
