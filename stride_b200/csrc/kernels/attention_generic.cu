@@ -156,8 +156,8 @@ paged_attention_generic_kernel(const T* __restrict__ q, int q_stride, T* __restr
 // key head, a warp NR of those (token, head) rows; 32 keys and values at a time come in by cp.async, the next ones while these are
 // worked through, and serve every row. A lane's chain over a key's numbers, the online softmax over a group of 32 keys and the order
 // of the values are those of the kernel above, so every row has the same bits whichever ran it. Bound by the chains: head size 128
-// costs 512 cycles a group, NR of them side by side. 301 tokens of 24 heads: 64 us (above: 175 us, where every (token, head) reads its
-// keys itself, lane by lane, and waits for every page number), two single tokens behind 151: 34 us (87).
+// costs 512 cycles a group, NR of them side by side. A prompt of 301 tokens, 24 heads on 8: 109 us (above: 342 us, where every (token, head)
+// reads its keys itself, lane by lane, and waits for every page number), a single token behind 151: 33 us (84).
 template <int TQ, int NW, int NR>
 __global__ void __launch_bounds__(NW * 32)
 paged_attention_tile_f32_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out, const float* __restrict__ k_pages,
@@ -337,8 +337,8 @@ int launch_tiles(const float* q, int q_stride, float* out, const float* k_pages,
 using namespace stride;
 
 // q: [tokens, q_stride] with head h at columns [h*hd, (h+1)*hd); out: [tokens, nq, vd];
-// key pages: [num_pages, nkv, page_size, hd], value pages the same with vd; block_table: [seqs, table_width]. portions: 0 where
-// (nearly) every row belongs to another request; the results are the same.
+// key pages: [num_pages, nkv, page_size, hd], value pages the same with vd; block_table: [seqs, table_width]. portions: which
+// kernel a 32-bit step takes, 0 a row a CTA, 1 eight rows a CTA, 2 a (row, head) a warp; the results are the same.
 extern "C" int stride_paged_attention_generic(const void* q, int q_stride, void* out, const void* k_pages, const void* v_pages,
                                               const int32_t* block_table, int table_width, const int32_t* seq_of_token,
                                               const int32_t* positions, int tokens, int nq, int nkv, int hd, int vd, int page_size,
@@ -349,7 +349,9 @@ extern "C" int stride_paged_attention_generic(const void* q, int q_stride, void*
     if (nq % nkv) return STRIDE_BAD_ARGUMENT;
     if (hd > kMaxHeadDim || vd > kMaxHeadDim) return STRIDE_UNSUPPORTED;
     if (tokens == 0) return 0;
-    const bool tile = dtype == STRIDE_DTYPE_F32 && hd % 4 == 0 && vd % 4 == 0 && hd <= kMaxTileDim && vd <= kMaxTileDim &&
+    // a warp reads its keys in packs of 16 bytes where a row is whole packs
+    if (hd % (dtype == STRIDE_DTYPE_F32 ? 4 : 8) == 0 && reinterpret_cast<uintptr_t>(k_pages) % 16) return STRIDE_UNSUPPORTED;
+    const bool tile = portions != 2 && dtype == STRIDE_DTYPE_F32 && hd % 4 == 0 && vd % 4 == 0 && hd <= kMaxTileDim && vd <= kMaxTileDim &&
                       (reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages)) % 16 == 0;
     if (tile) {
         const int gh = min(nq / nkv, 4), ctas_y = nkv * ((nq / nkv + gh - 1) / gh);

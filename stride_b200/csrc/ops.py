@@ -1822,15 +1822,43 @@ def _rel_args(rel, nq: int) -> tuple:
     return _dev(rel, "rel", torch.float32), rel.shape[1]
 
 
+# Kernels of ``paged_attention`` in 32 bits: a row a CTA, eight neighbouring rows a CTA, a (row, head) a warp.
+EXACT_ROWS, EXACT_TILES, EXACT_WARPS = 0, 1, 2
+
+
+def exact_attention_form(tokens: int, longest: int, keys: int, nq: int, nkv: int, hd: int, vd: int) -> int:
+    """The kernel for ``tokens`` neighbouring rows of requests that bring at most ``longest`` tokens each and hold at most ``keys``. A
+    row a CTA is fastest while its CTAs run at once; eight rows a CTA read keys once for all of them, but walk the runs of several
+    requests one after the other; a warp a (row, head) keeps the most warps in flight, which counts where keys are few or, with one or
+    two query heads a key head, single rows many. In us, rows / tiles / warps, head size 128: 24 query heads on 8 key heads, one request
+    of 8 tokens 6 / 12 / 9, 16 of 8 tokens 15 / 14 / 11, the same behind 300 tokens 213 / 103 / 300, 200 tokens 124 / 72 / 177; 32 on 32, 16
+    requests of 16 tokens 87 / 43 / 27, 8 tokens of each behind 300 681 / 173 / 388. (A captured step of single tokens gives its context
+    bucket as ``keys``: with few keys it loses up to 10 us a layer of 32 key heads to the warps.)"""
+    group = nq // nkv
+    ctas = tokens * nkv * -(-group // 4)
+    per_sm = 227 * 1024 // ((64 * (hd + 4) + 64 * vd + 4 * hd) * 4 + 1024)         # of a row each, by their shared memory
+    wave = 148 * max(1, min(16, per_sm))
+    if ctas <= 444 or (longest < 8 and ctas <= wave):
+        return EXACT_ROWS
+    if longest >= 8:
+        few = keys <= (48 if group == 1 else 32) and (longest < 16 or (group <= 2 and ctas > 7000))
+        return EXACT_WARPS if few else EXACT_TILES
+    if keys <= (96 if group <= 2 else 32):
+        return EXACT_WARPS
+    if group <= 2 and ctas > 4.7 * wave:
+        return EXACT_TILES if longest >= 4 else EXACT_WARPS
+    return EXACT_ROWS
+
+
 def paged_attention(q, q_stride: int, out, k_pages, v_pages, block_table, seq_of_token, positions, nq: int, nkv: int,
                     hd: int, page_size: int, scale: float, window: int = 0, softcap: float = 0.0, sinks=None, slopes=None,
-                    vd: int | None = None, rel=None, portions: bool = False) -> None:
+                    vd: int | None = None, rel=None, portions: int = 0) -> None:
     """Attention of every token in the flat batch over its request's pages.
     ``q`` holds head h of token t at ``q[t * q_stride + h * hd]``. ``softcap`` c > 0 caps the scaled scores at
     c tanh(s / c); ``sinks`` (float32 [nq]) adds exp(sink) of the head to the softmax's denominator; ``slopes`` (float32
     [nq]) takes slope_h times the key's distance off every score; ``vd`` is the values' width where it is not ``hd``;
-    ``rel`` (float32 [nq, n]) adds ``rel[h, min(distance, n - 1)]`` to every score of head h. ``portions``: neighbouring
-    tokens mostly belong to one request (only the time depends on it)."""
+    ``rel`` (float32 [nq, n]) adds ``rel[h, min(distance, n - 1)]`` to every score of head h. ``portions``: the kernel in
+    32 bits (``exact_attention_form``; only the time depends on it)."""
     tokens = out.shape[0]
     vd = hd if vd is None else int(vd)
     if out.shape[1] != nq * vd or k_pages.shape[-1] != hd or v_pages.shape[-1] != vd:
@@ -1839,7 +1867,7 @@ def paged_attention(q, q_stride: int, out, k_pages, v_pages, block_table, seq_of
         _dev(q, "q"), q_stride, _dev(out, "out"), _dev(k_pages, "k_pages"), _dev(v_pages, "v_pages"),
         _dev(block_table, "block_table", torch.int32), block_table.shape[1], _dev(seq_of_token, "seq_of_token", torch.int32),
         _dev(positions, "positions", torch.int32), tokens, nq, nkv, hd, vd, page_size, float(scale), int(window), float(softcap),
-        _opt(sinks, "sinks", torch.float32), _opt(slopes, "slopes", torch.float32), *_rel_args(rel, nq), 1 if portions else 0,
+        _opt(sinks, "sinks", torch.float32), _opt(slopes, "slopes", torch.float32), *_rel_args(rel, nq), int(portions),
         _code(q.dtype), _stream()), "paged_attention")
 
 

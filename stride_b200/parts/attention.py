@@ -480,9 +480,12 @@ class PagedAttention(Mixer):
         geometry = (self.nq, self.nkv, self.hd, cache.page_size, self.scale, self.window)
         if not self._fast:
             # the exact kernel: the whole 32-bit path, and bfloat16 sizes the tensor-core kernels refuse
-            ops.paged_attention(qkv, self.qkv_dim, attn, cache.k_pages, cache.v_pages, table, ctx.seq_of_token[:tokens],
-                                ctx.positions[:tokens], *geometry, self.softcap, self.sinks, self.slopes, self.vd, self.rel,
-                                portions=ctx.max_q_len >= 8)
+            split = min(ctx.decode_tail_start, tokens) if qkv.dtype == torch.float32 else 0     # portions before, single tokens after
+            for lo, hi, longest in ((0, split, ctx.max_q_len), (split, tokens, 1)):
+                if hi > lo:
+                    ops.paged_attention(qkv[lo:hi], self.qkv_dim, attn[lo:hi], cache.k_pages, cache.v_pages, table, ctx.seq_of_token[lo:hi],
+                                        ctx.positions[lo:hi], *geometry, self.softcap, self.sinks, self.slopes, self.vd, self.rel,
+                                        portions=ops.exact_attention_form(hi - lo, longest, ctx.context_bound, self.nq, self.nkv, self.hd, self.vd))
             return tokens
         split = min(ctx.decode_tail_start, tokens)          # portions before, single decoded tokens after
         if split > 0:

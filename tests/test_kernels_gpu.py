@@ -1101,3 +1101,43 @@ def test_attention_f32_in_tiles_gives_the_bits_of_single_rows(ops, nq, nkv, hd, 
     assert torch.equal(outs[0], outs[1]) and float(outs[0][tokens].abs().max()) == 0.0
     if not rules:
         close(outs[0][:tokens], want.reshape(tokens, -1), torch.float32)
+
+
+
+@pytest.mark.parametrize("nq,nkv,hd,window,rules", [(4, 2, 32, 0, False), (6, 1, 128, 40, True), (3, 3, 4, 0, True), (5, 1, 100, 33, False), (3, 3, 128, 0, False)])
+def test_attention_f32_has_the_same_bits_in_every_kernel(ops, nq, nkv, hd, window, rules):
+    """The kernels with the keys in shared memory (a row a CTA, eight rows a CTA) against the warp a (row, head): asked for, and taken because
+    the values do not start on 16 bytes. Keys that do not are refused where a row is read in packs of 16 bytes."""
+    g = torch.Generator().manual_seed(nq * hd + 1)
+    page = 8
+    q, k_pages, v_pages, table, seq_of, pos, _want = _paged_case(g, torch.float32, [(0, 100), (40, 9), (131, 1), (7, 1), (0, 33), (64, 2)], nq, nkv, hd,
+                                                                 page, window or None)
+    tokens = q.shape[0]
+    extra = dict(softcap=20.0, sinks=dev(torch.randn(nq, generator=g)), slopes=dev(torch.rand(nq, generator=g) * 0.1)) if rules else {}
+
+    def shifted(t):
+        room = torch.empty(t.numel() + 1, device="cuda")
+        return room[1:].view(t.shape).copy_(t)
+
+    def run(k, v, form):
+        out = torch.full((tokens, nq * hd), float("nan"), device="cuda")
+        ops.paged_attention(dev(q), nq * hd, out, k, v, dev(table), dev(seq_of), dev(pos), nq, nkv, hd, page, hd ** -0.5, window, portions=form, **extra)
+        return out
+
+    want = run(dev(k_pages), dev(v_pages), ops.EXACT_WARPS)
+    for form in (ops.EXACT_ROWS, ops.EXACT_TILES):
+        assert torch.equal(run(dev(k_pages), dev(v_pages), form), want)
+        assert torch.equal(run(dev(k_pages), shifted(v_pages), form), want)
+    with pytest.raises(ops.KernelError):
+        run(shifted(k_pages), dev(v_pages), ops.EXACT_TILES)
+
+
+def test_the_exact_attention_of_a_mixed_step_is_chosen_by_what_its_rows_hold(ops):
+    """Single tokens beside a portion never go eight requests to a CTA, and the choice follows rows, keys and query heads a key head."""
+    form = ops.exact_attention_form
+    for nq, nkv, hd in ((24, 8, 128), (32, 32, 128), (32, 32, 64), (4, 1, 32)):
+        assert all(form(n, 1, keys, nq, nkv, hd, hd) != ops.EXACT_TILES for n in (1, 20, 64, 256) for keys in (5, 300, 8192))
+        assert form(1, 1, 8192, nq, nkv, hd, hd) == ops.EXACT_ROWS
+        assert form(2048, 2048, 2048, nq, nkv, hd, hd) == ops.EXACT_TILES
+    assert form(16 * 8, 8, 8, 32, 32, 128, 128) == ops.EXACT_WARPS and form(16 * 8, 8, 308, 32, 32, 128, 128) == ops.EXACT_TILES
+    assert form(128, 1, 2048, 32, 32, 128, 128) == ops.EXACT_WARPS and form(128, 1, 2048, 24, 8, 128, 128) == ops.EXACT_ROWS
