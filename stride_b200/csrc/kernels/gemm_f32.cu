@@ -136,7 +136,13 @@ __device__ __forceinline__ float4 load_cluster_f4(const float* local, uint32_t r
     return v;
 }
 
-template <int BM, int BN, int TN, bool VEC>
+// ALONE: up to 128 columns a part is one tile of 16, and where the outputs alone fill the device a cluster's exchange is most of the time:
+// one CTA then takes all parts and adds them up as they come. 1,024 rows of 2048 x 64 11 us, 32 in clusters; 301 rows of 1000 x 33 5.6 and
+// 8.0; with fewer tiles than 64 both are level (100 rows 5.4 us) and from 65 columns on the clusters win by the parts side by side.
+// One tile of K has no parts to spread.
+__device__ __forceinline__ void add2(uint64_t& total, uint64_t part) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(total) : "l"(part)); }
+
+template <int BM, int BN, int TN, bool VEC, bool ALONE>
 __global__ void __launch_bounds__(BM / 8 * (BN / TN)) gemm_nt_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W,
                                                                               float* __restrict__ C, int M, int N, int K, int lda, int ldw,
                                                                               int ldc) {
@@ -151,7 +157,7 @@ __global__ void __launch_bounds__(BM / 8 * (BN / TN)) gemm_nt_f32_tile_kernel(co
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int row = (warp / WARPS_N) * 32 + (lane >> 3) * 4, col = (warp % WARPS_N) * WN + (lane & 7) * 4;
-    const int L = part_length(K), part = blockIdx.z, k_first = part * L, k_end = min(K, k_first + L);
+    const int L = part_length(K), part = blockIdx.z, k_first = ALONE ? 0 : part * L, k_end = ALONE ? K : min(K, k_first + L);
 
     auto fetch = [&](const float* __restrict__ from, int ld, int r, int limit, int k) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -196,6 +202,7 @@ __global__ void __launch_bounds__(BM / 8 * (BN / TN)) gemm_nt_f32_tile_kernel(co
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0;
+    uint64_t total[ALONE ? 8 : 1][ALONE ? TN / 2 : 1];
     fetch_w(k_first);
     pdl_wait();
     fetch_a(k_first);
@@ -226,6 +233,16 @@ __global__ void __launch_bounds__(BM / 8 * (BN / TN)) gemm_nt_f32_tile_kernel(co
                 for (int j = 0; j < TN / 2; ++j) fma2(acc[i][j], aa, w[j]);
             }
         }
+        if constexpr (ALONE) {  // the end of a part (a part without columns adds zero, which only makes -0 a 0)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < TN / 2; ++j) {
+                    if (k0 == 0) total[i][j] = acc[i][j];
+                    else add2(total[i][j], acc[i][j]);
+                    acc[i][j] = 0;
+                }
+        }
         if (more) {
             put(b ^ 1);         // last read one step ago, ahead of the barrier that ended it
             __syncthreads();
@@ -233,23 +250,42 @@ __global__ void __launch_bounds__(BM / 8 * (BN / TN)) gemm_nt_f32_tile_kernel(co
         }
     }
     __syncthreads();
+    if constexpr (ALONE) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < TN / 2; ++j) {
+                acc[i][j] = total[i][j];
+                if (K <= (PARTS - 1) * BK) add2(acc[i][j], 0);
+            }
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < TN / 4; ++j)
             *reinterpret_cast<ulonglong2*>(smem + (row + (i & 3) + (i >> 2) * 16) * LDS + col + 32 * j) = make_ulonglong2(acc[i][2 * j], acc[i][2 * j + 1]);
-    cluster_arrive();
-    cluster_wait();
+    if constexpr (ALONE) {
+        __syncthreads();
+    } else {
+        cluster_arrive();
+        cluster_wait();
+    }
     const bool wide = (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
-    for (int o = tid; o < BM / PARTS * (BN / 4); o += THREADS) {
-        const int r = part * (BM / PARTS) + o / (BN / 4), c = o % (BN / 4) * 4, m = m0 + r, n = n0 + c;
+    constexpr int ROWS = ALONE ? BM : BM / PARTS;
+    for (int o = tid; o < ROWS * (BN / 4); o += THREADS) {
+        const int r = (ALONE ? 0 : part * ROWS) + o / (BN / 4), c = o % (BN / 4) * 4, m = m0 + r, n = n0 + c;
         if (m >= M || n >= N) continue;
-        float4 v[PARTS];
+        float4 t;
+        if constexpr (ALONE) {
+            t = *reinterpret_cast<const float4*>(smem + r * LDS + c);
+        } else {
+            float4 v[PARTS];
 #pragma unroll
-        for (int p = 0; p < PARTS; ++p) v[p] = load_cluster_f4(smem + r * LDS + c, p);
-        float4 t = v[0];
+            for (int p = 0; p < PARTS; ++p) v[p] = load_cluster_f4(smem + r * LDS + c, p);
+            t = v[0];
 #pragma unroll
-        for (int p = 1; p < PARTS; ++p) { t.x += v[p].x; t.y += v[p].y; t.z += v[p].z; t.w += v[p].w; }
+            for (int p = 1; p < PARTS; ++p) { t.x += v[p].x; t.y += v[p].y; t.z += v[p].z; t.w += v[p].w; }
+        }
         float* const out = C + static_cast<size_t>(m) * ldc + n;
         if (wide && n + 3 < N) {
             *reinterpret_cast<float4*>(out) = t;
@@ -259,8 +295,10 @@ __global__ void __launch_bounds__(BM / 8 * (BN / TN)) gemm_nt_f32_tile_kernel(co
                 if (n + i < N) out[i] = e[i];
         }
     }
-    cluster_arrive();           // a CTA's shared memory stays until the others have read it
-    cluster_wait();
+    if constexpr (!ALONE) {
+        cluster_arrive();       // a CTA's shared memory stays until the others have read it
+        cluster_wait();
+    }
 }
 
 struct Args {
@@ -283,8 +321,14 @@ template <int BM, int BN, int TN>
 int run_tile(const Args& g, bool vec, cudaStream_t stream) {
     const dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, PARTS), block(BM / 8 * (BN / TN));
     if (grid.y > 65535) return STRIDE_UNSUPPORTED;
-    if (vec) stride::launch_clusters(gemm_nt_f32_tile_kernel<BM, BN, TN, true>, grid, block, 0, stream, PARTS, g.A, g.W, g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc);
-    else stride::launch_clusters(gemm_nt_f32_tile_kernel<BM, BN, TN, false>, grid, block, 0, stream, PARTS, g.A, g.W, g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc);
+    if (g.K <= 16 || (g.K <= PARTS * 16 && static_cast<long long>(grid.x) * grid.y >= 64)) {
+        const dim3 one(grid.x, grid.y);
+        if (vec) stride::launch(gemm_nt_f32_tile_kernel<BM, BN, TN, true, true>, dim3(one), dim3(block), 0, stream, g.A, g.W, g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc);
+        else stride::launch(gemm_nt_f32_tile_kernel<BM, BN, TN, false, true>, dim3(one), dim3(block), 0, stream, g.A, g.W, g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc);
+        return STRIDE_LAUNCH_STATUS();
+    }
+    if (vec) stride::launch_clusters(gemm_nt_f32_tile_kernel<BM, BN, TN, true, false>, grid, block, 0, stream, PARTS, g.A, g.W, g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc);
+    else stride::launch_clusters(gemm_nt_f32_tile_kernel<BM, BN, TN, false, false>, grid, block, 0, stream, PARTS, g.A, g.W, g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc);
     return STRIDE_LAUNCH_STATUS();
 }
 
@@ -297,13 +341,14 @@ extern "C" int stride_gemm_nt_f32(const float* A, const float* W, float* C, int 
     if (M == 0) return 0;
     const stride::f32::Args g{A, W, C, M, N, K, lda, ldw, ldc};
     const bool vec = (K & 3) == 0 && (lda & 3) == 0 && (ldw & 3) == 0 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
-    if (vec && M <= 16) {
+    if (vec && (M <= 4 || (M <= 16 && K > 16))) {
         if (M == 1) return stride::f32::run_stream<1, 6>(g, stream);
         if (M == 2) return stride::f32::run_stream<2, 5>(g, stream);
         if (M <= 4) return stride::f32::run_stream<4, 5>(g, stream);
         if (M <= 8) return stride::f32::run_stream<8, 4>(g, stream);
         return stride::f32::run_stream<16, 3>(g, stream);
     }
+    // (a row of W of one tile of K and 5 to 16 rows of A: tiles, 2.5 us for 16 rows of 2048 x 16, 3.5 streamed)
     // 3072 x 3072 in us, 32 x 64 (4 columns a thread) / 64 x 64 (4) / 64 x 64 (8): 20 rows 41 / 45 / 55, 48 rows 53 / 47 / 55,
     // 100 rows 79 / 68 / 62, 301 rows 172 / 146 / 148; 16384 x 3072: 102 / 148 / 148, 180 / 154 / 150, 348 / 296 / 277, 849 / 721 / 664
     if (M <= 32) return stride::f32::run_tile<32, 64, 4>(g, vec, stream);

@@ -1103,6 +1103,11 @@ def test_attention_f32_in_tiles_gives_the_bits_of_single_rows(ops, nq, nkv, hd, 
         close(outs[0][:tokens], want.reshape(tokens, -1), torch.float32)
 
 
+@pytest.mark.parametrize("n,k", [(2500, 4), (2500, 33), (1300, 112), (1300, 113), (2500, 128), (1000, 16), (70, 12)])
+def test_gemm_f32_gives_the_same_bits_for_short_k(ops, n, k):
+    """Up to 128 columns one CTA adds up all parts where the outputs fill the device, a cluster does elsewhere: with 131 rows and with few."""
+    test_gemm_f32_gives_the_same_bits_in_every_kernel(ops, n, k)
+
 
 @pytest.mark.parametrize("nq,nkv,hd,window,rules", [(4, 2, 32, 0, False), (6, 1, 128, 40, True), (3, 3, 4, 0, True), (5, 1, 100, 33, False), (3, 3, 128, 0, False)])
 def test_attention_f32_has_the_same_bits_in_every_kernel(ops, nq, nkv, hd, window, rules):
