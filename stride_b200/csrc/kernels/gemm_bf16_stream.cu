@@ -31,11 +31,13 @@ namespace stream_gemm {
 constexpr int kStepCols = 32;    // columns of K per warp step (a quad's four 16-byte pieces)
 constexpr int kUnroll = 2;       // steps per batch (one cp.async group)
 // 16-row tiles per CTA at most: five hold an 148th of 11,840 rows (with four a gate/up matrix of 11,008 rows went in 172 CTAs, two
-// rounds: 14.7 us a product of 2,048 columns against 10.3). With 9 to 16 tokens four: the ring and the partial sums of five do not fit.
+// rounds: 13.1 us a product of 2,048 columns and 3 tokens, back to back, against 7.9). With 9 to 16 tokens four: the ring and the
+// partial sums of five do not fit.
 constexpr int max_row_tiles(int nt) { return nt == 1 ? 5 : 4; }
 
-// Stages of two pieces of K, for up to kPairTiles row tiles. (2048 x 2048: 4.4 us among the kernels of a step, 5.5 piece by piece;
-// steps of the 2048-wide designs 3 to 9 % faster, the most at K = 8256. With two row tiles the ring is too coarse: the 8B layers lose 1.5 % a step.)
+// Stages of two pieces of K, for up to kPairTiles row tiles. (Back to back with 3 tokens, in pairs / piece by piece: 2048 x 2048 3.0 / 3.4 us,
+// 2048 x 5504 5.8 / 9.6, 2048 x 8256 7.8 / 15.0; a decode step of three requests of the Dopudra design 324 / 403 us. With two row tiles
+// the ring is too coarse: the 8B layers lose 1.5 % a step.)
 constexpr int kPairStages = 2;
 constexpr int kPairTiles = 1;
 
@@ -220,10 +222,11 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int my_turns = k_pieces > warp ? (k_pieces - warp + WARPS - 1) / WARPS : 0;
     const int whole = CH == 1 ? my_turns : k / (64 * WARPS), whole_stages = (whole + CH - 1) / CH;
     const int my_stages = whole_stages + (my_turns > whole ? 1 : 0);
-    // Stages asked for at a time. A warp whose share of K fits the ring has all of it on the way at once (K = 2048: 5.8 against 6.4 us
-    // for a 2048 x 2048 matrix among the kernels of a step; K = 4096: a step of the 8B layers 1 % faster); a longer one leaves a stage
-    // free (K = 8256: 9.3 us, with all four 11.3).
-    const int ahead = my_stages <= 2 * STAGES ? STAGES : STAGES - 1;
+    // Stages asked for at a time. The two stages of the paired ring both, or nothing is on the way while one is worked through (2048 x 8256
+    // back to back: 3 tokens 7.8 us, 16 tokens 8.3; with one of them 11.8 and 11.9). Of single pieces a warp whose share of K fits the
+    // ring twice has a whole ring on the way (4096 x 4096, two row tiles: 6.5 us, 6.9 with a stage left free); a longer one leaves a
+    // stage free.
+    const int ahead = CH > 1 || my_stages <= 2 * STAGES ? STAGES : STAGES - 1;
     unsigned char* my_ring = ring_bytes + warp * STAGES * STAGE_BYTES;
     bool alive = true;                                      // false once a bounded wait has run out
     auto request_stage = [&](int i, bool weights, bool tokens) {
