@@ -205,8 +205,8 @@ head_gemm_tc_kernel(const __nv_bfloat16* __restrict__ A, int lda, int a_hs, cons
 
 // The same for portions: 128 tokens x 128 columns a CTA, eight warps of 64 x 32, 64 columns of K at a time by cp.async, twice buffered;
 // weights whose output index is the contiguous one stay as they lie and are read with transposing fragment loads (the kernel above takes them
-// number by number). The terms come in the same order, so the bits are the same. 2,048 tokens of 16 heads, 128 x 512 and
-// 512 x 128: at most 31 us each, 243 with the tiles of 64 x 64.
+// number by number). The terms come in the same order, so the bits are the same. 2,048 tokens of 16 heads, back to back: to 512
+// columns from 128 24 us, 108 in tiles of 64 x 64; to 128 from 512 19 us and 48.
 constexpr int WM = 128, WN = 128, WLD = TK + 8, WLDT = WN + 8;
 constexpr int kWideStage = WM * WLD + (WN * WLD > TK * WLDT ? WN * WLD : TK * WLDT);       // elements
 template <bool N_CONTIGUOUS>
@@ -461,7 +461,11 @@ int stride_head_gemm(const void* A, int lda, int a_hs, const void* B, long long 
                        ldg, g_hs, g_ns, M, N, K);
     else if (dtype == STRIDE_DTYPE_BF16) {
         const long long b_ld = b_ns == 1 ? b_ks : b_ns;
-        const bool wide = M >= 128 && (b_ns == 1 || b_ks == 1) && K % 8 == 0 && N % 8 == 0 && lda % 8 == 0 && a_hs % 8 == 0 && b_hs % 8 == 0 && b_ld % 8 == 0 &&
+        // A CTA of the wide kernel walks K alone: where K is long, lies contiguous (which the narrow kernel reads well too) and the tiles are
+        // few, the narrow one's many CTAs win. 16 heads, to 128 columns from 512, wide / narrow: 128 tokens 12.5 / 9.8 us, 512 13.4 / 12.9,
+        // 1,024 17.5 / 24.6; to 512 from 128, 128 tokens, 5.7 / 6.6.
+        const long long wide_ctas = static_cast<long long>((N + WN - 1) / WN) * heads * ((M + WM - 1) / WM);
+        const bool wide = M >= 128 && (b_ns == 1 || K <= 128 || wide_ctas >= 128) && (b_ns == 1 || b_ks == 1) && K % 8 == 0 && N % 8 == 0 && lda % 8 == 0 && a_hs % 8 == 0 && b_hs % 8 == 0 && b_ld % 8 == 0 &&
                           ldc % 2 == 0 && c_hs % 2 == 0 && (reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) % 16 == 0 &&
                           reinterpret_cast<uintptr_t>(C) % 4 == 0;
         if (wide) {

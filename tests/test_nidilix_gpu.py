@@ -462,3 +462,25 @@ def test_per_head_products_of_portions_have_the_bits_of_short_ones(gpu, n, k, n_
         f = torch.sigmoid(gates[:, 8:].double())
         want = want * (f[:, :heads, None] if gate == "head" else f.view(tokens, heads, n))
     close(whole, want.reshape(tokens, -1), 1e-2)
+
+
+@pytest.mark.parametrize("gate", [None, "head"])
+def test_per_head_products_of_portions_with_a_long_k(gpu, gate):
+    """Enough tiles for the 128-wide kernel at more than 128 terms that lie as K does: the bits of launches of 64 rows."""
+    from stride_b200.csrc import ops
+    heads, tokens, n, k = 3, 2817, 136, 200
+    g = torch.Generator().manual_seed(77)
+    a = torch.randn(tokens, heads * k, generator=g).bfloat16().cuda()
+    b = torch.randn(heads, n, k, generator=g).bfloat16().cuda()
+    gates = torch.randn(tokens, 8, generator=g).bfloat16().cuda()
+    def run(lo, hi):
+        c = torch.full((hi - lo + 1, heads * n), 7.0, dtype=torch.bfloat16, device="cuda")
+        ops.head_gemm(a[lo:hi], heads * k, k, b, n * k, 1, k, c, heads * n, n, hi - lo, heads, n, k, gate=None if gate is None else gates[lo:hi], ldg=8, gate_off=3)
+        assert bool((c[hi - lo] == 7.0).all())
+        return c[:hi - lo]
+    whole = run(0, tokens)
+    assert torch.equal(whole, torch.cat([run(lo, min(tokens, lo + 64)) for lo in range(0, tokens, 64)]))
+    want = torch.einsum("thk,hnk->thn", a.double().view(tokens, heads, k), b.double())
+    if gate is not None:
+        want = want * torch.sigmoid(gates[:, 3:6].double())[:, :, None]
+    close(whole, want.reshape(tokens, -1), 1e-2)
