@@ -484,3 +484,14 @@ def test_per_head_products_of_portions_with_a_long_k(gpu, gate):
     if gate is not None:
         want = want * torch.sigmoid(gates[:, 3:6].double())[:, :, None]
     close(whole, want.reshape(tokens, -1), 1e-2)
+
+
+@pytest.mark.parametrize("tokens,blocks,bw", [(66, 1, 130), (65, 2, 200), (1100, 3, 72), (1099, 3, 72), (1070, 3, 72)])
+def test_recurrent_gates_at_the_edges_of_the_tensor_core_form(gpu, tokens, blocks, bw):
+    """Blocks of 128 inputs and more (rows of 2 and of 16 bytes), and the step length from which narrower blocks take it."""
+    test_recurrent_gates_of_long_steps_against_float64(gpu, tokens, blocks, bw)
+
+
+def test_recurrent_convolution_of_wide_long_steps(gpu):
+    """The form that keeps rows in registers, which narrow or short steps do not take."""
+    test_recurrent_convolution_of_long_steps(gpu, 2052)
