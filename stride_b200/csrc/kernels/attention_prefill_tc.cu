@@ -201,7 +201,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     const int x = rotated ? 0 : head0 * gate.head_stride + (is_k ? 0 : gate.v_off) + lane * 64;
                     for (int j = 0; j < n_tiles; ++j) {
                         const int st = j % stages;
-                        if (!mbar_wait(smem_u32(&empty[st]), (static_cast<uint32_t>(j / stages) & 1u) ^ 1u, status, is_k ? 11 : 18)) break;
+                        // (the warp gives up as one: a lane that went on alone would wait for the others below)
+                        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&empty[st]), (static_cast<uint32_t>(j / stages) & 1u) ^ 1u, status, is_k ? 11 : 18)))
+                            break;
                         const uint32_t bar = smem_u32(&full[st]);
                         if (lane == 0) mbar_expect_tx(bar, tile_bytes);
                         __syncwarp();

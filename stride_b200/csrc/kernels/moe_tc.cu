@@ -102,7 +102,9 @@ grouped_gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         const int row = lane == 0 ? m0 : e * N + n0;
         for (int i = 0; i < num_kb; ++i) {
             const int s = i % STAGES;
-            if (i >= STAGES && !mbar_wait(smem_u32(&empty_bar[s]), ((i / STAGES) & 1) ^ 1, status, 11)) break;
+            // (the warp gives up as one: a lane that went on alone would wait for the others below)
+            const bool free = i < STAGES || mbar_wait(smem_u32(&empty_bar[s]), ((i / STAGES) & 1) ^ 1, status, 11);
+            if (!__all_sync(0xffffffffu, free)) break;
             const uint32_t bar = smem_u32(&full_bar[s]);
             if (lane == 0) mbar_expect_tx(bar, STAGE_BYTES);
             __syncwarp();
