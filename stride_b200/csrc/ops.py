@@ -1830,22 +1830,29 @@ def exact_attention_form(tokens: int, longest: int, keys: int, nq: int, nkv: int
     """The kernel for ``tokens`` neighbouring rows of requests that bring at most ``longest`` tokens each and hold at most ``keys``. A
     row a CTA is fastest while its CTAs run at once; eight rows a CTA read keys once for all of them, but walk the runs of several
     requests one after the other; a warp a (row, head) keeps the most warps in flight, which counts where keys are few or, with one or
-    two query heads a key head, single rows many. In us, rows / tiles / warps, head size 128: 24 query heads on 8 key heads, one request
-    of 8 tokens 6 / 12 / 9, 16 of 8 tokens 15 / 14 / 11, the same behind 300 tokens 213 / 103 / 300, 200 tokens 124 / 72 / 177; 32 on 32, 16
-    requests of 16 tokens 87 / 43 / 27, 8 tokens of each behind 300 681 / 173 / 388. (A captured step of single tokens gives its context
-    bucket as ``keys``: with few keys it loses up to 10 us a layer of 32 key heads to the warps.)"""
+    two query heads a key head, single rows many. A row a CTA also gives every SM's shared memory another shape, which the products of
+    more than 16 rows around it wait for (some 25 us a layer), so there it takes many keys to pay.
+    Steps of two layers in us, rows / tiles / warps, head size 128, 24 query heads on 8 key heads: 8 tokens behind 300 354 / 417 / 902, 24
+    tokens 472 / 424 / 425, behind 300 620 / 629 / 1090, three requests of 8 472 / 422 / 412, eight of 8 behind 300 764 / 682 / 1183; 24 on
+    24, eight requests of 16 959 / 897 / 854. Launches alone, 32 on 32, 128 single tokens behind 300 681 / - / 388. (A captured step of
+    single tokens gives its context bucket as ``keys``: 32 tokens with 10 keys each take it 534 us, 482 with the warps; with 80 566
+    and 653.)"""
     group = nq // nkv
     ctas = tokens * nkv * -(-group // 4)
-    per_sm = 227 * 1024 // ((64 * (hd + 4) + 64 * vd + 4 * hd) * 4 + 1024)         # of a row each, by their shared memory
-    wave = 148 * max(1, min(16, per_sm))
-    if ctas <= 444 or (longest < 8 and ctas <= wave):
-        return EXACT_ROWS
     if longest >= 8:
-        few = keys <= (48 if group == 1 else 32) and (longest < 16 or (group <= 2 and ctas > 7000))
+        if ctas <= 444 and (keys >= 128 or tokens <= 16):
+            return EXACT_ROWS
+        few = keys <= 48 and (longest < 16 or (group <= 2 and ctas > (2500 if longest < 24 else 7000)))
         return EXACT_WARPS if few else EXACT_TILES
-    if keys <= (96 if group <= 2 else 32):
+    if keys <= 32 and tokens > 16:
         return EXACT_WARPS
-    if group <= 2 and ctas > 4.7 * wave:
+    per_sm = 227 * 1024 // ((64 * (hd + 4) + 64 * vd + 4 * hd) * 4 + 1024)         # CTAs of a row each, by their shared memory
+    wave = 148 * max(1, min(16, per_sm))
+    if ctas <= wave:
+        return EXACT_ROWS
+    if group <= 2 and keys <= 96:
+        return EXACT_WARPS
+    if group <= 2 and ctas > 6 * wave:
         return EXACT_TILES if longest >= 4 else EXACT_WARPS
     return EXACT_ROWS
 

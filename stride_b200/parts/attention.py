@@ -481,6 +481,8 @@ class PagedAttention(Mixer):
         if not self._fast:
             # the exact kernel: the whole 32-bit path, and bfloat16 sizes the tensor-core kernels refuse
             split = min(ctx.decode_tail_start, tokens) if qkv.dtype == torch.float32 else 0     # portions before, single tokens after
+            if 0 < split == tokens - 1:
+                split = tokens                              # one single token goes along
             for lo, hi, longest in ((0, split, ctx.max_q_len), (split, tokens, 1)):
                 if hi > lo:
                     ops.paged_attention(qkv[lo:hi], self.qkv_dim, attn[lo:hi], cache.k_pages, cache.v_pages, table, ctx.seq_of_token[lo:hi],

@@ -1146,3 +1146,12 @@ def test_the_exact_attention_of_a_mixed_step_is_chosen_by_what_its_rows_hold(ops
         assert form(2048, 2048, 2048, nq, nkv, hd, hd) == ops.EXACT_TILES
     assert form(16 * 8, 8, 8, 32, 32, 128, 128) == ops.EXACT_WARPS and form(16 * 8, 8, 308, 32, 32, 128, 128) == ops.EXACT_TILES
     assert form(128, 1, 2048, 32, 32, 128, 128) == ops.EXACT_WARPS and form(128, 1, 2048, 24, 8, 128, 128) == ops.EXACT_ROWS
+
+
+def test_a_row_a_cta_is_left_out_around_products_of_many_rows(ops):
+    """Short prompts of more than 16 rows with few keys stay off the kernel that reshapes every SM's shared memory."""
+    form = ops.exact_attention_form
+    for nq, nkv in ((24, 8), (24, 24), (4, 1)):
+        assert all(form(t, t, t, nq, nkv, 128, 128) != ops.EXACT_ROWS for t in (17, 20, 33, 48, 64))
+        assert form(20, 1, 10, nq, nkv, 128, 128) == ops.EXACT_WARPS and form(20, 1, 2048, nq, nkv, 128, 128) == ops.EXACT_ROWS
+    assert form(24, 24, 324, 24, 8, 128, 128) == ops.EXACT_ROWS and form(64, 64, 364, 24, 8, 128, 128) == ops.EXACT_TILES
