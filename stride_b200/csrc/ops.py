@@ -1840,7 +1840,7 @@ def exact_attention_form(tokens: int, longest: int, keys: int, nq: int, nkv: int
     group = nq // nkv
     ctas = tokens * nkv * -(-group // 4)
     if longest >= 8:
-        if ctas <= 444 and (keys >= 128 or tokens <= 16):
+        if ctas <= 444 and keys >= 128:
             return EXACT_ROWS
         few = keys <= 48 and (longest < 16 or (group <= 2 and ctas > (2500 if longest < 24 else 7000)))
         return EXACT_WARPS if few else EXACT_TILES
