@@ -65,7 +65,7 @@ constexpr long long kStaggerCycles = 1000;
 // (map_k and map_v both describe it), the rotated parts as rows of another (map_k2), the requests' rows one after the other; the
 // query's rotated part has a matrix of its own too (map_q2). A key tile is 24 KB: one stage for keys and two for values leave room
 // for two CTAs per SM, and the scores run two tiles ahead, which hides the one stage. An optional gate (LatentGate) multiplies the
-// result. 2,048 tokens of 16 heads: 42 us, beside 12 us for the product that expands and 4 us for the
+// result. 2,048 tokens of 16 heads: 42 us, beside 20 us for the product that expands (moe_tc.cu) and 4 us for the
 // gather; on the latents themselves (latent_attention_tc.cu and two products a head) 745 + 24 + 19 us.
 struct LatentGate {
     const __nv_bfloat16* values;        // null: none

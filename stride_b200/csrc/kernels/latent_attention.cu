@@ -82,14 +82,21 @@ latent_prepare_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ pr
 
 // ------------------------------------------------------------------------------------------------- gather
 // The latents and rotated key parts of the first `num_seqs` requests, position 0 on, request after request, out of their pages into
-// dense rows: what the product that expands keys and values reads. A warp a row, 16 bytes a lane.
+// dense rows: what the product that expands keys and values reads. A warp a row, 16 bytes a lane. range (or null): 0 and the number of rows
+// filled, which bound that product's work (a captured portion's `rows` are for the longest context that it may be replayed at).
 __global__ void __launch_bounds__(256)
 latent_gather_kernel(const uint4* __restrict__ latent_pages, const uint4* __restrict__ krot_pages, const int32_t* __restrict__ block_table,
                      int table_width, const int32_t* __restrict__ ctx_len, int num_seqs, int page_size, int rank16, int rot16, int rows,
-                     uint4* __restrict__ latent, uint4* __restrict__ krot) {
+                     uint4* __restrict__ latent, uint4* __restrict__ krot, int32_t* __restrict__ range) {
     pdl_trigger();
     pdl_wait();
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (range && blockIdx.x == 0 && threadIdx.x == 0) {
+        int total = 0;
+        for (int s = 0; s < num_seqs && total < rows; ++s) total += ctx_len[s];
+        range[0] = 0;
+        range[1] = min(total, rows);
+    }
     if (row >= rows) return;
     int key = row, seq = 0;
     while (seq < num_seqs && key >= ctx_len[seq]) key -= ctx_len[seq++];
@@ -490,7 +497,8 @@ int stride_head_gemm(const void* A, int lda, int a_hs, const void* B, long long 
 
 // Pages: latent [pages, page_size, rank], key part [pages, page_size, rot], bf16, rank and rot multiples of 8, 16-byte aligned.
 int stride_latent_gather(const void* latent_pages, const void* krot_pages, const int32_t* block_table, int table_width, const int32_t* ctx_len,
-                         int num_seqs, int page_size, int rank, int rot, int rows, void* latent, void* krot, cudaStream_t stream) {
+                         int num_seqs, int page_size, int rank, int rot, int rows, void* latent, void* krot, int32_t* range,
+                         cudaStream_t stream) {
     if (num_seqs < 0 || page_size <= 0 || table_width <= 0 || rank <= 0 || rot <= 0 || rows < 0) return STRIDE_BAD_ARGUMENT;
     if (rank % 8 || rot % 8 || (reinterpret_cast<uintptr_t>(latent_pages) | reinterpret_cast<uintptr_t>(krot_pages) | reinterpret_cast<uintptr_t>(latent) |
                                 reinterpret_cast<uintptr_t>(krot)) % 16)
@@ -498,7 +506,7 @@ int stride_latent_gather(const void* latent_pages, const void* krot_pages, const
     if (num_seqs == 0 || rows == 0) return 0;
     stride::launch(latent_gather_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, static_cast<const uint4*>(latent_pages),
                    static_cast<const uint4*>(krot_pages), block_table, table_width, ctx_len, num_seqs, page_size, rank / 8, rot / 8, rows,
-                   static_cast<uint4*>(latent), static_cast<uint4*>(krot));
+                   static_cast<uint4*>(latent), static_cast<uint4*>(krot), range);
     return STRIDE_LAUNCH_STATUS();
 }
 

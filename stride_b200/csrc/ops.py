@@ -103,7 +103,7 @@ _SIGNATURES = {
     "stride_latent_attention": ("latent_attention", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                                      c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p]),
     "stride_latent_gather": ("latent_attention", [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
-                                                  c_void_p, c_void_p]),
+                                                  c_void_p, c_void_p, c_void_p]),
     "stride_latent_prefill_tc": ("attention_prefill_tc", [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p,
                                                           c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
                                                           c_void_p, c_int, c_int, c_void_p, c_void_p]),
@@ -1137,15 +1137,15 @@ def latent_prefill_supported(dtype, dim: int, vdim: int, rot: int, rank: int) ->
     return dtype == torch.bfloat16 and dim == 128 and vdim == 128 and rot == 64 and rank % 8 == 0
 
 
-def latent_gather(latent_pages, krot_pages, block_table, ctx_len, num_seqs: int, page_size: int, latent, krot) -> None:
+def latent_gather(latent_pages, krot_pages, block_table, ctx_len, num_seqs: int, page_size: int, latent, krot, filled=None) -> None:
     """The cached latents and rotated key parts of the step's first ``num_seqs`` requests, every position of a request in order and the
     requests one after the other, as rows of ``latent`` [rows, rank] and ``krot`` [rows, rot] (rows past the last request's keys
-    are left as they are)."""
+    are left as they are). ``filled`` (int32 [2]) receives 0 and the number of rows filled."""
     _check(_fn("stride_latent_gather")(
         _dev(latent_pages, "latent_pages", torch.bfloat16), _dev(krot_pages, "krot_pages", torch.bfloat16),
         _dev(block_table, "block_table", torch.int32), block_table.shape[1], _dev(ctx_len, "ctx_len", torch.int32), num_seqs, page_size,
         latent.shape[1], krot.shape[1], latent.shape[0], _dev(latent, "latent", torch.bfloat16), _dev(krot, "krot", torch.bfloat16),
-        _stream()), "latent_gather")
+        _opt(filled, "filled", torch.int32), _stream()), "latent_gather")
 
 
 def latent_prefill_tc(q, q_off: int, q_rot, q_rot_off: int, q_rot_stride: int, kv, krot, out, q_start, q_len, ctx_len, num_seqs: int,

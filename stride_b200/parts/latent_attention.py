@@ -25,7 +25,7 @@ models):
 
     one product, latent_prepare  as above
     latent_gather                the requests' latents out of their pages
-    one product                  [W_uk ; W_uv] c: every head's keys and values
+    one product                  [W_uk ; W_uv] c: every head's keys and values (the experts' tcgen05 product, of one expert)
     latent_prefill_tc            attention over them, times the gate (tcgen05)
     output product               as above
 
@@ -59,12 +59,12 @@ class LatentAttention(Mixer):
     lazy_output = True
     # Portions go over expanded keys where one of their requests holds this many: the folded form walks a request's keys in one CTA, a
     # tile of 64 after the other at some 12 us each, however few the tokens. Two such layers of 16 heads and nothing else, a step on the
-    # latents / expanded: 33 tokens behind 2,000 841 / 449 us, 10 behind 30,000 9.3 / 1.5 ms, 2,000 alone 1738 / 577 us. Below it the
-    # folded form has fewer launches (256 alone 429 / 466 us, 64 requests of 8 561 / 651). Many requests make the product that
-    # expands long while the walk stays what the longest one's is (16 of 16 tokens behind 1,000 556 / 513 us): at most
+    # latents / expanded: 33 tokens behind 2,000 841 / 437 us, 10 behind 30,000 9.3 / 1.7 ms, 2,000 alone 1738 / 556 us. Below it the
+    # folded form has fewer launches (256 alone 400 / 450 us, 64 requests of 8 515 / 610). Many requests make the product that
+    # expands long while the walk stays what the longest one's is (16 of 16 tokens behind 1,000 556 / 580 us): at most
     # EXPAND_SHARE times the longest one's keys in all.
     EXPAND_KEYS = 512
-    EXPAND_SHARE = 16
+    EXPAND_SHARE = 8
     MAX_EXPANDED_BYTES = 1 << 28      # keys and values of a step, expanded, at most (the buffer, whose rows are a power of two)
 
     def __init__(self, spec, runtime):
@@ -249,8 +249,11 @@ class LatentAttention(Mixer):
         k_rot = self.rt.scratch("latent_dense_rot", rows * self.rot, self.rt.dtype)[:rows * self.rot].view(rows, self.rot)
         kv_dim = self.heads * (self.dim + self.vdim)
         kv = self.rt.scratch("latent_expanded", rows * kv_dim, self.rt.dtype)[:rows * kv_dim].view(rows, kv_dim)
-        ops.latent_gather(latent, key_rot, ctx.block_table[cache.group], ctx.ctx_len, seqs, cache.page_size, c[:keys], k_rot[:keys])
-        ops.linear(c[:keys], self.w_ukv, kv[:keys])
+        filled = self.rt.scratch("latent_filled", 2, torch.int32)
+        ops.latent_gather(latent, key_rot, ctx.block_table[cache.group], ctx.ctx_len, seqs, cache.page_size, c[:keys], k_rot[:keys], filled)
+        # the experts' product with one expert, whose rows are those that were filled
+        if not ops.grouped_gemm_tc(c, self.w_ukv.view(1, kv_dim, self.rank), filled, kv, rows):
+            raise ops.KernelError("the product that expands keys and values does not take the sizes")
         ops.latent_prefill_tc(q, q_off, qa, self.rank, self.rank + self.rot, kv, k_rot, out, ctx.q_start, ctx.q_len, ctx.ctx_len, seqs,
                               self.heads, self.scale, sinks=self.sinks, gate=proj if self.gated else None, gate_off=self.g_off,
                               gate_per_output=self.full_gate, kv_head_stride=self.dim, kv_v_off=self.heads * self.dim)

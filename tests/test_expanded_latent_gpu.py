@@ -177,7 +177,7 @@ def test_the_rule_and_the_byte_limit(gpu, models, expansions, monkeypatch):
     case = models[48]
     tokens = {key: seeded_tokens(n, case.cfg["vocab"], 720 + key) for key, n in ((1, 80), (2, 30), (3, 30))}
 
-    def run(expanded, keys=80, share=16, limit=1 << 28):
+    def run(expanded, keys=80, share=8, limit=1 << 28):
         for name, value in (("EXPAND_KEYS", keys), ("EXPAND_SHARE", share), ("MAX_EXPANDED_BYTES", limit)):
             monkeypatch.setattr(LatentAttention, name, value)
         engine = engine_for(case)
@@ -239,3 +239,21 @@ def test_query_latents_expand_unless_the_model_holds_a_matrix_lstm(gpu, expansio
         want = plain_netusun.forward(cfg, {k: v.bfloat16().double() for k, v in state.items()}, tokens)[list(range(0, 140, 7))]
         error = float((got.double() - want).norm() / want.norm())
         assert error <= 0.03, error         # bfloat16 through one layer; a lost key or rotation changes rows outright
+
+
+@pytest.mark.parametrize("lens,rows", [([5, 0, 17], 40), ([64], 64), ([100, 200], 150)])
+def test_the_gather_says_how_many_rows_it_filled(gpu, lens, rows):
+    """What the product that expands them is bounded by; never more than the rows there are."""
+    from stride_b200.csrc import ops
+    page, rank, rot = 16, 48, 64
+    pages = [-(-n // page) for n in lens]
+    table = torch.full((len(lens), max(pages)), -1, dtype=torch.int32)
+    for s, n in enumerate(pages):
+        table[s, :n] = torch.arange(n) + sum(pages[:s])
+    latent, key_rot = (torch.randn(sum(pages), 1, page, n, device="cuda").bfloat16() for n in (rank, rot))
+    c, k_rot = (torch.full((rows, n), 7.0, dtype=torch.bfloat16, device="cuda") for n in (rank, rot))
+    filled = torch.full((3,), -5, dtype=torch.int32, device="cuda")
+    ops.latent_gather(latent, key_rot, table.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), len(lens), page, c, k_rot, filled[:2])
+    total = min(sum(lens), rows)
+    assert filled.tolist() == [0, total, -5]
+    assert bool((c[total:] == 7.0).all()) and not bool((c[:total] == 7.0).all(1).any())
