@@ -719,8 +719,8 @@ def lstm_case(H, D, DV, lens, seed):
 
 @pytest.mark.parametrize("H,D,DV,lens", [(8, 128, 128, [500]), (8, 128, 128, [96, 130]), (4, 256, 128, [200]), (6, 100, 72, [300, 64])])
 def test_matrix_lstm_chunks_are_no_further_from_float64_than_the_chain(gpu, H, D, DV, lens):
-    """The median over a step's (token, head) rows, which single rows whose divisor all but vanishes do not move (over eight seeds the
-    ratio lay within 0.75 and 0.92)."""
+    """The median over a step's (token, head) rows, which single rows whose divisor all but vanishes do not move (over 16 seeds the
+    ratio lay within 0.72 and 0.92)."""
     run, want = lstm_case(H, D, DV, lens, 5)
     error = lambda o: float(((o.double().view(want.shape) - want).norm(dim=-1) / want.norm(dim=-1)).median())
     assert error(run()[0]) <= error(run(chunks=False)[0])
