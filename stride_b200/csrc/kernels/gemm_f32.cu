@@ -1,4 +1,4 @@
-// True float32 matrix product for the 32-bit path: C[M,N] = A[M,K] * W[N,K]^T.
+// True float32 matrix product for the 32-bit path: C[M,N] = A[M,K] * W[N,K]^T, for the matrices that gemm_f32_tc.cu leaves here.
 //
 // Plain FMA on the CUDA cores, no tensor-core mode of reduced precision. The terms of an output are cut into 8 parts of
 // 16 * ceil(K / 128) consecutive ones; a part is one chain of fused multiply-adds in the order of k, and the parts are added

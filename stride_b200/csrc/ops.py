@@ -39,6 +39,8 @@ _SIGNATURES = {
     "stride_silu_mul": ("elementwise", [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "stride_gemm_tc_gated": ("gemm_bf16_tc", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_float,
                                               c_int, c_float, c_float, c_void_p]),
+    "stride_gemm_nt_f32_tc": ("gemm_f32_tc", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p,
+                                              c_void_p]),
     "stride_gemm_nt_f32": ("gemm_f32", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "stride_paged_attention_generic": ("attention_generic", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
@@ -1450,7 +1452,8 @@ def tc_status(device=None) -> int:
 _WAIT_CODES = {1: "matrix product: producer", 2: "matrix product: tensor-core issuer", 3: "matrix product: epilogue",
                31: "decode attention: a tile copy", 41: "weight-streaming product: a tile copy",
                51: "tokens-as-rows product: activation copies", 52: "tokens-as-rows product: weight copies",
-               53: "tokens-as-rows product: tensor-core issuer", 54: "tokens-as-rows product: epilogue"}
+               53: "tokens-as-rows product: tensor-core issuer", 54: "tokens-as-rows product: epilogue",
+               61: "float32 product: copies", 62: "float32 product: tensor-core issuer", 63: "float32 product: cutting warps"}
 _WAIT_CODES.update({c: "prefill attention (attention_prefill_tc.cu)" for c in range(11, 22)})
 _OTHER_CODES = {32: "decode attention was given a token whose position is not below the context bound of its launch"}
 
@@ -1772,11 +1775,18 @@ def linear_qkv_rope(x, weight, qkv, bias, positions, slot_mapping, cos, sin, k_p
     return True
 
 
+# Weights from which on a float32 product runs on the tensor cores, whatever the rows (the bits of a row must not depend on them). Below, a
+# CTA's walk along its part of K, some 0.8 us a block of 64, is longer than the other kernels take: 1024 x 1024 21 us with 1 row and 34 with
+# 301, 8 and 29 there; 2504 x 1040 16 and 28, 10 and 53; 3072 x 3072 24 and 62, 17 and 143.
+F32_TC_WEIGHTS = 1 << 23
+
+
 def linear(x, weight, out) -> None:
     """``out = x @ weight.T`` for row-major ``weight`` [out_features, in_features].
 
-    float32 runs the package's own FMA kernel (true 32-bit, order of the sum
-    fixed). bfloat16 with few rows (decode steps) runs the package's own kernels:
+    float32 runs the package's own kernels (true 32-bit, order of the sum fixed by
+    the matrix alone): a large matrix as exact products of three bfloat16 parts on
+    the tensor cores, any other by FMA. bfloat16 with few rows (decode steps) runs the package's own kernels:
     the tcgen05 kernel for large matrices, the weight-streaming kernel for the
     others; with many rows it calls the library matrix product, as the
     reference's engine does (python/stride_worker/model.py:258-260). ``out`` may
@@ -1788,6 +1798,21 @@ def linear(x, weight, out) -> None:
     if weight.shape[1] != k or out.shape != (m, n):
         raise KernelError(f"linear: shapes {tuple(x.shape)} x {tuple(weight.shape)} -> {tuple(out.shape)} do not agree")
     if x.dtype == torch.float32:
+        if n * k >= F32_TC_WEIGHTS and n >= 512 and k >= 512:
+            # Beyond 48 rows their three parts go through memory (6 bytes a number), some 64 MB at a time: a row's bits do not depend on its batch.
+            slab = m if m <= 48 else min(m, max(160, (1 << 26) // (6 * k) // 160 * 160))
+            parts = torch.empty(6 * slab * k, dtype=torch.uint8, device=x.device) if m > 48 else None
+            fn = _fn("stride_gemm_nt_f32_tc", f"product {n}x{k} (float32, tcgen05)")
+            for lo in range(0, m, slab) if m else ():
+                rows = min(m, lo + slab) - lo
+                code = fn(_dev(x, "x", torch.float32) + lo * k * 4, _dev(weight, "weight", torch.float32), _dev(out, "out", torch.float32) + lo * n * 4,
+                          rows, n, k, k, k, n, None if parts is None else parts.data_ptr(), 0 if parts is None else parts.numel(),
+                          _status_ptr(x.device), _stream())
+                if code == -2:
+                    break           # it depends on the matrix alone, so this was the first slab
+                _check(code, "gemm_nt_f32_tc")
+            else:
+                return
         _check(_fn("stride_gemm_nt_f32", f"product {n}x{k} (float32)")(_dev(x, "x", torch.float32), _dev(weight, "weight", torch.float32),
                                          _dev(out, "out", torch.float32), m, n, k, k, k, n, _stream()), "gemm_nt_f32")
         return
