@@ -71,12 +71,15 @@ struct ScanArgs {
 // sets the pace of a prompt is the chain of dependent instructions a token costs a warp (shared-memory reads, the sums,
 // the shuffles), not the amount of arithmetic: the rows are spread over as many lanes as the head size allows, and the NC
 // columns of a thread are independent chains that fill one another's waits (they also share the reads of k, q and the decay).
-// PIECES false: the one chain only (mode 0), with nothing of the pieces' bookkeeping in its loop.
-template <int LANES, int R, int NC, int CHUNK, int RULE, bool PIECES>      // RULE: see MemoryRule
+// The delta rule's outputs of a token are added up over the lanes beside the next token's own sum, whose shuffles theirs then run with: one
+// after the other they were a second round of waits (16 heads of 128 x 128, 2,048 tokens of one request 791 us, now 654).
+// MODE: as ScanArgs::mode; 0 has nothing of the pieces' bookkeeping in its loop, 1 no outputs (nor their sums and shuffles).
+template <int LANES, int R, int NC, int CHUNK, int RULE, int MODE>      // RULE: see MemoryRule
 __global__ void __launch_bounds__(kScanThreads)
 scan_kernel(const ScanArgs p) {
     // Launched without programmatic dependent launch (launch_alone): no trigger, and nothing to wait for.
-    const int mode = PIECES ? p.mode : 0;
+    constexpr int mode = MODE;
+    constexpr bool PIECES = MODE != 0;
     constexpr int DP = R * LANES;                           // rows with padding
     constexpr int THREADS = kScanThreads;
     constexpr int COLS = THREADS / LANES;                   // columns of one pass over the threads
@@ -181,6 +184,16 @@ scan_kernel(const ScanArgs p) {
     stash(0);
     __syncthreads();
     int buf = 0;
+    float late[NC];                         // delta rule: this lane's share of the token before's outputs
+#pragma unroll
+    for (int c = 0; c < NC; ++c) late[c] = 0.f;
+    auto put = [&](int t, const float (&of)[NC]) {
+        if (il == 0) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                if (j0 + c * COLS < DV) p.o[(static_cast<size_t>(start + t) * H + h) * DV + j0 + c * COLS] = of[c];
+        }
+    };
     for (int c0 = first; c0 < len; c0 += CHUNK, buf ^= 1) {
         const int nt = min(CHUNK, len - c0);
         const bool more = c0 + CHUNK < len;
@@ -216,7 +229,11 @@ scan_kernel(const ScanArgs p) {
 #pragma unroll
                 for (int o = 1; o < LANES; o <<= 1)
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) u[c] += __shfl_xor_sync(0xffffffffu, u[c], o);
+                    for (int c = 0; c < NC; ++c) {
+                        u[c] += __shfl_xor_sync(0xffffffffu, u[c], o);
+                        if (mode != 1) late[c] += __shfl_xor_sync(0xffffffffu, late[c], o);
+                    }
+                if (mode != 1 && c0 + tt > first) put(c0 + tt - 1, late);
                 const float beta = s_beta[buf][tt];
 #pragma unroll
                 for (int c = 0; c < NC; ++c) u[c] = beta * (vj[c] - u[c]);
@@ -232,11 +249,11 @@ scan_kernel(const ScanArgs p) {
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             S[c][4 * g + e] = fmaf(kk[4 * g + e], u[c], S[c][4 * g + e]);
-                            acc[c][e] = fmaf(S[c][4 * g + e], qv[e], acc[c][e]);
+                            if (mode != 1) acc[c][e] = fmaf(S[c][4 * g + e], qv[e], acc[c][e]);
                         }
                 }
 #pragma unroll
-                for (int c = 0; c < NC; ++c) out[c] = (acc[c][0] + acc[c][1]) + (acc[c][2] + acc[c][3]);
+                for (int c = 0; c < NC; ++c) late[c] = (acc[c][0] + acc[c][1]) + (acc[c][2] + acc[c][3]);
             } else if (RULE == kChannelDecay || RULE == kConstantDecay || RULE == kTokenDecay) {
                 const float plain = RULE == kTokenDecay ? s_w[buf][tt][0] : fade;
                 float in[NC];           // what the memory takes of a value
@@ -280,29 +297,34 @@ scan_kernel(const ScanArgs p) {
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             const float kv = kv4[e] * vj[c];
-                            acc[c][e] = fmaf(rv[e], fmaf(bv[e], kv, S[c][4 * g + e]), acc[c][e]);
+                            if (mode != 1) acc[c][e] = fmaf(rv[e], fmaf(bv[e], kv, S[c][4 * g + e]), acc[c][e]);
                             S[c][4 * g + e] = fmaf(wv[e], S[c][4 * g + e], S[c][4 * g + e]) + kv;
                         }
                 }
 #pragma unroll
                 for (int c = 0; c < NC; ++c) out[c] = (acc[c][0] + acc[c][1]) + (acc[c][2] + acc[c][3]);
             }
+            if constexpr (RULE != kDeltaRule && mode != 1) {
 #pragma unroll
-            for (int o = 1; o < LANES; o <<= 1)
+                for (int o = 1; o < LANES; o <<= 1)
 #pragma unroll
-                for (int c = 0; c < NC; ++c) out[c] += __shfl_xor_sync(0xffffffffu, out[c], o);
-            if (RULE == kTokenDecay) {
+                    for (int c = 0; c < NC; ++c) out[c] += __shfl_xor_sync(0xffffffffu, out[c], o);
+                if (RULE == kTokenDecay) {
 #pragma unroll
-                for (int c = 0; c < NC; ++c) out[c] = fmaf(skip, vj[c], out[c]);
-            }
-            if (il == 0 && mode != 1) {
-#pragma unroll
-                for (int c = 0; c < NC; ++c)
-                    if (j0 + c * COLS < DV) p.o[(static_cast<size_t>(start + c0 + tt) * H + h) * DV + j0 + c * COLS] = out[c];
+                    for (int c = 0; c < NC; ++c) out[c] = fmaf(skip, vj[c], out[c]);
+                }
+                put(c0 + tt, out);
             }
         }
         if (more) stash(buf ^ 1);       // nobody reads that buffer: its chunk was finished before the last barrier
         __syncthreads();
+    }
+    if (RULE == kDeltaRule && mode != 1) {
+#pragma unroll
+        for (int o = 1; o < LANES; o <<= 1)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) late[c] += __shfl_xor_sync(0xffffffffu, late[c], o);
+        put(len - 1, late);
     }
     if (mode != 2) {
 #pragma unroll
@@ -380,43 +402,50 @@ pieces_combine_kernel(float* __restrict__ piece_s, const float* __restrict__ pie
     *S_g = S;
 }
 
-template <int LANES, int R, int CHUNK, int RULE>
+// WIDE: the columns a thread has where the head is wide enough to fill them.
+template <int LANES, int R, int WIDE, int CHUNK, int RULE>
 int launch_scan_as(const ScanArgs& p, int num_seqs, cudaStream_t stream) {
     constexpr int COLS = kScanThreads / LANES;
-    // four columns a thread where the head is wide enough to fill them
     if (p.mode) num_seqs *= p.max_pieces;
     if constexpr (RULE >= kChannelDecay) {      // one chain; long portions of these rules run chunk by chunk (decay_memory.cu)
         if (p.mode) return STRIDE_BAD_ARGUMENT;
-        const int cta_cols = p.DV >= 4 * COLS ? 4 * COLS : COLS;
-        stride::launch_alone(p.DV >= 4 * COLS ? scan_kernel<LANES, R, 4, CHUNK, RULE, false> : scan_kernel<LANES, R, 1, CHUNK, RULE, false>,
+        const int cta_cols = p.DV >= WIDE * COLS ? WIDE * COLS : COLS;
+        stride::launch_alone(p.DV >= WIDE * COLS ? scan_kernel<LANES, R, WIDE, CHUNK, RULE, 0> : scan_kernel<LANES, R, 1, CHUNK, RULE, 0>,
                              dim3((p.DV + cta_cols - 1) / cta_cols, p.H, num_seqs), dim3(kScanThreads), 0, stream, p);
-    } else if (p.DV >= 4 * COLS) {
-        const dim3 grid((p.DV + 4 * COLS - 1) / (4 * COLS), p.H, num_seqs);
+    } else if (p.DV >= WIDE * COLS) {
+        const dim3 grid((p.DV + WIDE * COLS - 1) / (WIDE * COLS), p.H, num_seqs);
         // The delta rule's token costs a thread two rounds of shuffles: with two columns a thread the chain is shorter, as long as the
-        // twice as many CTAs still run side by side, three an SM (16 heads of 128 x 128, four / two columns: 2,048 tokens of one request
-        // 881 / 788 us, 1,750 of three 417 / 385, 1,500 of six, 768 CTAs, 222 / 290; single tokens of three 8.6 / 7.1).
+        // twice as many CTAs still run side by side, three an SM (16 heads of 128 x 128, 1,750 tokens of three requests 347 us with two;
+        // 200 each of six, 768 CTAs, 154 with four and 203 with two; one column a thread takes 531 and 289).
         const long long narrow = (p.DV + 2 * COLS - 1) / (2 * COLS);
         if (RULE == kDeltaRule && !p.mode && narrow * p.H * num_seqs <= 3 * 148) {
-            stride::launch_alone(scan_kernel<LANES, R, 2, CHUNK, RULE, false>, dim3(static_cast<unsigned>(narrow), p.H, num_seqs), dim3(kScanThreads), 0, stream, p);
+            stride::launch_alone(scan_kernel<LANES, R, 2, CHUNK, RULE, 0>, dim3(static_cast<unsigned>(narrow), p.H, num_seqs), dim3(kScanThreads), 0, stream, p);
             return STRIDE_LAUNCH_STATUS();
         }
-        if (p.mode) stride::launch_alone(scan_kernel<LANES, R, 4, CHUNK, RULE, true>, grid, dim3(kScanThreads), 0, stream, p);
-        else stride::launch_alone(scan_kernel<LANES, R, 4, CHUNK, RULE, false>, grid, dim3(kScanThreads), 0, stream, p);
+        if (p.mode) stride::launch_alone(p.mode == 1 ? scan_kernel<LANES, R, WIDE, CHUNK, RULE, 1> : scan_kernel<LANES, R, WIDE, CHUNK, RULE, 2>, grid, dim3(kScanThreads), 0, stream, p);
+        else stride::launch_alone(scan_kernel<LANES, R, WIDE, CHUNK, RULE, 0>, grid, dim3(kScanThreads), 0, stream, p);
     } else {
         const dim3 grid((p.DV + COLS - 1) / COLS, p.H, num_seqs);
-        if (p.mode) stride::launch_alone(scan_kernel<LANES, R, 1, CHUNK, RULE, true>, grid, dim3(kScanThreads), 0, stream, p);
-        else stride::launch_alone(scan_kernel<LANES, R, 1, CHUNK, RULE, false>, grid, dim3(kScanThreads), 0, stream, p);
+        if (p.mode) stride::launch_alone(p.mode == 1 ? scan_kernel<LANES, R, 1, CHUNK, RULE, 1> : scan_kernel<LANES, R, 1, CHUNK, RULE, 2>, grid, dim3(kScanThreads), 0, stream, p);
+        else stride::launch_alone(scan_kernel<LANES, R, 1, CHUNK, RULE, 0>, grid, dim3(kScanThreads), 0, stream, p);
     }
     return STRIDE_LAUNCH_STATUS();
 }
 
 template <int RULE>
 int launch_scan(const ScanArgs& p, int num_seqs, cudaStream_t stream) {
-    if (p.D <= 16) return launch_scan_as<4, 4, 16, RULE>(p, num_seqs, stream);
-    if (p.D <= 32) return launch_scan_as<8, 4, 16, RULE>(p, num_seqs, stream);
-    if (p.D <= 64) return launch_scan_as<16, 4, 16, RULE>(p, num_seqs, stream);
-    if (p.D <= 128) return launch_scan_as<16, 8, 8, RULE>(p, num_seqs, stream);
-    if (p.D <= 256) return launch_scan_as<16, 16, 4, RULE>(p, num_seqs, stream);
+    if (p.D <= 16) return launch_scan_as<4, 4, 4, 16, RULE>(p, num_seqs, stream);
+    if (p.D <= 32) return launch_scan_as<8, 4, 4, 16, RULE>(p, num_seqs, stream);
+    if (p.D <= 64) {
+        // The bonus rule's chain through a token is one multiply-add a row, so few lanes and long rows cost it nothing and save shuffles: 4 lanes
+        // with two columns / 16 lanes with four, 32 heads of 64 x 64, both passes over pieces of 1,750 tokens of three requests 176 / 212 us
+        // (274 with outputs in both), of 2,048 of one 208 / 249 (321), eight single tokens 17.5 / 19.9, eight portions of 60 48 / 52; 4 lanes
+        // with one column 239, 8 lanes with two 210. The delta rule's two sums a token are shorter over 16 lanes (347 us, 408 over 4).
+        if constexpr (RULE == kBonusMemory) return launch_scan_as<4, 16, 2, 16, RULE>(p, num_seqs, stream);
+        else return launch_scan_as<16, 4, 4, 16, RULE>(p, num_seqs, stream);
+    }
+    if (p.D <= 128) return launch_scan_as<16, 8, 4, 8, RULE>(p, num_seqs, stream);
+    if (p.D <= 256) return launch_scan_as<16, 16, 4, 4, RULE>(p, num_seqs, stream);
     return STRIDE_UNSUPPORTED;
 }
 
