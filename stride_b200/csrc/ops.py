@@ -39,6 +39,8 @@ _SIGNATURES = {
     "stride_silu_mul": ("elementwise", [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "stride_gemm_tc_gated": ("gemm_bf16_tc", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_float,
                                               c_int, c_float, c_float, c_void_p]),
+    "stride_latent_attention_tc5": ("latent_attention_tc5", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                                             c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p]),
     "stride_gemm_nt_f32_tc": ("gemm_f32_tc", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p,
                                               c_void_p]),
     "stride_gemm_nt_f32": ("gemm_f32", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
@@ -1134,6 +1136,21 @@ def latent_attention_tc(qa, out, partial, latent_pages, krot_pages, block_table,
         _opt(sinks, "sinks", torch.float32), _stream()), "latent_attention_tc")
 
 
+def latent_attention_tc5(qa, out, latent_pages, krot_pages, block_table, q_start, q_len, ctx_len, num_seqs: int, max_q_len: int, heads: int,
+                         rank: int, rot: int, page_size: int, scale: float, sinks=None) -> bool:
+    """``latent_attention_tc`` for the portions of the step's first ``num_seqs`` requests, on tcgen05. Returns False when the kernel does
+    not take the sizes (rank a multiple of 128 up to 512, rot a multiple of 16 up to 64)."""
+    code = _fn("stride_latent_attention_tc5")(
+        _dev(qa, "qa", torch.bfloat16), _dev(out, "out", torch.bfloat16), _dev(latent_pages, "latent_pages", torch.bfloat16),
+        _dev(krot_pages, "krot_pages", torch.bfloat16), _dev(block_table, "block_table", torch.int32), block_table.shape[1],
+        _dev(q_start, "q_start", torch.int32), _dev(q_len, "q_len", torch.int32), _dev(ctx_len, "ctx_len", torch.int32), num_seqs, max_q_len,
+        heads, rank, rot, page_size, float(scale), _opt(sinks, "sinks", torch.float32), _status_ptr(qa.device), _stream())
+    if code == -2:
+        return False
+    _check(code, "latent_attention_tc5")
+    return True
+
+
 def latent_prefill_supported(dtype, dim: int, vdim: int, rot: int, rank: int) -> bool:
     """Sizes of the expanded form of latent attention (``latent_gather``, a product, ``latent_prefill_tc``)."""
     return dtype == torch.bfloat16 and dim == 128 and vdim == 128 and rot == 64 and rank % 8 == 0
@@ -1453,7 +1470,8 @@ _WAIT_CODES = {1: "matrix product: producer", 2: "matrix product: tensor-core is
                31: "decode attention: a tile copy", 41: "weight-streaming product: a tile copy",
                51: "tokens-as-rows product: activation copies", 52: "tokens-as-rows product: weight copies",
                53: "tokens-as-rows product: tensor-core issuer", 54: "tokens-as-rows product: epilogue",
-               61: "float32 product: copies", 62: "float32 product: tensor-core issuer", 63: "float32 product: cutting warps"}
+               61: "float32 product: copies", 62: "float32 product: tensor-core issuer", 63: "float32 product: cutting warps",
+               71: "latent attention: copies of keys", 72: "latent attention: tensor-core issuer", 73: "latent attention: softmax"}
 _WAIT_CODES.update({c: "prefill attention (attention_prefill_tc.cu)" for c in range(11, 22)})
 _OTHER_CODES = {32: "decode attention was given a token whose position is not below the context bound of its launch"}
 

@@ -58,7 +58,8 @@ from .base import CacheRequest, Mixer, Projection, TensorDecl, build_part, regis
 class LatentAttention(Mixer):
     lazy_output = True
     # Portions go over expanded keys where one of their requests holds this many: the folded form walks a request's keys in one CTA, a
-    # tile of 64 after the other at some 12 us each, however few the tokens. Two such layers of 16 heads and nothing else, a step on the
+    # tile of 64 after the other at some 12 us each on mma.sync (2.3 us on tcgen05 since, which leaves the rule where it was: the roundings
+    # of the two forms differ), however few the tokens. On mma.sync two such layers of 16 heads and nothing else, a step on the
     # latents / expanded: 33 tokens behind 2,000 841 / 437 us, 10 behind 30,000 9.3 / 1.7 ms, 2,000 alone 1738 / 556 us. Below it the
     # folded form has fewer launches (256 alone 400 / 450 us, 64 requests of 8 515 / 610). Many requests make the product that
     # expands long while the walk stays what the longest one's is (16 of 16 tokens behind 1,000 556 / 580 us): at most
@@ -268,7 +269,8 @@ class LatentAttention(Mixer):
             return
         geometry = (self.heads, self.rank, self.rot, cache.page_size, self.scale)
         split = min(ctx.decode_tail_start, tokens)          # portions before, single tokens after
-        if split > first:
+        if split > first and not ops.latent_attention_tc5(qa, mixed, latent, key_rot, table, ctx.q_start, ctx.q_len, ctx.ctx_len, ctx.decode_tail_seq,
+                                                          max(ctx.max_q_len, 2), *geometry, sinks=self.sinks):
             ops.latent_attention_tc(qa, mixed, None, latent, key_rot, table, ctx.q_start, ctx.q_len, ctx.ctx_len, ctx.seq_of_token, 0,
                                     ctx.decode_tail_seq, 0, split, max(ctx.max_q_len, 2), *geometry, sinks=self.sinks)
         if tokens > split:
