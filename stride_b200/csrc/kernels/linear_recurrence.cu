@@ -113,6 +113,142 @@ delta_prepare_kernel(const T* __restrict__ proj, int ld, const float* __restrict
     }
 }
 
+// The same for four taps and heads of up to 128 channels, the same sums in the same order: a warp takes RUN neighbouring tokens of a head, so
+// that a row of the projections is read once and not once a tap, and asks for all of its rows at once; decays and beta have warps of
+// their own, whose exponentials and logarithms otherwise ran on after the rest. Bound by those and by 93 MB of reads and writes (14 us):
+// 1,750 tokens of 16 + 16 + 16 heads of 128, among the kernels of a step, 53 us, 95 before; runs of eight with the decays in the values'
+// warps 78. One token a warp where runs of four would leave SMs without work (4 tokens 8.9 us, 9.4).
+constexpr int kPrepSlots = 4;       // channels a lane
+template <typename T, int RUN>
+__global__ void __launch_bounds__(kPrepWarps * 32)
+delta_prepare_rows_kernel(const T* __restrict__ proj, int ld, const float* __restrict__ conv_w, const float* __restrict__ low, int ld_low,
+                          const float* __restrict__ a_log, const float* __restrict__ dt_bias, const float* __restrict__ state,
+                          long long state_stride, long long tail_off, const int32_t* __restrict__ seq_of_token, const int32_t* __restrict__ q_start,
+                          const int32_t* __restrict__ state_slot, float* __restrict__ qk, float* __restrict__ v_out, float* __restrict__ beta,
+                          float* __restrict__ decay, int tokens, int G, int H, int D, int DV, float unit_eps) {
+    constexpr int TAPS = 4;
+    pdl_trigger();
+    const int t0 = blockIdx.x * RUN, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = blockIdx.y * kPrepWarps + warp;
+    if (head >= 2 * G + 2 * H) return;
+    const int GD = G * D, HV = H * DV, C = 2 * GD + HV;
+    if (head >= 2 * G + H) {            // the decays and beta of a head
+        const int h = head - 2 * G - H;
+        float bias[kPrepSlots], a[RUN][kPrepSlots];
+#pragma unroll
+        for (int r = 0; r < kPrepSlots; ++r) bias[r] = lane + 32 * r < D ? dt_bias[h * D + lane + 32 * r] : 0.f;
+        const float rate = expf(a_log[h]);
+        pdl_wait();
+#pragma unroll
+        for (int u = 0; u < RUN; ++u)
+#pragma unroll
+            for (int r = 0; r < kPrepSlots; ++r)
+                a[u][r] = t0 + u < tokens && lane + 32 * r < D ? low[static_cast<size_t>(t0 + u) * ld_low + h * D + lane + 32 * r] : 0.f;
+#pragma unroll
+        for (int u = 0; u < RUN; ++u) {
+            const int t = t0 + u;
+            if (t >= tokens) break;
+            const bool live = seq_of_token[t] >= 0;
+#pragma unroll
+            for (int r = 0; r < kPrepSlots; ++r)
+                if (lane + 32 * r < D)
+                    decay[static_cast<size_t>(t) * H * D + h * D + lane + 32 * r] = live ? expm1f(-rate * softplus_f(a[u][r] + bias[r])) : 0.f;
+            if (lane == 0) beta[static_cast<size_t>(t) * H + h] = live ? sigmoid_f(to_f32(proj[static_cast<size_t>(t) * ld + C + h])) : 0.f;
+        }
+        return;
+    }
+    const bool is_v = head >= 2 * G;
+    const int n = is_v ? DV : D, h = head - 2 * G;
+    const int c0 = is_v ? 2 * GD + h * DV : head * D;       // first channel of this head
+    float4 w[kPrepSlots];
+#pragma unroll
+    for (int r = 0; r < kPrepSlots; ++r) {
+        const int e = lane + 32 * r;
+        w[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e < n) {
+            const float* const at = conv_w + static_cast<size_t>(c0 + e) * TAPS;
+            w[r] = make_float4(at[0], at[1], at[2], at[3]);
+        }
+    }
+    pdl_wait();
+    // rows t0 - 3 .. t0 + RUN - 1 of the step, whosever they are
+    float x[RUN + TAPS - 1][kPrepSlots];
+    int seqs[RUN];
+#pragma unroll
+    for (int i = 0; i < RUN + TAPS - 1; ++i) {
+        const int t = t0 + i - (TAPS - 1);
+#pragma unroll
+        for (int r = 0; r < kPrepSlots; ++r) {
+            const int e = lane + 32 * r;
+            x[i][r] = t >= 0 && t < tokens && e < n ? to_f32(proj[static_cast<size_t>(t) * ld + c0 + e]) : 0.f;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < RUN; ++u) seqs[u] = t0 + u < tokens ? seq_of_token[t0 + u] : -1;
+#pragma unroll
+    for (int u = 0; u < RUN; ++u) {
+        const int t = t0 + u, seq = seqs[u];
+        if (t >= tokens) break;
+        float* const dst = is_v ? v_out + static_cast<size_t>(t) * HV + h * DV : qk + static_cast<size_t>(t) * 2 * GD + head * D;
+        if (seq < 0) {          // a padded row of a fixed-size batch
+            for (int e = lane; e < n; e += 32) dst[e] = 0.f;
+            continue;
+        }
+        const int local = t - q_start[seq];
+        float y[kPrepSlots], ss = 0.f;
+        if (local >= TAPS - 1) {
+#pragma unroll
+            for (int r = 0; r < kPrepSlots; ++r) {
+                y[r] = fmaf(w[r].x, x[u][r], 0.f);
+                y[r] = fmaf(w[r].y, x[u + 1][r], y[r]);
+                y[r] = fmaf(w[r].z, x[u + 2][r], y[r]);
+                y[r] = fmaf(w[r].w, x[u + 3][r], y[r]);
+            }
+        } else {                // the portion's first tokens: what lies before it is the state's tail
+            const float* const tail = state + static_cast<size_t>(state_slot[seq]) * state_stride + tail_off;
+#pragma unroll
+            for (int r = 0; r < kPrepSlots; ++r) {
+                const int e = lane + 32 * r;
+                const float taps[TAPS] = {w[r].x, w[r].y, w[r].z, w[r].w};
+                y[r] = 0.f;
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) {
+                    const int src = local - (TAPS - 1) + j;
+                    const float in = src >= 0 ? x[u + j][r] : e < n ? tail[static_cast<size_t>(TAPS - 1 + src) * C + c0 + e] : 0.f;
+                    y[r] = fmaf(taps[j], in, y[r]);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kPrepSlots; ++r)
+            if (lane + 32 * r < n) {
+                y[r] = silu_f(y[r]);
+                ss = fmaf(y[r], y[r], ss);
+            }
+        float mult = 1.f;
+        if (!is_v) {
+            ss = warp_sum(ss);
+            mult = 1.f / sqrtf(ss + unit_eps);
+            if (head < G) mult *= 1.f / sqrtf(static_cast<float>(D));
+        }
+#pragma unroll
+        for (int r = 0; r < kPrepSlots; ++r)
+            if (lane + 32 * r < n) dst[lane + 32 * r] = y[r] * mult;
+    }
+}
+
+template <typename T>
+static void launch_delta_rows(const T* proj, int ld, const float* conv_w, const float* low, int ld_low, const float* a_log, const float* dt_bias,
+                              const float* state, long long state_stride, long long tail_off, const int32_t* seq_of_token, const int32_t* q_start,
+                              const int32_t* state_slot, float* qk, float* v_out, float* beta, float* decay, int tokens, int G, int H, int D,
+                              int DV, float unit_eps, cudaStream_t stream) {
+    constexpr int RUN = 4;
+    const int blocks = (2 * G + 2 * H + kPrepWarps - 1) / kPrepWarps;
+    const bool runs = static_cast<long long>((tokens + RUN - 1) / RUN) * blocks >= 148;
+    stride::launch(runs ? delta_prepare_rows_kernel<T, RUN> : delta_prepare_rows_kernel<T, 1>, dim3(runs ? (tokens + RUN - 1) / RUN : tokens, blocks),
+                   dim3(kPrepWarps * 32), 0, stream, proj, ld, conv_w, low, ld_low, a_log, dt_bias, state, state_stride, tail_off, seq_of_token,
+                   q_start, state_slot, qk, v_out, beta, decay, tokens, G, H, D, DV, unit_eps);
+}
+
 // ---------------------------------------------------------------------------------------------------- shift_mix
 // x [tokens, width] (compute type); mu [mixes, width] float32; out [mixes, tokens, width] (compute type):
 // out[s, t] = x[t] + (prev - x[t]) * mu[s], prev = x[t - 1] inside a portion and the state's vector at its start. The CTA
@@ -373,6 +509,15 @@ int stride_delta_prepare(const void* proj, int ld, const float* conv_w, const fl
     if (tokens < 0 || G <= 0 || H <= 0 || D <= 0 || DV <= 0 || taps <= 0 || H % G) return STRIDE_BAD_ARGUMENT;
     if (D > 32 * kMaxPerLane || DV > 32 * kMaxPerLane) return STRIDE_UNSUPPORTED;
     if (tokens == 0) return 0;
+    if (taps == 4 && D <= 32 * kPrepSlots && DV <= 32 * kPrepSlots && (dtype == STRIDE_DTYPE_F32 || dtype == STRIDE_DTYPE_BF16)) {
+        if (dtype == STRIDE_DTYPE_F32)
+            launch_delta_rows(static_cast<const float*>(proj), ld, conv_w, low, ld_low, a_log, dt_bias, state, state_stride, tail_off, seq_of_token,
+                              q_start, state_slot, qk, v_out, beta, decay, tokens, G, H, D, DV, unit_eps, stream);
+        else
+            launch_delta_rows(static_cast<const __nv_bfloat16*>(proj), ld, conv_w, low, ld_low, a_log, dt_bias, state, state_stride, tail_off,
+                              seq_of_token, q_start, state_slot, qk, v_out, beta, decay, tokens, G, H, D, DV, unit_eps, stream);
+        return STRIDE_LAUNCH_STATUS();
+    }
     const dim3 grid(tokens, (2 * G + H + kPrepWarps - 1) / kPrepWarps), block(kPrepWarps * 32);
     if (dtype == STRIDE_DTYPE_F32)
         stride::launch(delta_prepare_kernel<float>, grid, block, 0, stream, static_cast<const float*>(proj), ld, conv_w, low, ld_low, a_log,
