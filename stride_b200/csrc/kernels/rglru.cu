@@ -198,8 +198,8 @@ rglru_gates_kernel(const float* __restrict__ u, const T* __restrict__ wa_t, cons
 // 1.2e-7 at 72 inputs): so the first parts' products of 16 inputs start from zero and are added up with rounded additions, and only
 // those of the second and third parts, 2^-8 and less of them, stay in an accumulator. A CTA: 64 tokens x 64 output channels
 // of one block, both gates; eight warps, 32 tokens x 16 channels each; 64 inputs at a time through shared memory. Bound by
-// the exponentials of its epilogue (22 us) and the products; 2,048 tokens x 10 blocks of 256: 114 us, 243 us with multiply-adds
-// (8 tokens x 128 channels a CTA).
+// the exponentials of its epilogue (22 us) and the products; 2,048 tokens x 10 blocks of 256: 102 us with the next 64 inputs on their way
+// during the products, 117 without, 243 us with multiply-adds (8 tokens x 128 channels a CTA).
 template <bool VEC>
 __global__ void __launch_bounds__(256, 2)
 rglru_gates_mma_kernel(const float* __restrict__ u, const __nv_bfloat16* __restrict__ wa_t, const __nv_bfloat16* __restrict__ wi_t,
@@ -216,24 +216,53 @@ rglru_gates_mma_kernel(const float* __restrict__ u, const __nv_bfloat16* __restr
     const float* const ub = u + static_cast<size_t>(b) * bw;
     float acc[2][4][4] = {}, low[2][4][4] = {};         // [16 tokens][gate, 8 channels][fragment]
     pdl_wait();
-    for (int k0 = 0; k0 < bw; k0 += 64) {
-        if (k0) __syncthreads();
-        for (int p = tid; p < 64 * 16; p += 256) {      // 4 inputs of a token
-            const int r = p >> 4, k = (p & 15) * 4;
+    float4 next_u[4];           // pieces of 4 inputs of a token
+    uint4 next_w[4];            // pieces of 8 channels of an input
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int p = tid + i * 256, r = p >> 4, k = k0 + (p & 15) * 4;
             float x[4] = {0.f, 0.f, 0.f, 0.f};
             if (t0 + r < tokens) {
-                const float* src = ub + static_cast<size_t>(t0 + r) * width + k0 + k;
+                const float* src = ub + static_cast<size_t>(t0 + r) * width + k;
                 if (VEC) {
-                    if (k0 + k < bw) {
+                    if (k < bw) {
                         const float4 v = *reinterpret_cast<const float4*>(src);
                         x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
                     }
                 } else {
 #pragma unroll
                     for (int e = 0; e < 4; ++e)
-                        if (k0 + k + e < bw) x[e] = src[e];
+                        if (k + e < bw) x[e] = src[e];
                 }
             }
+            next_u[i] = make_float4(x[0], x[1], x[2], x[3]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int p = tid + i * 256, gate = p >> 9, k = k0 + ((p >> 3) & 63), c = (p & 7) * 8;
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (k < bw) {
+                const __nv_bfloat16* src = wg[gate] + static_cast<size_t>(k) * bw + c0 + c;
+                if (VEC) {
+                    if (c0 + c < bw) v = *reinterpret_cast<const uint4*>(src);
+                } else {
+                    __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&v);
+#pragma unroll
+                    for (int n = 0; n < 8; ++n)
+                        if (c0 + c + n < bw) e[n] = src[n];
+                }
+            }
+            next_w[i] = v;
+        }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < bw; k0 += 64) {
+        if (k0) __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int p = tid + i * 256, r = p >> 4, k = (p & 15) * 4;
+            float x[4] = {next_u[i].x, next_u[i].y, next_u[i].z, next_u[i].w};
 #pragma unroll
             for (int part = 0; part < 3; ++part) {
                 __nv_bfloat162 h[2];
@@ -247,22 +276,12 @@ rglru_gates_mma_kernel(const float* __restrict__ u, const __nv_bfloat16* __restr
                 *reinterpret_cast<uint2*>(&us[part][r][k]) = make_uint2(*reinterpret_cast<uint32_t*>(&h[0]), *reinterpret_cast<uint32_t*>(&h[1]));
             }
         }
-        for (int p = tid; p < 2 * 64 * 8; p += 256) {   // 8 channels of an input
-            const int gate = p >> 9, k = (p >> 3) & 63, c = (p & 7) * 8;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (k0 + k < bw) {
-                const __nv_bfloat16* src = wg[gate] + static_cast<size_t>(k0 + k) * bw + c0 + c;
-                if (VEC) {
-                    if (c0 + c < bw) v = *reinterpret_cast<const uint4*>(src);
-                } else {
-                    __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&v);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (c0 + c + i < bw) e[i] = src[i];
-                }
-            }
-            *reinterpret_cast<uint4*>(&ws[gate][k][c]) = v;
+        for (int i = 0; i < 4; ++i) {
+            const int p = tid + i * 256, gate = p >> 9, k = (p >> 3) & 63, c = (p & 7) * 8;
+            *reinterpret_cast<uint4*>(&ws[gate][k][c]) = next_w[i];
         }
+        if (k0 + 64 < bw) fetch(k0 + 64);           // on their way while the products run
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < 64; k += 16) {
