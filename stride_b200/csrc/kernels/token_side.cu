@@ -67,6 +67,18 @@ __global__ void cast_rows_kernel(const float* __restrict__ src, T* __restrict__ 
         dst[i] = from_f32<T>(src[i]);
 }
 
+// The same to bfloat16, four numbers a thread (2,048 x 2,048 6.0 us among the kernels of a step, 11.8 a number a thread).
+__global__ void __launch_bounds__(256)
+cast_rows_vec_kernel(const float4* __restrict__ src, uint2* __restrict__ dst, size_t packs) {
+    pdl_trigger();
+    pdl_wait();
+    const size_t i = blockIdx.x * static_cast<size_t>(256) + threadIdx.x;
+    if (i >= packs) return;
+    const float4 v = src[i];
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    dst[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
 template <typename T>
 __global__ void side_gate_kernel(const T* __restrict__ pre, const int32_t* __restrict__ ids, const int32_t* __restrict__ seq_of_token,
                                  const T* __restrict__ table, int table_width, int offset, int vocab, T* __restrict__ out, int dim) {
@@ -144,6 +156,12 @@ using namespace stride;
 extern "C" int stride_cast_rows(const float* src, void* dst, long long n, int dtype, cudaStream_t stream) {
     if (n < 0) return STRIDE_BAD_ARGUMENT;
     if (n == 0) return 0;
+    if (dtype == STRIDE_DTYPE_BF16 && n % 4 == 0 && n / 1024 < 0x7fffffff && reinterpret_cast<uintptr_t>(src) % 16 == 0 && reinterpret_cast<uintptr_t>(dst) % 8 == 0) {
+        const size_t packs = static_cast<size_t>(n / 4);
+        stride::launch(cast_rows_vec_kernel, dim3(static_cast<unsigned>((packs + 255) / 256)), dim3(256), 0, stream, reinterpret_cast<const float4*>(src),
+                       static_cast<uint2*>(dst), packs);
+        return STRIDE_LAUNCH_STATUS();
+    }
     const unsigned blocks = static_cast<unsigned>(n / 256 >= 8192 ? 8192 : (n + 255) / 256);
     if (dtype == STRIDE_DTYPE_F32)
         stride::launch(cast_rows_kernel<float>, dim3(blocks), dim3(256), 0, stream, src, static_cast<float*>(dst), static_cast<size_t>(n));
