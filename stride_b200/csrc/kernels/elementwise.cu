@@ -554,6 +554,11 @@ __global__ void zero_fresh_state_kernel(const __grid_constant__ StateList list, 
     pdl_wait();
     const long long row_words = list.row_words[blockIdx.z];
     uint32_t* row = list.state[blockIdx.z] + static_cast<size_t>(slot) * row_words;
+    if (row_words % 4 == 0 && reinterpret_cast<uintptr_t>(list.state[blockIdx.z]) % 16 == 0) {      // 16 bytes a store (1 request, 1 MB a state: 3.4 us, 19 by words)
+        for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < row_words / 4; i += static_cast<long long>(gridDim.x) * blockDim.x)
+            reinterpret_cast<uint4*>(row)[i] = make_uint4(0u, 0u, 0u, 0u);
+        return;
+    }
     for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < row_words;
          i += static_cast<long long>(gridDim.x) * blockDim.x)
         row[i] = 0u;

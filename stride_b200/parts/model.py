@@ -19,7 +19,7 @@ from ..csrc import ops
 from ..weights import check_source, load_weights
 from .base import build_part
 from .copies import CopiedStream
-from .runtime import ResidualStream, Runtime
+from .runtime import ResidualStream, Runtime, sequence_slots
 
 
 def mixer_kinds(spec) -> set:
@@ -122,7 +122,8 @@ class DecoderModel:
         stream = CopiedStream(self.rt, tokens, self.hidden, self.copies) if self.copies else ResidualStream(self.rt, tokens, self.hidden)
         self.embedding.forward(ctx, stream.residual)
         # a request that starts in this step finds its state slots at zero
-        ops.zero_fresh_states(self._states(), ctx.state_slot, ctx.q_start, ctx.q_len, ctx.positions)
+        seqs = sequence_slots(ctx)
+        ops.zero_fresh_states(self._states(), ctx.state_slot[:seqs], ctx.q_start[:seqs], ctx.q_len[:seqs], ctx.positions)
         first = None
         if self.pass_input is not None:         # the embedding's output in the compute dtype, for every pass to come
             first = self.rt.buffer("embedding_out", tokens, self.hidden)
