@@ -301,9 +301,10 @@ latent_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict
     if (lane < splits) { m0 = src[lane * stride]; l0 = src[lane * stride + 1]; }
     if (lane + 32 < splits) { m1 = src[(lane + 32) * stride]; l1 = src[(lane + 32) * stride + 1]; }
     const float m = warp_max(fmaxf(m0, m1));
-    // a split without keys has the maximum -inf; the last ones are left out
-    const unsigned some0 = __ballot_sync(0xffffffffu, m0 != -INFINITY), some1 = __ballot_sync(0xffffffffu, m1 != -INFINITY);
-    const int live = some1 ? 64 - __clz(some1) : 32 - __clz(some0);
+    // a split without keys has the maximum -inf and the sum 0; the last ones are left out. (Scores that are no numbers leave the maximum alone, not
+    // the sum; and a row of nothing but -inf keeps one split, for 0 / 0 as without splits.)
+    const unsigned some0 = __ballot_sync(0xffffffffu, m0 != -INFINITY || l0 != 0.f), some1 = __ballot_sync(0xffffffffu, m1 != -INFINITY || l1 != 0.f);
+    const int live = some1 ? 64 - __clz(some1) : max(32 - __clz(some0), 1);
     float w0 = m0 == -INFINITY ? 0.f : expf(m0 - m), w1 = m1 == -INFINITY ? 0.f : expf(m1 - m);
     // the sum of the splits' sums in the order of the splits
     float l = 0.f;
