@@ -1,28 +1,36 @@
 // The float32 product C[M,N] = A[M,K] * W[N,K]^T of large matrices on the fifth-generation tensor cores.
 //
-// Every float32 is the exact sum of three bfloat16 (8 bits of its mantissa each), and a product of two bfloat16 is exact in float32. Of
-// the nine products of parts the six with a weight of 2^-16 and more are taken (the others are below 2^-22 of |a w|, of either sign).
-// The tensor cores cut their sums off towards zero, so the products of the first parts run from zero over 64 terms at a time, and those
-// sums are added up in registers by rounded additions; the five others, 2^-7 and less of the whole, stay in an accumulator of their
-// own over a part of K. K is cut into parts of at most 1,024 terms (longer ones beyond 8), a CTA each, which meet in a cluster and are
-// added up in order. K alone decides all this, so a row's bits do not depend on M, nor on the row's place in the batch.
+// A float32 is the sum of three bfloat16 (of 6, 8 and 8 bits of its mantissa and their signs; the splitting into bfloat16 is that of G. Henry,
+// P. T. P. Tang and A. Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations", 2019), and a
+// product of two bfloat16 is exact in float32. Eight of the nine products of parts are taken; third x third, 2^-30 of |a w|, is left out. The
+// numbers are worked on times 2^40, so that the parts of small ones, subnormal ones too, are no subnormal bfloat16 (whose steps of 2^-133 would
+// take their bits); numbers of 2^70 and sums of 2^48 and more become infinities on the way and are done again, see below.
+//
+// The tensor cores cut the terms of a sum off where they lie far below its largest, and every sum towards zero. So the products of first parts
+// run from zero over 64 terms at a time, whose 12 bits then lose nothing unless they lie 2^6 and more apart (parts of 8 bits made sums of terms
+// of one sign come out low, by 1.1e-7 to 1.5e-7), and those sums are added up in registers by rounded additions; the seven others, 2^-5 and
+// less of the whole and, by the rounding of the parts, of either sign, stay in an accumulator of their own over a part of K. K is cut into up to
+// eight parts, a CTA each, which meet in a cluster and are added up in order. N and K alone decide all this, so a row's bits do not depend on
+// M, nor on the row's place in the batch.
 //
 // D = W A^T: 128 rows of W are the M side, up to 160 rows of A (tokens) the N side, so that a few tokens cost few columns and a step's
 // weights are read once. W's parts go to tensor memory and not back to shared memory, whose reads would bound the products.
 //
-//   W warps (8)      cut W up: from the TMA ring (float32) into tensor memory, a lane a row, each warpgroup half of the 64 columns; and
-//                    add the finished sums of 64 terms to their registers, each warpgroup half of the tokens
+//   W warps (8)      cut W up: from the TMA ring (float32) into tensor memory, a lane a row; and add the finished sums of 64 terms to their
+//                    registers, each warpgroup half of the tokens. Up to 96 tokens the warpgroups take turns with W's blocks of 64 columns (a
+//                    wait, a fence or an arrival costs a warp some 100 cycles, and so comes half as often), beyond both cut half of each
 //   A warps (4 or 8) cut A up: from L2 through registers into swizzled shared memory; beyond 48 rows one warp brings the parts by TMA
 //   one warp         TMA: 128 x 64 float32 of W a stage
 //   one warp         tcgen05.mma, and the tensor memory
 //
-// An infinity and what is no number make a NaN here, also where the product itself has none: an element that comes out as NaN is
-// computed again as the chains of gemm_f32.cu.
+// What comes out as no finite number is computed again as the chains of gemm_f32.cu.
 //
-// 301 rows, us (gemm_f32.cu): 5120 x 3072 67 (227), 3072 x 3072 62 (143), 16384 x 3072 175 (668), 3072 x 8192 120 (363). Error against
-// 64 bits 1.3e-7 of the result (3.6e-7; 5.8e-7 with K = 8192). Cutting A up in every CTA cost issue slots that the tensor cores waited
-// for (81, 78, 217, 148 us), which is why more than 48 rows are cut once, by a kernel of its own. 2 rows: 25, 23, 63, 33 us
-// (27, 19, 57, 37), 128256 x 3072 287 (320).
+// us (gemm_f32.cu), one row: 5120 x 3072 15.0 (15.1), 3072 x 3072 11.0 (8.8), 16384 x 3072 35 (38), 3072 x 8192 24 (21), 128256 x 3072 249 (304); two rows
+// 15.2 (17.1), 11.0 (9.8), 36 (42), 24 (24), 251 (296); 301 rows 83 (223), 68 (146), 188 (665), 129 (376). Bound by the waits, fences and arrivals between
+// the warps where rows are few (some 0.75 us a block and CTA), by the products beyond (8 x 2 x 301 x 16384 x 3072 at 1.3 PFLOP/s). Six products of
+// parts of 8 bits took 301 rows in 58, 55, 166 and 110 us, with the errors named above. Error against 64 bits of sum |a w|, K = 3072, rms: normal
+// numbers 2.3e-9 (1.0e-8), of one sign 5.0e-8 (1.0e-7), one term 2.5e-8 (the same). One kind measured goes the other way: terms of one sign that lie very
+// far apart (log-normal, sigma 3, in both operands) 2.8e-7 to 3.0e-7 whatever K (1.1e-7 at 512, 1.6e-7 at 1024, 4.1e-7 at 3072, 1.2e-6 at 8192).
 //
 // Every wait on an mbarrier is bounded by a clock; a wait that runs out sets *status and the CTA winds down.
 #include "tcgen05.cuh"
@@ -32,24 +40,41 @@ namespace f32tc {
 
 using namespace tc;
 
-constexpr int kRows = 128, kBlockK = 64, kWThreads = 256, kPart = 1024;
+constexpr int kRows = 128, kBlockK = 64, kWThreads = 256, kMaxParts = 8;
+constexpr float kUp = 0x1p40f, kDown = 0x1p-80f;
 constexpr int kBoxBytes = kRows * 128, kStageBytes = 2 * kBoxBytes;       // 32 float32 of 128 rows a box
 
-__host__ __device__ __forceinline__ int parts_of(int K) {
-    const int p = (K + kPart - 1) / kPart;
-    return p > 8 ? 8 : p;
+// Parts of K, each with CTAs of its own: as many as make the shortest walk for up to 16 tokens, where two CTAs share an SM, some 256 run side by
+// side (clusters do not fill a GPC to the last SM; of seven they fill it worst) and beginning and end cost a CTA about four blocks. N and K
+// alone decide. One row, us, by parts: 3072 x 3072 1 38.9, 2 20.8, 4 12.6, 6 12.8, 8 11.0; 16384 x 3072 1 59, 2 35.4, 3 41.7, 8 46.6; 28672 x 4096 1 81, 2 90, 8
+// 97. With many rows fewer parts would do: 301 of 3072 x 3072 49 us in five and 68 in eight, of 5120 x 3072 68 in three and 83 in six.
+__host__ inline int parts_of(int N, int K) {
+    const long long tiles = (N + kRows - 1) / kRows;
+    const int blocks = (K + kBlockK - 1) / kBlockK;
+    int best = 1;
+    long long least = 0;
+    for (int p = 1; p <= kMaxParts && p <= blocks; ++p) {
+        const long long walk = (tiles * p + 255) / 256 * ((blocks + p - 1) / p + 4);
+        if (p != 7 && (p == 1 || walk < least)) {
+            best = p;
+            least = walk;
+        }
+    }
+    return best;
 }
 
-// Eight columns of 32 lanes.
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
-    uint32_t r[8];
+// Eight columns of 32 lanes; tmem_ld_wait() before anybody uses them.
+__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[8]) {      // (through r: nothing that uses it may come before)
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 :
+                 : "memory");
 }
 // Eight registers into eight columns; tmem_st_wait() before anybody reads them.
 __device__ __forceinline__ void tmem_st8_issue(uint32_t taddr, const uint32_t (&v)[8]) {
@@ -59,19 +84,30 @@ __device__ __forceinline__ void tmem_st8_issue(uint32_t taddr, const uint32_t (&
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Two float32 as three pairs of bfloat16 (the first number in the low half): x = first + second + third. The first is cut off (no
-// conversion, and nothing finite becomes an infinity), the second rounded, which leaves a third of either sign: what the products that
-// are left out add up to has no sign of its own.
-__device__ __forceinline__ uint32_t high_halves(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
+// Pairs of float32 in one instruction.
+__device__ __forceinline__ uint64_t pair(float x, float y) { uint64_t p; asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(x), "f"(y)); return p; }
+__device__ __forceinline__ void unpair(uint64_t p, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p)); }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(b), "l"(pair(-1.f, -1.f)), "l"(a));
+    return d;
+}
+
+// Two float32, times kUp, as three pairs of bfloat16 (the first number in the low half): x = first + second + third. The first has 6 bits
+// and is rounded (Veltkamp's splitting): a product of two firsts has 12, so 64 of them add up without a loss unless they lie far apart, and
+// what the seven other products add up to has no sign of its own. The second is rounded to its 8 bits, the third is what is left (8 bits: 24 in all).
 __device__ __forceinline__ void cut2(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-    p0 = high_halves(x, y);
-    x -= __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
-    y -= __uint_as_float(__float_as_uint(y) & 0xFFFF0000u);
+    const uint64_t v = pair(x, y), all = mul2(v, pair(kUp, kUp)), far = mul2(v, pair(kUp * 262145.f, kUp * 262145.f));     // 2^18 + 1
+    const uint64_t first = add2(far, sub2(all, far)), rest = sub2(all, first);
+    unpair(first, x, y);
+    p0 = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+    unpair(rest, x, y);
     const __nv_bfloat162 second = __floats2bfloat162_rn(x, y);
     p1 = *reinterpret_cast<const uint32_t*>(&second);
-    x -= __uint_as_float(p1 << 16);
-    y -= __uint_as_float(p1 & 0xFFFF0000u);
-    p2 = high_halves(x, y);
+    unpair(sub2(rest, pair(__uint_as_float(p1 << 16), __uint_as_float(p1 & 0xFFFF0000u))), x, y);
+    p2 = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
 }
 
 __device__ __forceinline__ float4 load_cluster_f4(const float* local, uint32_t rank) {
@@ -129,8 +165,10 @@ struct Shape {
     static constexpr int A_PART = TOKENS * 128, A_BYTES = 3 * A_PART;         // 64 bfloat16 a row; three parts
     static constexpr int RING = W_STAGES * kStageBytes + 2 * A_BYTES, OUT = TOKENS * kRows * 4;
     static constexpr int SMEM = (RING > OUT ? RING : OUT) + 1024;
-    static constexpr int COLS = 2 * TOKENS + 192 <= 256 ? 256 : 512;            // two accumulators, two stages of W's parts
+    static constexpr int MAINS = 3 * TOKENS + 192 <= 512 ? 2 : 1;                // accumulators of the first products
+    static constexpr int COLS = (MAINS + 1) * TOKENS + 192 <= 256 ? 256 : 512;   // those, the others', two stages of W's parts
     static constexpr int CTAS = COLS == 256 ? 2 : 1;
+    static constexpr bool TURNS = MAINS == 2;                     // the warpgroups take turns with W's blocks (else half of the columns each)
     static constexpr bool READY = HALF >= 48;                     // A comes cut up (cut_rows_kernel)
     static constexpr int A_THREADS = READY ? 32 : HALF == 8 ? 128 : 256;
     static constexpr int THREADS = kWThreads + A_THREADS + 64;
@@ -142,14 +180,14 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                       const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int blocks, int a_vec,
                       int* __restrict__ status) {
     using S = Shape<HALF>;
-    constexpr int TOKENS = S::TOKENS, W_STAGES = S::W_STAGES, A_THREADS = S::A_THREADS, PIECES = S::READY ? 1 : TOKENS * 16 / A_THREADS;
-    constexpr int CH = HALF % 16 == 0 ? 16 : 8;
+    constexpr int TOKENS = S::TOKENS, MAINS = S::MAINS, W_STAGES = S::W_STAGES, A_THREADS = S::A_THREADS, PIECES = S::READY ? 1 : TOKENS * 16 / A_THREADS;
+    constexpr int W_WARPS = S::TURNS ? 4 : 8, STEP = S::TURNS ? 2 : 1;         // warps that cut a block up, blocks from one of theirs to the next
     constexpr int TMA_WARP = (kWThreads + A_THREADS) / 32, MMA_WARP = TMA_WARP + 1;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* const smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* const a_s = smem + W_STAGES * kStageBytes;
     __shared__ __align__(8) uint64_t w_full[W_STAGES], w_empty[W_STAGES];
-    __shared__ __align__(8) uint64_t cut[2], used[2], a_full[2], main_done, main_read, all_done;
+    __shared__ __align__(8) uint64_t cut[2], used[2], a_full[2], main_done[S::MAINS], main_read[S::MAINS], all_done;
     __shared__ uint32_t tmem_slot;
 
     pdl_trigger();
@@ -159,15 +197,17 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (threadIdx.x == 0) {
         for (int s = 0; s < W_STAGES; ++s) {
             mbar_init(smem_u32(&w_full[s]), 1);
-            mbar_init(smem_u32(&w_empty[s]), kWThreads / 32);
+            mbar_init(smem_u32(&w_empty[s]), W_WARPS);
         }
         for (int s = 0; s < 2; ++s) {
-            mbar_init(smem_u32(&cut[s]), (kWThreads + (S::READY ? 0 : A_THREADS)) / 32);
+            mbar_init(smem_u32(&cut[s]), W_WARPS + (S::READY ? 0 : A_THREADS / 32));
             mbar_init(smem_u32(&used[s]), 1);
             mbar_init(smem_u32(&a_full[s]), 1);
         }
-        mbar_init(smem_u32(&main_done), 1);
-        mbar_init(smem_u32(&main_read), kWThreads / 32);
+        for (int s = 0; s < MAINS; ++s) {
+            mbar_init(smem_u32(&main_done[s]), 1);
+            mbar_init(smem_u32(&main_read[s]), kWThreads / 32);
+        }
         mbar_init(smem_u32(&all_done), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -175,7 +215,7 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot, t_main = tmem, t_cross = tmem + TOKENS, t_w = tmem + 2 * TOKENS;      // + 96 a stage, 32 a part
+    const uint32_t tmem = tmem_slot, t_main = tmem, t_cross = tmem + MAINS * TOKENS, t_w = t_cross + TOKENS;      // + 96 a stage, 32 a part
 
     bool ok = true;
     if (warp < kWThreads / 32) {
@@ -184,38 +224,57 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         float acc[HALF];
 #pragma unroll
         for (int i = 0; i < HALF; ++i) acc[i] = 0.f;
-        auto add = [&](uint32_t from) {
+        // sums of N accumulators, one after the other
+        auto add = [&](auto... from) {
+            constexpr int N = sizeof...(from);
+            const uint32_t at[N] = {from...};
 #pragma unroll
-            for (int j = 0; j < HALF; j += CH) {
-                float v[CH];
-                if constexpr (CH == 16) tmem_ld16(from + lanes + half * HALF + j, v);
-                else tmem_ld8(from + lanes + half * HALF + j, v);
+            for (int j = 0; j < HALF; j += 8) {
+                uint32_t v[N][8];
 #pragma unroll
-                for (int e = 0; e < CH; ++e) acc[j + e] += v[e];
+                for (int n = 0; n < N; ++n) tmem_ld8_issue(at[n] + lanes + half * HALF + j, v[n]);
+#pragma unroll
+                for (int n = 0; n < N; ++n) tmem_ld_wait(v[n]);
+#pragma unroll
+                for (int n = 0; n < N; ++n)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[j + e] += __uint_as_float(v[n][e]);
             }
         };
+        auto wait_main = [&](int i) { return mbar_wait(smem_u32(&main_done[i % MAINS]), (i / MAINS) & 1, status, 63); };
         auto take = [&](int i) {            // the finished sums of block i
-            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&main_done), i & 1, status, 63));
-            if (!ok) return;
+            if (!(ok = __all_sync(0xffffffffu, wait_main(i)))) return;
             tc_fence_after();
-            add(t_main);
+            add(t_main + i % MAINS * TOKENS);
             tc_fence_before();
-            warp_arrive(smem_u32(&main_read));
+            warp_arrive(smem_u32(&main_read[i % MAINS]));
         };
-        for (int i = 0; i < count; ++i) {
+        auto take2 = [&](int i) {           // of two blocks at once
+            if (!(ok = __all_sync(0xffffffffu, wait_main(i) && wait_main(i + 1)))) return;
+            tc_fence_after();
+            add(t_main + i % MAINS * TOKENS, t_main + (i + 1) % MAINS * TOKENS);
+            tc_fence_before();
+            __syncwarp();
+            if (lane < 2) mbar_arrive(smem_u32(&main_read[lane]));
+        };
+        int taken = 0;
+        for (int i = S::TURNS ? half : 0; i < count; i += STEP) {
             const int s = i & 1, ws = i % W_STAGES;
-            ok = mbar_wait(smem_u32(&w_full[ws]), (i / W_STAGES) & 1, status, 63);
-            ok = ok && (i < 2 || mbar_wait(smem_u32(&used[s]), ((i >> 1) & 1) ^ 1, status, 63));
+            // (in this order: a warpgroup that takes turns has not seen the phases of w_full that belong to the other's blocks, and a wait on a
+            // phase passes while the one before it is not over; that block i - 2 has been used tells that all blocks up to it have come)
+            ok = i < 2 || mbar_wait(smem_u32(&used[s]), ((i >> 1) & 1) ^ 1, status, 63);
+            ok = ok && mbar_wait(smem_u32(&w_full[ws]), (i / W_STAGES) & 1, status, 63);
             if (!(ok = __all_sync(0xffffffffu, ok))) break;
             tc_fence_after();
-            const unsigned char* const w_from = smem + ws * kStageBytes + half * kBoxBytes + row * 128;
-            const uint32_t to = t_w + lanes + s * 96 + half * 16;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            const unsigned char* const w_from = smem + ws * kStageBytes + row * 128;
+            const uint32_t to = t_w + lanes + s * 96;
+#pragma unroll 1
+            for (int g = 0; g < 2 * STEP; ++g) {        // 16 columns
+                const int h = S::TURNS ? g : 2 * half + g;
                 uint32_t p0[8], p1[8], p2[8];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const float4 x = *reinterpret_cast<const float4*>(w_from + (((4 * h + q) ^ (row & 7)) * 16));
+                    const float4 x = *reinterpret_cast<const float4*>(w_from + (h >> 1) * kBoxBytes + (((4 * (h & 1) + q) ^ (row & 7)) * 16));
                     cut2(x.x, x.y, p0[2 * q], p1[2 * q], p2[2 * q]);
                     cut2(x.z, x.w, p0[2 * q + 1], p1[2 * q + 1], p2[2 * q + 1]);
                 }
@@ -227,10 +286,16 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             tmem_st_wait();
             tc_fence_before();
             warp_arrive(smem_u32(&cut[s]));
-            if (i > 0) take(i - 1);
+            if constexpr (S::TURNS) {
+                if (taken + 2 == i) {
+                    take2(taken);
+                    taken = i;
+                }
+            }
+            for (; ok && taken < i; ++taken) take(taken);
             if (!ok) break;
         }
-        if (ok) take(count - 1);
+        for (; ok && taken < count; ++taken) take(taken);
         if (ok) ok = mbar_wait(smem_u32(&all_done), 0, status, 63);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
@@ -283,6 +348,7 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 #pragma unroll
                 for (int p = 0; p < PIECES; ++p) {
                     const int r = (tid >> 4) + p * (A_THREADS / 16);
+                    if (m0 + r >= M && i >= 2) continue;        // both buffers hold zeros there
                     uint2 x0, x1, x2;
                     cut2(next[p].x, next[p].y, x0.x, x1.x, x2.x);
                     cut2(next[p].z, next[p].w, x0.y, x1.y, x2.y);
@@ -322,7 +388,7 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             const int s = i & 1;
             ok = mbar_wait(smem_u32(&cut[s]), (i >> 1) & 1, status, 62);
             if (S::READY) ok = ok && mbar_wait(smem_u32(&a_full[s]), (i >> 1) & 1, status, 62);
-            ok = ok && (i == 0 || mbar_wait(smem_u32(&main_read), (i - 1) & 1, status, 62));
+            ok = ok && (i < MAINS || mbar_wait(smem_u32(&main_read[i % MAINS]), (i / MAINS - 1) & 1, status, 62));
             if (!(ok = __all_sync(0xffffffffu, ok))) break;
             tc_fence_after();
             const uint64_t a0 = smem_desc_sw128(smem_u32(a_s + s * S::A_BYTES));
@@ -330,11 +396,13 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             const uint32_t w0 = t_w + s * 96, w1 = w0 + 32, w2 = w0 + 64;
             if (issuer) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_bf16_tmem_a(t_main, w0 + 8 * k, a0 + 2 * k, idesc, k > 0 ? 1u : 0u);
-                umma_commit(smem_u32(&main_done));
+                for (int k = 0; k < 4; ++k) umma_bf16_tmem_a(t_main + i % MAINS * TOKENS, w0 + 8 * k, a0 + 2 * k, idesc, k > 0 ? 1u : 0u);
+                umma_commit(smem_u32(&main_done[i % MAINS]));
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {       // the smallest first
-                    umma_bf16_tmem_a(t_cross, w2 + 8 * k, a0 + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
+                    umma_bf16_tmem_a(t_cross, w2 + 8 * k, a1 + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
+                    umma_bf16_tmem_a(t_cross, w1 + 8 * k, a2 + 2 * k, idesc, 1u);
+                    umma_bf16_tmem_a(t_cross, w2 + 8 * k, a0 + 2 * k, idesc, 1u);
                     umma_bf16_tmem_a(t_cross, w0 + 8 * k, a2 + 2 * k, idesc, 1u);
                     umma_bf16_tmem_a(t_cross, w1 + 8 * k, a1 + 2 * k, idesc, 1u);
                     umma_bf16_tmem_a(t_cross, w1 + 8 * k, a0 + 2 * k, idesc, 1u);
@@ -358,18 +426,24 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     for (int o = threadIdx.x; o < share * (kRows / 4); o += S::THREADS) {
         const int t = part * share + o / (kRows / 4), col = o % (kRows / 4) * 4, n = n0 + col;
         if (t >= live || n >= N) continue;
-        float4 x = load_cluster_f4(sums + t * kRows + col, 0);
-        for (int p = 1; p < parts; ++p) {
-            const float4 y = load_cluster_f4(sums + t * kRows + col, p);
-            x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
-        }
-        float e[4] = {x.x, x.y, x.z, x.w};
+        float4 of[kMaxParts];               // all on their way at once
+#pragma unroll
+        for (int p = 0; p < kMaxParts; ++p)
+            if (p < parts) of[p] = load_cluster_f4(sums + t * kRows + col, p);
+        float4 x = of[0];
+#pragma unroll
+        for (int p = 1; p < kMaxParts; ++p)
+            if (p < parts) {
+                x.x += of[p].x; x.y += of[p].y; x.z += of[p].z; x.w += of[p].w;
+            }
+        float e[4] = {x.x * kDown, x.y * kDown, x.z * kDown, x.w * kDown};
         float* const out = C + static_cast<size_t>(m0 + t) * ldc + n;
-        if (isnan(x.x) || isnan(x.y) || isnan(x.z) || isnan(x.w)) {
+        if (!(isfinite(x.x) && isfinite(x.y) && isfinite(x.z) && isfinite(x.w))) {
 #pragma unroll 1
             for (int i = 0; i < 4; ++i) {
                 float y = i == 0 ? x.x : i == 1 ? x.y : i == 2 ? x.z : x.w;
-                if (isnan(y) && n + i < N) y = element(A + static_cast<size_t>(m0 + t) * lda, W + static_cast<size_t>(n + i) * ldw, K);
+                if (isfinite(y) || n + i >= N) continue;
+                y = element(A + static_cast<size_t>(m0 + t) * lda, W + static_cast<size_t>(n + i) * ldw, K);
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     if (i == j) e[j] = y;
@@ -422,7 +496,7 @@ int run(const Args& g, cudaStream_t stream) {
     } else {
         map_a = map;
     }
-    const int k_blocks = (g.K + kBlockK - 1) / kBlockK, blocks = (k_blocks + parts_of(g.K) - 1) / parts_of(g.K), parts = (k_blocks + blocks - 1) / blocks;
+    const int k_blocks = (g.K + kBlockK - 1) / kBlockK, blocks = (k_blocks + parts_of(g.N, g.K) - 1) / parts_of(g.N, g.K), parts = (k_blocks + blocks - 1) / blocks;
     // neighbouring CTAs share a tile of W: the second one finds it in L2
     const dim3 grid((g.M + S::TOKENS - 1) / S::TOKENS, (g.N + kRows - 1) / kRows, parts);
     const cudaError_t launched = stride::launch_clusters(gemm_nt_f32_tc_kernel<HALF>, grid, dim3(S::THREADS), S::SMEM, stream, parts, map, map_a, g.A,

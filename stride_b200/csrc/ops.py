@@ -1794,17 +1794,22 @@ def linear_qkv_rope(x, weight, qkv, bias, positions, slot_mapping, cos, sin, k_p
 
 
 # Weights from which on a float32 product runs on the tensor cores, whatever the rows (the bits of a row must not depend on them). Below, a
-# CTA's walk along its part of K, some 0.8 us a block of 64, is longer than the other kernels take: 1024 x 1024 21 us with 1 row and 34 with
-# 301, 8 and 29 there; 2504 x 1040 16 and 28, 10 and 53; 3072 x 3072 24 and 62, 17 and 143.
+# CTA's beginning and end and its walk along its part of K, some 0.75 us a block of 64, are longer than the other kernels take with the one or
+# two rows of most steps. 1, 2, 16 and 301 rows, us (by multiply-adds): 2048 x 2048 7, 7, 9, 42 (5, 6, 15, 73); 4096 x 2048, the line, 10, 11, 12, 70 (7, 7, 16, 127); 3072 x
+# 3072 11, 11, 12, 68 (9, 10, 23, 146); 5120 x 3072 15, 15, 16, 83 (15, 17, 37, 223). The layers of a 3072-wide model, one row: 85 us (83), two 85 (93).
 F32_TC_WEIGHTS = 1 << 23
 
 
 def linear(x, weight, out) -> None:
     """``out = x @ weight.T`` for row-major ``weight`` [out_features, in_features].
 
-    float32 runs the package's own kernels (true 32-bit, order of the sum fixed by
-    the matrix alone): a large matrix as exact products of three bfloat16 parts on
-    the tensor cores, any other by FMA. bfloat16 with few rows (decode steps) runs the package's own kernels:
+    float32 runs the package's own kernels (order of the sum fixed by the matrix
+    alone): any matrix below ``F32_TC_WEIGHTS`` by chains of FMA; a large one on the
+    tensor cores, whose every number is three bfloat16 parts that hold all its bits
+    (eight of the nine products of parts; the one left out is below 2^-30 of a
+    product), its sums of 64 terms cut off towards zero. Its error is no larger than
+    the chains', except for terms of one sign that spread over many powers of two
+    (the kernel's file has the figures). bfloat16 with few rows (decode steps) runs the package's own kernels:
     the tcgen05 kernel for large matrices, the weight-streaming kernel for the
     others; with many rows it calls the library matrix product, as the
     reference's engine does (python/stride_worker/model.py:258-260). ``out`` may
@@ -1816,7 +1821,7 @@ def linear(x, weight, out) -> None:
     if weight.shape[1] != k or out.shape != (m, n):
         raise KernelError(f"linear: shapes {tuple(x.shape)} x {tuple(weight.shape)} -> {tuple(out.shape)} do not agree")
     if x.dtype == torch.float32:
-        if n * k >= F32_TC_WEIGHTS and n >= 512 and k >= 512:
+        if n * k >= F32_TC_WEIGHTS and n >= 512 and k >= 512 and k % 8 == 0 and weight.data_ptr() % 16 == 0:
             # Beyond 48 rows their three parts go through memory (6 bytes a number), some 64 MB at a time: a row's bits do not depend on its batch.
             slab = m if m <= 48 else min(m, max(160, (1 << 26) // (6 * k) // 160 * 160))
             parts = torch.empty(6 * slab * k, dtype=torch.uint8, device=x.device) if m > 48 else None
