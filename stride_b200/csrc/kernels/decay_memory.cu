@@ -479,7 +479,7 @@ chunk_out_kernel(const ChunkArgs p) {
     bool safe = true;
     if (RULE == kChannelDecay) {
         int low = 0;
-        for (int d = threadIdx.x; d < D; d += kChunkThreads) low |= cum[static_cast<size_t>(nt - 1) * HD + d] < kSafeLog;
+        for (int d = threadIdx.x; d < D; d += kChunkThreads) low |= !(cum[static_cast<size_t>(nt - 1) * HD + d] >= kSafeLog);     // (no number: the tokens before it may lie low)
         safe = !__syncthreads_or(low);
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -663,12 +663,13 @@ chunk_out_kernel(const ChunkArgs p) {
     float acc[8][4];
 #pragma unroll
     for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
-    auto step = [&](const float* a_row, const float* b_row) {
+    auto step = [&](const float* a_row, const float* b_row, int from = 0) {     // the warp's tokens from ``from`` on
         const float4 lo = *reinterpret_cast<const float4*>(a_row), hi = *reinterpret_cast<const float4*>(a_row + 4);
         const float4 b = *reinterpret_cast<const float4*>(b_row);
         const float a[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
+            if (r < from) continue;
             acc[r][0] = fmaf(a[r], b.x, acc[r][0]);
             acc[r][1] = fmaf(a[r], b.y, acc[r][1]);
             acc[r][2] = fmaf(a[r], b.z, acc[r][2]);
@@ -720,17 +721,23 @@ chunk_out_kernel(const ChunkArgs p) {
     }
     stage_values<kChunkCols, RULE>(p, kT, row0, nt, h, col0);
     __syncthreads();
-    const int last = min(nt, 8 * warp + 8);         // later tokens have no weight in this warp's rows
+    // Tokens before this warp's eight, then the eight themselves: a later one of those has no weight in an earlier one's row and stays out of
+    // it (0 times a value that is no number would be none).
+    const int own = 8 * warp;
     if constexpr (RULE == kLstm) {
-        for (int j0 = 0; j0 < last; j0 += kRun) {
+        for (int j0 = 0; j0 < own && j0 < nt; j0 += kRun) {
 #pragma unroll 4
-            for (int j = j0; j < min(last, j0 + kRun); ++j) step(aT + j * kLd + 8 * warp, kT + j * kChunkCols + 4 * lane);
-            end_run();
+            for (int j = j0; j < min(min(nt, own), j0 + kRun); ++j) step(aT + j * kLd + own, kT + j * kChunkCols + 4 * lane);
+            if (j0 + kRun <= own) end_run();        // (the run of 16 that the warp's own tokens begin in goes on below)
         }
     } else {
 #pragma unroll 4
-        for (int j = 0; j < last; ++j) step(aT + j * kLd + 8 * warp, kT + j * kChunkCols + 4 * lane);
+        for (int j = 0; j < min(nt, own); ++j) step(aT + j * kLd + own, kT + j * kChunkCols + 4 * lane);
     }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+        if (own + u < nt) step(aT + (own + u) * kLd + own, kT + (own + u) * kChunkCols + 4 * lane, u);
+    if constexpr (RULE == kLstm) end_run();
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int i = 8 * warp + r;
