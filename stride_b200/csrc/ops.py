@@ -231,7 +231,7 @@ _CLASS_OF = {
     "stride_paged_prefill_attention_tc": "attention (prefill, tcgen05)", "stride_sample_rows": "sampling", "stride_sample_ranked": "sampling",
     "stride_add_dyt": "norm", "stride_add_scaled": "residual sum", "stride_token_side": "token side input",
     "stride_latent_prepare": "latent norm + rotation + cache write", "stride_head_gemm": "per-head product",
-    "stride_latent_attention": "attention (latent, exact kernel)", "stride_latent_attention_tc": "attention (latent, tensor cores)",
+    "stride_latent_attention": "attention (latent, exact kernel)", "stride_latent_attention_tc": "attention (latent, tensor cores)", "stride_latent_attention_tc5": "attention (latent, tensor cores)",
     "stride_side_gate": "token side input", "stride_side_norm_add": "token side input", "stride_cast_rows": "token side input",
     "stride_moe_select": "router", "stride_moe_select_sigmoid": "router", "stride_moe_select_groups": "router", "stride_head_gate": "gates and caps",
     "stride_add_sinusoid": "embedding", "stride_norm_add": "norm", "stride_qkv_unit_norm": "head norms + cache write",
