@@ -535,7 +535,8 @@ __global__ void scale_rows_kernel(const __nv_bfloat16* __restrict__ xt, const fl
 // A request's state slot starts at zero: a sequence whose first token of this step sits at position 0 is at its
 // beginning (a new request, or one that is recomputed after it was preempted), so the row of its slot is cleared
 // before any layer runs. Reads only the step's index arrays, so it can sit in a captured graph. One row of CTAs
-// per sequence of the layout (padded ones have q_len 0), 4-byte words.
+// per entry of the arrays, which are the step's requests, or a captured batch's slots (padded ones have q_len 0); 16 bytes a
+// store where rows are whole packs on their boundaries, else 4.
 // Several state tensors in one launch (grid z), each with rows of its own length.
 constexpr int kMaxStates = 64;
 struct StateList {
@@ -653,7 +654,7 @@ int stride_add_rmsnorm(float* residual, const void* delta, const float* weight, 
 }
 
 // Clears the state rows [num_slots, row_bytes] of the sequences that start at position 0 in this step.
-// `seq_cap`: entries of state_slot / q_start / q_len (the layout's capacity; padded sequences have q_len 0).
+// `seq_cap`: entries of state_slot / q_start / q_len (the step's requests, or a captured batch's slots; padded ones have q_len 0).
 // `count` state tensors of num_slots rows each: host arrays of their device pointers and row lengths in bytes.
 int stride_zero_fresh_states(void* const* states, const long long* row_bytes, int count, int num_slots, const int32_t* state_slot,
                              const int32_t* q_start, const int32_t* q_len, const int32_t* positions, int seq_cap, cudaStream_t stream) {

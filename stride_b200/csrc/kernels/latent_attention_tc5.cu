@@ -155,6 +155,8 @@ latent_attention_tc5_kernel(const __nv_bfloat16* __restrict__ qa, __nv_bfloat16*
                     f = expf(top - now);
                     top = now;
                 }
+                // (This wait may skip phases, and one on phase j - 1 would pass while phase j - 2 is not over. It is: the scores of tile j, which
+                // have been read above, were made from keys that came into the place of tile j - 2 only after its second product.)
                 ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&pv_done), (j - 1) & 1, status, 73));
                 if (!ok) break;
                 tc_fence_after();

@@ -58,12 +58,13 @@ from .base import CacheRequest, Mixer, Projection, TensorDecl, build_part, regis
 class LatentAttention(Mixer):
     lazy_output = True
     # Portions go over expanded keys where one of their requests holds this many: the folded form walks a request's keys in one CTA, a
-    # tile of 64 after the other at some 12 us each on mma.sync (2.3 us on tcgen05 since, which leaves the rule where it was: the roundings
-    # of the two forms differ), however few the tokens. On mma.sync two such layers of 16 heads and nothing else, a step on the
-    # latents / expanded: 33 tokens behind 2,000 841 / 437 us, 10 behind 30,000 9.3 / 1.7 ms, 2,000 alone 1738 / 556 us. Below it the
-    # folded form has fewer launches (256 alone 400 / 450 us, 64 requests of 8 515 / 610). Many requests make the product that
-    # expands long while the walk stays what the longest one's is (16 of 16 tokens behind 1,000 556 / 580 us): at most
-    # EXPAND_SHARE times the longest one's keys in all.
+    # tile of 64 after the other at 2.3 us each, however few the tokens. Two such layers of 16 heads and nothing else, a step on the latents /
+    # expanded, us: 2,000 tokens alone 911 / 586, 2,000 behind 8,000 3,644 / 1,034, 10 behind 30,000 2,937 / 1,831, 33 behind 2,000 512 / 498,
+    # 1,000 alone 525 / 496, 512 alone 405 / 457, 100 behind 600 373 / 420. The line was drawn when the folded form ran on mma.sync (12 us a tile,
+    # 2,000 alone 1,738); some 1,000 keys are where the forms are level now, and from 512 to there the latents would be 10 % faster. (The forms'
+    # roundings are alike: their outputs differ by 0.0013 to 0.0015, and neither is further from 64 bits.) Below it the folded form has
+    # fewer launches. Many requests make the product that expands long while the walk stays what the longest one's is: at most
+    # EXPAND_SHARE times the longest one's keys in all (on mma.sync 16 of 16 tokens behind 1,000 556 / 580).
     EXPAND_KEYS = 512
     EXPAND_SHARE = 8
     MAX_EXPANDED_BYTES = 1 << 28      # keys and values of a step, expanded, at most (the buffer, whose rows are a power of two)
