@@ -10,7 +10,7 @@
 // run from zero over 64 terms at a time, whose 12 bits then lose nothing unless they lie 2^6 and more apart (parts of 8 bits made sums of terms
 // of one sign come out low, by 1.1e-7 to 1.5e-7), and those sums are added up in registers by rounded additions; the seven others, 2^-5 and
 // less of the whole and, by the rounding of the parts, of either sign, stay in an accumulator of their own over a part of K. K is cut into up to
-// eight parts, a CTA each, which meet in a cluster and are added up in order. N and K alone decide all this, so a row's bits do not depend on
+// eight parts, a CTA (or half a CTA's time) each, which meet in a cluster and are added up by twos and then in order. N and K alone decide all this, so a row's bits do not depend on
 // M, nor on the row's place in the batch.
 //
 // D = W A^T: 128 rows of W are the M side, up to 160 rows of A (tokens) the N side, so that a few tokens cost few columns and a step's
@@ -26,7 +26,7 @@
 // What comes out as no finite number is computed again as the chains of gemm_f32.cu.
 //
 // us (gemm_f32.cu), one row: 5120 x 3072 15.0 (15.1), 3072 x 3072 11.0 (8.8), 16384 x 3072 35 (38), 3072 x 8192 24 (21), 128256 x 3072 249 (304); two rows
-// 15.2 (17.1), 11.0 (9.8), 36 (42), 24 (24), 251 (296); 301 rows 83 (223), 68 (146), 188 (665), 129 (376). Bound by the waits, fences and arrivals between
+// 15.2 (17.1), 11.0 (9.8), 36 (42), 24 (24), 251 (296); 301 rows 76 (223), 60 (146), 190 (665), 129 (376). Bound by the waits, fences and arrivals between
 // the warps where rows are few (some 0.75 us a block and CTA), by the products beyond (8 x 2 x 301 x 16384 x 3072 at 1.3 PFLOP/s). Six products of
 // parts of 8 bits took 301 rows in 58, 55, 166 and 110 us, with the errors named above. Error against 64 bits of sum |a w|, K = 3072, rms: normal
 // numbers 2.3e-9 (1.0e-8), of one sign 5.0e-8 (1.0e-7), one term 2.5e-8 (the same). One kind measured goes the other way: terms of one sign that lie very
@@ -47,7 +47,7 @@ constexpr int kBoxBytes = kRows * 128, kStageBytes = 2 * kBoxBytes;       // 32 
 // Parts of K, each with CTAs of its own: as many as make the shortest walk for up to 16 tokens, where two CTAs share an SM, some 256 run side by
 // side (clusters do not fill a GPC to the last SM; of seven they fill it worst) and beginning and end cost a CTA about four blocks. N and K
 // alone decide. One row, us, by parts: 3072 x 3072 1 38.9, 2 20.8, 4 12.6, 6 12.8, 8 11.0; 16384 x 3072 1 59, 2 35.4, 3 41.7, 8 46.6; 28672 x 4096 1 81, 2 90, 8
-// 97. With many rows fewer parts would do: 301 of 3072 x 3072 49 us in five and 68 in eight, of 5120 x 3072 68 in three and 83 in six.
+// 97. With many rows fewer parts would do (301 of 3072 x 3072 49 us in five, 60 in eight as four CTAs).
 __host__ inline int parts_of(int N, int K) {
     const long long tiles = (N + kRows - 1) / kRows;
     const int blocks = (K + kBlockK - 1) / kBlockK;
@@ -61,6 +61,21 @@ __host__ inline int parts_of(int N, int K) {
         }
     }
     return best;
+}
+
+// Parts that a CTA of 48 and more tokens, one an SM, takes one after the other, 1 or 2: the shorter walk, where beginning, end and exchange cost a
+// CTA about eight blocks and some 128 run side by side (148 in clusters of one or two). A row's bits are the same: two parts' sums are added up
+// first either way. us (one part a CTA): 4096 x 4096 48 rows 24 (38), 301 76 (102); 3072 x 3072 19 (23), 60 (68); 5120 x 3072 24 (27), 75 (83); 4096 x 14336 67 (101),
+// 231 (255). Of two parts in all 301 rows of 16384 x 3072 take 195 (188): left apart. 6144 x 4096, five parts, 48 rows: 65 in clusters of three, which do not
+// all fit at once, 37 in five.
+__host__ inline int parts_a_cta(int M, int N, int tokens, int parts, int blocks) {
+    if (parts < 3) return 1;
+    const long long tiles = static_cast<long long>((N + kRows - 1) / kRows) * ((M + tokens - 1) / tokens);
+    auto walk = [&](int per) {
+        const int ctas = (parts + per - 1) / per, room = ctas <= 2 ? 148 : 128;
+        return (tiles * ctas + room - 1) / room * (per * blocks + 7 + per);
+    };
+    return walk(2) <= walk(1) ? 2 : 1;
 }
 
 // Eight columns of 32 lanes; tmem_ld_wait() before anybody uses them.
@@ -174,7 +189,8 @@ struct Shape {
     static constexpr int THREADS = kWThreads + A_THREADS + 64;
 };
 
-template <int HALF>
+// PAIRS: a CTA has two parts of K, one after the other (see parts_a_cta). A kernel of its own: the first part's sums, kept meanwhile, cost the other 5 %.
+template <int HALF, bool PAIRS>
 __global__ void __launch_bounds__(Shape<HALF>::THREADS, Shape<HALF>::CTAS)
 gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const float* __restrict__ A,
                       const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc, int blocks, int a_vec,
@@ -187,13 +203,14 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     unsigned char* const smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* const a_s = smem + W_STAGES * kStageBytes;
     __shared__ __align__(8) uint64_t w_full[W_STAGES], w_empty[W_STAGES];
-    __shared__ __align__(8) uint64_t cut[2], used[2], a_full[2], main_done[S::MAINS], main_read[S::MAINS], all_done;
+    __shared__ __align__(8) uint64_t cut[2], used[2], a_full[2], main_done[S::MAINS], main_read[S::MAINS], all_done, cross_read;
     __shared__ uint32_t tmem_slot;
 
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * TOKENS, n0 = blockIdx.y * kRows, part = blockIdx.z, parts = gridDim.z;
-    const int k_blocks = (K + kBlockK - 1) / kBlockK, first = part * blocks, count = min(blocks, k_blocks - first);   // 64 columns each, one at least
+    const int m0 = blockIdx.x * TOKENS, n0 = blockIdx.y * kRows, part = blockIdx.z, parts = gridDim.z, span = PAIRS ? 2 * blocks : blocks;
+    const int k_blocks = (K + kBlockK - 1) / kBlockK, first = part * span, count = min(span, k_blocks - first);     // 64 columns each, one at least
+    const bool two = PAIRS && count > blocks;
     if (threadIdx.x == 0) {
         for (int s = 0; s < W_STAGES; ++s) {
             mbar_init(smem_u32(&w_full[s]), 1);
@@ -209,6 +226,7 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             mbar_init(smem_u32(&main_read[s]), kWThreads / 32);
         }
         mbar_init(smem_u32(&all_done), 1);
+        mbar_init(smem_u32(&cross_read), kWThreads / 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == MMA_WARP) tmem_alloc(smem_u32(&tmem_slot), S::COLS);
@@ -249,7 +267,7 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             tc_fence_before();
             warp_arrive(smem_u32(&main_read[i % MAINS]));
         };
-        auto take2 = [&](int i) {           // of two blocks at once
+        [[maybe_unused]] auto take2 = [&](int i) {           // of two blocks at once
             if (!(ok = __all_sync(0xffffffffu, wait_main(i) && wait_main(i + 1)))) return;
             tc_fence_after();
             add(t_main + i % MAINS * TOKENS, t_main + (i + 1) % MAINS * TOKENS);
@@ -257,7 +275,34 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             __syncwarp();
             if (lane < 2) mbar_arrive(smem_u32(&main_read[lane]));
         };
+        auto finish = [&](int phase) {      // a part's other products
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&all_done), phase, status, 63));
+            if (!ok) return;
+            tc_fence_after();
+            add(t_cross);
+            tc_fence_before();
+        };
+        float kept[PAIRS ? HALF : 1];    // the first part's sums
         int taken = 0;
+        auto take_to = [&](int end) {
+            if (S::TURNS && taken + 2 == end && !(two && (end == blocks || end == blocks + 1))) {
+                take2(taken);
+                taken = end;
+            }
+            for (; ok && taken < end; ++taken) {
+                take(taken);
+                if constexpr (PAIRS) {
+                    if (!ok || !two || taken + 1 != blocks) continue;
+                    finish(0);
+                    warp_arrive(smem_u32(&cross_read));
+#pragma unroll
+                    for (int j = 0; j < HALF; ++j) {
+                        kept[j] = acc[j];
+                        acc[j] = 0.f;
+                    }
+                }
+            }
+        };
         for (int i = S::TURNS ? half : 0; i < count; i += STEP) {
             const int s = i & 1, ws = i % W_STAGES;
             // (in this order: a warpgroup that takes turns has not seen the phases of w_full that belong to the other's blocks, and a wait on a
@@ -286,21 +331,17 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             tmem_st_wait();
             tc_fence_before();
             warp_arrive(smem_u32(&cut[s]));
-            if constexpr (S::TURNS) {
-                if (taken + 2 == i) {
-                    take2(taken);
-                    taken = i;
-                }
-            }
-            for (; ok && taken < i; ++taken) take(taken);
+            take_to(i);
             if (!ok) break;
         }
-        for (; ok && taken < count; ++taken) take(taken);
-        if (ok) ok = mbar_wait(smem_u32(&all_done), 0, status, 63);
-        ok = __all_sync(0xffffffffu, ok);
-        tc_fence_after();
-        if (ok) add(t_cross);
-        tc_fence_before();
+        if (ok) take_to(count);
+        if (ok) finish(two ? 1 : 0);
+        if constexpr (PAIRS) {
+            if (two) {
+#pragma unroll
+                for (int j = 0; j < HALF; ++j) acc[j] = kept[j] + acc[j];
+            }
+        }
         float* const to = reinterpret_cast<float*>(smem) + half * HALF * kRows + row;
         named_barrier(1, kWThreads);        // the last tile of W has been read by all of these warps: the sums take the ring's place
 #pragma unroll
@@ -383,12 +424,14 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         for (int j = i > W_STAGES ? i - W_STAGES : 0; j < i; ++j) mbar_wait(smem_u32(&w_full[j % W_STAGES]), (j / W_STAGES) & 1, status, 61);
     } else {
         const bool issuer = elect_one();
+        int phase = 0;
         const uint32_t idesc = instr_desc_bf16(kRows, min(TOKENS, (M - m0 + 15) / 16 * 16), false);
         for (int i = 0; i < count; ++i) {
             const int s = i & 1;
             ok = mbar_wait(smem_u32(&cut[s]), (i >> 1) & 1, status, 62);
             if (S::READY) ok = ok && mbar_wait(smem_u32(&a_full[s]), (i >> 1) & 1, status, 62);
             ok = ok && (i < MAINS || mbar_wait(smem_u32(&main_read[i % MAINS]), (i / MAINS - 1) & 1, status, 62));
+            if (two && i == blocks) ok = ok && mbar_wait(smem_u32(&cross_read), 0, status, 62);
             if (!(ok = __all_sync(0xffffffffu, ok))) break;
             tc_fence_after();
             const uint64_t a0 = smem_desc_sw128(smem_u32(a_s + s * S::A_BYTES));
@@ -400,7 +443,7 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 umma_commit(smem_u32(&main_done[i % MAINS]));
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {       // the smallest first
-                    umma_bf16_tmem_a(t_cross, w2 + 8 * k, a1 + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
+                    umma_bf16_tmem_a(t_cross, w2 + 8 * k, a1 + 2 * k, idesc, (i > 0 && !(two && i == blocks)) || k > 0 ? 1u : 0u);
                     umma_bf16_tmem_a(t_cross, w1 + 8 * k, a2 + 2 * k, idesc, 1u);
                     umma_bf16_tmem_a(t_cross, w2 + 8 * k, a0 + 2 * k, idesc, 1u);
                     umma_bf16_tmem_a(t_cross, w0 + 8 * k, a2 + 2 * k, idesc, 1u);
@@ -409,12 +452,14 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     umma_bf16_tmem_a(t_cross, w0 + 8 * k, a1 + 2 * k, idesc, 1u);
                 }
                 umma_commit(smem_u32(&used[s]));
+                if (two && i + 1 == blocks) umma_commit(smem_u32(&all_done));
             }
             __syncwarp();
+            if (two && i + 1 == blocks) phase = 1;
         }
         if (issuer) umma_commit(smem_u32(&all_done));
         __syncwarp();
-        mbar_wait(smem_u32(&all_done), 0, status, 62);
+        mbar_wait(smem_u32(&all_done), phase, status, 62);
     }
     float* const sums = reinterpret_cast<float*>(smem);     // [token][row of W]
     __syncthreads();
@@ -426,15 +471,25 @@ gemm_nt_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     for (int o = threadIdx.x; o < share * (kRows / 4); o += S::THREADS) {
         const int t = part * share + o / (kRows / 4), col = o % (kRows / 4) * 4, n = n0 + col;
         if (t >= live || n >= N) continue;
-        float4 of[kMaxParts];               // all on their way at once
+        float4 of[kMaxParts] = {};          // all on their way at once
 #pragma unroll
         for (int p = 0; p < kMaxParts; ++p)
             if (p < parts) of[p] = load_cluster_f4(sums + t * kRows + col, p);
-        float4 x = of[0];
+        // two parts' sums, and then those of the pairs in order
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int p = 1; p < kMaxParts; ++p)
+        for (int p = 0; p < kMaxParts; p += 2)
             if (p < parts) {
-                x.x += of[p].x; x.y += of[p].y; x.z += of[p].z; x.w += of[p].w;
+                const float4 a = of[p], b = of[p + 1];
+                const bool with = p + 1 < parts;
+                if (PAIRS) {                // of[p] is a pair's sum already
+                    x.x += a.x; x.y += a.y; x.z += a.z; x.w += a.w;
+                    if (with) { x.x += b.x; x.y += b.y; x.z += b.z; x.w += b.w; }
+                } else if (with) {
+                    x.x += a.x + b.x; x.y += a.y + b.y; x.z += a.z + b.z; x.w += a.w + b.w;
+                } else {
+                    x.x += a.x; x.y += a.y; x.z += a.z; x.w += a.w;
+                }
             }
         float e[4] = {x.x * kDown, x.y * kDown, x.z * kDown, x.w * kDown};
         float* const out = C + static_cast<size_t>(m0 + t) * ldc + n;
@@ -479,11 +534,18 @@ struct Args {
     int* status;
 };
 
+template <int HALF, bool PAIRS>
+cudaError_t launch_product(const Args& g, dim3 grid, const CUtensorMap& map, const CUtensorMap& map_a, int blocks, int a_vec, cudaStream_t stream) {
+    using S = Shape<HALF>;
+    const cudaError_t e = allow_shared<gemm_nt_f32_tc_kernel<HALF, PAIRS>>(S::SMEM);
+    if (e != cudaSuccess) return e;
+    return stride::launch_clusters(gemm_nt_f32_tc_kernel<HALF, PAIRS>, grid, dim3(S::THREADS), S::SMEM, stream, static_cast<int>(grid.z), map, map_a, g.A, g.W,
+                                   g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc, blocks, a_vec, g.status);
+}
+
 template <int HALF>
 int run(const Args& g, cudaStream_t stream) {
     using S = Shape<HALF>;
-    const cudaError_t e = allow_shared<gemm_nt_f32_tc_kernel<HALF>>(S::SMEM);
-    if (e != cudaSuccess) return static_cast<int>(e);
     CUtensorMap map, map_a;
     if (!make_map_f32(&map, g.W, g.N, g.K, g.ldw)) return STRIDE_UNSUPPORTED;
     const int a_vec = (g.lda & 3) == 0 && (reinterpret_cast<uintptr_t>(g.A) & 15) == 0;
@@ -496,11 +558,15 @@ int run(const Args& g, cudaStream_t stream) {
     } else {
         map_a = map;
     }
-    const int k_blocks = (g.K + kBlockK - 1) / kBlockK, blocks = (k_blocks + parts_of(g.N, g.K) - 1) / parts_of(g.N, g.K), parts = (k_blocks + blocks - 1) / blocks;
+    const int k_blocks = (g.K + kBlockK - 1) / kBlockK, wanted = parts_of(g.N, g.K), blocks = (k_blocks + wanted - 1) / wanted;
+    const int parts = (k_blocks + blocks - 1) / blocks, per = S::CTAS == 1 ? parts_a_cta(g.M, g.N, S::TOKENS, parts, blocks) : 1;
     // neighbouring CTAs share a tile of W: the second one finds it in L2
-    const dim3 grid((g.M + S::TOKENS - 1) / S::TOKENS, (g.N + kRows - 1) / kRows, parts);
-    const cudaError_t launched = stride::launch_clusters(gemm_nt_f32_tc_kernel<HALF>, grid, dim3(S::THREADS), S::SMEM, stream, parts, map, map_a, g.A,
-                                                         g.W, g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc, blocks, a_vec, g.status);
+    const dim3 grid((g.M + S::TOKENS - 1) / S::TOKENS, (g.N + kRows - 1) / kRows, (parts + per - 1) / per);
+    cudaError_t launched;
+    if constexpr (S::CTAS == 1)
+        launched = per == 2 ? launch_product<HALF, true>(g, grid, map, map_a, blocks, a_vec, stream) : launch_product<HALF, false>(g, grid, map, map_a, blocks, a_vec, stream);
+    else
+        launched = launch_product<HALF, false>(g, grid, map, map_a, blocks, a_vec, stream);
     return launched != cudaSuccess ? static_cast<int>(launched) : STRIDE_LAUNCH_STATUS();
 }
 
@@ -509,16 +575,14 @@ int run(const Args& g, cudaStream_t stream) {
 
 extern "C" {
 
-// Bytes of scratch for M rows of A: the parts of more rows than the product cuts up by itself.
-long long stride_gemm_nt_f32_tc_scratch(int M, int K) { return M > 48 ? 6LL * M * K : 0; }
-
-// Returns -2 for what it does not take, which depends on the matrix W alone.
+// Scratch: 6 bytes a number of A beyond 48 rows, the parts of more rows than the product cuts up by itself. Returns -2 for what it does not take, which
+// depends on the matrix W alone.
 int stride_gemm_nt_f32_tc(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, void* scratch,
                           long long scratch_bytes, int* status, cudaStream_t stream) {
     if (M < 0 || N <= 0 || K <= 0 || lda < K || ldw < K || ldc < N || status == nullptr) return STRIDE_BAD_ARGUMENT;
     if (N < 512 || K < 512 || K % 8 || ldw % 4 || reinterpret_cast<uintptr_t>(W) % 16 || N > 65535 * 128) return STRIDE_UNSUPPORTED;
     if (M == 0) return 0;
-    if (scratch_bytes < stride_gemm_nt_f32_tc_scratch(M, K) || reinterpret_cast<uintptr_t>(scratch) % 16) return STRIDE_BAD_ARGUMENT;
+    if (scratch_bytes < (M > 48 ? 6LL * M * K : 0) || reinterpret_cast<uintptr_t>(scratch) % 16) return STRIDE_BAD_ARGUMENT;
     const stride::f32tc::Args g{A, W, C, M, N, K, lda, ldw, ldc, static_cast<__nv_bfloat16*>(scratch), status};
     if (M <= 16) return stride::f32tc::run<8>(g, stream);
     if (M <= 48) return stride::f32tc::run<24>(g, stream);

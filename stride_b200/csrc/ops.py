@@ -1796,8 +1796,8 @@ def linear_qkv_rope(x, weight, qkv, bias, positions, slot_mapping, cos, sin, k_p
 
 # Weights from which on a float32 product runs on the tensor cores, whatever the rows (the bits of a row must not depend on them). Below, a
 # CTA's beginning and end and its walk along its part of K, some 0.75 us a block of 64, are longer than the other kernels take with the one or
-# two rows of most steps. 1, 2, 16 and 301 rows, us (by multiply-adds): 2048 x 2048 7, 7, 9, 42 (5, 6, 15, 73); 4096 x 2048, the line, 10, 11, 12, 70 (7, 7, 16, 127); 3072 x
-# 3072 11, 11, 12, 68 (9, 10, 23, 146); 5120 x 3072 15, 15, 16, 83 (15, 17, 37, 223). The layers of a 3072-wide model, one row: 85 us (83), two 85 (93).
+# two rows of most steps. 1, 2, 16 and 301 rows, us (by multiply-adds): 2048 x 2048 7, 7, 8, 25 (5, 6, 15, 73); 4096 x 2048, the line, 10, 11, 12, 48 (7, 7, 16, 127); 3072 x
+# 3072 11, 11, 12, 60 (9, 10, 23, 146); 5120 x 3072 15, 15, 16, 76 (15, 17, 37, 223). The layers of a 3072-wide model, one row: 85 us (83), two 85 (93).
 F32_TC_WEIGHTS = 1 << 23
 
 
