@@ -71,7 +71,7 @@ def test_a_decay_that_is_no_number_leaves_the_strong_decays_before_it():
     from stride_b200.csrc import ops
     proj, logit, gates, state = inputs(2)
     logit[:40] = -160.0         # e^-10 a token: their products fall below what float32 can turn round
-    logit[45, 7] = float("nan")
+    logit[45, :D] = float("nan")        # every channel of the first head: none is left to tell of the strong ones
     (o, _), (oc, _) = both(ops, "channel", proj, logit, gates, state)
     assert torch.equal(o.isnan(), oc.isnan()) and bool(oc[:45].isfinite().all()) and bool(oc[45, :DV].isnan().all())
     ok = o.isfinite()
