@@ -15,6 +15,9 @@
 // (q already times `q_scale`, the two gate logarithms computed once a token). The order of every sum depends on the token
 // only, so a token's output is bitwise the same in a whole prompt, in portions or decoded alone.
 //
+// All CTAs of a head start from the same n and m and end with the same new ones; the last of them to end stores these (a ticket a head and
+// request, which it leaves at zero): a CTA that came late, behind others that had ended, would otherwise start from what they stored.
+//
 // State row of a request: S [H, D, DV], then n [H, D], then m [H].
 #include "common.cuh"
 
@@ -36,6 +39,7 @@ struct LstmArgs {
     const int32_t* q_start;
     const int32_t* q_len;
     const int32_t* state_slot;
+    int* tickets;           // [requests, H], zero between launches
     int H, D, DV;
 };
 
@@ -205,9 +209,23 @@ mlstm_scan_kernel(const LstmArgs p) {
     for (int r = 0; r < R; ++r) {
         const int i = row_of(r);
         if (i < D && j < DV) S_g[static_cast<size_t>(i) * DV + j] = S[r];
-        if (blockIdx.x == 0 && jc == 0 && i < D) n_g[i] = nn[r];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *m_g = m;
+    __shared__ bool s_last;
+    if (threadIdx.x == 0) {         // (every thread of the CTA has read n and m: the barrier behind the last chunk)
+        __threadfence();
+        int* const ticket = p.tickets + static_cast<size_t>(seq) * H + h;
+        s_last = atomicAdd(ticket, 1) == static_cast<int>(gridDim.x) - 1;
+        if (s_last) {
+            *ticket = 0;
+            *m_g = m;
+        }
+    }
+    __syncthreads();
+    if (s_last && jc == 0) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (row_of(r) < D) n_g[row_of(r)] = nn[r];
+    }
 }
 
 }  // namespace stride
@@ -216,12 +234,12 @@ using namespace stride;
 
 extern "C" {
 
-// One launch for every request of the step (grid z: the step's sequence slots, empty ones return at once).
+// One launch for every request of the step (grid z: the step's sequence slots, empty ones return at once). `tickets`: num_seqs * H words, zero.
 int stride_mlstm_scan(const void* proj, int ld, int q_off, int k_off, int v_off, const float* gates, int ld_gates, const float* bias_i,
                       const float* bias_f, float cap, float q_scale, float* o, float* state, long long state_stride,
-                      const int32_t* q_start, const int32_t* q_len, const int32_t* state_slot, int num_seqs, int H, int D, int DV,
-                      int dtype, cudaStream_t stream) {
-    if (num_seqs < 0 || H <= 0 || D <= 0 || DV <= 0 || ld <= 0 || ld_gates < 2 * H || !(cap > 0.f) || q_off < 0 || k_off < 0 || v_off < 0)
+                      const int32_t* q_start, const int32_t* q_len, const int32_t* state_slot, int* tickets, int num_seqs, int H, int D,
+                      int DV, int dtype, cudaStream_t stream) {
+    if (tickets == nullptr || num_seqs < 0 || H <= 0 || D <= 0 || DV <= 0 || ld <= 0 || ld_gates < 2 * H || !(cap > 0.f) || q_off < 0 || k_off < 0 || v_off < 0)
         return STRIDE_BAD_ARGUMENT;
     if (dtype != STRIDE_DTYPE_F32 && dtype != STRIDE_DTYPE_BF16) return STRIDE_BAD_ARGUMENT;
     if (state_stride < static_cast<long long>(H) * D * DV + static_cast<long long>(H) * D + H) return STRIDE_BAD_ARGUMENT;
@@ -231,7 +249,7 @@ int stride_mlstm_scan(const void* proj, int ld, int q_off, int k_off, int v_off,
     a.proj = proj; a.ld = ld; a.q_off = q_off; a.k_off = k_off; a.v_off = v_off;
     a.gates = gates; a.ld_gates = ld_gates; a.bias_i = bias_i; a.bias_f = bias_f; a.cap = cap; a.q_scale = q_scale;
     a.o = o; a.state = state; a.state_stride = state_stride; a.q_start = q_start; a.q_len = q_len; a.state_slot = state_slot;
-    a.H = H; a.D = D; a.DV = DV;
+    a.tickets = tickets; a.H = H; a.D = D; a.DV = DV;
     const dim3 block(kLstmThreads);
     // a chain of tokens keeps few CTAs busy for long: launched without an early start behind the kernel before it.
     // Heads of up to 32 rows: 8 lanes a column; larger ones 16 lanes, so that a lane holds at most 16 rows.

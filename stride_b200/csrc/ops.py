@@ -190,7 +190,7 @@ _SIGNATURES = {
                                              c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                              c_void_p]),
     "stride_mlstm_scan": ("mlstm", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_float, c_void_p,
-                                    c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]),
+                                    c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "stride_pointwise": ("pointwise", [c_void_p, c_void_p, c_int, c_float, c_longlong, c_int, c_void_p]),
     "stride_weighted_sum": ("pointwise", [c_void_p, c_void_p, c_float, c_void_p, c_float, c_longlong, c_int, c_void_p]),
     "stride_delta_prepare": ("linear_recurrence", [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_longlong,
@@ -649,19 +649,24 @@ def mlstm_state_floats(H: int, D: int, DV: int) -> int:
 
 
 def mlstm_scan(proj, q_off: int, k_off: int, v_off: int, gates, bias_i, bias_f, cap: float, q_scale: float, o, state, q_start, q_len,
-               state_slot, num_seqs: int, H: int, D: int, DV: int) -> None:
+               state_slot, num_seqs: int, H: int, D: int, DV: int, tickets=None) -> None:
     """The matrix memory with exponential gates over every request of the step, in token order. ``proj`` [tokens, ld] holds
     q, k ([H, D]) and v ([H, DV]) from the given columns on; ``gates`` (float32 [tokens, >= 2H]) the projections of the input
     gates (columns 0..H-1) and the forget gates (H..2H-1), to which ``bias_i`` / ``bias_f`` are added before
-    ``cap * tanh(. / cap)``. ``o`` [tokens, H * DV] float32; ``state`` [slots, >= mlstm_state_floats]: S, n, m per head."""
+    ``cap * tanh(. / cap)``. ``o`` [tokens, H * DV] float32; ``state`` [slots, >= mlstm_state_floats]: S, n, m per head. ``tickets``: int32, zero
+    and left at zero, one a request and head (None: made for the call)."""
+    if tickets is None:
+        tickets = torch.zeros(int(num_seqs) * H, dtype=torch.int32, device=proj.device)
+    if tickets.numel() < int(num_seqs) * H:
+        raise KernelError("mlstm_scan: too few tickets")
     if state.shape[1] < mlstm_state_floats(H, D, DV) or o.shape[1] != H * DV or gates.shape[1] < 2 * H:
         raise KernelError("mlstm_scan: shapes do not agree")
     _check(_fn("stride_mlstm_scan")(
         _dev(proj, "proj"), proj.shape[1], int(q_off), int(k_off), int(v_off), _dev(gates, "gates", torch.float32), gates.shape[1],
         _dev(bias_i, "bias_i", torch.float32), _dev(bias_f, "bias_f", torch.float32), float(cap), float(q_scale),
         _dev(o, "o", torch.float32), *_state_rows(state), _dev(q_start, "q_start", torch.int32),
-        _dev(q_len, "q_len", torch.int32), _dev(state_slot, "state_slot", torch.int32), int(num_seqs), H, D, DV, _code(proj.dtype),
-        _stream()), "mlstm_scan")
+        _dev(q_len, "q_len", torch.int32), _dev(state_slot, "state_slot", torch.int32), _dev(tickets, "tickets", torch.int32), int(num_seqs), H, D, DV,
+        _code(proj.dtype), _stream()), "mlstm_scan")
 
 
 # Portions of at least this many tokens run chunk by chunk in bfloat16 models (0: none do).

@@ -121,7 +121,7 @@ class MatrixLstmMixer(Mixer):
             first = portions
         if slots > first:
             ops.mlstm_scan(proj, *columns, *gate_args, o, cache.state, ctx.q_start[first:], ctx.q_len[first:], ctx.state_slot[first:], slots - first,
-                           *sizes)
+                           *sizes, tickets=self.rt.scratch("mlstm_tickets", (slots - first) * self.H, torch.int32))
         mixed = self.rt.buffer("mlstm_mixed", tokens, self.HV)
         ops.head_norm_gate(o, self.norm_w, True, proj, "sigmoid_compute", mixed, self.H, self.DV, self.norm_eps, gate_off=self.g_off)
         if lazy_output:
