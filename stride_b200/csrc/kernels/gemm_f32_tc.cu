@@ -29,7 +29,7 @@
 // 15.2 (17.1), 11.0 (9.8), 36 (42), 24 (24), 251 (296); 301 rows 76 (223), 60 (146), 190 (665), 129 (376). Bound by the waits, fences and arrivals between
 // the warps where rows are few (some 0.75 us a block and CTA), by the products beyond (8 x 2 x 301 x 16384 x 3072 at 1.3 PFLOP/s). Six products of
 // parts of 8 bits took 301 rows in 58, 55, 166 and 110 us, with the errors named above. Error against 64 bits of sum |a w|, K = 3072, rms: normal
-// numbers 2.3e-9 (1.0e-8), of one sign 5.0e-8 (1.0e-7), one term 2.5e-8 (the same). One kind measured goes the other way: terms of one sign that lie very
+// numbers 2.2e-9 (1.0e-8), of one sign 4.4e-8 (1.0e-7), one term 2.5e-8 (the same). One kind measured goes the other way: terms of one sign that lie very
 // far apart (log-normal, sigma 3, in both operands) 2.8e-7 to 3.0e-7 whatever K (1.1e-7 at 512, 1.6e-7 at 1024, 4.1e-7 at 3072, 1.2e-6 at 8192).
 //
 // Every wait on an mbarrier is bounded by a clock; a wait that runs out sets *status and the CTA winds down.

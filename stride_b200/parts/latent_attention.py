@@ -62,7 +62,7 @@ class LatentAttention(Mixer):
     # expanded, us: 2,000 tokens alone 911 / 586, 2,000 behind 8,000 3,644 / 1,034, 10 behind 30,000 2,937 / 1,831, 33 behind 2,000 512 / 498,
     # 1,000 alone 525 / 496, 512 alone 405 / 457, 100 behind 600 373 / 420. The line was drawn when the folded form ran on mma.sync (12 us a tile,
     # 2,000 alone 1,738); some 1,000 keys are where the forms are level now, and from 512 to there the latents would be 10 % faster. (The forms'
-    # roundings are alike: their outputs differ by 0.0013 to 0.0015, and neither is further from 64 bits.) Below it the folded form has
+    # roundings are alike: their outputs differ by 0.0013 to 0.0015, the expanded form 1 % nearer to 64 bits.) Below it the folded form has
     # fewer launches. Many requests make the product that expands long while the walk stays what the longest one's is: at most
     # EXPAND_SHARE times the longest one's keys in all (on mma.sync 16 of 16 tokens behind 1,000 556 / 580).
     EXPAND_KEYS = 512
