@@ -759,6 +759,28 @@ ssm_chunk_out_kernel(const SsmChunkArgs p) {
             const int r = j0 + (lane & 7) + (((lane >> 3) & 1) << 3), c = n * 8 + ((lane >> 4) << 3);
             uint32_t b[4];
             ldmatrix_x4_trans(b, smem_addr(xs + r * kLdX + c));
+            if (j0 == i0) {
+                // The warp's own 16 tokens: a later one has the weight 0 in an earlier one's row, and 0 times a value that is infinite or no
+                // number would be none. Where there is such a value, the products go one by one and leave those rows out.
+                bool odd = false;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) odd |= (b[e] & 0x7F80u) == 0x7F80u || (b[e] & 0x7F800000u) == 0x7F800000u;
+                if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const int from = (lane & ~3) | ((j & 7) >> 1);
+                        const float wa = __shfl_sync(0xffffffffu, s[j >> 3][j & 1], from), wb = __shfl_sync(0xffffffffu, s[j >> 3][2 + (j & 1)], from);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float v = __bfloat162float(xs[(j0 + j) * kLdX + (n + (e >> 1)) * 8 + 2 * (lane & 3) + (e & 1)]);
+                            float* const to = acc[n + (e >> 1)] + (e & 1);
+                            if (j0 + j <= ia) to[0] = fmaf(wa, v, to[0]);
+                            if (j0 + j <= ib) to[2] = fmaf(wb, v, to[2]);
+                        }
+                    }
+                    continue;
+                }
+            }
             mma_bf16_16816(acc[n], ah, b[0], b[1]);
             mma_bf16_16816(acc[n], al, b[0], b[1]);
             mma_bf16_16816(acc[n + 1], ah, b[2], b[3]);

@@ -1,5 +1,5 @@
 """A chunk's tokens and a number that is none: it comes out of the token that brings it and of those after it, in its head (and, in a value, in its
-column), and of none before, as token by token. Constant decays, channel decays and the matrix LSTM."""
+column), and of none before, as token by token. Constant decays, channel decays, the matrix LSTM and the state space."""
 
 import pytest
 import torch
@@ -76,3 +76,30 @@ def test_a_decay_that_is_no_number_leaves_the_strong_decays_before_it():
     assert torch.equal(o.isnan(), oc.isnan()) and bool(oc[:45].isfinite().all()) and bool(oc[45, :DV].isnan().all())
     ok = o.isfinite()
     assert float((o[ok] - oc[ok]).abs().max()) < 300 * 2.0 ** -24 * float(o[ok].abs().max()) * D ** 0.5
+
+
+@pytest.mark.parametrize("what", ["value", "key", "infinite value"])
+@pytest.mark.parametrize("P,N", [(64, 64), (72, 128)])
+def test_state_space_chunks(P, N, what):
+    from stride_b200.csrc import ops
+    G, T = 1, sum(LENGTHS)
+    g = torch.Generator(device="cuda").manual_seed(P)
+    r = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    channels = H * P + 2 * G * N
+    shape = ops.SsmShape(H, G, N, P, 4, r(H), r(H), r(H), r(4, channels), r(channels))
+    u, raw, proj, state = r(T, channels).bfloat16(), r(T, H), r(T, channels).bfloat16(), 0.1 * r(2, shape.state_floats())
+    # the first, a middle and the last token of sixteen; a chunk's last and the next one's first; the second request's broken chunk
+    for t, head in ((0, 0), (5, 1), (127, 2), (LENGTHS[0] - 1, 0), (LENGTHS[0] + 63, 1), (LENGTHS[0] + 69, 2)):
+        u[t, H * P + 3 if what == "key" else head * P + 9] = float("inf") if what == "infinite value" else float("nan")
+    starts, lens, slots, positions = i32([0, LENGTHS[0]]), i32(LENGTHS), i32([1, 0]), i32([t for n in LENGTHS for t in range(n)])
+    y, yc = (torch.zeros(T, H * P, device="cuda") for _ in range(2))
+    s, sc = state.clone(), state.clone()
+    ops.ssm_scan(shape, u, raw, 0, y, s, starts, lens, slots, 2)
+    scratch = torch.zeros(ops.ssm_chunks_scratch_floats(shape, 2, max(LENGTHS)), device="cuda")
+    ops.ssm_chunks(shape, u, raw, 0, yc, sc, proj, 0, starts, lens, positions, slots, 2, max(LENGTHS), scratch)
+    memory = H * N * P
+    assert torch.equal(y.isfinite(), yc.isfinite()) and torch.equal(s[:, :memory].isfinite(), sc[:, :memory].isfinite())
+    ok = y.isfinite()
+    assert bool(ok[LENGTHS[0] + 62].all()) and not bool(ok[LENGTHS[0] + 63].all())
+    # operands of two bfloat16 parts (2^-16 of a term, of which a sum has N and 64)
+    assert float((y[ok] - yc[ok]).abs().max()) < 2.0 ** -13 * float(y[ok].abs().max())
